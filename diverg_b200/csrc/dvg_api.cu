@@ -8,6 +8,7 @@
 #include <string>
 
 #include "dvg_internal.h"
+#include "dvg_slots.h"
 
 namespace {
 thread_local std::string g_last_error;
@@ -628,6 +629,10 @@ dvg_matrix* create_distance_index(dvg_context* ctx, const dvg_matrix* a, unsigne
   // canonical only for canonical inputs, while the reference's squarings
   // canonicalise any input
   if (ctx->opt_dindex_schedule == 1 || (dlo == 0 && !a->canonical)) return distance_index_reference(ctx, a, dlo, dup);
+  if (ctx->opt_planned && ctx->opt_spgemm_mode == 0 && slots_suit(ctx, a)) {
+    if (dvg_matrix* t = slots_chain(ctx, a, dlo, dup)) return t;
+    ctx->stats.spgemm_reruns++;
+  }
   if (ctx->opt_planned && ctx->opt_spgemm_mode != 1 && a->nrows > 0) {
     PlannedBuild pb;
     bool planned = true;
@@ -773,6 +778,9 @@ dvg_status dvg_set_option(dvg_context* ctx, const char* key, int64_t value) {
     } else if (!std::strcmp(key, "planned_build")) {
       require(value == 0 || value == 1, "planned_build must be 0 or 1");
       ctx->opt_planned = value;
+    } else if (!std::strcmp(key, "row_slots")) {
+      require(value == 0 || value == 1, "row_slots must be 0 or 1");
+      ctx->opt_slots = value;
     } else if (!std::strcmp(key, "plan_growth")) {
       require(value >= 0 && value <= 100000, "plan_growth is a percentage in [0, 100000]");
       ctx->plan_growth = double(value) / 100.0;

@@ -79,6 +79,8 @@ struct dvg_context {
   uint32_t row_resident[3] = {0, 0, 0};  // resident CTAs of the row kernel per variant
   int64_t opt_planned = 1;            // 1: index builds run planned (no host round trips)
   double plan_growth = 3.0;           // planned builds: entry capacity per step / input entries
+  int64_t opt_slots = 1;              // chains of products over graph-like input run in the row-slot format
+  double slot_growth = 4.0;           // row-slot chains: ranges the arena holds / rows
   uint64_t max_product_entries = 0;   // largest product output since the last reset (read-back path)
   int64_t opt_autotune = 1;           // batches: tune the row kernel per (window, size class)
   std::map<std::tuple<unsigned, unsigned, int>, TuneChoice> tuned;

@@ -1,0 +1,1240 @@
+// dvg_slots.cu -- chains of range products in the row-slot format.
+//
+// An index build or a power is a chain of 8 to 20 products whose intermediate
+// matrices nobody sees, and on a sequence graph nearly every row of every one
+// of them is a single run of columns.  In range CRS such a row costs a row
+// pointer and a range to write, two row pointers and a range to read, and the
+// order in which rows are stored makes each product wait for the sizes of the
+// rows before.  Here an intermediate matrix is one 8-byte slot (x, y) a row
+// instead:
+//   x <= y               the run of columns x .. y
+//   (1, 0)               no column
+//   y + 1 < x < kMulti   the two columns y and x
+//   x >= kMulti          x - kMulti ranges from place y of an arena that the
+//                        whole chain shares
+// A row is then one load to read, one store to write, its position is its
+// number, and no product needs a prefix, a look-back or another block's
+// result.  Only the last pass counts its ranges, and k_slots_to_crs turns it
+// into range CRS.
+//
+// Rows are canonical (sorted, disjoint, non-adjacent runs), as the reference's
+// accumulators emit them (range_sparse.hpp:487-678, 1132-1442 in
+// cartoonist/diverg: merge rule start <= hi + 1), so the chain's result is the
+// matrix that the reference's sequence of range_spgemm / range_spadd gives.
+//
+// Measured on a B200 against the same builds product by product in range CRS:
+// 5.0e7 loci, window [400, 600]: 23.05 -> 2.78 ms; 1e6 loci, [0, 250]: 1.26 ->
+// 0.25 ms; 1e5 loci of a variant-dense graph, [100, 300]: 1.01 -> 0.18 ms.
+#include <algorithm>
+#include <cstring>
+
+#include "dvg_device.cuh"
+#include "dvg_slots.h"
+
+namespace dvg {
+namespace {
+
+constexpr int kSThreads = 256;  // streaming kernels
+constexpr int kSWarps = kSThreads / 32;
+constexpr int kWThreads = 128;  // kernels that walk rows
+constexpr int kWWarps = kWThreads / 32;
+constexpr int kSRows = 4;       // rows a lane of k_chain_rows takes
+constexpr int kSRuns = 8;       // runs of a lane's list
+constexpr int kSWin = 256;      // window words of a warp (8,192 columns)
+constexpr uint32_t kMulti = kSlotMulti;
+constexpr uint32_t kMultiMax = 0xFFFFFFFFu - kMulti - 1;  // ranges of one row
+constexpr uint32_t kCountRows = 32 * kSRows;  // rows whose ranges the last pass counts together
+constexpr uint32_t kSmallRows = 1u << 17;     // rows up to which a pass is one kernel
+constexpr double kChainReach = 1.28;          // branching * steps of a pass's left factors
+constexpr int kCrsRows = 1024;                // rows of a block of the conversion
+constexpr uint32_t kSuperGroups = 512;        // counts that k_slot_sums adds up
+
+__device__ __forceinline__ uint2 empty_slot() { return make_uint2(1u, 0u); }
+__device__ __forceinline__ bool is_multi(uint2 s) { return s.x >= kMulti; }
+__device__ __forceinline__ uint2 ld_slot(const uint2* __restrict__ p, size_t i) { return __ldg(p + i); }
+__device__ __forceinline__ bool is_run(uint2 s) { return s.x <= s.y; }
+__device__ __forceinline__ uint32_t slot_count(uint2 s) {
+  return is_run(s) ? 1u : is_multi(s) ? s.x - kMulti : s.x == s.y + 1 ? 0u : 2u;
+}
+// Range t of a slot that has it.
+__device__ __forceinline__ uint2 slot_range(const uint2* __restrict__ arena, uint2 s, uint32_t t) {
+  if (is_multi(s)) return __ldg(arena + s.y + t);
+  if (is_run(s)) return s;
+  return t ? make_uint2(s.x, s.x) : make_uint2(s.y, s.y);
+}
+// The slot of the two columns or equal columns c and d.
+__device__ __forceinline__ uint2 pair_slot(uint32_t c, uint32_t d) {
+  const uint32_t lo = min(c, d), hi = max(c, d);
+  return hi - lo <= 1 ? make_uint2(lo, hi) : make_uint2(hi, lo);
+}
+
+// v |= w for two runs that overlap or touch; false, v unchanged, for any other
+// two slots.  Columns are below kMulti, so y + 1 does not wrap.
+__device__ __forceinline__ bool unite(uint2& v, uint2 w) {
+  if (!is_run(v) || !is_run(w) || w.x > v.y + 1 || v.x > w.y + 1) return false;
+  v.x = min(v.x, w.x);
+  v.y = max(v.y, w.y);
+  return true;
+}
+
+// One pass: with S_0 = I and S_(j+1) = S_j M_j,
+//   s = S_k                         (where s is not null)
+//   c = union of S_j B over bits j  (where c is not null; B null: the identity)
+struct ChainArgs {
+  const uint2* m[kChainMax];
+  const uint2* b;
+  uint2* s;
+  uint2* c;
+  uint32_t k, bits;
+  uint2* arena;
+  unsigned long long* top;    // ranges taken from the arena
+  uint64_t arena_cap;
+  DeviceControl* ctl;
+  unsigned long long* abort;  // set when the arena is full: the rows that did not fit are left
+                              // empty, so that later passes stay in bounds, and the host drops the result
+  uint32_t* masks;            // bit r % 32 of word r / 32: k_chain_rows left row r to k_chain_walk
+  uint32_t* group_cnt;        // last pass: ranges and columns of c per kCountRows rows
+  unsigned long long* group_nnz;
+  uint32_t n;
+};
+
+// U * 32 rows from r0, all of them rows of the matrix: those that are one or
+// two columns in every S_j on the way, as nearly all rows of a sequence graph's
+// powers are.  A row of one column takes the next factor's row (at the end: B's)
+// as it is -- a row of several ranges keeps its place in the arena, rows are
+// never rewritten; a row of two takes two rows of one column each.  Returns the
+// rows that do not go through (bit u: row r0 + u * 32 + lane).
+template <bool OUTS, bool OUTC, bool COUNT, int U>
+__device__ __forceinline__ uint32_t chain_rows(const ChainArgs& p, uint32_t r0, uint32_t& cnt,
+                                               unsigned long long& nnz) {
+  const uint32_t r = r0 + lane_id();
+  uint32_t at[U], at2[U], bad = 0, two = 0;  // a row's column or two (bit u of two); of a bad row, its own number
+  uint2 acc[U];
+  bool pairs = false;                        // some row of the warp has two
+  bool have = OUTC && (p.bits & 1u) != 0;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    at[u] = at2[u] = r + u * 32;
+    acc[u] = have && p.b ? ld_slot(p.b, at[u]) : make_uint2(at[u], at[u]);
+  }
+  if (have && (p.bits & ~1u)) {  // only runs are united below
+#pragma unroll
+    for (int u = 0; u < U; ++u) bad |= (is_run(acc[u]) ? 0u : 1u) << u;
+  }
+#pragma unroll 1
+  for (uint32_t j = 0; j < p.k; ++j) {
+    const uint2* __restrict__ mat = p.m[j];
+    const bool last = j + 1 == p.k, gather = OUTC && ((p.bits >> (j + 1)) & 1u);
+    uint2 s[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) s[u] = ld_slot(mat, at[u]);
+    if (pairs) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (!((two >> u) & 1u)) continue;
+        const uint2 t = ld_slot(mat, at2[u]);
+        if (s[u].x == s[u].y && t.x == t.y) {
+          s[u] = pair_slot(s[u].x, t.x);
+        } else {  // (a marker is no column: never followed)
+          bad |= 1u << u;
+          s[u] = make_uint2(r + u * 32, r + u * 32);
+        }
+      }
+    }
+    if (OUTS && last) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (!((bad >> u) & 1u)) p.s[size_t(r) + u * 32] = s[u];
+    }
+    if (last && !gather) break;
+    uint32_t odd = 0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      odd |= s[u].x ^ s[u].y;
+      at[u] = s[u].x;
+    }
+    pairs = __any_sync(kFullMask, odd != 0);
+    if (pairs) {
+      two = 0;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        // one column, two neighbours, or two apart: x and y are the columns
+        const bool ok = is_run(s[u]) ? s[u].y - s[u].x <= 1 : s[u].x - s[u].y >= 2 && !is_multi(s[u]);
+        bad |= (ok ? 0u : 1u) << u;
+        const bool gone = (bad >> u) & 1u;
+        two |= (!gone && s[u].x != s[u].y ? 1u : 0u) << u;
+        at[u] = gone ? r + u * 32 : s[u].x;
+        at2[u] = s[u].y;
+      }
+    }
+    if (gather) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) s[u] = p.b ? ld_slot(p.b, at[u]) : make_uint2(at[u], at[u]);
+      if (pairs) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (!((two >> u) & 1u)) continue;
+          if (!unite(s[u], p.b ? ld_slot(p.b, at2[u]) : make_uint2(at2[u], at2[u]))) bad |= 1u << u;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (have) {
+          const bool touch = s[u].x <= min(s[u].y, acc[u].y + 1) && acc[u].x <= s[u].y + 1;
+          bad |= (touch ? 0u : 1u) << u;
+          acc[u].x = min(acc[u].x, s[u].x);
+          acc[u].y = max(acc[u].y, s[u].y);
+        } else {
+          acc[u] = s[u];
+        }
+      }
+      have = true;
+    }
+  }
+  if (OUTC) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if ((bad >> u) & 1u) continue;
+      p.c[size_t(r) + u * 32] = acc[u];
+      if (COUNT) {
+        const uint32_t c = slot_count(acc[u]);
+        cnt += c;
+        for (uint32_t t = 0; t < c; ++t) {
+          const uint2 v = slot_range(p.arena, acc[u], t);
+          nnz += v.y - v.x + 1;
+        }
+      }
+    }
+  }
+  return bad;
+}
+
+// ---- rows that need more than that -------------------------------------------
+
+// A warp's shared memory: the rows it walks next, and the lists of its
+// walks (entry k of lane t at [k * 32 + t]) or, for rows of more runs than
+// those hold, a bitmap window.
+struct WarpSmem {
+  union {
+    uint2 list[3][kSRuns * 32];
+    struct {
+      uint32_t bits[kSWin], reach[kSWin];
+    } win;
+  };
+  uint32_t todo[32];
+};
+
+// Merges v into the nr runs at L; returns their new number, or kFull.
+constexpr uint32_t kFull = 0xffffffffu;
+__device__ __noinline__ uint32_t list_merge(uint2* L, uint32_t nr, uint2 v) {
+  if (nr == 0 || L[(nr - 1) * 32].y + 1 < v.x) {  // past the last run
+    if (nr == uint32_t(kSRuns)) return kFull;
+    L[nr * 32] = v;
+    return nr + 1;
+  }
+  uint32_t k = 0;
+  while (L[k * 32].y + 1 < v.x) ++k;
+  if (v.y + 1 < L[k * 32].x) {
+    if (nr == uint32_t(kSRuns)) return kFull;
+    for (uint32_t m = nr; m > k; --m) L[m * 32] = L[(m - 1) * 32];
+    L[k * 32] = v;
+    return nr + 1;
+  }
+  uint2 w = L[k * 32];
+  w.x = min(w.x, v.x);
+  w.y = max(w.y, v.y);
+  uint32_t m = k + 1;
+  while (m < nr && w.y + 1 >= L[m * 32].x) {
+    w.y = max(w.y, L[m * 32].y);
+    ++m;
+  }
+  L[k * 32] = w;
+  const uint32_t gone = m - k - 1;
+  if (gone)
+    for (uint32_t q = m; q < nr; ++q) L[(q - gone) * 32] = L[q * 32];
+  return nr - gone;
+}
+
+// The nd runs at D |= the rows of `mat` that the ns runs at L name (mat null:
+// the runs themselves).  Returns their new number, or kFull.
+__device__ __noinline__ uint32_t list_product(const uint2* __restrict__ arena, const uint2* L, uint32_t ns,
+                                              const uint2* __restrict__ mat, uint2* D, uint32_t nd) {
+  uint2 run = empty_slot();
+  for (uint32_t k = 0; k < ns; ++k) {
+    const uint2 a = L[k * 32];
+    for (uint32_t x = a.x; x <= a.y; ++x) {
+      const uint2 s = mat ? ld_slot(mat, x) : a;
+      const uint32_t c = slot_count(s);
+      for (uint32_t t = 0; t < c; ++t) {
+        const uint2 v = slot_range(arena, s, t);
+        // extends the open run, or merges it into the list and opens another
+        if (v.x <= run.y + 1 && run.x <= v.y + 1) {
+          run.x = min(run.x, v.x);
+          run.y = max(run.y, v.y);
+        } else {
+          if (run.x <= run.y) {
+            nd = list_merge(D, nd, run);
+            if (nd == kFull) return kFull;
+          }
+          run = v;
+        }
+      }
+      if (!mat) break;
+    }
+  }
+  return run.x <= run.y ? list_merge(D, nd, run) : nd;
+}
+
+// The quick form of a walk.  The columns that a row's S_j holds lie close
+// together -- the ends of paths of one length -- so they are a 64-bit mask from
+// a base column, and a product ORs the named rows' ranges into the next mask.
+// c's row is at most two runs in registers.  Writes the runs of s and c to the
+// lists; false where the row does not fit.
+template <bool OUTS, bool OUTC>
+__device__ __forceinline__ bool quick_row(const ChainArgs& p, uint32_t row, uint2* Ls, uint32_t& ns, uint2* Lc,
+                                          uint32_t& nc) {
+  constexpr int kAhead = 2;
+  unsigned long long mask = 1ull;
+  uint32_t base = row;
+  uint2 r0 = empty_slot(), r1 = empty_slot();
+  bool ok = true;
+  auto add_c = [&](uint2 v) {
+    if (!is_run(r0)) {
+      r0 = v;
+    } else if (unite(r0, v)) {
+      if (unite(r0, r1)) r1 = empty_slot();
+    } else if (r1.x > r1.y) {
+      r1 = r0;
+      r0 = v;
+    } else if (unite(r1, v)) {
+      if (unite(r0, r1)) r1 = empty_slot();
+    } else {
+      ok = false;
+    }
+  };
+  // the ranges of the rows of `mat` that the mask names, four rows at a time so
+  // that their loads are in flight together
+  auto each = [&](const uint2* __restrict__ mat, auto&& f) {
+    for (unsigned long long w = mask; w;) {
+      uint2 s[kAhead];
+#pragma unroll
+      for (int q = 0; q < kAhead; ++q) {
+        s[q] = empty_slot();
+        if (w) {
+          s[q] = ld_slot(mat, base + uint32_t(__ffsll(w) - 1));
+          w &= w - 1;
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < kAhead; ++q) {
+        const uint32_t c = slot_count(s[q]);
+        for (uint32_t t = 0; t < c; ++t) f(slot_range(p.arena, s[q], t));
+      }
+    }
+  };
+  auto add_slot = [&](uint2 s) {
+    const uint32_t c = slot_count(s);
+    for (uint32_t t = 0; t < c; ++t) add_c(slot_range(p.arena, s, t));
+  };
+  // while the row is a single column
+  uint32_t j = 0;
+#pragma unroll 1
+  for (; j < p.k; ++j) {
+    const uint2 s = ld_slot(p.m[j], base);
+    if (OUTC && ((p.bits >> j) & 1u)) add_slot(p.b ? ld_slot(p.b, base) : make_uint2(base, base));
+    if (s.x != s.y) break;
+    base = s.x;
+  }
+  const uint32_t single = j;  // c has its part of S_0 .. S_(single - 1), and of S_single but for j = k
+#pragma unroll 1
+  for (; ok; ++j) {
+    if (OUTC && ((p.bits >> j) & 1u) && (j != single || j == p.k)) {
+      if (p.b) {
+        each(p.b, add_c);
+      } else {
+        for (unsigned long long w = mask; w;) {
+          const int lo = __ffsll(w) - 1, n = __ffsll(~(w >> lo)) - 1;  // (n < 0: all 64 columns)
+          const int hi = n < 0 ? 63 : lo + n - 1;
+          add_c(make_uint2(base + lo, base + hi));
+          w &= hi < 63 ? ~0ull << (hi + 1) : 0ull;
+        }
+      }
+    }
+    if (j == p.k) break;
+    unsigned long long to = 0;
+    uint32_t from = 0;
+    each(p.m[j], [&](uint2 v) {
+      if (!to) from = v.x > 16 ? v.x - 16 : 0;  // later rows may start a little before the first
+      if (v.x < from || v.y - from > 63) {
+        ok = false;
+        return;
+      }
+      to |= (~0ull << (v.x - from)) & (~0ull >> (63 - (v.y - from)));
+    });
+    mask = to;
+    base = from;
+  }
+  if (!ok) return false;
+  if (OUTS) {
+    ns = 0;
+    for (unsigned long long w = mask; w;) {
+      const int lo = __ffsll(w) - 1, n = __ffsll(~(w >> lo)) - 1;
+      const int hi = n < 0 ? 63 : lo + n - 1;
+      if (ns == uint32_t(kSRuns)) return false;
+      Ls[ns++ * 32] = make_uint2(base + lo, base + hi);
+      w &= hi < 63 ? ~0ull << (hi + 1) : 0ull;
+    }
+  }
+  if (OUTC) {
+    if (r1.x <= r1.y && r1.x < r0.x) {
+      const uint2 t = r0;
+      r0 = r1;
+      r1 = t;
+    }
+    nc = 0;
+    if (r0.x <= r0.y) Lc[nc++ * 32] = r0;
+    if (r1.x <= r1.y) Lc[nc++ * 32] = r1;
+  }
+  return true;
+}
+
+// The union of the rows of `mat` that the slot `left` names (mat null: none)
+// and of the slots d and e, by a warp, any number of runs: bitmap windows over
+// the columns that its ranges cover, the next window starting at the first
+// column past the last one.  Returns the row's slot (uniform).  The arena is
+// read past L1: a slot may be one that this warp has just written.
+__device__ uint2 warp_union(const ChainArgs& p, uint2 left, const uint2* __restrict__ mat, uint2 d, uint2 e,
+                            uint32_t* bits, uint32_t* reach) {
+  const int lane = lane_id();
+  // every range of the union, spread over the lanes
+  auto each = [&](auto&& f) {
+    auto range = [&](uint2 s, uint32_t t) { return is_multi(s) ? __ldcg(p.arena + s.y + t) : slot_range(p.arena, s, t); };
+    for (uint2 s : {d, e}) {
+      const uint32_t c = slot_count(s);
+      for (uint32_t t = lane; t < c; t += 32) f(range(s, t));
+    }
+    if (!mat) return;
+    auto rows = [&](uint64_t x, uint32_t end, uint32_t step) {
+      for (; x <= end; x += step) {
+        const uint2 s = ld_slot(mat, x);
+        const uint32_t c = slot_count(s);
+        for (uint32_t t = 0; t < c; ++t) f(range(s, t));
+      }
+    };
+    if (is_run(left)) {  // one long range: a lane takes single rows
+      rows(uint64_t(left.x) + lane, left.y, 32);
+    } else {  // a lane takes whole ranges of the left row
+      const uint32_t c = slot_count(left);
+      for (uint32_t t = lane; t < c; t += 32) {
+        const uint2 r = range(left, t);
+        rows(r.x, r.y, 1);
+      }
+    }
+  };
+  uint32_t first = 0xffffffffu;
+  each([&](uint2 v) { first = min(first, v.x); });
+  first = group_min<32>(kFullMask, first);
+  if (first == 0xffffffffu) return empty_slot();
+  uint64_t off = 0;
+  uint32_t total = 0;
+  for (int pass = 0; pass < 2; ++pass) {  // count, then write to the arena
+    uint32_t count = 0;                   // runs begun
+    uint2 open = empty_slot();            // y: the last column, where a run goes on past the words so far
+    uint32_t next = first;
+    while (next != 0xffffffffu) {
+      const uint64_t cb = next & ~31u, ce = cb + 32ull * kSWin - 1;
+      for (uint32_t w = lane; w < uint32_t(kSWin); w += 32) bits[w] = reach[w] = 0;
+      __syncwarp();
+      uint32_t after = 0xffffffffu;  // the first covered column past the window
+      each([&](uint2 v) {
+        if (uint64_t(v.y) > ce) after = min(after, max(v.x, uint32_t(ce + 1)));
+        if (uint64_t(v.y) < cb || uint64_t(v.x) > ce) return;
+        const uint32_t s = uint32_t(max(uint64_t(v.x), cb) - cb), t = uint32_t(min(uint64_t(v.y), ce) - cb);
+        const uint32_t ws = s >> 5, we = t >> 5;
+        const uint32_t lo = ~0u << (s & 31), hi = ~0u >> (31 - (t & 31));
+        if (ws == we) {
+          atomicOr(bits + ws, lo & hi);
+        } else {
+          atomicOr(bits + ws, lo);
+          atomicOr(bits + we, hi);
+          if (we > ws + 1) atomicMax(reach + ws + 1, we);
+        }
+      });
+      after = group_min<32>(kFullMask, after);
+      __syncwarp();
+      uint32_t run_reach = 0;
+      for (uint32_t wb = 0; wb < uint32_t(kSWin); wb += 32) {
+        const uint32_t w = wb + lane;
+        uint32_t x = bits[w];
+        const uint32_t rr = max(group_incl_max<32>(kFullMask, reach[w], lane), run_reach);
+        if (rr > w) x = ~0u;
+        run_reach = __shfl_sync(kFullMask, rr, 31);
+        const uint32_t prev = __shfl_up_sync(kFullMask, x, 1), after_word = __shfl_down_sync(kFullMask, x, 1);
+        const uint32_t col = uint32_t(cb) + 32 * w;
+        const bool carry = lane ? (prev >> 31) : (is_run(open) && open.y + 1 == col);
+        const uint32_t starts = x & ~((x << 1) | (carry ? 1u : 0u));
+        const uint32_t nb = __popc(starts);
+        const uint32_t incl = group_incl_sum<32>(kFullMask, nb, lane);
+        if (pass == 1) {
+          // starts in order; an end goes to the run that it closes, or to the
+          // last one begun before this word where that goes on here
+          uint32_t k = count + incl - nb;
+          for (uint32_t b = starts; b; b &= b - 1) p.arena[off + k++].x = col + uint32_t(__ffs(b) - 1);
+          uint32_t ends = x & ~(x >> 1);
+          if (lane < 31 && (after_word & 1u)) ends &= 0x7fffffffu;  // the next word ends it
+          uint32_t q = count + incl - nb - (carry && (x & 1u) ? 1u : 0u);
+          for (uint32_t b = ends; b; b &= b - 1) p.arena[off + q++].y = col + uint32_t(__ffs(b) - 1);
+          __syncwarp();  // the next words may prolong the last run
+        }
+        const uint32_t last = __shfl_sync(kFullMask, x, 31);
+        count += __shfl_sync(kFullMask, incl, 31);
+        open = last >> 31 ? make_uint2(0u, uint32_t(cb) + 32 * (wb + 31) + 31) : empty_slot();
+      }
+      __syncwarp();
+      next = after;
+    }
+    if (pass == 0) {
+      total = count;
+      if (lane == 0) off = atomicAdd(p.top, (unsigned long long)total);
+      off = __shfl_sync(kFullMask, off, 0);
+      if (total > kMultiMax || off + total > p.arena_cap) {
+        if (lane == 0) atomicOr(p.abort, 1ull);
+        return empty_slot();
+      }
+    }
+  }
+  __syncwarp();
+  return total == 1 ? __ldcg(p.arena + off) : make_uint2(kMulti + total, uint32_t(off));
+}
+
+// Walks the `batch` rows of the warp's list, a row a lane; rows of more runs
+// than a lane's lists hold go to the whole warp.
+// tally(row, ranges, columns) for each row of c that has any.
+template <bool OUTS, bool OUTC, class Tally>
+__device__ __forceinline__ void walk_batch(const ChainArgs& p, WarpSmem& S, uint32_t batch, Tally&& tally) {
+  const int lane = lane_id();
+  uint32_t row = 0, ns = 0, nc = 0, cur = 0;
+  bool done = false;
+  uint2* const C = S.list[2] + lane;
+  if (uint32_t(lane) < batch) {
+    row = S.todo[lane];
+    done = quick_row<OUTS, OUTC>(p, row, S.list[0] + lane, ns, C, nc);
+  }
+  __syncwarp();
+  if (uint32_t(lane) < batch && !done) {
+    S.list[0][lane] = make_uint2(row, row);
+    ns = 1;
+    nc = 0;
+#pragma unroll 1
+    for (uint32_t j = 0;; ++j) {
+      const uint2* L = S.list[cur] + lane;
+      if (OUTC && ((p.bits >> j) & 1u)) nc = list_product(p.arena, L, ns, p.b, C, nc);
+      if (j == p.k || nc == kFull) break;
+      ns = list_product(p.arena, L, ns, p.m[j], S.list[cur ^ 1u] + lane, 0);
+      if (ns == kFull) break;
+      cur ^= 1u;
+    }
+    done = ns != kFull && nc != kFull;
+  }
+  __syncwarp();
+  unsigned left = __ballot_sync(kFullMask, uint32_t(lane) < batch && !done);
+  // places in the arena for the rows of several runs, one request a warp
+  // (a row of two columns needs none)
+  const uint2* const T = S.list[cur] + lane;
+  auto place = [&](const uint2* L, uint32_t n) {
+    return n == 2 && L[0].x == L[0].y && L[32].x == L[32].y ? 0u : n > 1 ? n : 0u;
+  };
+  const uint32_t ws = OUTS && done ? place(T, ns) : 0u, wc = OUTC && done ? place(C, nc) : 0u;
+  const uint32_t incl = group_incl_sum<32>(kFullMask, ws + wc, lane);
+  const uint32_t all = __shfl_sync(kFullMask, incl, 31);
+  unsigned long long off = 0;
+  bool fits = true;
+  if (all) {
+    if (lane == 31) off = atomicAdd(p.top, (unsigned long long)all);
+    off = __shfl_sync(kFullMask, off, 31);
+    fits = off + all <= p.arena_cap;
+    if (!fits && lane == 0) atomicOr(p.abort, 1ull);
+    off += incl - ws - wc;
+  }
+  auto put = [&](uint2* to, const uint2* L, uint32_t n, uint32_t want) {
+    uint2 v = empty_slot();
+    if (n == 1) v = L[0];
+    else if (n == 2 && !want) v = make_uint2(L[32].x, L[0].x);
+    else if (want && fits) v = make_uint2(kMulti + n, uint32_t(off));
+    to[row] = v;
+    if (fits)
+      for (uint32_t k = 0; k < want; ++k) p.arena[off + k] = L[k * 32];
+    off += want;
+  };
+  if (done) {
+    if (OUTS) put(p.s, T, ns, ws);
+    if (OUTC) {
+      put(p.c, C, nc, wc);
+      unsigned long long z = 0;
+      for (uint32_t k = 0; k < nc; ++k) z += C[k * 32].y - C[k * 32].x + 1;
+      if (nc) tally(row, nc, z);
+    }
+  }
+  __syncwarp();
+  if (left && lane == 0) atomicAdd(&p.ctl->slow_rows, (unsigned long long)__popc(left));
+  for (; left; left &= left - 1) {
+    const uint32_t r = __shfl_sync(kFullMask, row, __ffs(left) - 1);
+    uint2 s = make_uint2(r, r), c = empty_slot();
+    for (uint32_t j = 0;; ++j) {
+      if (OUTC && ((p.bits >> j) & 1u))
+        c = p.b ? warp_union(p, s, p.b, c, empty_slot(), S.win.bits, S.win.reach)
+                : warp_union(p, s, nullptr, c, s, S.win.bits, S.win.reach);
+      if (j == p.k) break;
+      s = warp_union(p, s, p.m[j], empty_slot(), empty_slot(), S.win.bits, S.win.reach);
+    }
+    if (OUTS && lane == 0) p.s[r] = s;
+    if (OUTC) {
+      if (lane == 0) p.c[r] = c;
+      const uint32_t k = slot_count(c);
+      unsigned long long z = 0;
+      for (uint32_t q = lane; q < k; q += 32) {
+        const uint2 v = is_multi(c) ? __ldcg(p.arena + c.y + q) : slot_range(p.arena, c, q);
+        z += v.y - v.x + 1;
+      }
+      z = group_sum<32>(kFullMask, z);
+      if (lane == 0 && k) tally(r, k, z);
+    }
+  }
+  __syncwarp();
+}
+
+// ---- the passes ---------------------------------------------------------------
+// A pass over a large matrix is two kernels.  k_chain_rows streams it: nearly
+// all rows of a sequence graph's powers are a single column, and their part of
+// the pass is k + 1 dependent loads, each near the row's own diagonal, for
+// kSRows rows a lane at once.  It needs few registers, so that enough loads
+// are in flight to keep HBM busy, and leaves the other rows marked in a
+// bitmap.  k_chain_walk reads the bitmap and walks those, 32 at a time, a row a
+// lane, so that no lane waits for another's longer row and a walk's chain of
+// dependent loads is paid once for 32 rows.
+//
+// Bound: HBM, 8 bytes a row for each matrix read and written (all but the first
+// read of a matrix come from L2).  k_chain_rows on 1e7 rows: 51 to 72 us for
+// 190 to 300 MB, 3.8 to 5.2 TB/s, issue slots 45 to 60 % busy; six blocks an SM
+// (42 registers) against four: 2.75 and 2.90 ms a 5e7-locus build.  k_chain_walk: 27
+// to 56 us, the latency of a walk, whatever few rows there are.  Walking the
+// rows in the streaming kernel instead, behind a block's barrier or a warp at a
+// time, held the loads of its other rows back (8.9 and 4.1 ms a build).
+template <bool OUTS, bool OUTC, bool COUNT>
+__global__ void __launch_bounds__(kSThreads, 6) k_chain_rows(const __grid_constant__ ChainArgs p) {
+  const uint64_t r0 = (uint64_t(blockIdx.x) * kSWarps + (threadIdx.x >> 5)) * (32 * kSRows);
+  if (r0 >= p.n) return;
+  const int lane = lane_id();
+  uint32_t bad = 0, cnt = 0;
+  unsigned long long nnz = 0;
+  if (r0 + 32 * kSRows <= p.n) {
+    bad = chain_rows<OUTS, OUTC, COUNT, kSRows>(p, uint32_t(r0), cnt, nnz);
+  } else {  // the last, ragged rows are all walked
+#pragma unroll
+    for (int u = 0; u < kSRows; ++u) bad |= (r0 + u * 32 + lane < p.n ? 1u : 0u) << u;
+  }
+  uint32_t word = 0;
+#pragma unroll
+  for (int u = 0; u < kSRows; ++u) {
+    const uint32_t w = __ballot_sync(kFullMask, (bad >> u) & 1u);
+    if (lane == u) word = w;
+  }
+  if (lane < kSRows && r0 + lane * 32 < p.n) p.masks[r0 / 32 + lane] = word;
+  if (COUNT) {
+    cnt = __reduce_add_sync(kFullMask, cnt);
+    nnz = group_sum<32>(kFullMask, nnz);
+    if (lane == 0) {
+      p.group_cnt[r0 / kCountRows] = cnt;
+      p.group_nnz[r0 / kCountRows] = nnz;
+    }
+  }
+}
+
+template <bool OUTS, bool OUTC, bool COUNT>
+__global__ void __launch_bounds__(kWThreads) k_chain_walk(const __grid_constant__ ChainArgs p) {
+  __shared__ WarpSmem smem[kWWarps];
+  const int lane = lane_id(), warp = threadIdx.x >> 5;
+  WarpSmem& S = smem[warp];
+  // rows to walk come in clumps, the length of a left factor before a bubble:
+  // a warp's words lie a grid's width apart, so that each gets its share
+  const uint64_t words = (uint64_t(p.n) + 31) / 32, stride = gridDim.x * kWWarps;
+  uint64_t next = blockIdx.x * kWWarps + warp;
+  uint32_t x = 0, at = 0;  // a lane's word: its rows still to walk, and the first of its 32
+  while (true) {
+    const unsigned spent = __ballot_sync(kFullMask, x == 0);
+    uint32_t have = __reduce_add_sync(kFullMask, uint32_t(__popc(x)));
+    if (have < 32 && next < words) {  // lanes whose word is done take the next ones
+      const uint64_t w = next + __popc(spent & ((1u << lane) - 1u)) * stride;
+      if (x == 0 && w < words) {
+        x = p.masks[w];
+        at = uint32_t(w) * 32;
+      }
+      next += __popc(spent) * stride;
+      continue;
+    }
+    if (have == 0) break;
+    // the first 32 rows
+    uint32_t k = group_incl_sum<32>(kFullMask, uint32_t(__popc(x)), lane) - __popc(x);
+    for (; x && k < 32; x &= x - 1) S.todo[k++] = at + uint32_t(__ffs(x) - 1);
+    __syncwarp();
+    walk_batch<OUTS, OUTC>(p, S, min(have, 32u), [&](uint32_t row, uint32_t cnt, unsigned long long nnz) {
+      if (!COUNT) return;
+      atomicAdd(p.group_cnt + row / kCountRows, cnt);
+      atomicAdd(p.group_nnz + row / kCountRows, nnz);
+    });
+  }
+}
+
+// A pass over a small matrix, where a launch costs more than the rows: both in
+// one kernel, a block kCountRows rows, a warp 32 of them.
+template <bool OUTS, bool OUTC, bool COUNT>
+__global__ void __launch_bounds__(kWThreads) k_chain_small(const __grid_constant__ ChainArgs p) {
+  static_assert(kWThreads == kCountRows, "a block's rows are counted together");
+  __shared__ WarpSmem smem[kWWarps];
+  __shared__ unsigned long long sum[2];
+  const int lane = lane_id(), warp = threadIdx.x >> 5;
+  WarpSmem& S = smem[warp];
+  if (COUNT) {
+    if (threadIdx.x < 2) sum[threadIdx.x] = 0;
+    __syncthreads();
+  }
+  const uint64_t r0 = uint64_t(blockIdx.x) * kWThreads + warp * 32;
+  unsigned long long nnz = 0;
+  uint32_t cnt = 0;
+  if (r0 < p.n) {
+    uint32_t bad;
+    if (r0 + 32 <= p.n) bad = chain_rows<OUTS, OUTC, COUNT, 1>(p, uint32_t(r0), cnt, nnz);
+    else bad = r0 + lane < p.n ? 1u : 0u;
+    const unsigned who = __ballot_sync(kFullMask, bad != 0);
+    if (bad) S.todo[__popc(who & ((1u << lane) - 1u))] = uint32_t(r0) + lane;
+    __syncwarp();
+    if (who)
+      walk_batch<OUTS, OUTC>(p, S, __popc(who), [&](uint32_t, uint32_t c, unsigned long long z) {
+        cnt += c;
+        nnz += z;
+      });
+  }
+  if (COUNT) {
+    cnt = __reduce_add_sync(kFullMask, cnt);
+    nnz = group_sum<32>(kFullMask, nnz);
+    if (lane == 0) {
+      atomicAdd(&sum[0], (unsigned long long)cnt);
+      atomicAdd(&sum[1], nnz);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      p.group_cnt[blockIdx.x] = uint32_t(sum[0]);
+      p.group_nnz[blockIdx.x] = sum[1];
+    }
+  }
+}
+
+// Range CRS -> slots.  Canonical input: a row of several ranges is copied to
+// the arena as it is.
+__global__ void __launch_bounds__(kSThreads) k_crs_to_slots(const uint64_t* __restrict__ rowmap,
+                                                            const uint32_t* __restrict__ entries,
+                                                            const __grid_constant__ ChainArgs p) {
+  const uint64_t stride = uint64_t(gridDim.x) * kSThreads;
+  const int lane = lane_id();
+  for (uint64_t b0 = blockIdx.x * uint64_t(kSThreads) + (threadIdx.x & ~31u); b0 < p.n; b0 += stride) {
+    const uint64_t r = b0 + lane;
+    uint64_t a0 = 0, cnt = 0;
+    uint2 v = empty_slot();
+    if (r < p.n) {
+      a0 = __ldg(rowmap + r) >> 1;
+      cnt = (__ldg(rowmap + r + 1) >> 1) - a0;
+      if (cnt == 1) v = load_range(entries, a0);
+    }
+    uint64_t want = cnt > 1 ? cnt : 0;
+    if (cnt == 2) {
+      const uint2 a = load_range(entries, a0), b = load_range(entries, a0 + 1);
+      if (a.x == a.y && b.x == b.y) {
+        v = make_uint2(b.x, a.x);
+        want = 0;
+      }
+    }
+    if (__any_sync(kFullMask, want != 0)) {
+      const uint64_t incl = group_incl_sum<32>(kFullMask, want, lane);
+      unsigned long long off = 0;
+      if (lane == 31) off = atomicAdd(p.top, (unsigned long long)incl);
+      off = __shfl_sync(kFullMask, off, 31) + incl - want;
+      if (want) {
+        if (want > kMultiMax || off + want > p.arena_cap) {
+          atomicOr(p.abort, 1ull);
+        } else {
+          for (uint64_t k = 0; k < want; ++k) p.arena[off + k] = load_range(entries, a0 + k);
+          v = make_uint2(kMulti + uint32_t(want), uint32_t(off));
+        }
+      }
+    }
+    if (r < p.n) p.s[r] = v;
+  }
+}
+
+// Sums of kSuperGroups counts each, a block a sum; the totals of the result.
+__global__ void __launch_bounds__(kSThreads) k_slot_sums(const uint32_t* __restrict__ cnt,
+                                                         const unsigned long long* __restrict__ nnz, uint64_t groups,
+                                                         unsigned long long* __restrict__ sums, DeviceControl* ctl) {
+  __shared__ unsigned long long part[2][kSWarps];
+  unsigned long long s = 0, z = 0;
+  for (uint32_t k = threadIdx.x; k < kSuperGroups; k += kSThreads) {
+    const uint64_t g = uint64_t(blockIdx.x) * kSuperGroups + k;
+    if (g < groups) {
+      s += cnt[g];
+      z += nnz[g];
+    }
+  }
+  s = group_sum<32>(kFullMask, s);
+  z = group_sum<32>(kFullMask, z);
+  if (lane_id() == 0) {
+    part[0][threadIdx.x >> 5] = s;
+    part[1][threadIdx.x >> 5] = z;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kSWarps; ++w) {
+      s += part[0][w];
+      z += part[1][w];
+    }
+    sums[blockIdx.x] = s;
+    atomicAdd(&ctl->total, 2 * s);
+    atomicAdd(&ctl->nnz, z);
+  }
+}
+
+// Slots -> range CRS.  A block takes kCrsRows rows; the ranges before them are
+// the sums of the super groups before its own and the counts of the groups
+// before it in that one, so no block waits for another.  A warp takes 32
+// consecutive rows at a time.
+__global__ void __launch_bounds__(kSThreads) k_slots_to_crs(const uint2* __restrict__ slots,
+                                                            const uint2* __restrict__ arena,
+                                                            const unsigned long long* __restrict__ sums,
+                                                            const uint32_t* __restrict__ group_cnt, uint32_t n,
+                                                            uint64_t* __restrict__ rowmap,
+                                                            uint32_t* __restrict__ entries, uint64_t cap,
+                                                            DeviceControl* ctl) {
+  constexpr int kIter = kCrsRows / kSThreads;
+  __shared__ unsigned long long pre[kSWarps];
+  __shared__ uint32_t wsum[kSWarps];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t tile = blockIdx.x, g0 = tile * (kCrsRows / kCountRows), sup = g0 / kSuperGroups;
+  unsigned long long before = 0;
+  for (uint32_t k = tid; k < sup; k += kSThreads) before += sums[k];
+  for (uint32_t k = sup * kSuperGroups + tid; k < g0; k += kSThreads) before += group_cnt[k];
+  // the warp's rows: kIter groups of 32
+  const uint64_t w0 = uint64_t(tile) * kCrsRows + uint64_t(warp) * (kIter * 32);
+  uint2 v[kIter];
+  uint32_t c[kIter];
+#pragma unroll
+  for (int u = 0; u < kIter; ++u) {
+    const uint64_t r = w0 + u * 32 + lane;
+    v[u] = r < n ? ld_slot(slots, r) : empty_slot();
+  }
+  uint32_t sum = 0;
+#pragma unroll
+  for (int u = 0; u < kIter; ++u) {
+    const uint32_t k = slot_count(v[u]);
+    c[u] = group_incl_sum<32>(kFullMask, k, lane);  // inclusive within the group
+    sum += __shfl_sync(kFullMask, c[u], 31);
+  }
+  before = group_sum<32>(kFullMask, before);
+  if (lane == 0) {
+    pre[warp] = before;
+    wsum[warp] = sum;
+  }
+  __syncthreads();
+  unsigned long long at = 0;
+#pragma unroll
+  for (int w = 0; w < kSWarps; ++w) {
+    at += pre[w];
+    if (w < warp) at += wsum[w];
+  }
+  uint2* const out = reinterpret_cast<uint2*>(entries);
+#pragma unroll
+  for (int u = 0; u < kIter; ++u) {
+    const uint64_t r = w0 + u * 32 + lane;
+    const uint32_t tot = __shfl_sync(kFullMask, c[u], 31);
+    if (r < n) {
+      rowmap[r + 1] = 2 * (at + c[u]);
+      if (r == 0) rowmap[0] = 0;
+      if (2 * (at + c[u]) > cap) {
+        atomicOr(&ctl->status, 256ull);
+      } else if (is_run(v[u])) {
+        out[at + c[u] - 1] = v[u];
+      } else {
+        const uint32_t k = slot_count(v[u]);
+        for (uint32_t q = 0; q < k; ++q) out[at + c[u] - k + q] = slot_range(arena, v[u], q);
+      }
+    }
+    at += tot;
+  }
+}
+
+template <bool OUTS, bool OUTC, bool COUNT>
+void launch_pass(dvg_context* ctx, const ChainArgs& p) {
+  // one kernel while a warp a 32 rows fits the chip at once; the second
+  // kernel's launch costs more than it saves there
+  if (p.n <= kSmallRows) {
+    k_chain_small<OUTS, OUTC, COUNT><<<(p.n + kWThreads - 1) / kWThreads, kWThreads, 0, ctx->stream>>>(p);
+    DVG_CUDA(cudaGetLastError());
+    ctx->stats.kernel_launches++;
+    return;
+  }
+  k_chain_rows<OUTS, OUTC, COUNT><<<unsigned((uint64_t(p.n) + kSThreads * kSRows - 1) / (kSThreads * kSRows)),
+                                    kSThreads, 0, ctx->stream>>>(p);
+  DVG_CUDA(cudaGetLastError());
+  const uint64_t want = (uint64_t(p.n) + 32 * kWWarps - 1) / (32 * kWWarps);
+  k_chain_walk<OUTS, OUTC, COUNT><<<unsigned(std::min<uint64_t>(want, 7ull * ctx->num_sms)), kWThreads, 0,
+                                    ctx->stream>>>(p);
+  DVG_CUDA(cudaGetLastError());
+  ctx->stats.kernel_launches += 2;
+}
+
+}  // namespace
+
+// What the left factors of one pass may add up to in steps of A: past it most
+// rows would have left the single column on the way, and walking a product of
+// several factors a row repeats what one factor at a time shares between rows.
+static unsigned chain_reach(double branching) {
+  const double r = kChainReach / std::max(branching, 1e-9);
+  return r >= 1e9 ? 1000000000u : std::max(1u, unsigned(r));
+}
+
+SlotPlan plan_slots(unsigned dlo, unsigned dup, double branching) {
+  SlotPlan pl;
+  const unsigned K = dup - dlo, reach = chain_reach(branching);
+  auto top_bit = [](unsigned v) { return v ? 31 - __builtin_clz(v) : -1; };
+  struct Power {
+    unsigned e;  // A^e
+    int mat;
+  };
+  std::vector<Power> P{{1u, 0}};
+  auto pass = [&](const std::vector<Power>& left, int b, unsigned bits, bool s, bool c) {
+    SlotStep st;
+    st.k = int(left.size());
+    for (int j = 0; j < st.k; ++j) st.m[j] = left[j].mat;
+    st.b = b;
+    st.bits = bits;
+    if (s) st.s = pl.nmats++;
+    if (c) st.c = pl.nmats++;
+    pl.steps.push_back(st);
+  };
+  // (A + I)^(2^t) = Q by doubling, with the powers of A on the way: from A^e and
+  // (A + I)^e to their f-th powers in one pass, f = 4 while the reach allows
+  const int t = top_bit(K);
+  const unsigned q_top = K > 0 ? 1u << t : 0u;
+  const unsigned rest = K > 0 ? K - q_top : 0;
+  // from A^e on the way to A^top (and, first, to (A + I)^q_top): the next power
+  auto factor = [&](unsigned e, unsigned top) {
+    return 4ull * e <= (e < q_top ? q_top : top) && 4ull * e <= reach ? 4u : 2u;
+  };
+  auto levels = [&](unsigned top) {
+    std::vector<unsigned> v{1u};
+    for (unsigned e = 1; e < std::max(top, q_top);) {
+      e *= factor(e, top);
+      if (e <= top) v.push_back(e);
+    }
+    return v;
+  };
+  // passes that multiply by A^v, its factors the largest powers that fit
+  auto passes = [&](unsigned v, const std::vector<unsigned>& have) {
+    unsigned n = 0, k = 0;
+    unsigned long long sum = 0;
+    for (size_t j = have.size(); j-- > 0;)
+      for (; v >= have[j]; v -= have[j]) {
+        if (n == 0 || k == kChainMax || sum + have[j] > reach) {
+          ++n;
+          k = 0;
+          sum = 0;
+        }
+        ++k;
+        sum += have[j];
+      }
+    return n;
+  };
+  // powers up to half of Q's, and further where that saves passes over A^dlo
+  unsigned p_top = q_top > 1 ? q_top / 2 : 1;
+  if (rest) p_top = std::max(p_top, 1u << top_bit(rest));
+  unsigned best = ~0u;
+  for (unsigned long long top = p_top; top <= std::max<unsigned long long>(p_top, dlo); top *= 2) {
+    const std::vector<unsigned> have = levels(unsigned(top));
+    unsigned cost = passes(rest, have) + passes(dlo, have);
+    for (unsigned e = 1; e < std::max(unsigned(top), q_top); ++cost) e *= factor(e, unsigned(top));
+    if (cost < best) {
+      best = cost;
+      p_top = unsigned(top);
+    }
+  }
+  int Q = -1;
+  unsigned e = 1;  // the last power and the sum stand at e
+  while (e < std::max(p_top, q_top)) {
+    const unsigned f = factor(e, p_top);
+    const bool s = e * f <= p_top, c = K > 0 && e * f <= q_top;
+    if (!s && !c) break;
+    const Power last = P.back();
+    // the factors S_1 .. S_f; c needs S_0 .. S_(f-1) times (A + I)^e, for e = 1
+    // that is S_0 .. S_f itself
+    const unsigned bits = e == 1 ? (1u << (f + 1)) - 1 : (1u << f) - 1;
+    const unsigned k = s || e == 1 ? f : f - 1;
+    pass(std::vector<Power>(k, last), e == 1 ? -1 : Q, c ? bits : 0u, s, c);
+    if (s) P.push_back({e * f, pl.steps.back().s});
+    if (c) Q = pl.steps.back().c;
+    e *= f;
+  }
+  // the fewest factors whose exponents add up to v, the largest first
+  auto factors = [&](unsigned v) {
+    std::vector<Power> f;
+    for (int j = int(P.size()) - 1; j >= 0; --j)
+      for (; v >= P[j].e; v -= P[j].e) f.push_back(P[j]);
+    return f;
+  };
+  // takes the next pass's factors off the list
+  auto next = [&](std::vector<Power>& f) {
+    std::vector<Power> g;
+    unsigned long long sum = 0;
+    while (!f.empty() && int(g.size()) < kChainMax && (g.empty() || sum + f.back().e <= reach)) {
+      sum += f.back().e;
+      g.push_back(f.back());
+      f.pop_back();
+    }
+    return g;
+  };
+  int R = Q;
+  if (K == 1) {  // I + A
+    pass({P[0]}, -1, 3u, false, true);
+    R = pl.steps.back().c;
+  }
+  // (A + I)^(v + w) = (A + I)^v + A^w (A + I)^v for w <= v + 1
+  for (std::vector<Power> f = factors(rest); !f.empty();) {
+    const std::vector<Power> g = next(f);
+    pass(g, R, 1u | (1u << g.size()), false, true);
+    R = pl.steps.back().c;
+  }
+  // A^dlo from the left: the right operand is a sum of powers, whose rows are
+  // one run, not a power, whose rows fall apart
+  std::vector<Power> f = factors(dlo);
+  if (R < 0) {  // A^dlo alone: its largest factor is the first right operand
+    R = f.front().mat;
+    f.erase(f.begin());
+  }
+  while (!f.empty()) {
+    const std::vector<Power> g = next(f);
+    pass(g, R, 1u << g.size(), false, true);
+    R = pl.steps.back().c;
+  }
+  // the last pass counts the result
+  if (pl.steps.empty() || pl.steps.back().s >= 0 || pl.steps.back().c != R) {
+    pass({}, R, 1u, false, true);
+    R = pl.steps.back().c;
+  }
+  pl.out = R;
+  return pl;
+}
+
+// Rows of a sequence graph's adjacency hold about one range of one or two
+// columns.  Where A has more than 1.5 ranges a row or ranges of more than two
+// columns on average, the powers' rows soon leave the slots for the arena, or
+// name so many rows that a thread walks them for long: such input, input whose
+// rows are not canonical, and matrices whose columns reach the marker of a
+// several-run row stay with the range-CRS row kernel.
+bool slots_suit(const dvg_context* ctx, const dvg_matrix* a) {
+  const uint64_t ranges = a->nentries / 2;
+  return a->canonical && a->nrows == a->ncols && a->nrows > 0 && a->ncols < kSlotMulti &&
+         2 * ranges <= 3ull * a->nrows && a->nnz <= 2 * ranges && ctx->opt_slots != 0;
+}
+
+// Columns of a row beyond its first, on average: how fast rows leave the single column.
+static double branching(const dvg_matrix* a) {
+  return a->nnz > a->nrows ? double(a->nnz - a->nrows) / double(a->nrows) : 0.0;
+}
+
+SlotBuild prepare_slots(dvg_context* ctx, const SlotPlan& plan, uint32_t n) {
+  SlotBuild sb;
+  sb.plan = plan;
+  sb.n = n;
+  sb.mat.assign(plan.nmats, nullptr);
+  sb.live.assign(plan.nmats, 0);
+  const uint64_t groups = (uint64_t(n) + kCountRows - 1) / kCountRows;
+  const uint64_t supers = (groups + kSuperGroups - 1) / kSuperGroups;
+  const size_t sums_off = 512, nnz_off = sums_off + supers * 8, cnt_off = nnz_off + groups * 8;
+  const size_t masks_off = cnt_off + groups * 4;
+  static_assert(sizeof(DeviceControl) <= 256, "the counters come first");
+  std::vector<int> last(plan.nmats, -1);
+  auto reads = [&](const SlotStep& s, auto&& f) {
+    for (int j = 0; j < s.k; ++j) f(s.m[j]);
+    if (s.b >= 0) f(s.b);
+  };
+  for (size_t i = 0; i < plan.steps.size(); ++i) reads(plan.steps[i], [&](int k) { last[k] = int(i); });
+  // (below kMulti, so that the slot of a row of several runs has y < x)
+  sb.arena_cap = std::min<uint64_t>(uint64_t(ctx->slot_growth * double(n)) + 4096, kMulti);
+  const double room = 0.5 * double(device_free_bytes(ctx) + ctx->cached_bytes);
+  if (double(sb.arena_cap) * 8.0 > room) sb.arena_cap = uint64_t(room / 8.0) + 4096;
+  auto take = [&](int k) {
+    sb.mat[k] = static_cast<uint2*>(dalloc(ctx, size_t(n) * sizeof(uint2)));
+    sb.live[k] = 1;
+  };
+  try {
+    sb.scratch = dalloc(ctx, masks_off + (uint64_t(n) + 31) / 32 * 4);
+    char* base = static_cast<char*>(sb.scratch);
+    sb.ctl = reinterpret_cast<DeviceControl*>(base);
+    sb.top = reinterpret_cast<unsigned long long*>(base + 256);
+    sb.abort = sb.top + 1;
+    sb.sums = reinterpret_cast<unsigned long long*>(base + sums_off);
+    sb.group_nnz = reinterpret_cast<unsigned long long*>(base + nnz_off);
+    sb.group_cnt = reinterpret_cast<uint32_t*>(base + cnt_off);
+    sb.masks = reinterpret_cast<uint32_t*>(base + masks_off);
+    sb.arena = static_cast<uint2*>(dalloc(ctx, sb.arena_cap * sizeof(uint2)));
+    take(0);
+    for (size_t i = 0; i < plan.steps.size(); ++i) {
+      if (plan.steps[i].s >= 0) take(plan.steps[i].s);
+      if (plan.steps[i].c >= 0) take(plan.steps[i].c);
+      // a matrix whose last reader is this step goes back now: stream order
+      // makes the reuse of its block by later steps safe
+      reads(plan.steps[i], [&](int k) {
+        if (last[k] == int(i) && k != plan.out && sb.live[k]) {
+          dfree(ctx, sb.mat[k]);
+          sb.live[k] = 0;
+        }
+      });
+    }
+  } catch (...) {
+    release_slots(ctx, sb);
+    throw;
+  }
+  return sb;
+}
+
+void release_slots(dvg_context* ctx, SlotBuild& sb) {
+  for (size_t k = 0; k < sb.mat.size(); ++k) {
+    if (sb.live[k]) dfree(ctx, sb.mat[k]);
+    sb.live[k] = 0;
+  }
+  if (sb.arena) dfree(ctx, sb.arena);
+  sb.arena = nullptr;
+  if (sb.scratch) dfree(ctx, sb.scratch);
+  sb.scratch = nullptr;
+}
+
+void launch_slots(dvg_context* ctx, SlotBuild& sb, const uint64_t* rowmap, const uint32_t* entries) {
+  const uint64_t t0 = now_ns();
+  DVG_CUDA(cudaMemsetAsync(sb.scratch, 0, 512, ctx->stream));
+  ctx->stats.kernel_launches++;
+  ChainArgs p{};
+  p.arena = sb.arena;
+  p.top = sb.top;
+  p.arena_cap = sb.arena_cap;
+  p.ctl = sb.ctl;
+  p.abort = sb.abort;
+  p.masks = sb.masks;
+  p.group_cnt = sb.group_cnt;
+  p.group_nnz = sb.group_nnz;
+  p.n = sb.n;
+  p.s = sb.mat[0];
+  const unsigned blocks =
+      unsigned(std::min<uint64_t>((uint64_t(sb.n) + kSThreads - 1) / kSThreads, 16ull * ctx->num_sms));
+  k_crs_to_slots<<<blocks, kSThreads, 0, ctx->stream>>>(rowmap, entries, p);
+  DVG_CUDA(cudaGetLastError());
+  ctx->stats.kernel_launches++;
+  for (size_t i = 0; i < sb.plan.steps.size(); ++i) {
+    const SlotStep& st = sb.plan.steps[i];
+    p.k = uint32_t(st.k);
+    p.bits = st.bits;
+    for (int j = 0; j < kChainMax; ++j) p.m[j] = j < st.k ? sb.mat[st.m[j]] : nullptr;
+    p.b = st.b >= 0 ? sb.mat[st.b] : nullptr;
+    p.s = st.s >= 0 ? sb.mat[st.s] : nullptr;
+    p.c = st.c >= 0 ? sb.mat[st.c] : nullptr;
+    cudaEvent_t ev = span_begin(ctx);
+    if (i + 1 == sb.plan.steps.size()) launch_pass<false, true, true>(ctx, p);
+    else if (p.s && p.c) launch_pass<true, true, false>(ctx, p);
+    else if (p.s) launch_pass<true, false, false>(ctx, p);
+    else launch_pass<false, true, false>(ctx, p);
+    span_end(ctx, ev, kProduct);
+  }
+  const uint64_t groups = (uint64_t(sb.n) + kCountRows - 1) / kCountRows;
+  k_slot_sums<<<unsigned((groups + kSuperGroups - 1) / kSuperGroups), kSThreads, 0, ctx->stream>>>(
+      sb.group_cnt, sb.group_nnz, groups, sb.sums, sb.ctl);
+  DVG_CUDA(cudaGetLastError());
+  ctx->stats.kernel_launches++;
+  ctx->stats.host_launch_ns += now_ns() - t0;
+}
+
+dvg_matrix* finish_slots(dvg_context* ctx, SlotBuild& sb) {
+  struct Counters {
+    DeviceControl ctl;
+    char pad[256 - sizeof(DeviceControl)];
+    unsigned long long top, abort;
+  };
+  auto* h = static_cast<Counters*>(host_stage(ctx, sizeof(Counters)));
+  dvg_matrix* m = nullptr;
+  try {
+    DVG_CUDA(cudaMemcpyAsync(h, sb.scratch, sizeof(Counters), cudaMemcpyDeviceToHost, ctx->stream));
+    const uint64_t t0 = now_ns();
+    DVG_CUDA(cudaStreamSynchronize(ctx->stream));
+    ctx->stats.host_sync_ns += now_ns() - t0;
+    ctx->stats.host_syncs++;
+    resolve_spans(ctx);
+    if (h->abort) {
+      // more rows of several runs than the arena was sized for: the caller
+      // takes the range-CRS path, later chains a larger arena
+      ctx->slot_growth = std::min(2.0 * ctx->slot_growth, 64.0);
+      release_slots(ctx, sb);
+      return nullptr;
+    }
+    const Counters c = *h;
+    m = new_matrix(ctx, sb.n, sb.n, c.ctl.total);
+    m->nnz = c.ctl.nnz;
+    m->canonical = true;
+    k_slots_to_crs<<<unsigned((uint64_t(sb.n) + kCrsRows - 1) / kCrsRows), kSThreads, 0, ctx->stream>>>(
+        sb.mat[sb.plan.out], sb.arena, sb.sums, sb.group_cnt, sb.n, m->rowmap, m->entries, m->nentries, ctx->d_ctl);
+    DVG_CUDA(cudaGetLastError());
+    ctx->stats.kernel_launches++;
+    // statistics: what every pass had to move, 8 bytes a row for each matrix it
+    // reads or writes, and the products that it stands for
+    uint64_t bytes = 0, products = 0, adds = 0;
+    for (const SlotStep& st : sb.plan.steps) {
+      std::vector<int> seen;
+      auto once = [&](int k) {
+        if (k < 0 || std::find(seen.begin(), seen.end(), k) != seen.end()) return;
+        seen.push_back(k);
+        bytes += 8ull * sb.n;
+      };
+      for (int j = 0; j < st.k; ++j) once(st.m[j]);
+      for (int k : {st.b, st.s, st.c}) once(k);
+      const int gathers = __builtin_popcount(st.bits >> 1);
+      products += st.s >= 0 ? std::max(st.k - 1, 0) : 0;
+      if (st.c >= 0) products += st.b >= 0 ? gathers + (st.s >= 0 ? 0 : st.k - 1) : (st.s >= 0 ? 0 : st.k);
+      adds += st.c >= 0 && (st.bits & (st.bits - 1)) ? __builtin_popcount(st.bits) - 1 : 0;
+    }
+    ctx->stats.alg_bytes += bytes;
+    ctx->stats.spgemm_alg_bytes += bytes;
+    ctx->stats.spgemm_calls += products;
+    ctx->stats.spgemm_light += products;
+    ctx->stats.spgemm_fused_adds += adds;
+    ctx->stats.spgemm_slow_rows += c.ctl.slow_rows;
+  } catch (...) {
+    free_matrix(ctx, m);
+    release_slots(ctx, sb);
+    throw;
+  }
+  release_slots(ctx, sb);
+  return m;
+}
+
+dvg_matrix* slots_chain(dvg_context* ctx, const dvg_matrix* a, unsigned dlo, unsigned dup) {
+  SlotBuild sb;
+  try {
+    sb = prepare_slots(ctx, plan_slots(dlo, dup, branching(a)), a->nrows);
+  } catch (const Error& e) {
+    if (e.status != DVG_ERR_OOM) throw;
+    return nullptr;
+  }
+  try {
+    launch_slots(ctx, sb, a->rowmap, a->entries);
+  } catch (...) {
+    release_slots(ctx, sb);
+    throw;
+  }
+  return finish_slots(ctx, sb);
+}
+
+}  // namespace dvg

@@ -1,0 +1,119 @@
+"""GPU: index builds as passes over row slots against the oracle and against
+the same builds in range CRS (option "row_slots" 0): sizes around the edges of
+warps, count groups, conversion blocks and the one-kernel limit, rows of more
+runs than a lane's list and of columns wider apart than its mask, and input that
+stays in range CRS."""
+import numpy as np
+import pytest
+
+from diverg_b200 import CRSMatrix, gen
+from diverg_b200.runtime import Context
+from oracle import pyoracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = Context(0)
+    yield c
+    c.close()
+
+
+def omat(m):
+    return orc.OMat(m.numRows(), m.numCols(), m.rowmap, m.entries, m.nnz())
+
+
+def check(ctx, a, window, slots=True):
+    want = orc.dindex(omat(a), *window, algo="hbv")
+    da = ctx.upload(a)
+    ctx.reset_stats()
+    got = ctx.distance_index(da, *window).download()
+    st = ctx.stats()
+    ctx.set_option("row_slots", 0)
+    try:
+        ctx.reset_stats()
+        crs = ctx.distance_index(da, *window).download()
+        crs_st = ctx.stats()
+    finally:
+        ctx.set_option("row_slots", 1)
+    for m in (got, crs):
+        assert np.array_equal(m.rowmap, want.rowmap), window
+        assert np.array_equal(m.entries, want.entries), window
+        assert m.nnz() == want.nnz, window
+    # the two forms move different bytes
+    assert slots == (st["spgemm_alg_bytes"] != crs_st["spgemm_alg_bytes"])
+
+
+def rows(a, n):
+    """The first n rows and columns of a."""
+    rm = a.rowmap[:n + 1]
+    e = a.entries[:int(rm[-1])].copy().reshape(-1, 2)
+    keep = e[:, 0] < n
+    e[:, 1] = np.minimum(e[:, 1], n - 1)
+    cnt = np.add.reduceat(np.append(keep, False).astype(np.int64), (rm[:-1] // 2).astype(np.int64)) if n else []
+    empty = rm[1:] == rm[:-1]
+    cnt = np.where(empty, 0, cnt)
+    return CRSMatrix(n, e[keep].reshape(-1), np.concatenate(([0], np.cumsum(2 * cnt))).astype(np.uint64))
+
+
+GRAPH = None
+
+
+def graph():
+    global GRAPH
+    if GRAPH is None:
+        GRAPH, _ = gen.graph_adjacency(gen.small_graph_spec(300_000, seed=61))
+    return GRAPH
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 127, 128, 129, 1023, 1024, 1025, 65_535, 65_537,
+                               131_071, 131_072, 131_073, 131_200, 262_145])
+@pytest.mark.parametrize("window", [(3, 11), (0, 70)])
+def test_sizes(ctx, n, window):
+    check(ctx, rows(graph(), n), window)
+
+
+@pytest.mark.parametrize("n", [5_000, 140_001])
+@pytest.mark.parametrize("window", [(0, 1), (1, 1), (1, 2), (2, 2), (0, 2), (0, 5), (64, 64), (9, 11), (100, 300),
+                                    (0, 250), (350, 650), (1000, 1003)])
+def test_windows(ctx, n, window):
+    check(ctx, rows(graph(), n), window)
+
+
+@pytest.mark.parametrize("spec", [
+    gen.GraphSpec(150_000, 0.02, 0.05, 0.5, 1, 60, 0.0, 0.0, 100, 2000, 5),     # many runs a row
+    gen.GraphSpec(150_000, 0.001, 0.004, 0.5, 1, 10, 0.0, 0.5, 100, 4000, 6),   # runs far apart
+    gen.GraphSpec(400_000, 0.001, 0.0005, 0.2, 1, 10, 0.0, 0.6, 9000, 20000, 7),  # and past a window
+])
+@pytest.mark.parametrize("window", [(100, 140), (0, 90), (300, 300)])
+def test_branching_graphs(ctx, spec, window):
+    a, _ = gen.graph_adjacency(spec)
+    check(ctx, a, window)
+
+
+@pytest.mark.parametrize("hw", [40, 3_000])
+@pytest.mark.parametrize("window", [(2, 5), (0, 4)])
+def test_columns_anywhere_near(ctx, hw, window):
+    # about one short range a row at random in the band: rows fill up quickly
+    a = gen.banded(140_500, hw, 1.2, 1.2, seed=63)
+    assert a.entries.size <= 3 * a.numRows() and a.nnz() <= a.entries.size
+    check(ctx, a, window)
+
+
+def test_a_full_arena_falls_back(ctx):
+    # rows of random columns double with every factor: more ranges than the
+    # arena holds, and the build runs again in range CRS
+    a = gen.banded(3_000, 3_000, 1.4, 1.0, seed=64)
+    want = orc.dindex(omat(a), 12, 12, algo="hbv")
+    ctx.reset_stats()
+    got = ctx.distance_index(ctx.upload(a), 12, 12).download()
+    assert np.array_equal(got.rowmap, want.rowmap) and np.array_equal(got.entries, want.entries)
+    assert ctx.stats()["spgemm_reruns"] >= 1
+
+
+def test_dense_and_noncanonical_input_stays_in_range_crs(ctx):
+    check(ctx, gen.random_matrix(2_000, 8_000, seed=65), (1, 3), slots=False)   # 4 ranges a row
+    check(ctx, gen.banded(2_000, 200, 1.0, 12.0, seed=66), (1, 3), slots=False)  # ranges of 12 columns
+    split = CRSMatrix(6, np.array([1, 1, 2, 3, 3, 3, 5, 5], np.uint32), np.array([0, 4, 6, 6, 8, 8, 8], np.uint64))
+    check(ctx, split, (1, 3), slots=False)
