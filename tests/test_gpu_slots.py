@@ -117,3 +117,13 @@ def test_dense_and_noncanonical_input_stays_in_range_crs(ctx):
     check(ctx, gen.banded(2_000, 200, 1.0, 12.0, seed=66), (1, 3), slots=False)  # ranges of 12 columns
     split = CRSMatrix(6, np.array([1, 1, 2, 3, 3, 3, 5, 5], np.uint32), np.array([0, 4, 6, 6, 8, 8, 8], np.uint64))
     check(ctx, split, (1, 3), slots=False)
+
+
+@pytest.mark.parametrize("n", [33, 131_073])
+@pytest.mark.parametrize("k", [0, 1, 2, 3, 63, 64, 100])
+def test_powers(ctx, n, k):
+    a = rows(graph(), n)
+    want = orc.power(omat(a), k, algo="hbv")
+    got = ctx.power(ctx.upload(a), k).download()
+    assert np.array_equal(got.rowmap, want.rowmap) and np.array_equal(got.entries, want.entries)
+    assert got.nnz() == want.nnz
