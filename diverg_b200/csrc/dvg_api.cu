@@ -735,6 +735,8 @@ dvg_status dvg_shutdown(dvg_context* ctx) {
     resolve_spans(ctx);
     for (cudaEvent_t e : ctx->event_pool) cudaEventDestroy(e);
     ctx->event_pool.clear();
+    for (cudaEvent_t e : ctx->side_events) cudaEventDestroy(e);
+    for (cudaStream_t t : ctx->side_streams) cudaStreamDestroy(t);
     DVG_CUDA(cudaFree(ctx->d_ctl));
     DVG_CUDA(cudaFreeHost(ctx->h_ctl));
     if (ctx->h_stage) DVG_CUDA(cudaFreeHost(ctx->h_stage));

@@ -10,6 +10,13 @@
 // graph's index is then cut out of its group's result (rows rebased, columns
 // shifted back), giving exactly what a build of that graph alone gives.
 //
+// Graph-like input (slots_suit) is built as passes over row slots
+// (dvg_slots.cu): a window's graphs go side by side into one chain, laid out and
+// cut apart again by the chain's own conversions, and the chains of different
+// windows are branches of the CUDA graph that run side by side.  The other
+// graphs are assembled in range CRS, built as planned sequences of products one
+// window after another, and cut apart.
+//
 // The reference builds graphs one at a time (dindex.hpp:46-189 per
 // component); its own combination of components (crs_matrix.hpp:1448-1518
 // builds rows component by component) is the layout used here.
@@ -22,6 +29,7 @@
 #include <tuple>
 
 #include "dvg_internal.h"
+#include "dvg_slots.h"
 
 namespace dvg {
 namespace {
@@ -136,6 +144,60 @@ struct Group {
   size_t table_off = 0;            // slices in the device table (GraphSlice units)
 };
 
+// Graphs of one window that run as one chain over row slots.
+struct SlotGroup {
+  unsigned dlo, dup;
+  std::vector<uint32_t> members;
+  std::vector<SlotPart> parts;     // one a member
+  std::vector<uint32_t> part_of;   // one a kSlotPartRows rows
+  uint64_t n = 0, nnz = 0;
+  SlotBuild sb;
+  SlotParts table{};               // on the device
+  unsigned long long* totals = nullptr;
+  bool ready = false;
+};
+
+// Issues a context's work on another stream while in scope.
+struct OnStream {
+  dvg_context* ctx;
+  cudaStream_t kept;
+  OnStream(dvg_context* c, cudaStream_t s) : ctx(c), kept(c->stream) { ctx->stream = s; }
+  ~OnStream() { ctx->stream = kept; }
+};
+
+// Chains that run side by side: most of a chain's passes over small graphs are
+// bound by latency, so a few at once cost little more than one.
+constexpr size_t kSideStreams = 4;
+
+void make_side_streams(dvg_context* ctx, size_t n) {
+  while (ctx->side_streams.size() < n) {
+    cudaStream_t t;
+    DVG_CUDA(cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking));
+    ctx->side_streams.push_back(t);
+  }
+  while (ctx->side_events.size() < n + 1) {
+    cudaEvent_t e;
+    DVG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    ctx->side_events.push_back(e);
+  }
+}
+
+// Lays the members' rows side by side, each from a multiple of kSlotPartRows on.
+void lay_out(SlotGroup& g, const dvg_matrix* const* graphs) {
+  for (uint32_t k : g.members) {
+    SlotPart part{};
+    part.rowmap = graphs[k]->rowmap;
+    part.entries = graphs[k]->entries;
+    part.row0 = uint32_t(g.n);
+    part.n = graphs[k]->nrows;
+    const uint32_t blocks = uint32_t((uint64_t(part.n) + kSlotPartRows - 1) / kSlotPartRows);
+    g.part_of.insert(g.part_of.end(), blocks, uint32_t(g.parts.size()));
+    g.parts.push_back(part);
+    g.n += uint64_t(blocks) * kSlotPartRows;
+    g.nnz += graphs[k]->nnz + (uint64_t(blocks) * kSlotPartRows - part.n);
+  }
+}
+
 }  // namespace
 
 // Times planned builds of `a` over the candidate kernel shapes and keeps the
@@ -193,7 +255,7 @@ void batch_distance_index(dvg_context* ctx, uint32_t ngraphs, const dvg_matrix* 
                           const unsigned* dmax, dvg_matrix** out) {
   for (uint32_t k = 0; k < ngraphs; ++k) out[k] = nullptr;
   // ---- validation and grouping -------------------------------------------------
-  std::map<std::pair<unsigned, unsigned>, std::vector<uint32_t>> by_window;
+  std::map<std::pair<unsigned, unsigned>, std::vector<uint32_t>> by_window, slots_by_window;
   std::vector<uint32_t> alone;  // built one by one (non-canonical input with dmin = 0)
   for (uint32_t k = 0; k < ngraphs; ++k) {
     const dvg_matrix* a = graphs[k];
@@ -203,6 +265,8 @@ void batch_distance_index(dvg_context* ctx, uint32_t ngraphs, const dvg_matrix* 
     if ((dmin[k] == 0 && !a->canonical) || !ctx->opt_planned || ctx->opt_spgemm_mode == 1 ||
         ctx->opt_dindex_schedule != 0)
       alone.push_back(k);
+    else if (ctx->opt_spgemm_mode == 0 && slots_suit(ctx, a))
+      slots_by_window[{dmin[k], dmax[k]}].push_back(k);
     else
       by_window[{dmin[k], dmax[k]}].push_back(k);
   }
@@ -225,7 +289,24 @@ void batch_distance_index(dvg_context* ctx, uint32_t ngraphs, const dvg_matrix* 
     }
     if (!cur.members.empty()) groups.push_back(std::move(cur));
   }
-  if (groups.empty()) {
+  std::vector<SlotGroup> chains;
+  for (auto& kv : slots_by_window) {
+    // at most as many rows as columns have numbers
+    uint64_t rows = 0;
+    for (uint32_t k : kv.second) {
+      const uint64_t n = (uint64_t(graphs[k]->nrows) + kSlotPartRows - 1) / kSlotPartRows * kSlotPartRows;
+      if (rows == 0 || rows + n >= kSlotMulti) {
+        chains.emplace_back();
+        rows = 0;
+      }
+      chains.back().dlo = kv.first.first;
+      chains.back().dup = kv.first.second;
+      chains.back().members.push_back(k);
+      rows += n;
+    }
+  }
+  for (auto& g : chains) lay_out(g, graphs);
+  if (groups.empty() && chains.empty()) {
     try {
       for (uint32_t k : alone) out[k] = create_distance_index(ctx, graphs[k], dmin[k], dmax[k]);
     } catch (...) {
@@ -238,6 +319,10 @@ void batch_distance_index(dvg_context* ctx, uint32_t ngraphs, const dvg_matrix* 
     return;
   }
   auto cleanup = [&]() {
+    for (auto& g : chains) {
+      if (g.ready) release_slots(ctx, g.sb);
+      g.ready = false;
+    }
     for (auto& g : groups) {
       if (g.planned) release_build(ctx, g.pb);
       g.planned = false;
@@ -247,9 +332,45 @@ void batch_distance_index(dvg_context* ctx, uint32_t ngraphs, const dvg_matrix* 
     }
   };
   void* d_table = nullptr;
+  void* d_parts = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   try {
+    // ---- the chains' buffers ------------------------------------------------------
+    // (before any planned build's: those hand blocks back that their own later
+    // steps, on the one stream, still write; a chain beside them must not get one)
+    for (auto it = chains.begin(); it != chains.end();) {
+      try {
+        it->sb = prepare_slots(ctx, plan_slots(it->dlo, it->dup, branching(it->nnz, it->n)), uint32_t(it->n));
+        it->ready = true;
+        ++it;
+      } catch (const Error& e) {
+        if (e.status != DVG_ERR_OOM) throw;
+        alone.insert(alone.end(), it->members.begin(), it->members.end());  // too large together
+        it = chains.erase(it);
+      }
+    }
+    // their tables: parts, part of every block, totals
+    size_t nparts = 0, nblocks = 0;
+    for (auto& g : chains) {
+      nparts += g.parts.size();
+      nblocks += g.part_of.size();
+    }
+    const size_t part_bytes = nparts * sizeof(SlotPart) + nblocks * 4;
+    const size_t totals_off = (part_bytes + 255) & ~size_t(255);
+    if (nparts) {
+      d_parts = dalloc(ctx, totals_off + nparts * 16);
+      size_t p0 = 0, b0 = nparts * sizeof(SlotPart), t0 = totals_off;
+      for (auto& g : chains) {
+        char* base = static_cast<char*>(d_parts);
+        g.table.table = reinterpret_cast<SlotPart*>(base + p0);
+        g.table.part_of = reinterpret_cast<uint32_t*>(base + b0);
+        g.totals = reinterpret_cast<unsigned long long*>(base + t0);
+        p0 += g.parts.size() * sizeof(SlotPart);
+        b0 += g.part_of.size() * 4;
+        t0 += g.parts.size() * 16;
+      }
+    }
     // ---- the block-diagonal inputs ---------------------------------------------
     size_t nslices = 0;
     for (auto& g : groups) {
@@ -270,10 +391,26 @@ void batch_distance_index(dvg_context* ctx, uint32_t ngraphs, const dvg_matrix* 
     const size_t table_bytes = std::max<size_t>(nslices, 1) * sizeof(GraphSlice);
     d_table = dalloc(ctx, table_bytes);
     {
-      auto* h = static_cast<GraphSlice*>(host_stage(ctx, table_bytes));
+      char* stage = static_cast<char*>(host_stage(ctx, part_bytes + 8 + table_bytes));
+      char* to = stage;
+      for (auto& g : chains) {
+        std::memcpy(to, g.parts.data(), g.parts.size() * sizeof(SlotPart));
+        to += g.parts.size() * sizeof(SlotPart);
+      }
+      for (auto& g : chains) {
+        std::memcpy(to, g.part_of.data(), g.part_of.size() * 4);
+        to += g.part_of.size() * 4;
+      }
+      if (part_bytes) {
+        DVG_CUDA(cudaMemcpyAsync(d_parts, stage, part_bytes, cudaMemcpyHostToDevice, ctx->stream));
+        ctx->stats.h2d_bytes += part_bytes;
+      }
+      auto* h = reinterpret_cast<GraphSlice*>(stage + ((part_bytes + 7) & ~size_t(7)));
       for (auto& g : groups) std::memcpy(h + g.table_off, g.slices.data(), g.slices.size() * sizeof(GraphSlice));
-      DVG_CUDA(cudaMemcpyAsync(d_table, h, nslices * sizeof(GraphSlice), cudaMemcpyHostToDevice, ctx->stream));
-      ctx->stats.h2d_bytes += nslices * sizeof(GraphSlice);
+      if (nslices) {
+        DVG_CUDA(cudaMemcpyAsync(d_table, h, nslices * sizeof(GraphSlice), cudaMemcpyHostToDevice, ctx->stream));
+        ctx->stats.h2d_bytes += nslices * sizeof(GraphSlice);
+      }
     }
     auto* table = static_cast<GraphSlice*>(d_table);
     auto assemble = [&](Group& g) {
@@ -299,11 +436,25 @@ void batch_distance_index(dvg_context* ctx, uint32_t ngraphs, const dvg_matrix* 
       g.planned = true;
     }
     // ---- one CUDA graph: every group's assembly and build ------------------------
+    const size_t nside = std::min(chains.size(), kSideStreams);
+    if (nside) make_side_streams(ctx, nside);
     DVG_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     try {
+      if (nside) DVG_CUDA(cudaEventRecord(ctx->side_events[nside], ctx->stream));
+      for (size_t k = 0; k < nside; ++k)
+        DVG_CUDA(cudaStreamWaitEvent(ctx->side_streams[k], ctx->side_events[nside], 0));
+      for (size_t k = 0; k < chains.size(); ++k) {
+        OnStream on(ctx, ctx->side_streams[k % nside]);
+        launch_slots(ctx, chains[k].sb, chains[k].table, false);
+        launch_slots_totals(ctx, chains[k].sb, chains[k].table, uint32_t(chains[k].parts.size()), chains[k].totals);
+      }
       for (auto& g : groups) {
         assemble(g);
         launch_build(ctx, g.pb, false);
+      }
+      for (size_t k = 0; k < nside; ++k) {
+        DVG_CUDA(cudaEventRecord(ctx->side_events[k], ctx->side_streams[k]));
+        DVG_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->side_events[k], 0));
       }
     } catch (...) {
       cudaGraph_t dropped = nullptr;
@@ -326,13 +477,67 @@ void batch_distance_index(dvg_context* ctx, uint32_t ngraphs, const dvg_matrix* 
       free_matrix(ctx, g.g);
       g.g = nullptr;
     }
+    if (!chains.empty()) {
+      // every chain's counters and its graphs' sizes: one read-back for all
+      auto* hc = static_cast<SlotCounters*>(host_stage(ctx, chains.size() * sizeof(SlotCounters) + nparts * 16));
+      auto* ht = reinterpret_cast<unsigned long long*>(hc + chains.size());
+      for (size_t k = 0; k < chains.size(); ++k)
+        DVG_CUDA(cudaMemcpyAsync(hc + k, chains[k].sb.scratch, sizeof(SlotCounters), cudaMemcpyDeviceToHost, ctx->stream));
+      DVG_CUDA(cudaMemcpyAsync(ht, chains[0].totals, nparts * 16, cudaMemcpyDeviceToHost, ctx->stream));
+      const uint64_t ts = now_ns();
+      DVG_CUDA(cudaStreamSynchronize(ctx->stream));
+      ctx->stats.host_sync_ns += now_ns() - ts;
+      ctx->stats.host_syncs++;
+      std::vector<SlotPart> table;
+      size_t part = 0;
+      std::vector<char> whole(chains.size());
+      for (size_t k = 0; k < chains.size(); ++k) {
+        SlotGroup& g = chains[k];
+        whole[k] = check_slots(ctx, g.sb, hc[k]);
+        unsigned long long before = 0;
+        for (size_t j = 0; j < g.parts.size(); ++j, ++part) {
+          if (whole[k]) {
+            const uint32_t id = g.members[j];
+            dvg_matrix* m = new_matrix(ctx, graphs[id]->nrows, graphs[id]->ncols, 2 * ht[2 * part]);
+            out[id] = m;
+            m->nnz = ht[2 * part + 1];
+            m->canonical = true;
+            g.parts[j].c_rowmap = m->rowmap;
+            g.parts[j].c_entries = m->entries;
+            g.parts[j].c_ranges = ht[2 * part];
+            g.parts[j].before = before;
+            const uint64_t next = j + 1 < g.parts.size() ? g.parts[j + 1].row0 : g.n;
+            before += ht[2 * part] + (next - g.parts[j].row0 - g.parts[j].n);
+          }
+          table.push_back(g.parts[j]);
+        }
+      }
+      auto* hp = static_cast<SlotPart*>(host_stage(ctx, nparts * sizeof(SlotPart)));
+      std::memcpy(hp, table.data(), nparts * sizeof(SlotPart));
+      DVG_CUDA(cudaMemcpyAsync(d_parts, hp, nparts * sizeof(SlotPart), cudaMemcpyHostToDevice, ctx->stream));
+      ctx->stats.h2d_bytes += nparts * sizeof(SlotPart);
+      for (size_t k = 0; k < chains.size(); ++k) {
+        SlotGroup& g = chains[k];
+        if (whole[k]) launch_slots_out(ctx, g.sb, g.table);
+        release_slots(ctx, g.sb);
+        g.ready = false;
+        if (!whole[k]) {  // its graphs one by one
+          ctx->stats.spgemm_reruns++;
+          alone.insert(alone.end(), g.members.begin(), g.members.end());
+        }
+      }
+      // what follows uses the staging again: the table must have been read
+      if (!groups.empty() || !alone.empty()) DVG_CUDA(cudaStreamSynchronize(ctx->stream));
+      dfree(ctx, d_parts);
+      d_parts = nullptr;
+    }
     DVG_CUDA(cudaGraphExecDestroy(exec));
     exec = nullptr;
     DVG_CUDA(cudaGraphDestroy(graph));
     graph = nullptr;
     // where every graph's index starts in its group's, and its nnz: one
     // read-back for all
-    {
+    if (!groups.empty()) {
       const size_t nb = std::max<size_t>(nslices, 1);
       auto* d_bounds = static_cast<unsigned long long*>(dalloc(ctx, 2 * nb * 8));
       unsigned long long* d_nnz = d_bounds + nb;
@@ -397,6 +602,7 @@ void batch_distance_index(dvg_context* ctx, uint32_t ngraphs, const dvg_matrix* 
     if (graph) cudaGraphDestroy(graph);
     cleanup();
     if (d_table) dfree(ctx, d_table);
+    if (d_parts) dfree(ctx, d_parts);
     for (uint32_t k = 0; k < ngraphs; ++k) {
       free_matrix(ctx, out[k]);
       out[k] = nullptr;

@@ -101,6 +101,10 @@ struct dvg_context {
   std::unordered_map<void*, size_t> live_blocks;  // block -> bytes
   size_t cached_bytes = 0;
   size_t owned_bytes = 0;   // device memory this context holds (live + cached)
+  // streams and events of a batch's chains that run side by side, made on first
+  // use, given back at shutdown
+  std::vector<cudaStream_t> side_streams;
+  std::vector<cudaEvent_t> side_events;
   // the last cudaMemGetInfo answer, when it was taken, and owned_bytes then
   size_t mi_free = 0, mi_owned = 0;
   uint64_t mi_ns = 0;

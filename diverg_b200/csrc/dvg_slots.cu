@@ -46,7 +46,7 @@ constexpr uint32_t kMultiMax = 0xFFFFFFFFu - kMulti - 1;  // ranges of one row
 constexpr uint32_t kCountRows = 32 * kSRows;  // rows whose ranges the last pass counts together
 constexpr uint32_t kSmallRows = 1u << 17;     // rows up to which a pass is one kernel
 constexpr double kChainReach = 1.28;          // branching * steps of a pass's left factors
-constexpr int kCrsRows = 1024;                // rows of a block of the conversion
+constexpr int kCrsRows = kSlotPartRows;        // rows of a block of the conversions
 constexpr uint32_t kSuperGroups = 512;        // counts that k_slot_sums adds up
 
 __device__ __forceinline__ uint2 empty_slot() { return make_uint2(1u, 0u); }
@@ -729,27 +729,53 @@ __global__ void __launch_bounds__(kWThreads) k_chain_small(const __grid_constant
   }
 }
 
+// The matrices of a chain laid side by side on the diagonal, each from a
+// multiple of kCrsRows rows on, so that every block of the conversions below
+// works on one of them: block b's is number part_of[b] (a null table: all
+// blocks are `one`'s, the only one).
+struct Parts {
+  const SlotPart* __restrict__ table;
+  const uint32_t* __restrict__ part_of;
+  SlotPart one;
+};
+__device__ __forceinline__ SlotPart my_part(const Parts& q) { return q.table ? q.table[q.part_of[blockIdx.x]] : q.one; }
+
 // Range CRS -> slots.  Canonical input: a row of several ranges is copied to
-// the arena as it is.
-__global__ void __launch_bounds__(kSThreads) k_crs_to_slots(const uint64_t* __restrict__ rowmap,
-                                                            const uint32_t* __restrict__ entries,
+// the arena as it is.  Rows past a part's last are rows of the identity: one
+// column each, whatever the pass.
+__global__ void __launch_bounds__(kSThreads) k_crs_to_slots(const __grid_constant__ Parts q,
                                                             const __grid_constant__ ChainArgs p) {
-  const uint64_t stride = uint64_t(gridDim.x) * kSThreads;
+  constexpr int kIter = kCrsRows / kSThreads;
+  const SlotPart part = my_part(q);
   const int lane = lane_id();
-  for (uint64_t b0 = blockIdx.x * uint64_t(kSThreads) + (threadIdx.x & ~31u); b0 < p.n; b0 += stride) {
-    const uint64_t r = b0 + lane;
-    uint64_t a0 = 0, cnt = 0;
-    uint2 v = empty_slot();
-    if (r < p.n) {
-      a0 = __ldg(rowmap + r) >> 1;
-      cnt = (__ldg(rowmap + r + 1) >> 1) - a0;
-      if (cnt == 1) v = load_range(entries, a0);
+  const uint64_t b0 = uint64_t(blockIdx.x) * kCrsRows + threadIdx.x;
+  uint64_t a0[kIter], cnt[kIter];
+#pragma unroll
+  for (int u = 0; u < kIter; ++u) {
+    const uint64_t i = b0 + u * kSThreads - part.row0;
+    a0[u] = cnt[u] = 0;
+    if (i < part.n) {
+      a0[u] = __ldg(part.rowmap + i) >> 1;
+      cnt[u] = (__ldg(part.rowmap + i + 1) >> 1) - a0[u];
     }
-    uint64_t want = cnt > 1 ? cnt : 0;
-    if (cnt == 2) {
-      const uint2 a = load_range(entries, a0), b = load_range(entries, a0 + 1);
-      if (a.x == a.y && b.x == b.y) {
-        v = make_uint2(b.x, a.x);
+  }
+  auto range = [&](uint64_t k) {
+    uint2 v = load_range(part.entries, k);
+    v.x += part.row0;
+    v.y += part.row0;
+    return v;
+  };
+  uint2 v[kIter];
+#pragma unroll
+  for (int u = 0; u < kIter; ++u) v[u] = cnt[u] ? range(a0[u]) : empty_slot();
+#pragma unroll
+  for (int u = 0; u < kIter; ++u) {
+    const uint64_t r = b0 + u * kSThreads;
+    uint64_t want = cnt[u] > 1 ? cnt[u] : 0;
+    if (cnt[u] == 2) {
+      const uint2 w = range(a0[u] + 1);
+      if (v[u].x == v[u].y && w.x == w.y) {
+        v[u] = make_uint2(w.x, v[u].x);
         want = 0;
       }
     }
@@ -761,13 +787,14 @@ __global__ void __launch_bounds__(kSThreads) k_crs_to_slots(const uint64_t* __re
       if (want) {
         if (want > kMultiMax || off + want > p.arena_cap) {
           atomicOr(p.abort, 1ull);
+          v[u] = empty_slot();
         } else {
-          for (uint64_t k = 0; k < want; ++k) p.arena[off + k] = load_range(entries, a0 + k);
-          v = make_uint2(kMulti + uint32_t(want), uint32_t(off));
+          for (uint64_t k = 0; k < want; ++k) p.arena[off + k] = range(a0[u] + k);
+          v[u] = make_uint2(kMulti + uint32_t(want), uint32_t(off));
         }
       }
     }
-    if (r < p.n) p.s[r] = v;
+    if (r < p.n) p.s[r] = r - part.row0 < part.n ? v[u] : make_uint2(uint32_t(r), uint32_t(r));
   }
 }
 
@@ -802,20 +829,51 @@ __global__ void __launch_bounds__(kSThreads) k_slot_sums(const uint32_t* __restr
   }
 }
 
+// Ranges and columns of every part's result, a block a part (its last rows of
+// the identity are no part of it).
+__global__ void __launch_bounds__(kSThreads) k_part_totals(const Parts q, const uint32_t* __restrict__ cnt,
+                                                           const unsigned long long* __restrict__ nnz, uint32_t n,
+                                                           unsigned long long* __restrict__ totals) {
+  __shared__ unsigned long long sum[2][kSWarps];
+  const SlotPart part = q.table[blockIdx.x];
+  const uint64_t end = min((uint64_t(part.row0) + part.n + kCrsRows - 1) / kCrsRows * kCrsRows, uint64_t(n));
+  unsigned long long s = 0, z = 0;
+  for (uint64_t g = part.row0 / kCountRows + threadIdx.x; g < (end + kCountRows - 1) / kCountRows; g += kSThreads) {
+    s += cnt[g];
+    z += nnz[g];
+  }
+  s = group_sum<32>(kFullMask, s);
+  z = group_sum<32>(kFullMask, z);
+  if (lane_id() == 0) {
+    sum[0][threadIdx.x >> 5] = s;
+    sum[1][threadIdx.x >> 5] = z;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kSWarps; ++w) {
+      s += sum[0][w];
+      z += sum[1][w];
+    }
+    const uint64_t pad = end - part.row0 - part.n;
+    totals[2 * blockIdx.x] = s - pad;
+    totals[2 * blockIdx.x + 1] = z - pad;
+  }
+}
+
 // Slots -> range CRS.  A block takes kCrsRows rows; the ranges before them are
 // the sums of the super groups before its own and the counts of the groups
-// before it in that one, so no block waits for another.  A warp takes 32
-// consecutive rows at a time.
-__global__ void __launch_bounds__(kSThreads) k_slots_to_crs(const uint2* __restrict__ slots,
+// before it in that one, less those before its part, so no block waits for
+// another.  A warp takes 32 consecutive rows at a time.
+__global__ void __launch_bounds__(kSThreads) k_slots_to_crs(const __grid_constant__ Parts q,
+                                                            const uint2* __restrict__ slots,
                                                             const uint2* __restrict__ arena,
                                                             const unsigned long long* __restrict__ sums,
-                                                            const uint32_t* __restrict__ group_cnt, uint32_t n,
-                                                            uint64_t* __restrict__ rowmap,
-                                                            uint32_t* __restrict__ entries, uint64_t cap,
+                                                            const uint32_t* __restrict__ group_cnt,
                                                             DeviceControl* ctl) {
   constexpr int kIter = kCrsRows / kSThreads;
   __shared__ unsigned long long pre[kSWarps];
   __shared__ uint32_t wsum[kSWarps];
+  const SlotPart part = my_part(q);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t tile = blockIdx.x, g0 = tile * (kCrsRows / kCountRows), sup = g0 / kSuperGroups;
   unsigned long long before = 0;
@@ -828,7 +886,7 @@ __global__ void __launch_bounds__(kSThreads) k_slots_to_crs(const uint2* __restr
 #pragma unroll
   for (int u = 0; u < kIter; ++u) {
     const uint64_t r = w0 + u * 32 + lane;
-    v[u] = r < n ? ld_slot(slots, r) : empty_slot();
+    v[u] = r - part.row0 < part.n ? ld_slot(slots, r) : empty_slot();
   }
   uint32_t sum = 0;
 #pragma unroll
@@ -843,27 +901,30 @@ __global__ void __launch_bounds__(kSThreads) k_slots_to_crs(const uint2* __restr
     wsum[warp] = sum;
   }
   __syncthreads();
-  unsigned long long at = 0;
+  unsigned long long at = 0ull - part.before;
 #pragma unroll
   for (int w = 0; w < kSWarps; ++w) {
     at += pre[w];
     if (w < warp) at += wsum[w];
   }
-  uint2* const out = reinterpret_cast<uint2*>(entries);
+  uint2* const out = reinterpret_cast<uint2*>(part.c_entries);
 #pragma unroll
   for (int u = 0; u < kIter; ++u) {
-    const uint64_t r = w0 + u * 32 + lane;
+    const uint64_t i = w0 + u * 32 + lane - part.row0;
     const uint32_t tot = __shfl_sync(kFullMask, c[u], 31);
-    if (r < n) {
-      rowmap[r + 1] = 2 * (at + c[u]);
-      if (r == 0) rowmap[0] = 0;
-      if (2 * (at + c[u]) > cap) {
+    if (i < part.n) {
+      part.c_rowmap[i + 1] = 2 * (at + c[u]);
+      if (i == 0) part.c_rowmap[0] = 0;
+      if (at + c[u] > part.c_ranges) {
         atomicOr(&ctl->status, 256ull);
-      } else if (is_run(v[u])) {
-        out[at + c[u] - 1] = v[u];
       } else {
         const uint32_t k = slot_count(v[u]);
-        for (uint32_t q = 0; q < k; ++q) out[at + c[u] - k + q] = slot_range(arena, v[u], q);
+        for (uint32_t t = 0; t < k; ++t) {
+          uint2 w = slot_range(arena, v[u], t);
+          w.x -= part.row0;
+          w.y -= part.row0;
+          out[at + c[u] - k + t] = w;
+        }
       }
     }
     at += tot;
@@ -1043,22 +1104,18 @@ bool slots_suit(const dvg_context* ctx, const dvg_matrix* a) {
          2 * ranges <= 3ull * a->nrows && a->nnz <= 2 * ranges && ctx->opt_slots != 0;
 }
 
-// Columns of a row beyond its first, on average: how fast rows leave the single column.
-static double branching(const dvg_matrix* a) {
-  return a->nnz > a->nrows ? double(a->nnz - a->nrows) / double(a->nrows) : 0.0;
-}
+static unsigned conversion_blocks(const SlotBuild& sb) { return unsigned((uint64_t(sb.n) + kCrsRows - 1) / kCrsRows); }
 
 SlotBuild prepare_slots(dvg_context* ctx, const SlotPlan& plan, uint32_t n) {
   SlotBuild sb;
   sb.plan = plan;
   sb.n = n;
   sb.mat.assign(plan.nmats, nullptr);
-  sb.live.assign(plan.nmats, 0);
   const uint64_t groups = (uint64_t(n) + kCountRows - 1) / kCountRows;
   const uint64_t supers = (groups + kSuperGroups - 1) / kSuperGroups;
   const size_t sums_off = 512, nnz_off = sums_off + supers * 8, cnt_off = nnz_off + groups * 8;
   const size_t masks_off = cnt_off + groups * 4;
-  static_assert(sizeof(DeviceControl) <= 256, "the counters come first");
+  static_assert(sizeof(SlotCounters) <= 512, "the counters come first");
   std::vector<int> last(plan.nmats, -1);
   auto reads = [&](const SlotStep& s, auto&& f) {
     for (int j = 0; j < s.k; ++j) f(s.m[j]);
@@ -1069,9 +1126,16 @@ SlotBuild prepare_slots(dvg_context* ctx, const SlotPlan& plan, uint32_t n) {
   sb.arena_cap = std::min<uint64_t>(uint64_t(ctx->slot_growth * double(n)) + 4096, kMulti);
   const double room = 0.5 * double(device_free_bytes(ctx) + ctx->cached_bytes);
   if (double(sb.arena_cap) * 8.0 > room) sb.arena_cap = uint64_t(room / 8.0) + 4096;
+  // a matrix takes the buffer of one whose last reader is an earlier pass (the
+  // chain's own buffers only: chains that run side by side share none)
+  std::vector<uint2*> spare;
   auto take = [&](int k) {
-    sb.mat[k] = static_cast<uint2*>(dalloc(ctx, size_t(n) * sizeof(uint2)));
-    sb.live[k] = 1;
+    if (spare.empty()) {
+      sb.buffers.push_back(static_cast<uint2*>(dalloc(ctx, size_t(n) * sizeof(uint2))));
+      spare.push_back(sb.buffers.back());
+    }
+    sb.mat[k] = spare.back();
+    spare.pop_back();
   };
   try {
     sb.scratch = dalloc(ctx, masks_off + (uint64_t(n) + 31) / 32 * 4);
@@ -1088,14 +1152,11 @@ SlotBuild prepare_slots(dvg_context* ctx, const SlotPlan& plan, uint32_t n) {
     for (size_t i = 0; i < plan.steps.size(); ++i) {
       if (plan.steps[i].s >= 0) take(plan.steps[i].s);
       if (plan.steps[i].c >= 0) take(plan.steps[i].c);
-      // a matrix whose last reader is this step goes back now: stream order
-      // makes the reuse of its block by later steps safe
+      std::vector<int> done;
       reads(plan.steps[i], [&](int k) {
-        if (last[k] == int(i) && k != plan.out && sb.live[k]) {
-          dfree(ctx, sb.mat[k]);
-          sb.live[k] = 0;
-        }
+        if (last[k] == int(i) && k != plan.out && std::find(done.begin(), done.end(), k) == done.end()) done.push_back(k);
       });
+      for (int k : done) spare.push_back(sb.mat[k]);
     }
   } catch (...) {
     release_slots(ctx, sb);
@@ -1105,17 +1166,15 @@ SlotBuild prepare_slots(dvg_context* ctx, const SlotPlan& plan, uint32_t n) {
 }
 
 void release_slots(dvg_context* ctx, SlotBuild& sb) {
-  for (size_t k = 0; k < sb.mat.size(); ++k) {
-    if (sb.live[k]) dfree(ctx, sb.mat[k]);
-    sb.live[k] = 0;
-  }
+  for (uint2* b : sb.buffers) dfree(ctx, b);
+  sb.buffers.clear();
   if (sb.arena) dfree(ctx, sb.arena);
   sb.arena = nullptr;
   if (sb.scratch) dfree(ctx, sb.scratch);
   sb.scratch = nullptr;
 }
 
-void launch_slots(dvg_context* ctx, SlotBuild& sb, const uint64_t* rowmap, const uint32_t* entries) {
+void launch_slots(dvg_context* ctx, SlotBuild& sb, const SlotParts& parts, bool timed) {
   const uint64_t t0 = now_ns();
   DVG_CUDA(cudaMemsetAsync(sb.scratch, 0, 512, ctx->stream));
   ctx->stats.kernel_launches++;
@@ -1130,9 +1189,7 @@ void launch_slots(dvg_context* ctx, SlotBuild& sb, const uint64_t* rowmap, const
   p.group_nnz = sb.group_nnz;
   p.n = sb.n;
   p.s = sb.mat[0];
-  const unsigned blocks =
-      unsigned(std::min<uint64_t>((uint64_t(sb.n) + kSThreads - 1) / kSThreads, 16ull * ctx->num_sms));
-  k_crs_to_slots<<<blocks, kSThreads, 0, ctx->stream>>>(rowmap, entries, p);
+  k_crs_to_slots<<<conversion_blocks(sb), kSThreads, 0, ctx->stream>>>(Parts{parts.table, parts.part_of, parts.one}, p);
   DVG_CUDA(cudaGetLastError());
   ctx->stats.kernel_launches++;
   for (size_t i = 0; i < sb.plan.steps.size(); ++i) {
@@ -1143,7 +1200,7 @@ void launch_slots(dvg_context* ctx, SlotBuild& sb, const uint64_t* rowmap, const
     p.b = st.b >= 0 ? sb.mat[st.b] : nullptr;
     p.s = st.s >= 0 ? sb.mat[st.s] : nullptr;
     p.c = st.c >= 0 ? sb.mat[st.c] : nullptr;
-    cudaEvent_t ev = span_begin(ctx);
+    cudaEvent_t ev = timed ? span_begin(ctx) : nullptr;
     if (i + 1 == sb.plan.steps.size()) launch_pass<false, true, true>(ctx, p);
     else if (p.s && p.c) launch_pass<true, true, false>(ctx, p);
     else if (p.s) launch_pass<true, false, false>(ctx, p);
@@ -1158,59 +1215,86 @@ void launch_slots(dvg_context* ctx, SlotBuild& sb, const uint64_t* rowmap, const
   ctx->stats.host_launch_ns += now_ns() - t0;
 }
 
-dvg_matrix* finish_slots(dvg_context* ctx, SlotBuild& sb) {
-  struct Counters {
-    DeviceControl ctl;
-    char pad[256 - sizeof(DeviceControl)];
-    unsigned long long top, abort;
-  };
-  auto* h = static_cast<Counters*>(host_stage(ctx, sizeof(Counters)));
+void launch_slots_totals(dvg_context* ctx, const SlotBuild& sb, const SlotParts& parts, uint32_t nparts,
+                         unsigned long long* totals) {
+  k_part_totals<<<nparts, kSThreads, 0, ctx->stream>>>(Parts{parts.table, parts.part_of, parts.one}, sb.group_cnt,
+                                                       sb.group_nnz, sb.n, totals);
+  DVG_CUDA(cudaGetLastError());
+  ctx->stats.kernel_launches++;
+}
+
+void launch_slots_out(dvg_context* ctx, const SlotBuild& sb, const SlotParts& parts) {
+  k_slots_to_crs<<<conversion_blocks(sb), kSThreads, 0, ctx->stream>>>(
+      Parts{parts.table, parts.part_of, parts.one}, sb.mat[sb.plan.out], sb.arena, sb.sums, sb.group_cnt, ctx->d_ctl);
+  DVG_CUDA(cudaGetLastError());
+  ctx->stats.kernel_launches++;
+}
+
+bool check_slots(dvg_context* ctx, const SlotBuild& sb, const SlotCounters& c) {
+  if (c.abort) {
+    // more rows of several runs than the arena was sized for: the caller takes
+    // the range-CRS path, later chains a larger arena
+    ctx->slot_growth = std::min(2.0 * ctx->slot_growth, 8.0);
+    return false;
+  }
+  // statistics: what every pass had to move, 8 bytes a row for each matrix it
+  // reads or writes, and the products that it stands for
+  uint64_t bytes = 0, products = 0, adds = 0;
+  for (const SlotStep& st : sb.plan.steps) {
+    std::vector<int> seen;
+    auto once = [&](int k) {
+      if (k < 0 || std::find(seen.begin(), seen.end(), k) != seen.end()) return;
+      seen.push_back(k);
+      bytes += 8ull * sb.n;
+    };
+    for (int j = 0; j < st.k; ++j) once(st.m[j]);
+    for (int k : {st.b, st.s, st.c}) once(k);
+    const int gathers = __builtin_popcount(st.bits >> 1);
+    products += st.s >= 0 ? std::max(st.k - 1, 0) : 0;
+    if (st.c >= 0) products += st.b >= 0 ? gathers + (st.s >= 0 ? 0 : st.k - 1) : (st.s >= 0 ? 0 : st.k);
+    adds += st.c >= 0 && (st.bits & (st.bits - 1)) ? __builtin_popcount(st.bits) - 1 : 0;
+  }
+  ctx->stats.alg_bytes += bytes;
+  ctx->stats.spgemm_alg_bytes += bytes;
+  ctx->stats.spgemm_calls += products;
+  ctx->stats.spgemm_light += products;
+  ctx->stats.spgemm_fused_adds += adds;
+  ctx->stats.spgemm_slow_rows += c.ctl.slow_rows;
+  return true;
+}
+
+dvg_matrix* slots_chain(dvg_context* ctx, const dvg_matrix* a, unsigned dlo, unsigned dup) {
+  SlotBuild sb;
+  try {
+    sb = prepare_slots(ctx, plan_slots(dlo, dup, branching(a->nnz, a->nrows)), a->nrows);
+  } catch (const Error& e) {
+    if (e.status != DVG_ERR_OOM) throw;
+    return nullptr;
+  }
   dvg_matrix* m = nullptr;
   try {
-    DVG_CUDA(cudaMemcpyAsync(h, sb.scratch, sizeof(Counters), cudaMemcpyDeviceToHost, ctx->stream));
+    SlotParts parts{};
+    parts.one.rowmap = a->rowmap;
+    parts.one.entries = a->entries;
+    parts.one.n = a->nrows;
+    launch_slots(ctx, sb, parts, ctx->opt_timing);
+    auto* h = static_cast<SlotCounters*>(host_stage(ctx, sizeof(SlotCounters)));
+    DVG_CUDA(cudaMemcpyAsync(h, sb.scratch, sizeof(SlotCounters), cudaMemcpyDeviceToHost, ctx->stream));
     const uint64_t t0 = now_ns();
     DVG_CUDA(cudaStreamSynchronize(ctx->stream));
     ctx->stats.host_sync_ns += now_ns() - t0;
     ctx->stats.host_syncs++;
     resolve_spans(ctx);
-    if (h->abort) {
-      // more rows of several runs than the arena was sized for: the caller
-      // takes the range-CRS path, later chains a larger arena
-      ctx->slot_growth = std::min(2.0 * ctx->slot_growth, 64.0);
-      release_slots(ctx, sb);
-      return nullptr;
+    const SlotCounters c = *h;
+    if (check_slots(ctx, sb, c)) {
+      m = new_matrix(ctx, a->nrows, a->ncols, c.ctl.total);
+      m->nnz = c.ctl.nnz;
+      m->canonical = true;
+      parts.one.c_rowmap = m->rowmap;
+      parts.one.c_entries = m->entries;
+      parts.one.c_ranges = m->nentries / 2;
+      launch_slots_out(ctx, sb, parts);
     }
-    const Counters c = *h;
-    m = new_matrix(ctx, sb.n, sb.n, c.ctl.total);
-    m->nnz = c.ctl.nnz;
-    m->canonical = true;
-    k_slots_to_crs<<<unsigned((uint64_t(sb.n) + kCrsRows - 1) / kCrsRows), kSThreads, 0, ctx->stream>>>(
-        sb.mat[sb.plan.out], sb.arena, sb.sums, sb.group_cnt, sb.n, m->rowmap, m->entries, m->nentries, ctx->d_ctl);
-    DVG_CUDA(cudaGetLastError());
-    ctx->stats.kernel_launches++;
-    // statistics: what every pass had to move, 8 bytes a row for each matrix it
-    // reads or writes, and the products that it stands for
-    uint64_t bytes = 0, products = 0, adds = 0;
-    for (const SlotStep& st : sb.plan.steps) {
-      std::vector<int> seen;
-      auto once = [&](int k) {
-        if (k < 0 || std::find(seen.begin(), seen.end(), k) != seen.end()) return;
-        seen.push_back(k);
-        bytes += 8ull * sb.n;
-      };
-      for (int j = 0; j < st.k; ++j) once(st.m[j]);
-      for (int k : {st.b, st.s, st.c}) once(k);
-      const int gathers = __builtin_popcount(st.bits >> 1);
-      products += st.s >= 0 ? std::max(st.k - 1, 0) : 0;
-      if (st.c >= 0) products += st.b >= 0 ? gathers + (st.s >= 0 ? 0 : st.k - 1) : (st.s >= 0 ? 0 : st.k);
-      adds += st.c >= 0 && (st.bits & (st.bits - 1)) ? __builtin_popcount(st.bits) - 1 : 0;
-    }
-    ctx->stats.alg_bytes += bytes;
-    ctx->stats.spgemm_alg_bytes += bytes;
-    ctx->stats.spgemm_calls += products;
-    ctx->stats.spgemm_light += products;
-    ctx->stats.spgemm_fused_adds += adds;
-    ctx->stats.spgemm_slow_rows += c.ctl.slow_rows;
   } catch (...) {
     free_matrix(ctx, m);
     release_slots(ctx, sb);
@@ -1218,23 +1302,6 @@ dvg_matrix* finish_slots(dvg_context* ctx, SlotBuild& sb) {
   }
   release_slots(ctx, sb);
   return m;
-}
-
-dvg_matrix* slots_chain(dvg_context* ctx, const dvg_matrix* a, unsigned dlo, unsigned dup) {
-  SlotBuild sb;
-  try {
-    sb = prepare_slots(ctx, plan_slots(dlo, dup, branching(a)), a->nrows);
-  } catch (const Error& e) {
-    if (e.status != DVG_ERR_OOM) throw;
-    return nullptr;
-  }
-  try {
-    launch_slots(ctx, sb, a->rowmap, a->entries);
-  } catch (...) {
-    release_slots(ctx, sb);
-    throw;
-  }
-  return finish_slots(ctx, sb);
 }
 
 }  // namespace dvg

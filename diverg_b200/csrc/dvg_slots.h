@@ -25,20 +25,46 @@ struct SlotPlan {
   int nmats = 1;
   int out = 0;
 };
-// A^dlo (A + I)^(dup - dlo) as passes over powers of A.
-SlotPlan plan_slots(unsigned dlo, unsigned dup);
+// A^dlo (A + I)^(dup - dlo) as passes over powers of A, for an A whose rows have
+// `branching` columns beyond their first on average.
+SlotPlan plan_slots(unsigned dlo, unsigned dup, double branching);
 
 // Whether a chain over `a` runs in the row-slot format.
 bool slots_suit(const dvg_context* ctx, const dvg_matrix* a);
 
+// A chain may run over several matrices at once, side by side on the diagonal
+// (a power of a block-diagonal matrix has the blocks' powers as blocks): each
+// from a multiple of kSlotPartRows rows on, the rows between filled with the
+// identity's.
+constexpr uint32_t kSlotPartRows = 1024;
+struct SlotPart {
+  const uint64_t* rowmap;      // the part, range CRS
+  const uint32_t* entries;
+  uint64_t* c_rowmap;          // its result
+  uint32_t* c_entries;
+  unsigned long long c_ranges; // ranges that c_entries holds
+  unsigned long long before;   // ranges of the chain's result before the part's
+  uint32_t row0, n;            // its first row in the chain, and its rows
+};
+struct SlotParts {
+  const SlotPart* table;       // device; null: one part, `one`
+  const uint32_t* part_of;     // device: part of every kSlotPartRows rows
+  SlotPart one;
+};
+
+struct SlotCounters {          // the head of a chain's scratch
+  DeviceControl ctl;
+  char pad[256 - sizeof(DeviceControl)];
+  unsigned long long top, abort;
+};
 struct SlotBuild {
   SlotPlan plan;
   uint32_t n = 0;
-  std::vector<uint2*> mat;   // per matrix, as the launches use them
-  std::vector<char> live;
+  std::vector<uint2*> mat;     // per matrix, as the launches use them
+  std::vector<uint2*> buffers; // theirs
   uint2* arena = nullptr;
-  uint64_t arena_cap = 0;    // ranges
-  void* scratch = nullptr;   // counters | sums of the counts | counts of the result's ranges
+  uint64_t arena_cap = 0;      // ranges
+  void* scratch = nullptr;     // counters | sums of the counts | counts of the result | bitmap
   DeviceControl* ctl = nullptr;
   unsigned long long* top = nullptr;
   unsigned long long* abort = nullptr;
@@ -49,17 +75,27 @@ struct SlotBuild {
 };
 
 // Allocates what the chain needs (no device work beyond stream-ordered
-// allocation), issues it (no host round trip: it may be captured), and after
-// the stream has been waited for turns the result into range CRS.
+// allocation); issues it (no host round trip: it may be captured).
 SlotBuild prepare_slots(dvg_context* ctx, const SlotPlan& plan, uint32_t n);
-void launch_slots(dvg_context* ctx, SlotBuild& sb, const uint64_t* rowmap, const uint32_t* entries);
-// Reads the counters back (one synchronisation), allocates the result and
-// issues its conversion; null when the arena ran full (all buffers released,
-// the context's estimate raised).
-dvg_matrix* finish_slots(dvg_context* ctx, SlotBuild& sb);
+void launch_slots(dvg_context* ctx, SlotBuild& sb, const SlotParts& parts, bool timed);
+// Ranges and columns of each part's result (device, two words a part), once
+// the chain has run.
+void launch_slots_totals(dvg_context* ctx, const SlotBuild& sb, const SlotParts& parts, uint32_t nparts,
+                         unsigned long long* totals);
+// The parts' results, into the arrays that the table now names.
+void launch_slots_out(dvg_context* ctx, const SlotBuild& sb, const SlotParts& parts);
+// Books a finished chain's counters; false when its arena ran full and there is
+// no result.
+bool check_slots(dvg_context* ctx, const SlotBuild& sb, const SlotCounters& c);
 void release_slots(dvg_context* ctx, SlotBuild& sb);
 
-// prepare, launch and finish; null when the chain did not fit its arena.
+// The chain over `a`, waited for once (for the result's size); null when it did
+// not fit its arena.
 dvg_matrix* slots_chain(dvg_context* ctx, const dvg_matrix* a, unsigned dlo, unsigned dup);
+
+// Columns of a row beyond its first, on average: how fast rows leave the single column.
+inline double branching(uint64_t nnz, uint64_t nrows) {
+  return nnz > nrows ? double(nnz - nrows) / double(nrows) : 0.0;
+}
 
 }  // namespace dvg

@@ -42,7 +42,8 @@ def check(ctx, a, window, slots=True):
         assert np.array_equal(m.entries, want.entries), window
         assert m.nnz() == want.nnz, window
     # the two forms move different bytes
-    assert slots == (st["spgemm_alg_bytes"] != crs_st["spgemm_alg_bytes"])
+    if slots is not None:
+        assert slots == (st["spgemm_alg_bytes"] != crs_st["spgemm_alg_bytes"])
 
 
 def rows(a, n):
@@ -96,9 +97,10 @@ def test_branching_graphs(ctx, spec, window):
 @pytest.mark.parametrize("window", [(2, 5), (0, 4)])
 def test_columns_anywhere_near(ctx, hw, window):
     # about one short range a row at random in the band: rows fill up quickly
+    # (and may fill the arena: the build then falls back)
     a = gen.banded(140_500, hw, 1.2, 1.2, seed=63)
     assert a.entries.size <= 3 * a.numRows() and a.nnz() <= a.entries.size
-    check(ctx, a, window)
+    check(ctx, a, window, slots=None)
 
 
 def test_a_full_arena_falls_back(ctx):
@@ -127,3 +129,23 @@ def test_powers(ctx, n, k):
     got = ctx.power(ctx.upload(a), k).download()
     assert np.array_equal(got.rowmap, want.rowmap) and np.array_equal(got.entries, want.entries)
     assert got.nnz() == want.nnz
+
+
+def test_a_batch_of_chains_beside_range_crs_builds(ctx):
+    # parts of a chain around the edges of its blocks, several windows side by
+    # side, graphs that stay in range CRS, and one whose chain runs full
+    windows = [(100, 300), (0, 50), (3, 3), (1, 1), (0, 1), (200, 500)]
+    graphs = [rows(graph(), n) for n in (1, 50, 1023, 1024, 1025, 2048, 3000, 20_000, 70_001, 1024, 31, 4096)]
+    ws = [windows[k % len(windows)] for k in range(len(graphs))]
+    graphs += [gen.random_matrix(500, 2_500, seed=67), gen.banded(3_000, 3_000, 1.4, 1.0, seed=64),
+               CRSMatrix(0, np.zeros(0, np.uint32), np.zeros(1, np.uint64))]
+    ws += [(1, 3), (12, 12), (1, 3)]
+    for _ in range(2):
+        ctx.reset_stats()
+        got = ctx.batch_distance_index([ctx.upload(g) for g in graphs], ws)
+        assert ctx.stats()["graph_launches"] == 1
+        for k, (g, w) in enumerate(zip(graphs, ws)):
+            want = orc.dindex(omat(g), *w, algo="hbv")
+            m = got[k].download()
+            assert np.array_equal(m.rowmap, want.rowmap) and np.array_equal(m.entries, want.entries), (k, w)
+            assert m.nnz() == want.nnz, (k, w)
