@@ -256,13 +256,15 @@ void batch_distance_index(dvg_context* ctx, uint32_t ngraphs, const dvg_matrix* 
   for (uint32_t k = 0; k < ngraphs; ++k) out[k] = nullptr;
   // ---- validation and grouping -------------------------------------------------
   std::map<std::pair<unsigned, unsigned>, std::vector<uint32_t>> by_window, slots_by_window;
-  std::vector<uint32_t> alone;  // built one by one (non-canonical input with dmin = 0)
+  std::vector<uint32_t> alone;  // built one by one (no rows, or non-canonical input with dmin = 0)
   for (uint32_t k = 0; k < ngraphs; ++k) {
     const dvg_matrix* a = graphs[k];
     require(a != nullptr, "batch: null graph");
     require(a->nrows == a->ncols, "batch: adjacency matrix is not square");
     require(dmin[k] <= dmax[k] && dmax[k] != 0, "batch: requires dmin <= dmax and dmax != 0");
-    if ((dmin[k] == 0 && !a->canonical) || !ctx->opt_planned || ctx->opt_spgemm_mode == 1 ||
+    // (a window whose graphs have no row at all would be split by row pointers that
+    // no product has written)
+    if (a->nrows == 0 || (dmin[k] == 0 && !a->canonical) || !ctx->opt_planned || ctx->opt_spgemm_mode == 1 ||
         ctx->opt_dindex_schedule != 0)
       alone.push_back(k);
     else if (ctx->opt_spgemm_mode == 0 && slots_suit(ctx, a))
