@@ -310,9 +310,28 @@ static dvg_matrix* range_spgemm_fused(dvg_context* ctx, const dvg_matrix* a, boo
       levels = build_levels(ctx, b, nlv);
     }
   }
+  // long A ranges, a warp per row: bitmaps of unions of B's rows
+  struct BandGuard {
+    dvg_context* ctx;
+    BandTables t;
+    ~BandGuard() {
+      if (t.mem) dfree(ctx, t.mem);
+    }
+  } band{ctx, {}};
+  if (!a_identity && !d && ctx->opt_spgemm_mode == 0 && levels.empty() && has_long_ranges(a))
+    band.t = build_band_tables(ctx, a, b);
   // speculative output capacity; an overflow is detected and re-run exactly
   const uint64_t a_ent = a_identity ? 2ull * n : a->nentries;
   uint64_t cap = std::max<uint64_t>({2 * a_ent, 2 * b->nentries, d ? 2 * d->nentries : 0, 4ull * n, 64});
+  // unions of many short ranges hold 3 to 13 times the larger input's entries; a
+  // product run twice costs more than room for what the last one took
+  const bool grows = !a_identity && has_long_ranges(a);
+  const uint64_t larger = std::max<uint64_t>({a_ent, b->nentries, 1});
+  const uint64_t usual = cap;
+  if (grows) {
+    const uint64_t want = uint64_t(ctx->product_growth * double(larger));
+    if (want > cap && want < (device_free_bytes(ctx) + ctx->cached_bytes) / 16) cap = want;
+  }
   dvg_matrix* c = new_matrix(ctx, n, b->ncols, cap);
   try {
     DVG_CUDA(cudaMemsetAsync(c->rowmap, 0, sizeof(uint64_t), ctx->stream));
@@ -320,7 +339,8 @@ static dvg_matrix* range_spgemm_fused(dvg_context* ctx, const dvg_matrix* a, boo
     for (int attempt = 0; attempt < 2; ++attempt) {
       reset_control(ctx);
       cudaEvent_t t0 = span_begin(ctx);
-      launch_spgemm_fused(ctx, a, a_identity, b, d, c->rowmap, c->entries, cap, levels.empty() ? nullptr : &levels);
+      launch_spgemm_fused(ctx, a, a_identity, b, d, c->rowmap, c->entries, cap, levels.empty() ? nullptr : &levels,
+                          band.t.mem ? &band.t : nullptr);
       span_end(ctx, t0, kProduct);
       ctl = read_control(ctx);
       if (ctl.timeout) throw Error(DVG_ERR_TIMEOUT, "range_spgemm: tile look-back wait expired");
@@ -331,6 +351,18 @@ static dvg_matrix* range_spgemm_fused(dvg_context* ctx, const dvg_matrix* a, boo
       dfree(ctx, c->entries);
       c->entries = nullptr;
       c->entries = static_cast<uint32_t*>(dalloc(ctx, entries_alloc_bytes(cap)));
+    }
+    if (grows) ctx->product_growth = std::min(std::max(2.0, 1.25 * double(ctl.total) / double(larger)), 16.0);
+    if (cap > usual && cap / 2 > ctl.total) {  // (the room was for another product's result)
+      auto* exact = static_cast<uint32_t*>(dalloc(ctx, entries_alloc_bytes(ctl.total)));
+      if (ctl.total) {
+        const cudaError_t e = cudaMemcpyAsync(exact, c->entries, ctl.total * sizeof(uint32_t), cudaMemcpyDeviceToDevice,
+                                              ctx->stream);
+        if (e != cudaSuccess) dfree(ctx, exact);
+        DVG_CUDA(e);
+      }
+      dfree(ctx, c->entries);
+      c->entries = exact;
     }
     c->nentries = ctl.total;
     c->nnz = ctl.nnz;

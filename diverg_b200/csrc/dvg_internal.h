@@ -81,6 +81,7 @@ struct dvg_context {
   double plan_growth = 3.0;           // planned builds: entry capacity per step / input entries
   int64_t opt_slots = 1;              // chains of products over graph-like input run in the row-slot format
   double slot_growth = 4.0;           // row-slot chains: ranges the arena holds / rows
+  double product_growth = 2.0;        // products with long A ranges: entry capacity / the larger input's entries
   uint64_t max_product_entries = 0;   // largest product output since the last reset (read-back path)
   int64_t opt_autotune = 1;           // batches: tune the row kernel per (window, size class)
   std::map<std::tuple<unsigned, unsigned, int>, TuneChoice> tuned;
@@ -173,6 +174,26 @@ void launch_spadd_single_pass(dvg_context* ctx, const dvg_matrix* a, const dvg_m
 void launch_query(dvg_context* ctx, const dvg_matrix* idx, const uint32_t* d_pairs, uint64_t npairs, uint8_t* d_out,
                   DeviceControl* ctl = nullptr);
 
+// Bitmaps of unions of B's rows for the warp-per-row SpGEMM: table k holds the unions
+// of 1, 4, 8, 16, 32 and 64 rows (k = 0 .. 5) from every row on.  The rows of block
+// b = j / kBandBlock lie from 16-byte word k * table + b * kBandBlock * stride / 4 of t
+// on, y words each for (x, y) = blk[b], of 32 columns each from word x of B's columns
+// on; x, y and the stride, the largest y, are multiples of four.
+constexpr int kBandLevels = 6;
+constexpr uint32_t kBandBlock = 64;
+struct BandTables {
+  const uint4* t;
+  const uint2* blk;
+  uint64_t table;
+  uint32_t stride;
+  void* mem;
+};
+// Whether the automatic choice takes a warp per row for products from the left by a.
+bool has_long_ranges(const dvg_matrix* a);
+// Builds them where they pay for the product a b (one read-back for B's widest
+// band); mem is null where they do not.
+BandTables build_band_tables(dvg_context* ctx, const dvg_matrix* a, const dvg_matrix* b);
+
 // Fused single-pass SpGEMM (dvg_spgemm_fused.cu): writes c_rowmap fully and
 // c_entries up to `cap` entries; the control block receives the total entry
 // count, the nnz and an overflow flag when total > cap.
@@ -180,14 +201,15 @@ void launch_query(dvg_context* ctx, const dvg_matrix* idx, const uint32_t* d_pai
 // `levels` (row kernel only): union levels of b, level k + 1 at index k.
 void launch_spgemm_fused(dvg_context* ctx, const dvg_matrix* a, bool a_identity, const dvg_matrix* b,
                          const dvg_matrix* d, uint64_t* c_rowmap, uint32_t* c_entries, uint64_t cap,
-                         const std::vector<dvg_matrix*>* levels = nullptr);
+                         const std::vector<dvg_matrix*>* levels = nullptr, const BandTables* band = nullptr);
 // C = U + S U with S the identity shifted by `shift` rows (row j of C is the
 // union of U's rows j and j + shift): one union level from the previous one.
 // The warp-per-row SpGEMM for rows that name many B ranges (dvg_spgemm_wide.cu):
 // desc holds spgemm_wide_desc_bytes(a->nrows) zeroed bytes, ticket a zeroed word.
 size_t spgemm_wide_desc_bytes(uint32_t nrows);
 void launch_spgemm_wide(dvg_context* ctx, const dvg_matrix* a, const dvg_matrix* b, const dvg_matrix* d,
-                        uint64_t* c_rowmap, uint32_t* c_entries, uint64_t cap, void* desc, unsigned* ticket);
+                        uint64_t* c_rowmap, uint32_t* c_entries, uint64_t cap, void* desc, unsigned* ticket,
+                        const BandTables* band);
 // Range operations a second the warp-per-row kernel's inner work sustains on
 // this device (measured; synchronises the context's stream).
 double calibrate_range_ops(dvg_context* ctx);

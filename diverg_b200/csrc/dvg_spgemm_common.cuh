@@ -77,6 +77,8 @@ struct FusedArgs {
   uint32_t stage_cap;
   // polls a look-back waits before it gives up (0: kSpinLimit)
   uint32_t spin_limit;
+  // warp-per-row kernel: bitmaps of unions of B rows (null: none), see BandTables
+  BandTables band;
 };
 
 // Row `row` of the (shifted) identity: column row + a_shift, or an empty

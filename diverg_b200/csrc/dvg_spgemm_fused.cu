@@ -583,8 +583,11 @@ __global__ void __launch_bounds__(kThreads, 2) k_spgemm_fused(FusedArgs p) {
 
 }  // namespace
 
-// Mean A range length above which the automatic mode stages tiles.
+// Mean A range length above which the automatic mode takes a warp per row.
 constexpr double kWideRangeMean = 8.0;
+bool has_long_ranges(const dvg_matrix* a) {
+  return a->nentries > 0 && double(a->nnz) > kWideRangeMean * double(a->nentries / 2);
+}
 
 // Scratch for one single-pass product on the context: the chunk descriptors
 // (zeroed) and the ticket (zeroed).
@@ -646,19 +649,18 @@ void launch_row_shifted_sum(dvg_context* ctx, const dvg_matrix* u, uint32_t shif
 
 void launch_spgemm_fused(dvg_context* ctx, const dvg_matrix* a, bool a_identity, const dvg_matrix* b,
                          const dvg_matrix* d, uint64_t* c_rowmap, uint32_t* c_entries, uint64_t cap,
-                         const std::vector<dvg_matrix*>* levels) {
+                         const std::vector<dvg_matrix*>* levels, const BandTables* band) {
   const uint32_t n = a_identity ? b->nrows : a->nrows;
   if (n == 0) return;
   // mode 1 forces the tile-staged kernel, mode 2 the row kernel, mode 3 the
   // warp-per-row kernel; automatic (0) takes the warp-per-row kernel when A's
   // ranges are long on average (a row then names many B ranges) and the row
   // kernel otherwise.  An addend needs the row or the warp-per-row kernel.
-  const bool long_ranges = !a_identity && !(levels && !levels->empty()) && a->nentries > 0 &&
-                           double(a->nnz) > kWideRangeMean * double(a->nentries / 2);
+  const bool long_ranges = !a_identity && !(levels && !levels->empty()) && has_long_ranges(a);
   if ((ctx->opt_spgemm_mode == 3 || (ctx->opt_spgemm_mode == 0 && long_ranges)) && !a_identity &&
       !(levels && !levels->empty())) {
     void* desc = chunk_scratch(ctx, spgemm_wide_desc_bytes(n));
-    launch_spgemm_wide(ctx, a, b, d, c_rowmap, c_entries, cap, desc, ctx->d_ticket);
+    launch_spgemm_wide(ctx, a, b, d, c_rowmap, c_entries, cap, desc, ctx->d_ticket, band);
     return;
   }
   bool row_mode = ctx->opt_spgemm_mode != 1;

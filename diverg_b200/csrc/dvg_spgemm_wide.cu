@@ -43,6 +43,11 @@ namespace {
 constexpr int kWThreads = DVG_WIDE_THREADS;
 constexpr int kWWarps = kWThreads / 32;
 constexpr int kWRows = DVG_WIDE_ROWS;  // rows of a chunk
+// With the tables a chunk is 64 rows: 128 are 3 % faster where a row holds few runs
+// (1.06 against 1.09 ms on 2^20 rows of 9 entries), but a chunk of more than 2,048
+// entries misses its image and waits for its place (16 entries a row: 4.3 ms
+// against 1.3; 22 a row: 1.9 against 1.1).
+constexpr uint32_t kWBandRows = 64, kWRowsMin = 64;
 constexpr int kWRowsLane = kWRows / 32;  // rows of the chunk prefix a lane sums
 static_assert(kWRows % 32 == 0 && kWRowsLane >= 1, "chunk rows are a multiple of 32");
 constexpr int kWWin = 128;     // window words of a warp (4,096 columns)
@@ -50,8 +55,8 @@ constexpr int kWBuf = 256;     // run entries of a warp's rows kept from the cou
 constexpr int kWImage = 2048;  // output entries of a chunk held for its deferred write-out
 
 struct WideSmem {
-  uint32_t bits[kWWarps][kWWin];
-  uint32_t reach[kWWarps][kWWin];
+  // a warp's windows: one row's bits and reach, or four rows' bits
+  uint32_t win[kWWarps][4 * kWWin];
   uint32_t buf[kWWarps][kWBuf];  // runs of the warp's rows of the counted chunk, in row order
   uint32_t img[2][kWImage];      // images of the counted and the pending chunk
   uint32_t incl[2][kWRows];      // their chunk-local inclusive row counts
@@ -120,27 +125,253 @@ __device__ void wide_lookback(unsigned long long* out, const FusedArgs& p, uint3
   }
 }
 
-__global__ void __launch_bounds__(kWThreads, DVG_WIDE_MINB) k_spgemm_wide(FusedArgs p) {
+// Four consecutive rows of C = A B, from `row` on (`rows` of them), from the tables
+// of unions of B rows, eight lanes a row: an A range [s, f] is the rows' union in
+// steps of the largest table that fits (the last step ends at f and may overlap
+// the one before).  A step ORs a table's row into the row's window in shared
+// memory, 16 bytes a lane: window quad q belongs to lane q % 8, so that no two
+// lanes meet on one, and a step is ORed in once the next one's loads are under
+// way.  Runs out: keep(place, value) for entry `place` of the four rows' runs
+// together; cnt[g] takes row g's entries, or kByRange where the row has more A
+// ranges than kBandRanges or is wider than the window and has to be walked range
+// by range.
+//
+// Bound: instructions, about 460 a row where an A range takes two steps instead
+// of the 1,300 of ORing each of its ~100 B ranges with two shared atomics.  On the
+// banded product of 4.2e6 rows (half-width 512, four ranges of ~32 columns a row)
+// 6.54 -> 4.00 ms, 1.0 of it the tables; 3.2e6 rows whose products hold 16 entries
+// a row, 37.1 -> 3.7 ms.  A warp a row, its window in registers,
+// took 930 (a word a lane) and 720 instructions a row (16 bytes a lane): a step
+// covers ten 16-byte words, so most lanes were idle.
+constexpr uint32_t kBandMaxWords = 64;  // of a table's row: two quads for each of a row's eight lanes
+constexpr uint32_t kByRange = 0xffffffffu;
+// The table that a range of `len` rows steps in, and the rows of a step.
+__device__ __forceinline__ uint32_t band_level(uint32_t len) {
+  return len >= 4 ? min(30u - uint32_t(__clz(len)), uint32_t(kBandLevels) - 1) : 0u;  // 4: 1, 8: 2, .. 64: 5
+}
+__device__ __forceinline__ uint32_t band_by(uint32_t level) { return level ? 2u << level : 1u; }
+constexpr uint32_t kBandRanges = 64;
+template <class Keep>
+__device__ __forceinline__ void band_rows(const FusedArgs& p, uint64_t row, uint32_t rows, uint4* window, uint32_t* cnt,
+                                          unsigned long long& nnz, Keep&& keep) {
+  static_assert(kWWin == 128, "sixteen window words a lane");
+  const int lane = lane_id(), g = lane >> 3, l = lane & 7;
+  uint4* const win = window + g * (kWWin / 4);
+  uint64_t a0 = 0, a1 = 0;
+  if (uint32_t(g) < rows) {
+    a0 = __ldg(p.a_rowmap + row + g) >> 1;
+    a1 = __ldg(p.a_rowmap + row + g + 1) >> 1;
+  }
+  // a step: where its table's row starts, and its box (the quads that it covers)
+  const uint32_t quads = p.band.stride / 4;
+  auto place = [&](uint32_t level, uint32_t j, uint2 box) {
+    return level * uint32_t(p.band.table) + j / kBandBlock * (kBandBlock * quads) + j % kBandBlock * (box.y / 4);
+  };
+  // a range's first and last step, and whether it has more between them
+  struct Range {
+    uint32_t q[2];
+    uint2 box[2];
+    uint32_t steps;  // 0: no range
+    bool more;
+  };
+  auto range = [&](uint64_t k) {
+    Range r{{0, 0}, {make_uint2(0u, 0u), make_uint2(0u, 0u)}, 0, false};
+    if (k >= a1) return r;
+    const uint2 ar = load_range(p.a_entries, k);
+    if (ar.y < ar.x) return r;
+    const uint32_t level = band_level(ar.y - ar.x + 1), last = ar.y + 1 - band_by(level);
+    r.box[0] = __ldg(p.band.blk + ar.x / kBandBlock);
+    r.box[1] = __ldg(p.band.blk + last / kBandBlock);
+    r.q[0] = place(level, ar.x, r.box[0]);
+    r.q[1] = place(level, last, r.box[1]);
+    r.steps = last == ar.x ? 1u : 2u;
+    r.more = last - ar.x > band_by(level);
+    return r;
+  };
+  uint32_t lo = 0xffffffffu, hi = 0;
+  auto cover = [&](uint2 w) {
+    if (w.y) {
+      lo = min(lo, w.x);
+      hi = max(hi, w.x + w.y);
+    }
+  };
+  const Range mine = range(a0 + l);
+  const bool many = a1 - a0 > kBandRanges;
+  bool more = false;  // some range of the row has steps between its first and last
+  for (uint64_t k = a0 + l; k < a1 && !many; k += 8) {
+    const Range w = k == a0 + l ? mine : range(k);
+    if (!w.steps) continue;
+    cover(w.box[0]);
+    cover(w.box[1]);
+    more |= w.more;
+    if (w.more) {
+      const uint2 ar = load_range(p.a_entries, k);
+      for (uint32_t b = ar.x / kBandBlock + 1; b < ar.y / kBandBlock; ++b) cover(__ldg(p.band.blk + b));
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) {
+    lo = min(lo, __shfl_xor_sync(kFullMask, lo, o));
+    hi = max(hi, __shfl_xor_sync(kFullMask, hi, o));
+  }
+  // the window's last word stays empty, which ends the last run
+  const bool walk = many || (lo < hi && hi - lo > uint32_t(kWWin) - 4);
+#pragma unroll
+  for (int i = 0; i < kWWin / 32; ++i) win[i * 8 + l] = make_uint4(0u, 0u, 0u, 0u);
+  uint4 v0 = make_uint4(0u, 0u, 0u, 0u), v1 = v0;
+  uint32_t to0 = l, to1 = l;  // where they go (quads of the lane's)
+  auto flush = [&](uint32_t to, uint4 v) {
+    uint4 x = win[to];
+    x.x |= v.x;
+    x.y |= v.y;
+    x.z |= v.z;
+    x.w |= v.w;
+    win[to] = x;
+  };
+  // (at, n): the step's first quad in the window, and how many
+  auto step = [&](uint32_t q, uint32_t at, uint32_t n) {
+    const uint32_t k = (l - at) & 7u;
+    const uint4* __restrict__ t = p.band.t + (q + k);
+    uint4 n0 = make_uint4(0u, 0u, 0u, 0u), n1 = n0;
+    if (k < n) n0 = __ldg(t);
+    if (k + 8 < n) n1 = __ldg(t + 8);
+    flush(to0, v0);
+    flush(to1, v1);
+    v0 = n0;
+    v1 = n1;
+    if (k < n) to0 = at + k;
+    if (k + 8 < n) to1 = at + k + 8;
+  };
+  auto boxed = [&](uint2 b) { return b.y ? (b.x - lo) / 4 << 16 | b.y / 4 : 0u; };
+  // every range's first and last step, range k's from lane k % 8 of its row (the
+  // trip counts are the warp's, so that its lanes stay together)
+  const uint32_t count = walk ? 0u : uint32_t(a1 - a0);
+  const uint32_t most = __reduce_max_sync(kFullMask, count);
+  Range r = mine;
+  uint32_t box0 = boxed(r.box[0]), box1 = boxed(r.box[1]);
+  for (uint32_t k = 0; k < most; ++k) {
+    const int src = (lane & 24) + (k & 7);
+    if (k >= 8 && (k & 7) == 0) {  // (rows of more than eight ranges)
+      r = range(a0 + k + l);
+      box0 = boxed(r.box[0]);
+      box1 = boxed(r.box[1]);
+    }
+    const uint32_t steps = __shfl_sync(kFullMask, r.steps, src);
+    const uint32_t q0 = __shfl_sync(kFullMask, r.q[0], src), q1 = __shfl_sync(kFullMask, r.q[1], src);
+    const uint32_t w0 = __shfl_sync(kFullMask, box0, src), w1 = __shfl_sync(kFullMask, box1, src);
+    if (k < count) {
+      step(q0, w0 >> 16, steps ? w0 & 0xffffu : 0u);
+      if (steps > 1) step(q1, w1 >> 16, w1 & 0xffffu);
+    }
+    __syncwarp();
+  }
+  // the steps between, of ranges of 128 rows and more
+  if (__any_sync(kFullMask, more && !walk)) {
+    for (uint32_t k = 0; k < most; ++k) {
+      if (k >= count) continue;
+      const uint2 ar = load_range(p.a_entries, a0 + k);
+      if (ar.y < ar.x) continue;
+      const uint32_t level = band_level(ar.y - ar.x + 1), by = band_by(level);
+      for (uint32_t j = ar.x + by; j < ar.y + 1 - by; j += by) {
+        const uint2 b = __ldg(p.band.blk + j / kBandBlock);
+        const uint32_t w = boxed(b);
+        step(place(level, j, b), w >> 16, w & 0xffffu);
+      }
+    }
+    __syncwarp();
+  }
+  flush(to0, v0);
+  flush(to1, v1);
+  __syncwarp();
+  // runs: the lane takes words 16 l .. 16 l + 15; where a column differs from the one
+  // before, a run starts or has ended
+  uint32_t n = 0, some = 0;
+  const uint32_t* const words = reinterpret_cast<const uint32_t*>(win);
+  if (!walk && lo < hi && 16 * l <= int(hi - lo)) {
+    uint32_t prev = l ? words[16 * l - 1] : 0u;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint4 x = win[4 * l + i];
+      const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint32_t b = w[k] ^ __funnelshift_l(prev, w[k], 1);
+        n += __popc(b);
+        some |= (b ? 1u : 0u) << (4 * i + k);
+        nnz += __popc(w[k]);
+        prev = w[k];
+      }
+    }
+  }
+  __syncwarp();
+  uint32_t incl = group_incl_sum<32>(kFullMask, n, lane);
+  const uint32_t before = incl - n;
+  const uint32_t ends = __shfl_sync(kFullMask, incl, lane | 7);
+  uint32_t start = __shfl_sync(kFullMask, incl, ((lane & 24) - 1) & 31);
+  if (g == 0) start = 0;
+  if (l == 0 && uint32_t(g) < rows) cnt[g] = walk ? kByRange : ends - start;
+  uint32_t k = before;
+  for (; some; some &= some - 1) {
+    const int i = __ffs(some) - 1;
+    const uint32_t w = words[16 * l + i], prev = 16 * l + i ? words[16 * l + i - 1] : 0u;
+    const uint32_t col = 32u * (lo + 16u * l + i);
+    for (uint32_t d = w ^ __funnelshift_l(prev, w, 1); d; d &= d - 1, ++k)
+      keep(k, col + uint32_t(__ffs(d) - 1) - ((k - start) & 1u));
+  }
+  __syncwarp();
+}
+
+template <bool BAND>
+__global__ void __launch_bounds__(kWThreads, DVG_WIDE_MINB) k_spgemm_wide(const __grid_constant__ FusedArgs p) {
   extern __shared__ __align__(16) unsigned char wide_smem_raw[];
   WideSmem& S = *reinterpret_cast<WideSmem*>(wide_smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  uint32_t* const bits = S.bits[warp];
-  uint32_t* const reach = S.reach[warp];
+  uint32_t* const bits = S.win[warp];
+  uint32_t* const reach = bits + kWWin;
   uint32_t* const buf = S.buf[warp];
   unsigned long long nnz_acc = 0;
+  // the warp's rows of a chunk, in the order in which its buffer keeps them
+  constexpr uint32_t kRun = BAND ? 4 : 1;  // consecutive ones
+  auto each_row = [&](uint32_t crows, auto&& f) {
+    for (uint32_t r0 = warp * kRun; r0 < crows; r0 += kWWarps * kRun)
+      for (uint32_t r = r0; r < min(r0 + kRun, crows); ++r) f(r);
+  };
   if (tid == 0) S.next = atomicAdd(p.ticket, 1u);
   wide_sync();
   uint32_t t = S.next, b = 0;
   bool pend = false;  // a counted chunk waits in image buffer b ^ 1
   while (t < p.nchunks || pend) {
     const bool have = t < p.nchunks;
-    const uint32_t c0 = have ? t * uint32_t(kWRows) : 0u;
-    const uint32_t crows = have ? min(uint32_t(kWRows), p.nrows - c0) : 0u;
+    const uint32_t c0 = have ? t * p.chunk_rows : 0u;
+    const uint32_t crows = have ? min(p.chunk_rows, p.nrows - c0) : 0u;
     uint32_t cnt = 0;
     bool imaged = false;
     if (have) {
       // 1. count: warp w walks rows w, w + kWWarps, ...; their runs go to its buffer
       uint32_t bpos = 0;
+      if constexpr (BAND) {
+        uint4* const window = reinterpret_cast<uint4*>(S.win[warp]);
+        for (uint32_t r = warp * kRun; r < crows; r += kWWarps * kRun) {
+          const uint32_t start = bpos, rows = min(kRun, crows - r);
+          band_rows(p, uint64_t(c0) + r, rows, window, S.cnt_row + r, nnz_acc, [&](uint32_t k, uint32_t v) {
+            if (start + k < uint32_t(kWBuf)) buf[start + k] = v;
+          });
+          __syncwarp();
+          const uint32_t c = uint32_t(lane) < rows ? S.cnt_row[r + lane] : 0u;
+          const unsigned walk = __ballot_sync(kFullMask, c == kByRange);
+          const uint32_t upto = bpos + group_incl_sum<32>(kFullMask, c == kByRange ? 0u : c, lane);
+          if (uint32_t(lane) < rows) S.kept[r + lane] = c != kByRange && upto <= uint32_t(kWBuf) ? 1u : 0u;
+          // (rows that fit lie where they are even if the buffer has no room for later ones)
+          bpos = __shfl_sync(kFullMask, upto, 31);
+          for (unsigned m = walk; m; m &= m - 1) {
+            const uint32_t j = __ffs(m) - 1;
+            const uint64_t n = wide_row<kWWin>(p, uint64_t(c0) + r + j, bits, reach, &nnz_acc, [](uint64_t, uint32_t) {});
+            if (n > 0xfffffffeull) raise_flag(p, &p.ctl->status, 16ull);
+            if (lane == 0) S.cnt_row[r + j] = uint32_t(n);
+          }
+        }
+      } else
       for (uint32_t r = warp; r < crows; r += kWWarps) {
         const uint32_t start = bpos;
         const uint64_t c = wide_row<kWWin>(p, uint64_t(c0) + r, bits, reach, &nnz_acc, [&](uint64_t k, uint32_t v) {
@@ -195,7 +426,7 @@ __global__ void __launch_bounds__(kWThreads, DVG_WIDE_MINB) k_spgemm_wide(FusedA
       if (imaged) {
         uint32_t* img = S.img[b];
         uint32_t bp = 0;
-        for (uint32_t r = warp; r < crows; r += kWWarps) {
+        auto image_row = [&](uint32_t r) {
           const uint32_t n = S.cnt_row[r], o = r ? S.incl[b][r - 1] : 0u;
           if (S.kept[r]) {
             for (uint32_t k = lane; k < n; k += 32) img[o + k] = buf[bp + k];
@@ -208,6 +439,17 @@ __global__ void __launch_bounds__(kWThreads, DVG_WIDE_MINB) k_spgemm_wide(FusedA
             });
             if (bad || c != n) raise_flag(p, &p.ctl->status, 8ull);
           }
+        };
+        for (uint32_t r0 = warp * kRun; r0 < crows; r0 += kWWarps * kRun) {
+          const uint32_t rows = min(kRun, crows - r0);
+          if (kRun > 1 && __all_sync(kFullMask, uint32_t(lane) >= rows || S.kept[r0 + lane])) {
+            // consecutive rows in the buffer and in the image
+            const uint32_t o = r0 ? S.incl[b][r0 - 1] : 0u, n = S.incl[b][r0 + rows - 1] - o;
+            for (uint32_t k = lane; k < n; k += 32) img[o + k] = buf[bp + k];
+            bp += n;
+          } else {
+            for (uint32_t r = r0; r < r0 + rows; ++r) image_row(r);
+          }
         }
       }
     }
@@ -218,7 +460,7 @@ __global__ void __launch_bounds__(kWThreads, DVG_WIDE_MINB) k_spgemm_wide(FusedA
       wide_sync();
       const unsigned long long prefix = S.prefix[0];
       for (uint32_t r = tid; r < prow; r += kWThreads)
-        p.c_rowmap[uint64_t(pt) * kWRows + r + 1] = prefix + S.incl[b ^ 1u][r];
+        p.c_rowmap[uint64_t(pt) * p.chunk_rows + r + 1] = prefix + S.incl[b ^ 1u][r];
       if (pt == 0 && tid == 0) p.c_rowmap[0] = 0;
       if (prefix + pcnt <= p.cap) {
         uint32_t* dst = p.c_entries + prefix;
@@ -236,7 +478,7 @@ __global__ void __launch_bounds__(kWThreads, DVG_WIDE_MINB) k_spgemm_wide(FusedA
       for (uint32_t r = tid; r < crows; r += kWThreads) p.c_rowmap[uint64_t(c0) + r + 1] = prefix + S.incl[b][r];
       if (t == 0 && tid == 0) p.c_rowmap[0] = 0;
       uint32_t bp = 0;
-      for (uint32_t r = warp; r < crows; r += kWWarps) {
+      each_row(crows, [&](uint32_t r) {
         const uint32_t n = S.cnt_row[r], o = r ? S.incl[b][r - 1] : 0u;
         const bool kept = S.kept[r] != 0;
         if (n && prefix + o + n > p.cap) {
@@ -254,7 +496,7 @@ __global__ void __launch_bounds__(kWThreads, DVG_WIDE_MINB) k_spgemm_wide(FusedA
           if (bad || c != n) raise_flag(p, &p.ctl->status, 8ull);
         }
         if (kept) bp += n;
-      }
+      });
     }
     if (have && imaged) {
       if (tid == 0) {
@@ -276,14 +518,167 @@ __global__ void __launch_bounds__(kWThreads, DVG_WIDE_MINB) k_spgemm_wide(FusedA
   if (lane == 0 && nnz_acc) atomicAdd(&p.ctl->nnz, nnz_acc);
 }
 
+// ---- the tables -----------------------------------------------------------------
+
+// blk[b]: the words, in whole fours, that the ranges of the rows cover that a union
+// from block b reaches (the block's and the 63 after them), a warp a block; the
+// widest into *widest.
+constexpr uint32_t kBandReach = kBandBlock + 63;
+__global__ void __launch_bounds__(kWThreads) k_band_blocks(const uint64_t* __restrict__ rowmap,
+                                                           const uint32_t* __restrict__ entries, uint32_t nrows,
+                                                           uint2* __restrict__ blk, unsigned long long* widest) {
+  const int lane = lane_id();
+  const uint64_t b = (uint64_t(blockIdx.x) * kWThreads + threadIdx.x) >> 5, r0 = b * kBandBlock;
+  if (r0 >= nrows) return;
+  const uint64_t e0 = __ldg(rowmap + r0) >> 1, e1 = __ldg(rowmap + min(r0 + kBandReach, uint64_t(nrows))) >> 1;
+  uint32_t lo = 0xffffffffu, hi = 0;
+  for (uint64_t e = e0 + lane; e < e1; e += 32) {
+    const uint2 r = load_range(entries, e);
+    if (r.y < r.x) continue;
+    lo = min(lo, (r.x >> 5) & ~3u);
+    hi = max(hi, ((r.y >> 5) & ~3u) + 4u);
+  }
+  lo = group_min<32>(kFullMask, lo);
+  hi = group_max<32>(kFullMask, hi);
+  if (lane == 0) {
+    blk[b] = lo < hi ? make_uint2(lo, hi - lo) : make_uint2(0u, 0u);
+    if (lo < hi) atomicMax(widest, (unsigned long long)(hi - lo));
+  }
+}
+
+// The unions from a block's rows: the rows that they reach as bitmaps in shared
+// memory, then in place 4 rows' unions from those, 8 from 4 and so on to 64, each
+// written out on the way.
+// Bound: the tables' writes, 24 bytes a word of a row's band.
+constexpr uint32_t kBandRows = kBandBlock + 64;  // rows in shared memory (the last of them empty)
+__global__ void __launch_bounds__(kWThreads) k_band_tables(const uint64_t* __restrict__ rowmap,
+                                                           const uint32_t* __restrict__ entries, uint32_t nrows,
+                                                           BandTables t, uint4* __restrict__ out) {
+  extern __shared__ __align__(16) uint4 band_smem[];
+  static_assert(2 * kBandRows == kWThreads, "two threads a row");
+  constexpr int kMine = kBandMaxWords / 4 * kBandRows / kWThreads;  // quads of a thread
+  const uint32_t r0 = kBandBlock * blockIdx.x, tid = threadIdx.x;
+  const uint2 box = t.blk[blockIdx.x];
+  const uint32_t v = box.y / 4;  // 16-byte words of a row
+  if (v == 0) return;            // nothing there: no step reads these
+  const uint32_t all = kBandRows * v;
+  for (uint32_t k = tid; k < all; k += kWThreads) band_smem[k] = make_uint4(0u, 0u, 0u, 0u);
+  __syncthreads();
+  const uint32_t r = tid / 2;
+  if (r < kBandReach && uint64_t(r0) + r < nrows) {
+    uint32_t* const bits = reinterpret_cast<uint32_t*>(band_smem + r * v);
+    const uint64_t e1 = __ldg(rowmap + r0 + r + 1) >> 1;
+    for (uint64_t e = (__ldg(rowmap + r0 + r) >> 1) + tid % 2; e < e1; e += 2) {
+      const uint2 c = load_range(entries, e);
+      if (c.y < c.x) continue;
+      const uint32_t ws = (c.x >> 5) - box.x, we = (c.y >> 5) - box.x;
+      const uint32_t lo = ~0u << (c.x & 31), hi = ~0u >> (31 - (c.y & 31));
+      for (uint32_t k = ws; k <= we; ++k) atomicOr(bits + k, (k == ws ? lo : ~0u) & (k == we ? hi : ~0u));
+    }
+  }
+  __syncthreads();
+  // the thread's quads tid, tid + kWThreads, ... of the block's rows, kept in
+  // registers while the others' are read
+  const uint32_t mine = min(kBandBlock, nrows - r0) * v;  // quads that are written out
+  uint4* const to = out + size_t(r0) * (t.stride / 4);  // the block's rows, v quads each
+  auto either = [](uint4 a, uint4 b) { return make_uint4(a.x | b.x, a.y | b.y, a.z | b.z, a.w | b.w); };
+  uint4 q[kMine];
+#pragma unroll
+  for (int i = 0; i < kMine; ++i) {
+    const uint32_t k = tid + i * kWThreads;
+    if (k < all) q[i] = band_smem[k];
+    if (k < mine) to[k] = q[i];
+  }
+#pragma unroll 1
+  for (int level = 1; level < kBandLevels; ++level) {
+    // rows of the level before that one of this level takes besides its own
+    const uint32_t by = level == 1 ? 1u : 1u << level, n = level == 1 ? 3u : 1u;
+#pragma unroll
+    for (int i = 0; i < kMine; ++i) {
+      const uint32_t k = tid + i * kWThreads;
+      if (k >= all) break;
+      for (uint32_t m = 1; m <= n; ++m)
+        if (k + m * by * v < all) q[i] = either(q[i], band_smem[k + m * by * v]);
+      if (k < mine) to[size_t(level) * t.table + k] = q[i];
+    }
+    if (level + 1 == kBandLevels) break;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kMine; ++i) {
+      const uint32_t k = tid + i * kWThreads;
+      if (k < all) band_smem[k] = q[i];
+    }
+    __syncthreads();
+  }
+}
+
 }  // namespace
 
+// The tables cost about 0.25 us a 1,000 B rows of 40 words, a row walked range by
+// range 1.5 ns for each B row that it names: a product has to name B's rows often
+// (at 45 times each it gains 13 %, at 113 times 26 % with 1.3e5 rows and 70 % with
+// 4.2e6), and one that names fewer than 2^21 is over before the read-back is.
+constexpr uint64_t kBandMinUses = 32, kBandMinRows = 1u << 21;
+
+BandTables build_band_tables(dvg_context* ctx, const dvg_matrix* a, const dvg_matrix* b) {
+  BandTables none{};
+  if (b->nrows == 0 || b->nentries == 0 || a->nnz < kBandMinRows || a->nnz < kBandMinUses * b->nrows) return none;
+  const uint32_t blocks = uint32_t((uint64_t(b->nrows) + kBandBlock - 1) / kBandBlock);
+  const size_t blk_bytes = (size_t(blocks) * sizeof(uint2) + 255) & ~size_t(255);
+  void *head = nullptr, *mem = nullptr;
+  try {
+    head = dalloc(ctx, blk_bytes + 256);
+    auto* blk = static_cast<uint2*>(head);
+    auto* widest = reinterpret_cast<unsigned long long*>(static_cast<char*>(head) + blk_bytes);
+    DVG_CUDA(cudaMemsetAsync(widest, 0, 8, ctx->stream));
+    k_band_blocks<<<(blocks + kWWarps - 1) / kWWarps, kWThreads, 0, ctx->stream>>>(b->rowmap, b->entries, b->nrows, blk,
+                                                                                widest);
+    DVG_CUDA(cudaGetLastError());
+    auto* h = static_cast<unsigned long long*>(host_stage(ctx, 8));
+    DVG_CUDA(cudaMemcpyAsync(h, widest, 8, cudaMemcpyDeviceToHost, ctx->stream));
+    DVG_CUDA(cudaStreamSynchronize(ctx->stream));
+    ctx->stats.host_syncs++;
+    ctx->stats.kernel_launches += 2;
+    const uint64_t words = *h;
+    const size_t table = size_t(b->nrows) * words * 4;
+    if (words == 0 || words > kBandMaxWords || kBandLevels * table / 16 > 0xffffffffull ||
+        kBandLevels * table > (device_free_bytes(ctx) + ctx->cached_bytes) / 4) {
+      dfree(ctx, head);
+      return none;
+    }
+    mem = dalloc(ctx, blk_bytes + kBandLevels * table);
+    auto* out = reinterpret_cast<uint4*>(static_cast<char*>(mem) + blk_bytes);
+    BandTables t{};
+    t.t = out;
+    t.table = table / 16;
+    t.blk = static_cast<const uint2*>(mem);
+    t.stride = uint32_t(words);
+    t.mem = mem;
+    DVG_CUDA(cudaMemcpyAsync(mem, head, blk_bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+    const int smem = int(kBandRows * words * 4);
+    DVG_CUDA(cudaFuncSetAttribute(k_band_tables, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    cudaEvent_t ev = span_begin(ctx);
+    k_band_tables<<<blocks, kWThreads, smem, ctx->stream>>>(b->rowmap, b->entries, b->nrows, t, out);
+    span_end(ctx, ev, kLevels);
+    DVG_CUDA(cudaGetLastError());
+    ctx->stats.kernel_launches++;
+    dfree(ctx, head);
+    return t;
+  } catch (const Error& e) {
+    if (head) dfree(ctx, head);
+    if (mem) dfree(ctx, mem);
+    if (e.status == DVG_ERR_OOM) return none;  // range by range instead
+    throw;
+  }
+}
+
 size_t spgemm_wide_desc_bytes(uint32_t nrows) {
-  return size_t((uint64_t(nrows) + kWRows - 1) / kWRows) * sizeof(ChunkDesc);
+  return size_t((uint64_t(nrows) + kWRowsMin - 1) / kWRowsMin) * sizeof(ChunkDesc);
 }
 
 void launch_spgemm_wide(dvg_context* ctx, const dvg_matrix* a, const dvg_matrix* b, const dvg_matrix* d,
-                        uint64_t* c_rowmap, uint32_t* c_entries, uint64_t cap, void* desc, unsigned* ticket) {
+                        uint64_t* c_rowmap, uint32_t* c_entries, uint64_t cap, void* desc, unsigned* ticket,
+                        const BandTables* band) {
   const uint32_t n = a->nrows;
   if (n == 0) return;
   FusedArgs p{};
@@ -300,15 +695,17 @@ void launch_spgemm_wide(dvg_context* ctx, const dvg_matrix* a, const dvg_matrix*
   p.ticket = ticket;
   p.ctl = ctx->d_ctl;
   p.nrows = n;
-  p.chunk_rows = kWRows;
-  p.nchunks = uint32_t((uint64_t(n) + kWRows - 1) / kWRows);
+  p.chunk_rows = band ? kWBandRows : kWRows;
+  p.nchunks = uint32_t((uint64_t(n) + p.chunk_rows - 1) / p.chunk_rows);
+  if (band) p.band = *band;
+  auto kern = band ? k_spgemm_wide<true> : k_spgemm_wide<false>;
   const int smem = int(sizeof(WideSmem));
-  DVG_CUDA(cudaFuncSetAttribute(k_spgemm_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  DVG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   int per_sm = 0;
-  DVG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_spgemm_wide, kWThreads, smem));
+  DVG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWThreads, smem));
   if (per_sm < 1) throw Error(DVG_ERR_DEVICE, "wide spgemm: shared memory layout does not fit");
   const unsigned grid = unsigned(std::min<uint64_t>(p.nchunks, uint64_t(per_sm) * ctx->num_sms));
-  k_spgemm_wide<<<grid, kWThreads, smem, ctx->stream>>>(p);
+  kern<<<grid, kWThreads, smem, ctx->stream>>>(p);
   DVG_CUDA(cudaGetLastError());
   ctx->stats.kernel_launches++;
 }

@@ -135,3 +135,57 @@ def test_range_operation_calibration(ctx):
     assert np.isfinite(rate) and 1e9 < rate < 1e14, rate
     a = gen.banded(1 << 12, 64, 4.0, 16.0, seed=13)
     assert_same(product(ctx, a, a), orc.spgemm(omat(a), omat(a)), "after calibration")
+
+
+def named(ctx, a, b):
+    """The automatic product of operands that name enough B rows for the tables of unions."""
+    assert a.nnz() >= 1 << 21 and a.nnz() >= 32 * b.numRows()
+    ctx.reset_stats()
+    got = product(ctx, a, b, mode=0)
+    st = ctx.stats()
+    assert st["spgemm_calls"] == 1 and st["spgemm_light"] == 0
+    return got
+
+
+@pytest.mark.parametrize("n,hw,ranges,length", [(20_033, 512, 4.0, 32.0), (65_536, 128, 2.0, 40.0),
+                                                (30_000, 700, 6.0, 20.0), (12_345, 300, 12.0, 200.0),
+                                                (40_001, 256, 10.0, 12.0)])
+def test_unions_of_b_rows(ctx, n, hw, ranges, length):
+    a = gen.banded(n, hw, ranges, length, seed=15)
+    b = gen.banded(n, hw, ranges, length, seed=16)
+    assert_same(named(ctx, a, b), orc.spgemm(omat(a), omat(b)), f"banded {n} {hw}")
+
+
+def test_unions_with_rows_that_need_walking(ctx):
+    # ranges of 1 to 400 rows (every table, steps between the first and the last),
+    # rows of more than 8 and of more than 64 ranges, empty rows, ranges given out of
+    # order, and rows whose ranges lie too far apart for the window
+    rng = np.random.default_rng(17)
+    n = 9_000
+    brows = [[(max(0, min(n - 1, i + int(d))), max(0, min(n - 1, i + int(d) + int(rng.integers(0, 9)))))
+              for d in rng.integers(-300, 300, int(rng.integers(0, 4)))] for i in range(n)]
+    b = from_rows(brows, n)
+    arows = []
+    for i in range(n):
+        kind = i % 9
+        if kind == 0:
+            r = []
+        elif kind == 1:
+            r = [(max(0, i - 400), min(n - 1, i + 399))]
+        elif kind == 2:  # 80 short ranges
+            r = [(j, min(n - 1, j + 5)) for j in range(max(0, i - 400), min(n, i + 400), 10)]
+        elif kind == 3:  # 20 ranges, last first
+            r = [(j, min(n - 1, j + 24)) for j in range(max(0, i - 400), min(n, i + 400), 40)][::-1]
+        elif kind == 4:  # far apart
+            r = [(max(0, i - 300), i), (min(n - 1, i + 4000), min(n - 1, i + 4400))]
+        else:
+            r = []
+            for _ in range(4):
+                s = min(n - 1, max(0, i - 300 + int(rng.integers(0, 400))))
+                r.append((s, min(n - 1, s + int(rng.choice([0, 1, 2, 3, 6, 7, 8, 15, 16, 31, 63, 64, 127, 128, 200, 399])))))
+        arows.append(r)
+    a = from_rows(arows, n)
+    assert_same(named(ctx, a, b), orc.spgemm(omat(a), omat(b)), "mixed rows")
+    # B's band wider than a table's row: range by range
+    wide = from_rows([[(int(c), int(min(n - 1, c + 20))) for c in np.sort(rng.integers(0, n, 3))] for _ in range(n)], n)
+    assert_same(named(ctx, a, wide), orc.spgemm(omat(a), omat(wide)), "wide B")
