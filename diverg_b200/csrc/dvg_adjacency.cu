@@ -15,12 +15,19 @@
 //     repeated successor yields a repeated single-column range, as in append.
 // nnz is the number of Basic entries, (loci - nodes) + edges.
 //
-// Kernels: edges are counted per source node and scattered into per-node
-// segments (counting sort, any edge order), each node sorts its segment and
-// counts its ranges, a scan gives every node's first entry, then one thread
-// per locus writes the row map and the inner rows and one thread per node
-// writes its last row.  All of it is streaming integer work on HBM.
+// Kernels: edges are checked, counted per source node and scattered into
+// per-node segments (counting sort, any edge order), each node sorts its segment
+// and counts its ranges, a scan gives every node's first entry, then a thread
+// per locus writes the row map and its row.  The output is allocated for the
+// most entries that so many bases and edges can have (a few more than there
+// are), so nothing is waited for until the end; a node range's edges are counted
+// first.
+//
+// Bound: the matrix's writes, 16 bytes a locus; below ~1e6 loci the launches and
+// the one wait.  1e7 loci of 3.4e4 nodes and 4.6e4 edges: 449 -> 187 us a call, of which
+// k_adj_rows 128 -> 45 us (a binary search over all nodes for every locus before).
 #include <algorithm>
+#include <cstring>
 #include <vector>
 
 #include "dvg_device.cuh"
@@ -30,6 +37,7 @@ namespace dvg {
 namespace {
 
 constexpr int kAdjThreads = 256;
+constexpr size_t kAdjStaged = 8u << 20;  // input bytes up to which they go through pinned staging
 
 unsigned adj_grid(dvg_context* ctx, uint64_t n) {
   const uint64_t want = (n + kAdjThreads - 1) / kAdjThreads;
@@ -53,17 +61,18 @@ struct AdjArgs {
   DeviceControl* ctl;
 };
 
-// start[v + 1] = node_len[v] (scanned afterwards)
-__global__ void k_adj_lengths(AdjArgs p) {
-  for (uint64_t v = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; v < p.nnodes; v += uint64_t(gridDim.x) * blockDim.x)
-    p.start[v + 1] = p.node_len[v];
-}
-
-// eoff[v + 1] = out-degree of node v within the range; a successor outside
-// the range is an error (its column would not exist)
-__global__ void k_adj_degrees(AdjArgs p) {
-  for (uint64_t e = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; e < p.nedges; e += uint64_t(gridDim.x) * blockDim.x) {
+// start[v + 1] = node_len[v], eoff[v + 1] = out-degree of node v within the range
+// (scanned afterwards).  Bit 2 of invalid: an endpoint that is no node; bit 1: a
+// successor outside the range of a node inside it (its column would not exist).
+__global__ void k_adj_counts(AdjArgs p, uint32_t all_nodes) {
+  const uint64_t t0 = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x, stride = uint64_t(gridDim.x) * blockDim.x;
+  for (uint64_t v = t0; v < p.nnodes; v += stride) p.start[v + 1] = p.node_len[v];
+  for (uint64_t e = t0; e < p.nedges; e += stride) {
     const uint32_t from = p.edges[2 * e], to = p.edges[2 * e + 1];
+    if (from < 1 || from > all_nodes || to < 1 || to > all_nodes) {
+      atomicOr(&p.ctl->invalid, 2ull);
+      continue;
+    }
     if (from < p.lower || from >= p.upper) continue;
     if (to < p.lower || to >= p.upper) {
       atomicOr(&p.ctl->invalid, 1ull);
@@ -73,10 +82,57 @@ __global__ void k_adj_degrees(AdjArgs p) {
   }
 }
 
+// In-place inclusive scans of a[1 .. n] and b[1 .. n] (b null: a alone), a block
+// each: for the node counts of most graphs one launch beats the three that a
+// scan over the whole chip takes (two scans of 3.4e4 nodes: 33 -> 18 us).
+constexpr uint32_t kAdjScanThreads = 1024, kAdjScanMax = 1u << 17;
+__global__ void __launch_bounds__(kAdjScanThreads) k_adj_scan(uint64_t* a, uint64_t* b, uint32_t n) {
+  constexpr int kAhead = 8;
+  __shared__ uint64_t warps[kAdjScanThreads / 32];
+  uint64_t* const x = (blockIdx.x ? b : a) + 1;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // a warp's consecutive elements, 32 at a time
+  const uint32_t per = ((n + kAdjScanThreads - 1) / kAdjScanThreads) * 32, i0 = min(warp * per, n), i1 = min(i0 + per, n);
+  uint64_t sum = 0;
+  for (uint32_t i = i0 + lane; i < i1; i += 32 * kAhead) {
+    uint64_t v[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) v[k] = i + 32 * k < i1 ? x[i + 32 * k] : 0;
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) sum += v[k];
+  }
+  sum = group_sum<32>(kFullMask, sum);
+  if (lane == 0) warps[warp] = sum;
+  __syncthreads();
+  uint64_t run = group_sum<32>(kFullMask, lane < warp ? warps[lane] : uint64_t(0));
+  for (uint32_t i = i0; i < i1; i += 32 * kAhead) {
+    uint64_t v[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) v[k] = i + 32 * k + lane < i1 ? x[i + 32 * k + lane] : 0;
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      v[k] = run + group_incl_sum<32>(kFullMask, v[k], int(lane));
+      run = __shfl_sync(kFullMask, v[k], 31);
+      if (i + 32 * k + lane < i1) x[i + 32 * k + lane] = v[k];
+    }
+  }
+}
+
+void scan_nodes(dvg_context* ctx, uint64_t* a, uint64_t* b, uint32_t n) {
+  if (n <= kAdjScanMax) {
+    k_adj_scan<<<b ? 2 : 1, kAdjScanThreads, 0, ctx->stream>>>(a, b, n);
+    DVG_CUDA(cudaGetLastError());
+    ctx->stats.kernel_launches++;
+    return;
+  }
+  launch_rowmap_scan(ctx, a, n);
+  if (b) launch_rowmap_scan(ctx, b, n);
+}
+
 // each edge's successor locus into its source node's segment
 __global__ void k_adj_scatter(AdjArgs p) {
   for (uint64_t e = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; e < p.nedges; e += uint64_t(gridDim.x) * blockDim.x) {
-    const uint32_t from = p.edges[2 * e], to = p.edges[2 * e + 1];
+    const uint32_t from = p.edges[2 * e], to = p.edges[2 * e + 1];  // (what k_adj_counts counted)
     if (from < p.lower || from >= p.upper || to < p.lower || to >= p.upper) continue;
     const uint32_t v = from - p.lower;
     const uint64_t slot = atomicAdd(reinterpret_cast<unsigned long long*>(p.cursor + v), 1ull);
@@ -150,56 +206,68 @@ __global__ void k_adj_nodes(AdjArgs p) {
   }
 }
 
-// per locus: the row map, and the single range of every row but a node's last
-__global__ void k_adj_rows(AdjArgs p, uint64_t nloci) {
-  for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < nloci; i += uint64_t(gridDim.x) * blockDim.x) {
-    // the node holding locus i: the last v with start[v] <= i
-    uint32_t lo = 0, hi = p.nnodes;  // start[lo] <= i < start[hi]
+// Per locus: the row map and the row's ranges.  A block takes kAdjTile consecutive
+// loci; their nodes -- the last one that starts at or before the first locus, and
+// every one that starts after it within the tile -- are found once, and a locus
+// searches only those.
+constexpr uint32_t kAdjTile = 1024;
+__global__ void __launch_bounds__(kAdjThreads) k_adj_rows(AdjArgs p, uint64_t nloci) {
+  __shared__ uint32_t first[kAdjTile + 1];  // first loci of its nodes, from the tile's first (the first node: 0)
+  const uint64_t i0 = uint64_t(blockIdx.x) * kAdjTile;
+  const uint32_t rows = uint32_t(min(uint64_t(kAdjTile), nloci - i0));
+  // the last of `len` nodes from v on that starts at or before x (v does): every
+  // thread tries one, a few rounds for any graph
+  auto last_at = [&](uint64_t x, uint32_t v, uint32_t len) {
+    while (len > 1) {
+      const uint32_t step = (len + kAdjThreads - 1) / kAdjThreads, k = threadIdx.x * step;
+      const uint32_t c = uint32_t(__syncthreads_count(k < len && p.start[v + k] <= x)) - 1;
+      v += c * step;
+      len = min(step, len - c * step);
+    }
+    return v;
+  };
+  const uint32_t v0 = last_at(i0, 0, p.nnodes);
+  // (every node has a locus: at most `rows` nodes)
+  const uint32_t n = last_at(i0 + rows - 1, v0, min(rows, p.nnodes - v0)) - v0 + 1;
+  for (uint32_t v = threadIdx.x; v < n; v += kAdjThreads) first[v] = v ? uint32_t(p.start[v0 + v] - i0) : 0u;
+  __syncthreads();
+  for (uint32_t t = threadIdx.x; t < rows; t += kAdjThreads) {
+    uint32_t lo = 0, hi = n;
     while (hi - lo > 1) {
-      const uint32_t mid = lo + (hi - lo) / 2;
-      if (p.start[mid] <= i) lo = mid;
+      const uint32_t mid = (lo + hi) / 2;
+      if (first[mid] <= t) lo = mid;
       else hi = mid;
     }
-    const uint64_t k = i - p.start[lo];
-    const uint64_t len = p.node_len[lo];
-    if (k + 1 < len) {
-      const uint64_t at = p.base[lo] + 2 * k;
-      p.c_entries[at] = uint32_t(i + 1);
-      p.c_entries[at + 1] = uint32_t(i + 1);
+    const uint32_t v = v0 + lo;
+    const uint64_t i = i0 + t, k = i - p.start[v];
+    const uint64_t at = p.base[v] + 2 * k;
+    if (k + 1 < p.node_len[v]) {
+      *reinterpret_cast<uint2*>(p.c_entries + at) = make_uint2(uint32_t(i + 1), uint32_t(i + 1));
       p.c_rowmap[i + 1] = at + 2;
-    } else {
-      p.c_rowmap[i + 1] = p.base[lo + 1];
+    } else {  // the node's last row: its successors
+      const uint32_t* a = p.cols + p.eoff[v];
+      const uint64_t ns = p.eoff[v + 1] - p.eoff[v], end_at = p.base[v + 1];
+      uint64_t w = at;
+      auto put = [&](uint32_t lo_col, uint32_t hi_col) {
+        if (w + 2 <= end_at) *reinterpret_cast<uint2*>(p.c_entries + w) = make_uint2(lo_col, hi_col);
+        w += 2;
+      };
+      bool open = false;
+      uint32_t begin = 0, end = 0;
+      for (uint64_t q = 0; q < ns; ++q) {
+        if (open && uint64_t(a[q]) == uint64_t(end) + 1) {
+          ++end;
+          continue;
+        }
+        if (open) put(begin, end);
+        begin = end = a[q];
+        open = true;
+      }
+      if (open) put(begin, end);
+      if (w != end_at) atomicOr(&p.ctl->status, 32ull);
+      p.c_rowmap[i + 1] = end_at;
     }
     if (i == 0) p.c_rowmap[0] = 0;
-  }
-}
-
-// per node: the ranges of its last row
-__global__ void k_adj_last_rows(AdjArgs p) {
-  for (uint64_t v = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; v < p.nnodes; v += uint64_t(gridDim.x) * blockDim.x) {
-    const uint32_t* a = p.cols + p.eoff[v];
-    const uint64_t n = p.eoff[v + 1] - p.eoff[v];
-    uint32_t* out = p.c_entries + p.base[v] + 2 * (uint64_t(p.node_len[v]) - 1);
-    const uint32_t* stop = p.c_entries + p.base[v + 1];
-    uint64_t w = 0;
-    auto put = [&](uint32_t x) {
-      if (out + w < stop) out[w] = x;
-      ++w;
-    };
-    bool open = false;
-    uint32_t end = 0;
-    for (uint64_t i = 0; i < n; ++i) {
-      if (open && uint64_t(a[i]) == uint64_t(end) + 1) {
-        ++end;
-        continue;
-      }
-      if (open) put(end);
-      put(a[i]);
-      end = a[i];
-      open = true;
-    }
-    if (open) put(end);
-    if (out + w != stop) atomicOr(&p.ctl->status, 32ull);
   }
 }
 
@@ -214,10 +282,12 @@ dvg_matrix* adjacency_from_graph(dvg_context* ctx, uint32_t nnodes, const uint32
   const uint32_t m = upper - lower;
   const uint32_t* lens = node_len + (lower - 1);
   uint64_t nloci = 0;
+  uint32_t shortest = 0xffffffffu;
   for (uint32_t v = 0; v < m; ++v) {
-    if (lens[v] == 0) throw Error(DVG_ERR_INVALID_ARG, "adjacency: a node has length 0");
     nloci += lens[v];
+    shortest = std::min(shortest, lens[v]);
   }
+  if (shortest == 0) throw Error(DVG_ERR_INVALID_ARG, "adjacency: a node has length 0");
   if (nloci > 0xFFFFFFFEull) throw Error(DVG_ERR_OVERFLOW, "adjacency: more loci than 32-bit columns hold");
 
   AdjArgs p{};
@@ -234,61 +304,76 @@ dvg_matrix* adjacency_from_graph(dvg_context* ctx, uint32_t nnodes, const uint32
   };
   dvg_matrix* out = nullptr;
   try {
-    uint32_t* d_len = static_cast<uint32_t*>(grab(size_t(m) * 4));
-    uint32_t* d_edges = nedges ? static_cast<uint32_t*>(grab(nedges * 8)) : nullptr;
-    p.start = static_cast<uint64_t*>(grab((size_t(m) + 1) * 8));
-    p.eoff = static_cast<uint64_t*>(grab((size_t(m) + 1) * 8));
-    p.cursor = static_cast<uint64_t*>(grab(size_t(m) * 8));
-    p.base = static_cast<uint64_t*>(grab((size_t(m) + 1) * 8));
-    DVG_CUDA(cudaMemcpyAsync(d_len, lens, size_t(m) * 4, cudaMemcpyHostToDevice, ctx->stream));
-    if (nedges) DVG_CUDA(cudaMemcpyAsync(d_edges, edges, nedges * 8, cudaMemcpyHostToDevice, ctx->stream));
-    ctx->stats.h2d_bytes += uint64_t(m) * 4 + nedges * 8;
-    p.node_len = d_len;
-    p.edges = d_edges;
+    // the edges, then the lengths
+    const size_t edge_bytes = nedges * 8, len_bytes = size_t(m) * 4;
+    char* d_in = static_cast<char*>(grab(edge_bytes + len_bytes));
+    if (edge_bytes + len_bytes <= kAdjStaged) {
+      // one copy from pinned memory, under way while the rest is prepared (two
+      // copies of pageable memory are waited for in turn)
+      char* h = static_cast<char*>(host_stage(ctx, edge_bytes + len_bytes));
+      if (nedges) std::memcpy(h, edges, edge_bytes);
+      std::memcpy(h + edge_bytes, lens, len_bytes);
+      DVG_CUDA(cudaMemcpyAsync(d_in, h, edge_bytes + len_bytes, cudaMemcpyHostToDevice, ctx->stream));
+    } else {
+      if (nedges) DVG_CUDA(cudaMemcpyAsync(d_in, edges, edge_bytes, cudaMemcpyHostToDevice, ctx->stream));
+      DVG_CUDA(cudaMemcpyAsync(d_in + edge_bytes, lens, len_bytes, cudaMemcpyHostToDevice, ctx->stream));
+    }
+    ctx->stats.h2d_bytes += edge_bytes + len_bytes;
+    p.edges = reinterpret_cast<const uint32_t*>(d_in);
+    p.node_len = reinterpret_cast<const uint32_t*>(d_in + edge_bytes);
+    // start | eoff | cursor | base, all zero at first
+    const size_t words = size_t(m) + 1;
+    p.start = static_cast<uint64_t*>(grab(4 * words * 8));
+    p.eoff = p.start + words;
+    p.cursor = p.eoff + words;
+    p.base = p.cursor + words;
+    uint64_t* h_sizes = reinterpret_cast<uint64_t*>(ctx->h_ctl + 1);
+    uint64_t most_edges = nedges;  // of the range
+    auto allocate = [&]() {
+      p.cols = static_cast<uint32_t*>(grab(std::max<uint64_t>(most_edges, 1) * 4));
+      // at most a range a base but the last of a node, and one an edge
+      out = new_matrix(ctx, uint32_t(nloci), uint32_t(nloci), 2 * (nloci - m) + 2 * most_edges);
+      p.c_rowmap = out->rowmap;
+      p.c_entries = out->entries;
+    };
+    const bool whole = m == nnodes;
+    if (whole) allocate();
     reset_control(ctx);
-    DVG_CUDA(cudaMemsetAsync(p.start, 0, 8, ctx->stream));
-    DVG_CUDA(cudaMemsetAsync(p.eoff, 0, (size_t(m) + 1) * 8, ctx->stream));
-    DVG_CUDA(cudaMemsetAsync(p.cursor, 0, size_t(m) * 8, ctx->stream));
-    DVG_CUDA(cudaMemsetAsync(p.base, 0, 8, ctx->stream));
-    k_adj_lengths<<<adj_grid(ctx, m), kAdjThreads, 0, ctx->stream>>>(p);
+    DVG_CUDA(cudaMemsetAsync(p.start, 0, 4 * words * 8, ctx->stream));
+    k_adj_counts<<<adj_grid(ctx, std::max<uint64_t>(m, nedges)), kAdjThreads, 0, ctx->stream>>>(p, nnodes);
     DVG_CUDA(cudaGetLastError());
-    if (nedges) {
-      k_adj_degrees<<<adj_grid(ctx, nedges), kAdjThreads, 0, ctx->stream>>>(p);
-      DVG_CUDA(cudaGetLastError());
+    scan_nodes(ctx, p.start, p.eoff, m);
+    if (!whole) {  // a component may hold few of the graph's edges: its own number sizes the result
+      DVG_CUDA(cudaMemcpyAsync(h_sizes, p.eoff + m, 8, cudaMemcpyDeviceToHost, ctx->stream));
+      read_control(ctx);
+      most_edges = h_sizes[0];
+      allocate();
     }
-    launch_rowmap_scan(ctx, p.start, m);
-    launch_rowmap_scan(ctx, p.eoff, m);
-    // the range's edges: one read-back sizes the segment array
-    uint64_t nedges_in = 0;
-    DVG_CUDA(cudaMemcpyAsync(&ctx->h_ctl[1], p.eoff + m, 8, cudaMemcpyDeviceToHost, ctx->stream));
-    {
-      const DeviceControl c = read_control(ctx);
-      nedges_in = *reinterpret_cast<const uint64_t*>(&ctx->h_ctl[1]);
-      if (c.invalid & 1) throw Error(DVG_ERR_INVALID_ARG, "adjacency: an edge leaves the node range [lower, upper)");
-    }
-    p.cols = static_cast<uint32_t*>(grab(std::max<uint64_t>(nedges_in, 1) * 4));
     if (nedges) {
       k_adj_scatter<<<adj_grid(ctx, nedges), kAdjThreads, 0, ctx->stream>>>(p);
       DVG_CUDA(cudaGetLastError());
     }
     k_adj_nodes<<<adj_grid(ctx, m), kAdjThreads, 0, ctx->stream>>>(p);
     DVG_CUDA(cudaGetLastError());
-    launch_rowmap_scan(ctx, p.base, m);
-    DVG_CUDA(cudaMemcpyAsync(&ctx->h_ctl[1], p.base + m, 8, cudaMemcpyDeviceToHost, ctx->stream));
-    const DeviceControl c = read_control(ctx);
-    const uint64_t nentries = *reinterpret_cast<const uint64_t*>(&ctx->h_ctl[1]);
-    out = new_matrix(ctx, uint32_t(nloci), uint32_t(nloci), nentries);
+    scan_nodes(ctx, p.base, nullptr, m);
+    k_adj_rows<<<unsigned((nloci + kAdjTile - 1) / kAdjTile), kAdjThreads, 0, ctx->stream>>>(p, nloci);
+    DVG_CUDA(cudaGetLastError());
+    ctx->stats.kernel_launches += 4 + (nedges ? 1 : 0);
+    DVG_CUDA(cudaMemcpyAsync(h_sizes, p.base + m, 8, cudaMemcpyDeviceToHost, ctx->stream));
+    DVG_CUDA(cudaMemcpyAsync(h_sizes + 1, p.eoff + m, 8, cudaMemcpyDeviceToHost, ctx->stream));
+    DVG_CUDA(cudaMemcpyAsync(ctx->h_ctl, ctx->d_ctl, sizeof(DeviceControl), cudaMemcpyDeviceToHost, ctx->stream));
+    const uint64_t t0 = now_ns();
+    DVG_CUDA(cudaStreamSynchronize(ctx->stream));
+    ctx->stats.host_sync_ns += now_ns() - t0;
+    ctx->stats.host_syncs++;
+    resolve_spans(ctx);
+    const DeviceControl c = *ctx->h_ctl;
+    if (c.invalid & 2) throw Error(DVG_ERR_INVALID_ARG, "edge endpoint is not a node id in 1..nnodes");
+    if (c.invalid & 1) throw Error(DVG_ERR_INVALID_ARG, "adjacency: an edge leaves the node range [lower, upper)");
+    if (c.status) throw Error(DVG_ERR_DEVICE, "adjacency: internal consistency check failed on the device");
+    out->nentries = h_sizes[0];
     out->canonical = !(c.invalid & 16);
-    out->nnz = (nloci - m) + nedges_in;
-    p.c_rowmap = out->rowmap;
-    p.c_entries = out->entries;
-    k_adj_rows<<<adj_grid(ctx, nloci), kAdjThreads, 0, ctx->stream>>>(p, nloci);
-    DVG_CUDA(cudaGetLastError());
-    k_adj_last_rows<<<adj_grid(ctx, m), kAdjThreads, 0, ctx->stream>>>(p);
-    DVG_CUDA(cudaGetLastError());
-    ctx->stats.kernel_launches += 5 + (nedges ? 2 : 0);
-    const DeviceControl done = read_control(ctx);
-    if (done.status) throw Error(DVG_ERR_DEVICE, "adjacency: internal consistency check failed on the device");
+    out->nnz = (nloci - m) + h_sizes[1];
   } catch (...) {
     for (void* q : scratch) dfree(ctx, q);
     if (out) free_matrix(ctx, out);

@@ -1132,8 +1132,6 @@ dvg_status dvg_adjacency_from_graph(dvg_context* ctx, uint32_t nnodes, const uin
     Lock lk(ctx);
     require(out != nullptr, "null argument");
     require(nedges == 0 || edges != nullptr, "null edges");
-    for (uint64_t e = 0; e < 2 * nedges; ++e)
-      require(edges[e] >= 1 && edges[e] <= nnodes, "edge endpoint is not a node id in 1..nnodes");
     *out = adjacency_from_graph(ctx, nnodes, node_len, nedges, edges, lower, upper);
   });
 }

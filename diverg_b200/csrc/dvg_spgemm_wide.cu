@@ -54,9 +54,10 @@ constexpr int kWWin = 128;     // window words of a warp (4,096 columns)
 constexpr int kWBuf = 256;     // run entries of a warp's rows kept from the count
 constexpr int kWImage = 2048;  // output entries of a chunk held for its deferred write-out
 
+template <bool BAND>
 struct WideSmem {
   // a warp's windows: one row's bits and reach, or four rows' bits
-  uint32_t win[kWWarps][4 * kWWin];
+  uint32_t win[kWWarps][(BAND ? 4 : 2) * kWWin];
   uint32_t buf[kWWarps][kWBuf];  // runs of the warp's rows of the counted chunk, in row order
   uint32_t img[2][kWImage];      // images of the counted and the pending chunk
   uint32_t incl[2][kWRows];      // their chunk-local inclusive row counts
@@ -325,7 +326,7 @@ __device__ __forceinline__ void band_rows(const FusedArgs& p, uint64_t row, uint
 template <bool BAND>
 __global__ void __launch_bounds__(kWThreads, DVG_WIDE_MINB) k_spgemm_wide(const __grid_constant__ FusedArgs p) {
   extern __shared__ __align__(16) unsigned char wide_smem_raw[];
-  WideSmem& S = *reinterpret_cast<WideSmem*>(wide_smem_raw);
+  auto& S = *reinterpret_cast<WideSmem<BAND>*>(wide_smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint32_t* const bits = S.win[warp];
   uint32_t* const reach = bits + kWWin;
@@ -334,8 +335,12 @@ __global__ void __launch_bounds__(kWThreads, DVG_WIDE_MINB) k_spgemm_wide(const 
   // the warp's rows of a chunk, in the order in which its buffer keeps them
   constexpr uint32_t kRun = BAND ? 4 : 1;  // consecutive ones
   auto each_row = [&](uint32_t crows, auto&& f) {
-    for (uint32_t r0 = warp * kRun; r0 < crows; r0 += kWWarps * kRun)
-      for (uint32_t r = r0; r < min(r0 + kRun, crows); ++r) f(r);
+    if constexpr (!BAND) {
+      for (uint32_t r = warp; r < crows; r += kWWarps) f(r);
+    } else {
+      for (uint32_t r0 = warp * kRun; r0 < crows; r0 += kWWarps * kRun)
+        for (uint32_t r = r0; r < min(r0 + kRun, crows); ++r) f(r);
+    }
   };
   if (tid == 0) S.next = atomicAdd(p.ticket, 1u);
   wide_sync();
@@ -440,16 +445,20 @@ __global__ void __launch_bounds__(kWThreads, DVG_WIDE_MINB) k_spgemm_wide(const 
             if (bad || c != n) raise_flag(p, &p.ctl->status, 8ull);
           }
         };
-        for (uint32_t r0 = warp * kRun; r0 < crows; r0 += kWWarps * kRun) {
-          const uint32_t rows = min(kRun, crows - r0);
-          if (kRun > 1 && __all_sync(kFullMask, uint32_t(lane) >= rows || S.kept[r0 + lane])) {
-            // consecutive rows in the buffer and in the image
-            const uint32_t o = r0 ? S.incl[b][r0 - 1] : 0u, n = S.incl[b][r0 + rows - 1] - o;
-            for (uint32_t k = lane; k < n; k += 32) img[o + k] = buf[bp + k];
-            bp += n;
-          } else {
-            for (uint32_t r = r0; r < r0 + rows; ++r) image_row(r);
+        if constexpr (BAND) {
+          for (uint32_t r0 = warp * kRun; r0 < crows; r0 += kWWarps * kRun) {
+            const uint32_t rows = min(kRun, crows - r0);
+            if (__all_sync(kFullMask, uint32_t(lane) >= rows || S.kept[r0 + lane])) {
+              // consecutive rows in the buffer and in the image
+              const uint32_t o = r0 ? S.incl[b][r0 - 1] : 0u, n = S.incl[b][r0 + rows - 1] - o;
+              for (uint32_t k = lane; k < n; k += 32) img[o + k] = buf[bp + k];
+              bp += n;
+            } else {
+              for (uint32_t r = r0; r < r0 + rows; ++r) image_row(r);
+            }
           }
+        } else {
+          each_row(crows, image_row);
         }
       }
     }
@@ -699,7 +708,7 @@ void launch_spgemm_wide(dvg_context* ctx, const dvg_matrix* a, const dvg_matrix*
   p.nchunks = uint32_t((uint64_t(n) + p.chunk_rows - 1) / p.chunk_rows);
   if (band) p.band = *band;
   auto kern = band ? k_spgemm_wide<true> : k_spgemm_wide<false>;
-  const int smem = int(sizeof(WideSmem));
+  const int smem = int(band ? sizeof(WideSmem<true>) : sizeof(WideSmem<false>));
   DVG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   int per_sm = 0;
   DVG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWThreads, smem));

@@ -186,3 +186,22 @@ def test_bad_graphs_fail_with_invalid_argument(ctx):
         assert e.value.status == N.INVALID_ARG, (lo, hi)
     # the context stays usable
     assert same(ctx.adjacency_from_graph(lens, ok).download(), orc.adjacency(lens, ok))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,longest", [(1, 1), (1, 5000), (2, 1024), (255, 9), (1023, 1), (1024, 1), (1025, 1), (1024, 2),
+                                       (40_000, 60), (131_072, 2), (131_073, 2), (200_000, 1)])
+def test_tiles_and_scans_at_their_edges(ctx, n, longest):
+    # loci around a block's tile, nodes longer than one, node counts on both
+    # sides of the one-launch scan, and the second half alone where it is closed
+    rng = np.random.default_rng(n + longest)
+    lens = (np.full(n, longest, np.uint32) if n <= 2 else rng.integers(1, longest + 1, n).astype(np.uint32))
+    src = rng.integers(1, n + 1, n)
+    dst = np.minimum(n, src + rng.integers(1, 5, n))
+    half = n // 2 + 1
+    keep = (src < dst) & ((src < half) == (dst < half))
+    edges = np.stack([src[keep], dst[keep]], 1).astype(np.uint32).reshape(-1, 2)
+    assert same(ctx.adjacency_from_graph(lens, edges).download(), orc.adjacency(lens, edges))
+    if n > 1:
+        assert same(ctx.adjacency_from_graph(lens, edges, half, n + 1).download(),
+                    orc.adjacency(lens, edges, half, n + 1))
