@@ -422,7 +422,7 @@ dvg_matrix* range_spadd(dvg_context* ctx, const dvg_matrix* a, const dvg_matrix*
     dvg_matrix* c = new_matrix(ctx, n, a->ncols, cap);
     void* scratch = nullptr;
     try {
-      scratch = dalloc(ctx, spadd_single_pass_scratch(n));
+      scratch = dalloc(ctx, spadd_single_pass_scratch(a, b, b_identity));
       reset_control(ctx);
       cudaEvent_t t0 = span_begin(ctx);
       launch_spadd_single_pass(ctx, a, b, b_identity, c->rowmap, c->entries, cap, scratch);

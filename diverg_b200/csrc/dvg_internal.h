@@ -166,8 +166,8 @@ void launch_spadd(dvg_context* ctx, const dvg_matrix* a, const dvg_matrix* b, bo
 // C = A + B (B the identity when b_identity) in one pass: c_rowmap written
 // fully, c_entries up to `cap` entries (a.nentries + b's entries always
 // suffice); the control block receives the total entries, the nnz and a
-// timeout flag.  `scratch`: spadd_single_pass_scratch(a->nrows) bytes.
-uint64_t spadd_single_pass_scratch(uint32_t nrows);
+// timeout flag.  `scratch`: spadd_single_pass_scratch(a, b, b_identity) bytes.
+uint64_t spadd_single_pass_scratch(const dvg_matrix* a, const dvg_matrix* b, bool b_identity);
 void launch_spadd_single_pass(dvg_context* ctx, const dvg_matrix* a, const dvg_matrix* b, bool b_identity,
                               uint64_t* c_rowmap, uint32_t* c_entries, uint64_t cap, void* scratch);
 // Out-of-range pairs are counted into ctl->invalid (ctx->d_ctl when null).

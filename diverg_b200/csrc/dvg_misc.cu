@@ -254,29 +254,34 @@ __global__ void __launch_bounds__(kThreads) k_spadd(SpaddArgs p) {
 
 // ---- SpAdd in one pass ----------------------------------------------------------
 // The same rows as k_spadd (the merge of spadd_row), with no counting pass and
-// no scan: a persistent CTA takes chunks of kAddThreads rows from a ticket,
+// no scan: a persistent CTA takes chunks of up to kAddThreads rows from a ticket,
 // copies the chunk's row pointers and ranges of A and B -- contiguous in HBM --
-// into shared memory with asynchronous copies, merges a row per thread
-// (count), takes the chunk-local prefix, publishes the chunk's entry count
-// for later chunks' look-backs and merges again into a shared image of the
-// chunk's output.  The image waits in shared memory (two buffers) and is
-// resolved one iteration later: by then the chunks before it have long
-// published their counts, so its decoupled look-back rarely waits, and it is
-// written out with coalesced stores.  Rows whose ranges lie past the stages
-// read HBM; a chunk whose output exceeds its image buffer is resolved and
-// written straight to C in its own iteration.  Reads A and B once, writes C
-// once.
+// into shared memory with asynchronous copies and merges a row per thread.  A
+// row's result holds at most its two rows' ranges, so it goes to a place that
+// the row pointers give before anything is counted: the chunk's image in shared
+// memory, where it waits (two buffers) until the next iteration.  Meanwhile the
+// chunk-local prefix is taken and the chunk's entry count published; by the time
+// of its decoupled look-back the chunks before it have long published theirs, so
+// that rarely waits, and every thread then writes its row out.  Rows whose ranges
+// lie past the stages read HBM; a chunk with more ranges than its image holds is
+// resolved and written straight to C in its own iteration, merging a second time.
+// Reads A and B once, writes C once.
+//
+// Bound: instructions, most of them the merges' (lanes of a warp take as long as
+// the longest row).  Merging once instead of twice, the next chunk's ranges on
+// their way behind the pending one's write-out, and one stage for both operands
+// (8 CTAs an SM instead of 7): 614 -> 527 us for the banded sum of 2^23 rows,
+// 1.25 -> 1.66 instructions a cycle.  (Merging once alone: 602 us.)
 constexpr int kAddThreads = 128;
-constexpr int kAddStage = 6 * kAddThreads;   // ranges of each operand staged per chunk
-constexpr int kAddImage = 16 * kAddThreads;  // output entries of a chunk held in an image buffer
+constexpr int kAddImage = 8 * kAddThreads;   // ranges that a chunk's image has places for, and its stage
 constexpr unsigned long long kAddFlag = 1ull << 63;
 constexpr uint32_t kAddSpinLimit = 1u << 22;
 
 struct AddSmem {
-  uint2 a[kAddStage];
-  uint2 b[kAddStage];
-  uint2 img[2][kAddImage / 2];            // images of the counted and the pending chunk (ranges)
+  uint2 stage[kAddImage];                 // the chunk's ranges of A, then of B
+  uint2 img[2][kAddImage];                // results of the counted and the pending chunk, each row at its place
   uint32_t incl[2][kAddThreads];          // their chunk-local inclusive row counts
+  uint16_t at[2][kAddThreads];            // their rows' places
   unsigned long long arow[kAddThreads + 1];  // the chunk's row pointers (entry offsets)
   unsigned long long brow[kAddThreads + 1];
   uint32_t wsum[kAddThreads / 32];
@@ -312,6 +317,7 @@ struct SpaddChunkArgs {
   DeviceControl* ctl;
   uint64_t cap;              // entries C can hold
   uint32_t nrows, nchunks;
+  uint32_t chunk_rows;       // at most kAddThreads
   uint32_t spin_limit;       // polls a look-back waits before it gives up (0: kAddSpinLimit)
 };
 
@@ -377,11 +383,32 @@ __global__ void __launch_bounds__(kAddThreads) k_spadd_chunks(SpaddChunkArgs p) 
   add_sync();
   uint32_t t = S.next, b = 0;
   bool pend = false;  // a counted chunk waits in image buffer b ^ 1
+  bool pre = false;   // chunk t's row pointers and ranges were requested in the last iteration
+  auto rows_of = [&](uint32_t chunk) { return min(p.chunk_rows, p.nrows - chunk * p.chunk_rows); };
+  auto request_rows = [&](uint32_t chunk) {
+    const uint64_t c0 = uint64_t(chunk) * p.chunk_rows;
+    for (uint32_t k = tid; k <= rows_of(chunk); k += kAddThreads) {
+      add_cp8(&S.arow[k], p.a_rowmap + c0 + k);
+      if (!B_ID) add_cp8(&S.brow[k], p.b_rowmap + c0 + k);
+    }
+  };
+  // (rows start at even entries: a range is one 8-byte copy)
+  auto request_ranges = [&](uint32_t crows) {
+    const uint64_t abase = S.arow[0];
+    const uint32_t nas = uint32_t(min((S.arow[crows] - abase) / 2, (unsigned long long)kAddImage));
+    for (uint32_t k = tid; k < nas; k += kAddThreads) add_cp8(&S.stage[k], p.a_entries + abase + 2 * uint64_t(k));
+    if (!B_ID) {
+      const uint64_t bbase = S.brow[0];
+      const uint32_t nbs = uint32_t(min((S.brow[crows] - bbase) / 2, (unsigned long long)(kAddImage - nas)));
+      for (uint32_t k = tid; k < nbs; k += kAddThreads)
+        add_cp8(&S.stage[nas + k], p.b_entries + bbase + 2 * uint64_t(k));
+    }
+  };
   while (t < p.nchunks || pend) {
     const bool have = t < p.nchunks;
-    const uint32_t c0 = have ? t * uint32_t(kAddThreads) : 0u;
-    const uint32_t crows = have ? min(uint32_t(kAddThreads), p.nrows - c0) : 0u;
-    uint32_t cnt = 0, excl = 0, cnt_r = 0;
+    const uint32_t c0 = have ? t * p.chunk_rows : 0u;
+    const uint32_t crows = have ? rows_of(t) : 0u;
+    uint32_t cnt = 0, excl = 0, cnt_r = 0, taken = 0xffffffffu;
     bool imaged = false;
     const uint2* ap = nullptr;
     const uint2* bp = nullptr;
@@ -390,43 +417,56 @@ __global__ void __launch_bounds__(kAddThreads) k_spadd_chunks(SpaddChunkArgs p) 
     const uint32_t r = tid;
     const bool has = r < crows;
     if (have) {
-      // 1. the chunk's row pointers
-      for (uint32_t k = tid; k <= crows; k += kAddThreads) {
-        add_cp8(&S.arow[k], p.a_rowmap + uint64_t(c0) + k);
-        if (!B_ID) add_cp8(&S.brow[k], p.b_rowmap + uint64_t(c0) + k);
+      if (tid == 0) taken = atomicAdd(p.ticket, 1u);  // the next chunk (the reply comes while this one is merged)
+      // 1. the chunk's row pointers and ranges
+      if (!pre) {
+        request_rows(t);
+        add_cp_wait();
+        add_sync();
+        request_ranges(crows);
       }
       add_cp_wait();
       add_sync();
       const uint64_t abase = S.arow[0], bbase = B_ID ? 0 : S.brow[0];
       const uint64_t ra = (S.arow[crows] - abase) / 2, rb = B_ID ? 0 : (S.brow[crows] - bbase) / 2;
-      const uint32_t nas = ra < uint64_t(kAddStage) ? uint32_t(ra) : uint32_t(kAddStage);
-      const uint32_t nbs = rb < uint64_t(kAddStage) ? uint32_t(rb) : uint32_t(kAddStage);
-      // 2. their ranges (rows start at even entries: a range is one 8-byte copy)
-      for (uint32_t k = tid; k < nas; k += kAddThreads) add_cp8(&S.a[k], p.a_entries + abase + 2 * uint64_t(k));
-      if (!B_ID)
-        for (uint32_t k = tid; k < nbs; k += kAddThreads) add_cp8(&S.b[k], p.b_entries + bbase + 2 * uint64_t(k));
-      add_cp_wait();
-      add_sync();
-      // 3. count this thread's row
+      const uint32_t nas = uint32_t(min(ra, uint64_t(kAddImage)));
+      const uint32_t nbs = uint32_t(min(rb, uint64_t(kAddImage - nas)));
+      const uint2* const sb = S.stage + nas;
+      // 2. this thread's row, merged into its place: past the ranges of the rows before
+      const uint64_t places = ra + (B_ID ? crows : rb);
+      imaged = places <= uint64_t(kAddImage);
       if (has) {
         const uint64_t a0 = (S.arow[r] - abase) / 2, a1 = (S.arow[r + 1] - abase) / 2;
         na = uint32_t(a1 - a0);
-        ap = a1 <= nas ? S.a + a0 : reinterpret_cast<const uint2*>(p.a_entries + abase) + a0;
+        const uint2* const ga = reinterpret_cast<const uint2*>(p.a_entries + abase) + a0;
+        const uint2* gb = &id;
+        uint64_t b0 = r, b1 = r + 1;
         if (B_ID) {
           id = make_uint2(c0 + r, c0 + r);
-          bp = &id;
           nb = 1;
         } else {
-          const uint64_t b0 = (S.brow[r] - bbase) / 2, b1 = (S.brow[r + 1] - bbase) / 2;
+          b0 = (S.brow[r] - bbase) / 2;
+          b1 = (S.brow[r + 1] - bbase) / 2;
           nb = uint32_t(b1 - b0);
-          bp = b1 <= nbs ? S.b + b0 : reinterpret_cast<const uint2*>(p.b_entries + bbase) + b0;
+          gb = reinterpret_cast<const uint2*>(p.b_entries + bbase) + b0;
         }
-        spadd_row(reinterpret_cast<const uint32_t*>(ap), 2ull * na, reinterpret_cast<const uint32_t*>(bp), 2ull * nb, [&](uint32_t lo, uint32_t hi) {
-          cnt_r += 2;
-          nnz_cta += uint64_t(hi - lo) + 1;
-        });
+        ap = a1 <= nas ? S.stage + a0 : ga;
+        bp = B_ID ? &id : b1 <= nbs ? sb + b0 : gb;
+        const uint32_t place = uint32_t(a0 + b0);
+        if (imaged) S.at[b][r] = uint16_t(place);
+        auto merge = [&](const uint2* x, const uint2* y) {
+          uint32_t k = imaged ? place : 0u;
+          spadd_row(reinterpret_cast<const uint32_t*>(x), 2ull * na, reinterpret_cast<const uint32_t*>(y), 2ull * nb,
+                    [&](uint32_t lo, uint32_t hi) {
+                      if (imaged) S.img[b][k++] = make_uint2(lo, hi);
+                      cnt_r += 2;
+                      nnz_cta += uint64_t(hi - lo) + 1;
+                    });
+        };
+        if (!B_ID && a1 <= nas && b1 <= nbs) merge(S.stage + a0, sb + b0);  // (shared-memory loads)
+        else merge(ap, bp);
       }
-      // 4. chunk-local prefix; the aggregate for later chunks at once
+      // 3. chunk-local prefix; the aggregate for later chunks at once
       uint32_t incl = cnt_r;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -446,35 +486,41 @@ __global__ void __launch_bounds__(kAddThreads) k_spadd_chunks(SpaddChunkArgs p) 
       if (tid == 0) {
         asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p.desc + 2 * size_t(t)), "l"(kAddFlag | cnt)
                      : "memory");
-        S.next = atomicAdd(p.ticket, 1u);  // the next chunk, taken once this one is counted
+        S.next = taken;
       }
-      // 5. the chunk's image in buffer b (its inclusive row counts beside it)
-      imaged = cnt <= uint32_t(kAddImage);
-      if (imaged) {
-        S.incl[b][r] = excl + cnt_r;
-        if (has)
-          spadd_row(reinterpret_cast<const uint32_t*>(ap), 2ull * na, reinterpret_cast<const uint32_t*>(bp), 2ull * nb, [&, k = excl / 2](uint32_t lo, uint32_t hi) mutable {
-            S.img[b][k++] = make_uint2(lo, hi);
-          });
-      }
+      if (imaged) S.incl[b][r] = excl + cnt_r;
     }
-    // 6. the pending chunk (counted last iteration): look-back, row map, entries
+    // every thread is done with the stages (but for a chunk written in place
+    // below, whose successor is then not requested ahead); S.next is visible
+    add_sync();
+    const uint32_t next = have ? S.next : 0xffffffffu;
+    pre = imaged && next < p.nchunks;
+    // 4. the next chunk's row pointers come behind the pending chunk's look-back,
+    // its ranges behind the pending chunk's write-out
+    if (pre) request_rows(next);
+    const uint32_t pt = S.pend_t[b ^ 1u], prow = S.pend_rows[b ^ 1u], pcnt = S.pend_cnt[b ^ 1u];
+    if (pend && warp == 0) add_lookback(&S.prefix[0], p, pt, pcnt);
+    if (pre) add_cp_wait();
+    add_sync();
+    if (pre) request_ranges(rows_of(next));
+    // 5. the pending chunk (counted last iteration): row map, entries
     if (pend) {
-      const uint32_t pt = S.pend_t[b ^ 1u], prow = S.pend_rows[b ^ 1u], pcnt = S.pend_cnt[b ^ 1u];
-      if (warp == 0) add_lookback(&S.prefix[0], p, pt, pcnt);
-      add_sync();
       const unsigned long long prefix = S.prefix[0];
-      if (uint32_t(tid) < prow) p.c_rowmap[uint64_t(pt) * kAddThreads + tid + 1] = prefix + S.incl[b ^ 1u][tid];
+      if (uint32_t(tid) < prow) p.c_rowmap[uint64_t(pt) * p.chunk_rows + tid + 1] = prefix + S.incl[b ^ 1u][tid];
       if (pt == 0 && tid == 0) p.c_rowmap[0] = 0;
       if (prefix + pcnt <= p.cap) {
-        uint2* dst = reinterpret_cast<uint2*>(p.c_entries + prefix);  // prefix is even: 8-byte aligned
-        for (uint32_t k = tid; k < pcnt / 2; k += kAddThreads) dst[k] = S.img[b ^ 1u][k];
+        if (uint32_t(tid) < prow) {
+          const uint32_t o = tid ? S.incl[b ^ 1u][tid - 1] : 0u, n = (S.incl[b ^ 1u][tid] - o) / 2;
+          uint2* dst = reinterpret_cast<uint2*>(p.c_entries + prefix + o);  // (even: 8-byte aligned)
+          const uint2* src = S.img[b ^ 1u] + S.at[b ^ 1u][tid];
+          for (uint32_t k = 0; k < n; ++k) dst[k] = src[k];
+        }
       } else if (tid == 0 && pcnt) {
         atomicOr(&p.ctl->overflow, 1ull);
       }
       pend = false;
     }
-    // 7. a chunk whose output does not fit its image: resolved now, in place
+    // 6. a chunk whose output does not fit its image: resolved now, in place
     if (have && !imaged) {
       if (warp == 0) add_lookback(&S.prefix[1], p, t, cnt);
       add_sync();
@@ -491,6 +537,7 @@ __global__ void __launch_bounds__(kAddThreads) k_spadd_chunks(SpaddChunkArgs p) 
           k += 2;
         });
       }
+      add_sync();  // (its stages are free for the next chunk)
     }
     if (have && imaged) {
       if (tid == 0) {
@@ -501,10 +548,7 @@ __global__ void __launch_bounds__(kAddThreads) k_spadd_chunks(SpaddChunkArgs p) 
       pend = true;
       b ^= 1u;
     }
-    // every thread is done with the stages and the images it needs; S.next
-    // (written after the prefix) and the pending record are visible
-    add_sync();
-    t = have ? S.next : 0xffffffffu;
+    t = next;
   }
   // the product's nnz: one atomic per CTA
 #pragma unroll
@@ -786,18 +830,30 @@ void launch_spadd(dvg_context* ctx, const dvg_matrix* a, const dvg_matrix* b, bo
   ctx->stats.kernel_launches++;
 }
 
-uint64_t spadd_single_pass_scratch(uint32_t nrows) {
-  const uint64_t nchunks = (uint64_t(nrows) + kAddThreads - 1) / kAddThreads;
-  return nchunks * 16 + 256;
+// Rows of a chunk: one a thread, or half as many, and so on, where a chunk would
+// have more ranges than its image on average -- its rows are then merged in place
+// and wait for their offset.  2^20 rows of 8.8, 17.7 and 53 ranges of each operand
+// (64, 16 and 8 rows a chunk): 488 -> 272, 1456 -> 579 and, for 2^19, 3976 -> 979 us.
+static uint32_t add_chunk_rows(const dvg_matrix* a, const dvg_matrix* b, bool b_identity) {
+  const uint64_t n = a->nrows, ranges = (a->nentries + (b_identity ? 2 * n : b->nentries)) / 2;
+  uint32_t rows = kAddThreads;
+  while (rows > 1 && ranges * rows > n * (8ull * kAddImage / 9)) rows /= 2;
+  return ranges * rows > n * (8ull * kAddImage / 9) ? uint32_t(kAddThreads) : rows;
+}
+
+uint64_t spadd_single_pass_scratch(const dvg_matrix* a, const dvg_matrix* b, bool b_identity) {
+  const uint32_t rows = add_chunk_rows(a, b, b_identity);
+  return (uint64_t(a->nrows) + rows - 1) / rows * 16 + 256;
 }
 
 void launch_spadd_single_pass(dvg_context* ctx, const dvg_matrix* a, const dvg_matrix* b, bool b_identity,
                               uint64_t* c_rowmap, uint32_t* c_entries, uint64_t cap, void* scratch) {
   const uint32_t n = a->nrows;
   if (n == 0) return;
-  const uint32_t nchunks = uint32_t((uint64_t(n) + kAddThreads - 1) / kAddThreads);
+  const uint32_t chunk_rows = add_chunk_rows(a, b, b_identity);
+  const uint32_t nchunks = uint32_t((uint64_t(n) + chunk_rows - 1) / chunk_rows);
   // per chunk 16 bytes of descriptors, then the ticket
-  DVG_CUDA(cudaMemsetAsync(scratch, 0, spadd_single_pass_scratch(n), ctx->stream));
+  DVG_CUDA(cudaMemsetAsync(scratch, 0, size_t(nchunks) * 16 + 4, ctx->stream));
   SpaddChunkArgs p{};
   p.a_rowmap = a->rowmap;
   p.a_entries = a->entries;
@@ -811,6 +867,7 @@ void launch_spadd_single_pass(dvg_context* ctx, const dvg_matrix* a, const dvg_m
   p.cap = cap;
   p.nrows = n;
   p.nchunks = nchunks;
+  p.chunk_rows = chunk_rows;
   const int smem = int(sizeof(AddSmem));
   DVG_CUDA(cudaFuncSetAttribute(k_spadd_chunks<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   DVG_CUDA(cudaFuncSetAttribute(k_spadd_chunks<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));

@@ -600,3 +600,25 @@ def test_random_read_calibration(ctx):
     a, _ = gen.graph_adjacency(gen.small_graph_spec(20_000, seed=334))
     pairs = np.array([[k, k + 1] for k in range(0, 2000, 7)], np.uint32)
     assert np.array_equal(ctx.query(ctx.upload(a), pairs), orc.query(omat(a), pairs))
+
+
+@pytest.mark.parametrize("ranges", [1.0, 4.5, 7.0, 14.0, 28.0, 60.0, 120.0, 250.0, 450.0, 1200.0])
+@pytest.mark.parametrize("n", [2, 37, 5000])
+def test_spadd_chunks_of_fewer_rows(ctx, n, ranges):
+    # the denser the rows, the fewer a chunk of the one-pass sum takes (128 down
+    # to 1, and past that 128 merged in place); the last chunk is ragged, and some
+    # rows hold several times the average
+    a = gen.banded(n, 6000, ranges, 1.0, seed=90)
+    b = gen.banded(n, 6000, ranges / 3, 1.0, seed=91)
+    want = orc.spadd(omat(a), omat(b))
+    assert_same(ctx.spadd(ctx.upload(a), ctx.upload(b)).download(), want.rowmap, want.entries, want.nnz)
+    # a few rows full, the rest empty: chunks far from the average
+    k = max(1, n // 50)
+    full = np.arange(0, 2 * n, 2, dtype=np.uint32)
+    rowmap = np.zeros(n + 1, np.uint64)
+    rowmap[-k:] = 2 * n * np.arange(1, k + 1, dtype=np.uint64)
+    m = CRSMatrix(2 * n, np.tile(np.repeat(full, 2), k), rowmap)
+    o = CRSMatrix(2 * n, np.tile(np.repeat(full + 1, 2), k)[:0], np.zeros(n + 1, np.uint64))
+    for x, y in ((m, o), (o, m), (m, m)):
+        want = orc.spadd(omat(x), omat(y))
+        assert_same(ctx.spadd(ctx.upload(x), ctx.upload(y)).download(), want.rowmap, want.entries, want.nnz)
