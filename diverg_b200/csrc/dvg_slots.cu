@@ -288,8 +288,14 @@ __device__ __noinline__ uint32_t list_product(const uint2* __restrict__ arena, c
 // The quick form of a walk.  The columns that a row's S_j holds lie close
 // together -- the ends of paths of one length -- so they are a 64-bit mask from
 // a base column, and a product ORs the named rows' ranges into the next mask.
-// c's row is at most two runs in registers.  Writes the runs of s and c to the
-// lists; false where the row does not fit.
+// A product's loads -- the named rows of the factor and, where c takes S_j, of B --
+// are requested together, two columns at a time, so a factor is one trip to memory
+// for most rows, and one copy of the code handles the columns in turn.  The walk of
+// a row is a chain of such trips, and the slowest warp's chain bounds a small pass.
+// (Against a separate form for rows of a single column, then two trips a factor:
+// 238 -> 220 us for A^10 at 1e6 nodes, 193 -> 178 for the build at 1e5; 3, 4 and 6
+// columns at a time cost up to 6 % more.)  c's row is at most two runs in registers.
+// Writes the runs of s and c to the lists; false where the row does not fit.
 template <bool OUTS, bool OUTC>
 __device__ __forceinline__ bool quick_row(const ChainArgs& p, uint32_t row, uint2* Ls, uint32_t& ns, uint2* Lc,
                                           uint32_t& nc) {
@@ -303,7 +309,7 @@ __device__ __forceinline__ bool quick_row(const ChainArgs& p, uint32_t row, uint
       r0 = v;
     } else if (unite(r0, v)) {
       if (unite(r0, r1)) r1 = empty_slot();
-    } else if (r1.x > r1.y) {
+    } else if (!is_run(r1)) {
       r1 = r0;
       r0 = v;
     } else if (unite(r1, v)) {
@@ -312,65 +318,60 @@ __device__ __forceinline__ bool quick_row(const ChainArgs& p, uint32_t row, uint
       ok = false;
     }
   };
-  // the ranges of the rows of `mat` that the mask names, four rows at a time so
-  // that their loads are in flight together
-  auto each = [&](const uint2* __restrict__ mat, auto&& f) {
-    for (unsigned long long w = mask; w;) {
-      uint2 s[kAhead];
-#pragma unroll
-      for (int q = 0; q < kAhead; ++q) {
-        s[q] = empty_slot();
-        if (w) {
-          s[q] = ld_slot(mat, base + uint32_t(__ffsll(w) - 1));
-          w &= w - 1;
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < kAhead; ++q) {
-        const uint32_t c = slot_count(s[q]);
-        for (uint32_t t = 0; t < c; ++t) f(slot_range(p.arena, s[q], t));
-      }
-    }
-  };
-  auto add_slot = [&](uint2 s) {
-    const uint32_t c = slot_count(s);
-    for (uint32_t t = 0; t < c; ++t) add_c(slot_range(p.arena, s, t));
-  };
-  // while the row is a single column
-  uint32_t j = 0;
 #pragma unroll 1
-  for (; j < p.k; ++j) {
-    const uint2 s = ld_slot(p.m[j], base);
-    if (OUTC && ((p.bits >> j) & 1u)) add_slot(p.b ? ld_slot(p.b, base) : make_uint2(base, base));
-    if (s.x != s.y) break;
-    base = s.x;
-  }
-  const uint32_t single = j;  // c has its part of S_0 .. S_(single - 1), and of S_single but for j = k
-#pragma unroll 1
-  for (; ok; ++j) {
-    if (OUTC && ((p.bits >> j) & 1u) && (j != single || j == p.k)) {
-      if (p.b) {
-        each(p.b, add_c);
-      } else {
-        for (unsigned long long w = mask; w;) {
-          const int lo = __ffsll(w) - 1, n = __ffsll(~(w >> lo)) - 1;  // (n < 0: all 64 columns)
-          const int hi = n < 0 ? 63 : lo + n - 1;
-          add_c(make_uint2(base + lo, base + hi));
-          w &= hi < 63 ? ~0ull << (hi + 1) : 0ull;
-        }
-      }
-    }
-    if (j == p.k) break;
+  for (uint32_t j = 0;; ++j) {
+    const bool gather = OUTC && ((p.bits >> j) & 1u), go = j < p.k;
+    if (!gather && !go) break;
+    const uint2* __restrict__ mat = go ? p.m[j] : nullptr;
     unsigned long long to = 0;
     uint32_t from = 0;
-    each(p.m[j], [&](uint2 v) {
+    auto add_s = [&](uint2 v) {
       if (!to) from = v.x > 16 ? v.x - 16 : 0;  // later rows may start a little before the first
-      if (v.x < from || v.y - from > 63) {
+      const uint32_t lo = v.x - from, hi = v.y - from;
+      if (lo > 63 || hi > 63) {
         ok = false;
         return;
       }
-      to |= (~0ull << (v.x - from)) & (~0ull >> (63 - (v.y - from)));
-    });
+      to |= (~0ull << lo) & (~0ull >> (63 - hi));
+    };
+    for (unsigned long long w = mask; w;) {
+      uint32_t x[kAhead];
+      uint2 sm[kAhead], sb[kAhead];
+      int n = 0;
+#pragma unroll
+      for (int q = 0; q < kAhead; ++q) {
+        x[q] = base + uint32_t(__ffsll(w) - 1);
+        n += w ? 1 : 0;
+        w &= w - 1;
+      }
+#pragma unroll
+      for (int q = 0; q < kAhead; ++q) {
+        sm[q] = go && q < n ? ld_slot(mat, x[q]) : empty_slot();
+        sb[q] = gather && q < n ? (p.b ? ld_slot(p.b, x[q]) : make_uint2(x[q], x[q])) : empty_slot();
+      }
+#pragma unroll 1
+      for (int q = 0; q < n; ++q) {  // (one copy of the code for the columns in turn)
+        const uint2 s = sm[0], b = sb[0];
+#pragma unroll
+        for (int i = 0; i + 1 < kAhead; ++i) {
+          sm[i] = sm[i + 1];
+          sb[i] = sb[i + 1];
+        }
+        if (is_run(s)) {
+          add_s(s);
+        } else {
+          const uint32_t c = slot_count(s);
+          for (uint32_t t = 0; t < c; ++t) add_s(slot_range(p.arena, s, t));
+        }
+        if (is_run(b)) {
+          add_c(b);
+        } else {
+          const uint32_t c = slot_count(b);
+          for (uint32_t t = 0; t < c; ++t) add_c(slot_range(p.arena, b, t));
+        }
+      }
+    }
+    if (!go || !ok) break;
     mask = to;
     base = from;
   }
@@ -378,7 +379,7 @@ __device__ __forceinline__ bool quick_row(const ChainArgs& p, uint32_t row, uint
   if (OUTS) {
     ns = 0;
     for (unsigned long long w = mask; w;) {
-      const int lo = __ffsll(w) - 1, n = __ffsll(~(w >> lo)) - 1;
+      const int lo = __ffsll(w) - 1, n = __ffsll(~(w >> lo)) - 1;  // (n < 0: all 64 columns)
       const int hi = n < 0 ? 63 : lo + n - 1;
       if (ns == uint32_t(kSRuns)) return false;
       Ls[ns++ * 32] = make_uint2(base + lo, base + hi);
@@ -386,14 +387,14 @@ __device__ __forceinline__ bool quick_row(const ChainArgs& p, uint32_t row, uint
     }
   }
   if (OUTC) {
-    if (r1.x <= r1.y && r1.x < r0.x) {
+    if (is_run(r1) && r1.x < r0.x) {
       const uint2 t = r0;
       r0 = r1;
       r1 = t;
     }
     nc = 0;
-    if (r0.x <= r0.y) Lc[nc++ * 32] = r0;
-    if (r1.x <= r1.y) Lc[nc++ * 32] = r1;
+    if (is_run(r0)) Lc[nc++ * 32] = r0;
+    if (is_run(r1)) Lc[nc++ * 32] = r1;
   }
   return true;
 }
