@@ -361,6 +361,7 @@ static dvg_matrix* range_spgemm_fused(dvg_context* ctx, const dvg_matrix* a, boo
         if (e != cudaSuccess) dfree(ctx, exact);
         DVG_CUDA(e);
       }
+      DVG_CUDA(cudaStreamSynchronize(ctx->stream));  // the caller waits no more
       dfree(ctx, c->entries);
       c->entries = exact;
     }
@@ -654,7 +655,8 @@ static dvg_matrix* distance_index_powersum(dvg_context* ctx, const dvg_matrix* a
   }
 }
 
-dvg_matrix* create_distance_index(dvg_context* ctx, const dvg_matrix* a, unsigned dlo, unsigned dup) {
+dvg_matrix* create_distance_index(dvg_context* ctx, const dvg_matrix* a, unsigned dlo, unsigned dup,
+                                  bool* settled) {
   require(dlo <= dup && dup != 0, "create_distance_index: requires dmin <= dmax and dmax != 0");
   require(a->nrows == a->ncols, "create_distance_index: adjacency matrix is not square");
   // the sum-of-powers schedule ends on SpAdds when dlo == 0; those keep rows
@@ -662,7 +664,7 @@ dvg_matrix* create_distance_index(dvg_context* ctx, const dvg_matrix* a, unsigne
   // canonicalise any input
   if (ctx->opt_dindex_schedule == 1 || (dlo == 0 && !a->canonical)) return distance_index_reference(ctx, a, dlo, dup);
   if (ctx->opt_planned && ctx->opt_spgemm_mode == 0 && slots_suit(ctx, a)) {
-    if (dvg_matrix* t = slots_chain(ctx, a, dlo, dup)) return t;
+    if (dvg_matrix* t = slots_chain(ctx, a, dlo, dup, settled)) return t;
     ctx->stats.spgemm_reruns++;
   }
   if (ctx->opt_planned && ctx->opt_spgemm_mode != 1 && a->nrows > 0) {
@@ -1064,9 +1066,18 @@ dvg_status dvg_range_spgemm(dvg_context* ctx, const dvg_matrix* a, const dvg_mat
   return guarded([&] {
     Lock lk(ctx);
     require(a && b && c, "null argument");
-    dvg_matrix* r = range_spgemm(ctx, a, false, b);
+    dvg_matrix* r = nullptr;
+    bool settled = false;
+    if (ctx->opt_planned && ctx->opt_spgemm_mode == 0 && slots_product_suits(ctx, a, b)) {
+      r = slots_product(ctx, a, b, &settled);
+      if (!r) ctx->stats.spgemm_reruns++;
+    }
+    if (!r) {
+      r = range_spgemm(ctx, a, false, b);  // (has read its counters, after its last kernel)
+      settled = true;
+    }
     try {
-      read_control(ctx);
+      if (!settled) read_control(ctx);
     } catch (...) {
       free_matrix(ctx, r);
       throw;
@@ -1083,13 +1094,14 @@ dvg_status dvg_range_power(dvg_context* ctx, const dvg_matrix* a, unsigned k, dv
     // (1e6 loci of a variant-dense graph, k = 100: 0.87 -> 0.25 ms); with k = 1
     // there is a single product, and with k = 0 none
     dvg_matrix* r = nullptr;
+    bool settled = false;
     if (k > 1 && ctx->opt_planned && ctx->opt_spgemm_mode == 0 && slots_suit(ctx, a)) {
-      r = slots_chain(ctx, a, k, k);
+      r = slots_chain(ctx, a, k, k, &settled);
       if (!r) ctx->stats.spgemm_reruns++;
     }
     if (!r) r = range_power(ctx, a, k);
     try {
-      read_control(ctx);
+      if (!settled) read_control(ctx);
     } catch (...) {
       free_matrix(ctx, r);
       throw;
@@ -1141,9 +1153,10 @@ dvg_status dvg_create_distance_index(dvg_context* ctx, const dvg_matrix* ra, uns
   return guarded([&] {
     Lock lk(ctx);
     require(ra && out, "null argument");
-    dvg_matrix* r = create_distance_index(ctx, ra, dmin, dmax);
+    bool settled = false;
+    dvg_matrix* r = create_distance_index(ctx, ra, dmin, dmax, &settled);
     try {
-      read_control(ctx);
+      if (!settled) read_control(ctx);
     } catch (...) {
       free_matrix(ctx, r);
       throw;

@@ -268,7 +268,9 @@ void selftest_bounded_wait(dvg_context* ctx, uint32_t spin_limit);
 dvg_matrix* range_spgemm(dvg_context* ctx, const dvg_matrix* a, bool a_identity, const dvg_matrix* b);
 dvg_matrix* range_spadd(dvg_context* ctx, const dvg_matrix* a, const dvg_matrix* b, bool b_identity);
 dvg_matrix* range_power(dvg_context* ctx, const dvg_matrix* a, unsigned k);
-dvg_matrix* create_distance_index(dvg_context* ctx, const dvg_matrix* a, unsigned dlo, unsigned dup);
+// Sets *settled where the result's kernels have ended and been checked.
+dvg_matrix* create_distance_index(dvg_context* ctx, const dvg_matrix* a, unsigned dlo, unsigned dup,
+                                  bool* settled = nullptr);
 // Host range-CRS -> device (H2D, validation with one read-back).
 dvg_matrix* upload_matrix(dvg_context* ctx, uint32_t nrows, uint32_t ncols, const uint64_t* rowmap,
                           const uint32_t* entries, uint64_t nnz);

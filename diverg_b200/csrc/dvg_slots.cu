@@ -46,6 +46,16 @@ constexpr uint32_t kMultiMax = 0xFFFFFFFFu - kMulti - 1;  // ranges of one row
 constexpr uint32_t kCountRows = 32 * kSRows;  // rows whose ranges the last pass counts together
 constexpr uint32_t kSmallRows = 1u << 17;     // rows up to which a pass is one kernel
 constexpr double kChainReach = 1.28;          // branching * steps of a pass's left factors
+// A result of up to so many rows gets room for two ranges a row and is written
+// before its size is known, so that the host waits once.  A second wait and the
+// gap before it are 20 us: from 2^24 rows on, under 3 % of a product.
+constexpr uint32_t kEarlyRows = 1u << 24;
+// A single product goes through slots from so many rows on.  The conversions are
+// launches of their own, 3 to 7 us more than the row kernel's one at 1e4 rows, equal
+// at 2e4; A^2 of a sequence graph's A takes 39 in place of 62 us at 1e5 rows, 54 of
+// 83 at 1e6, 166 of 223 at 1e7 and 546 of 785 at 4e7.  With two different factors,
+// both converted: 41, 58, 218 and 732 us against 63, 83, 233 and 823.
+constexpr uint32_t kProductRows = 3u << 13;
 constexpr int kCrsRows = kSlotPartRows;        // rows of a block of the conversions
 constexpr uint32_t kSuperGroups = 512;        // counts that k_slot_sums adds up
 
@@ -1140,6 +1150,7 @@ SlotBuild prepare_slots(dvg_context* ctx, const SlotPlan& plan, uint32_t n) {
   sb.arena_cap = std::min<uint64_t>(uint64_t(ctx->slot_growth * double(n)) + 4096, kMulti);
   const double room = 0.5 * double(device_free_bytes(ctx) + ctx->cached_bytes);
   if (double(sb.arena_cap) * 8.0 > room) sb.arena_cap = uint64_t(room / 8.0) + 4096;
+  if (n <= kEarlyRows && 16.0 * double(n) < room / 8.0) sb.early = 2ull * n;
   // a matrix takes the buffer of one whose last reader is an earlier pass (the
   // chain's own buffers only: chains that run side by side share none)
   std::vector<uint2*> spare;
@@ -1162,7 +1173,7 @@ SlotBuild prepare_slots(dvg_context* ctx, const SlotPlan& plan, uint32_t n) {
     sb.group_cnt = reinterpret_cast<uint32_t*>(base + cnt_off);
     sb.masks = reinterpret_cast<uint32_t*>(base + masks_off);
     sb.arena = static_cast<uint2*>(dalloc(ctx, sb.arena_cap * sizeof(uint2)));
-    take(0);
+    for (int k = 0; k < plan.inputs; ++k) take(k);
     for (size_t i = 0; i < plan.steps.size(); ++i) {
       if (plan.steps[i].s >= 0) take(plan.steps[i].s);
       if (plan.steps[i].c >= 0) take(plan.steps[i].c);
@@ -1188,7 +1199,7 @@ void release_slots(dvg_context* ctx, SlotBuild& sb) {
   sb.scratch = nullptr;
 }
 
-void launch_slots(dvg_context* ctx, SlotBuild& sb, const SlotParts& parts, bool timed) {
+void launch_slots(dvg_context* ctx, SlotBuild& sb, const SlotParts& parts, bool timed, const SlotPart* right) {
   const uint64_t t0 = now_ns();
   DVG_CUDA(cudaMemsetAsync(sb.scratch, 0, 512, ctx->stream));
   ctx->stats.kernel_launches++;
@@ -1206,6 +1217,12 @@ void launch_slots(dvg_context* ctx, SlotBuild& sb, const SlotParts& parts, bool 
   k_crs_to_slots<<<conversion_blocks(sb), kSThreads, 0, ctx->stream>>>(Parts{parts.table, parts.part_of, parts.one}, p);
   DVG_CUDA(cudaGetLastError());
   ctx->stats.kernel_launches++;
+  if (right) {
+    p.s = sb.mat[1];
+    k_crs_to_slots<<<conversion_blocks(sb), kSThreads, 0, ctx->stream>>>(Parts{nullptr, nullptr, *right}, p);
+    DVG_CUDA(cudaGetLastError());
+    ctx->stats.kernel_launches++;
+  }
   for (size_t i = 0; i < sb.plan.steps.size(); ++i) {
     const SlotStep& st = sb.plan.steps[i];
     p.k = uint32_t(st.k);
@@ -1237,9 +1254,10 @@ void launch_slots_totals(dvg_context* ctx, const SlotBuild& sb, const SlotParts&
   ctx->stats.kernel_launches++;
 }
 
-void launch_slots_out(dvg_context* ctx, const SlotBuild& sb, const SlotParts& parts) {
+void launch_slots_out(dvg_context* ctx, const SlotBuild& sb, const SlotParts& parts, DeviceControl* ctl) {
   k_slots_to_crs<<<conversion_blocks(sb), kSThreads, 0, ctx->stream>>>(
-      Parts{parts.table, parts.part_of, parts.one}, sb.mat[sb.plan.out], sb.arena, sb.sums, sb.group_cnt, ctx->d_ctl);
+      Parts{parts.table, parts.part_of, parts.one}, sb.mat[sb.plan.out], sb.arena, sb.sums, sb.group_cnt,
+      ctl ? ctl : ctx->d_ctl);
   DVG_CUDA(cudaGetLastError());
   ctx->stats.kernel_launches++;
 }
@@ -1277,10 +1295,19 @@ bool check_slots(dvg_context* ctx, const SlotBuild& sb, const SlotCounters& c) {
   return true;
 }
 
-dvg_matrix* slots_chain(dvg_context* ctx, const dvg_matrix* a, unsigned dlo, unsigned dup) {
+static SlotPart whole(const dvg_matrix* a) {
+  SlotPart p{};
+  p.rowmap = a->rowmap;
+  p.entries = a->entries;
+  p.n = a->nrows;
+  return p;
+}
+
+static dvg_matrix* run_slots(dvg_context* ctx, const SlotPlan& plan, const dvg_matrix* a, const dvg_matrix* b,
+                             bool* settled) {
   SlotBuild sb;
   try {
-    sb = prepare_slots(ctx, plan_slots(dlo, dup, branching(a->nnz, a->nrows)), a->nrows);
+    sb = prepare_slots(ctx, plan, a->nrows);
   } catch (const Error& e) {
     if (e.status != DVG_ERR_OOM) throw;
     return nullptr;
@@ -1288,10 +1315,22 @@ dvg_matrix* slots_chain(dvg_context* ctx, const dvg_matrix* a, unsigned dlo, uns
   dvg_matrix* m = nullptr;
   try {
     SlotParts parts{};
-    parts.one.rowmap = a->rowmap;
-    parts.one.entries = a->entries;
-    parts.one.n = a->nrows;
-    launch_slots(ctx, sb, parts, ctx->opt_timing);
+    parts.one = whole(a);
+    const SlotPart right = b ? whole(b) : SlotPart{};
+    launch_slots(ctx, sb, parts, ctx->opt_timing, b ? &right : nullptr);
+    auto out = [&](uint64_t ranges, DeviceControl* ctl) {
+      m = new_matrix(ctx, a->nrows, a->ncols, 2 * ranges);
+      m->canonical = true;
+      parts.one.c_rowmap = m->rowmap;
+      parts.one.c_entries = m->entries;
+      parts.one.c_ranges = ranges;
+      launch_slots_out(ctx, sb, parts, ctl);
+    };
+    try {
+      if (sb.early) out(sb.early, sb.ctl);
+    } catch (const Error& e) {
+      if (e.status != DVG_ERR_OOM) throw;
+    }
     auto* h = static_cast<SlotCounters*>(host_stage(ctx, sizeof(SlotCounters)));
     DVG_CUDA(cudaMemcpyAsync(h, sb.scratch, sizeof(SlotCounters), cudaMemcpyDeviceToHost, ctx->stream));
     const uint64_t t0 = now_ns();
@@ -1300,14 +1339,21 @@ dvg_matrix* slots_chain(dvg_context* ctx, const dvg_matrix* a, unsigned dlo, uns
     ctx->stats.host_syncs++;
     resolve_spans(ctx);
     const SlotCounters c = *h;
-    if (check_slots(ctx, sb, c)) {
-      m = new_matrix(ctx, a->nrows, a->ncols, c.ctl.total);
+    const bool whole_chain = check_slots(ctx, sb, c);
+    if (m && (!whole_chain || c.ctl.total > m->nentries)) {
+      free_matrix(ctx, m);
+      m = nullptr;
+    }
+    if (m) {
+      if (c.ctl.status)
+        throw Error(DVG_ERR_DEVICE, "row slots: a result and its counts differ (code " + std::to_string(c.ctl.status) + ")");
+      if (settled) *settled = true;
+    } else if (whole_chain) {
+      out(c.ctl.total / 2, nullptr);
+    }
+    if (m) {
+      m->nentries = c.ctl.total;
       m->nnz = c.ctl.nnz;
-      m->canonical = true;
-      parts.one.c_rowmap = m->rowmap;
-      parts.one.c_entries = m->entries;
-      parts.one.c_ranges = m->nentries / 2;
-      launch_slots_out(ctx, sb, parts);
     }
   } catch (...) {
     free_matrix(ctx, m);
@@ -1316,6 +1362,29 @@ dvg_matrix* slots_chain(dvg_context* ctx, const dvg_matrix* a, unsigned dlo, uns
   }
   release_slots(ctx, sb);
   return m;
+}
+
+dvg_matrix* slots_chain(dvg_context* ctx, const dvg_matrix* a, unsigned dlo, unsigned dup, bool* settled) {
+  return run_slots(ctx, plan_slots(dlo, dup, branching(a->nnz, a->nrows)), a, nullptr, settled);
+}
+
+bool slots_product_suits(const dvg_context* ctx, const dvg_matrix* a, const dvg_matrix* b) {
+  return a->nrows >= kProductRows && a->nrows == b->nrows && slots_suit(ctx, a) && slots_suit(ctx, b);
+}
+
+dvg_matrix* slots_product(dvg_context* ctx, const dvg_matrix* a, const dvg_matrix* b, bool* settled) {
+  SlotPlan pl;
+  pl.inputs = a == b ? 1 : 2;
+  pl.out = pl.inputs;
+  pl.nmats = pl.inputs + 1;
+  SlotStep st;  // c = S_1 B, S_1 = A
+  st.k = 1;
+  st.m[0] = 0;
+  st.b = pl.inputs - 1;
+  st.bits = 2;
+  st.c = pl.out;
+  pl.steps.push_back(st);
+  return run_slots(ctx, pl, a, a == b ? nullptr : b, settled);
 }
 
 }  // namespace dvg

@@ -12,7 +12,7 @@ constexpr int kChainMax = 6;  // left factors of one pass
 
 // One pass over the rows: with S_0 = I and S_(j+1) = S_j m[j], s = S_k and
 // c = union of S_j b over the set bits j (b = -1: the identity).  Matrices are
-// numbered, 0 is the input; -1: no such output.
+// numbered, the inputs first; -1: no such output.
 struct SlotStep {
   int k = 0;
   int m[kChainMax] = {-1, -1, -1, -1, -1, -1};
@@ -22,6 +22,7 @@ struct SlotStep {
 };
 struct SlotPlan {
   std::vector<SlotStep> steps;
+  int inputs = 1;
   int nmats = 1;
   int out = 0;
 };
@@ -64,6 +65,7 @@ struct SlotBuild {
   std::vector<uint2*> buffers; // theirs
   uint2* arena = nullptr;
   uint64_t arena_cap = 0;      // ranges
+  uint64_t early = 0;          // room for the result's ranges before their number is known; 0: none
   void* scratch = nullptr;     // counters | sums of the counts | counts of the result | bitmap
   DeviceControl* ctl = nullptr;
   unsigned long long* top = nullptr;
@@ -76,22 +78,29 @@ struct SlotBuild {
 
 // Allocates what the chain needs (no device work beyond stream-ordered
 // allocation); issues it (no host round trip: it may be captured).
+// A plan of two inputs takes `right` as its second.
 SlotBuild prepare_slots(dvg_context* ctx, const SlotPlan& plan, uint32_t n);
-void launch_slots(dvg_context* ctx, SlotBuild& sb, const SlotParts& parts, bool timed);
+void launch_slots(dvg_context* ctx, SlotBuild& sb, const SlotParts& parts, bool timed, const SlotPart* right = nullptr);
 // Ranges and columns of each part's result (device, two words a part), once
 // the chain has run.
 void launch_slots_totals(dvg_context* ctx, const SlotBuild& sb, const SlotParts& parts, uint32_t nparts,
                          unsigned long long* totals);
-// The parts' results, into the arrays that the table now names.
-void launch_slots_out(dvg_context* ctx, const SlotBuild& sb, const SlotParts& parts);
+// The parts' results, into the arrays that the table now names; `ctl` (null: the
+// context's) takes a status where an array is too small.
+void launch_slots_out(dvg_context* ctx, const SlotBuild& sb, const SlotParts& parts, DeviceControl* ctl = nullptr);
 // Books a finished chain's counters; false when its arena ran full and there is
 // no result.
 bool check_slots(dvg_context* ctx, const SlotBuild& sb, const SlotCounters& c);
 void release_slots(dvg_context* ctx, SlotBuild& sb);
 
-// The chain over `a`, waited for once (for the result's size); null when it did
-// not fit its arena.
-dvg_matrix* slots_chain(dvg_context* ctx, const dvg_matrix* a, unsigned dlo, unsigned dup);
+// The chain over `a`, waited for once; null when it did not fit its arena.  Sets
+// *settled where that wait has seen all of the result's kernels end, and checked them.
+dvg_matrix* slots_chain(dvg_context* ctx, const dvg_matrix* a, unsigned dlo, unsigned dup, bool* settled);
+
+// A B alone, where that is faster than the range-CRS row kernel; null and
+// *settled likewise.
+bool slots_product_suits(const dvg_context* ctx, const dvg_matrix* a, const dvg_matrix* b);
+dvg_matrix* slots_product(dvg_context* ctx, const dvg_matrix* a, const dvg_matrix* b, bool* settled);
 
 // Columns of a row beyond its first, on average: how fast rows leave the single column.
 inline double branching(uint64_t nnz, uint64_t nrows) {

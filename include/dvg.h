@@ -99,9 +99,10 @@ dvg_status dvg_synchronize(dvg_context* ctx);
  * default; 1 = the reference's squaring of A + I; both give the same index),
  * "planned_build" (1 = index builds run as a planned sequence of products with
  * pre-allocated buffers and no host round trip between them, the default; 0 =
- * one read-back per product), "row_slots" (1 = planned builds and powers of graph-like
- * input -- canonical rows, at most 1.5 ranges a row and two columns a range on
- * average -- run as passes over matrices of one 8-byte slot a row, the default;
+ * one read-back per product), "row_slots" (1 = planned builds, powers, and
+ * products of 24,576 rows or more, of graph-like input -- canonical rows, at most
+ * 1.5 ranges a row and two columns a range on average -- run as passes over
+ * matrices of one 8-byte slot a row, the default;
  * 0 = every product in range CRS), "plan_growth" (planned builds: the entry
  * capacity of every step as a percentage of the input's entries, 300 by
  * default and adapted after each build; a step that outgrows it makes the

@@ -149,3 +149,57 @@ def test_a_batch_of_chains_beside_range_crs_builds(ctx):
             m = got[k].download()
             assert np.array_equal(m.rowmap, want.rowmap) and np.array_equal(m.entries, want.entries), (k, w)
             assert m.nnz() == want.nnz, (k, w)
+
+
+def product_forms(n, seed):
+    """Factors that single products take in slots, and their neighbours that they
+    do not: a row of several short ranges, rows split or out of order, ranges of
+    12 columns, a wide matrix."""
+    a = rows(graph(), n)
+    yield "square", a, a, True
+    yield "another factor", a, gen.banded(n, 50, 1.2, 1.2, seed=seed), True
+    yield "and before it", gen.banded(n, 50, 1.2, 1.2, seed=seed), a, True
+    yield "dense left", gen.random_matrix(n, 3 * n, seed=seed + 1), a, False
+    yield "dense right", a, gen.banded(n, 200, 1.0, 12.0, seed=seed + 2), False
+    i = np.arange(n - 1, dtype=np.uint32)  # [i, i], and in every third row [i + 1, i + 1] beside it
+    both = np.stack([i, i, i + 1, i + 1], 1)
+    entries = both[np.repeat((i % 3 == 0)[:, None], 4, 1) | np.array([True, True, False, False])]
+    at = np.concatenate(([0], np.cumsum(np.where(i % 3 == 0, 4, 2)))).astype(np.uint64)
+    yield "split rows", CRSMatrix(n, entries, np.append(at, at[-1])), a, False
+
+
+@pytest.mark.parametrize("n", [24_575, 24_576, 24_577, 33_023, 131_072, 131_073])
+def test_single_products(ctx, n):
+    for what, a, b, slots in product_forms(n, 71):
+        da = ctx.upload(a)
+        db = da if b is a else ctx.upload(b)
+        want = orc.spgemm(omat(a), omat(b))
+        ctx.reset_stats()
+        got = ctx.spgemm(da, db).download()
+        here = ctx.stats()["kernel_launches"]
+        ctx.set_option("row_slots", 0)
+        try:
+            ctx.reset_stats()
+            crs = ctx.spgemm(da, db).download()
+            there = ctx.stats()["kernel_launches"]
+        finally:
+            ctx.set_option("row_slots", 1)
+        for m in (got, crs):
+            assert np.array_equal(m.rowmap, want.rowmap), what
+            assert np.array_equal(m.entries, want.entries), what
+            assert m.nnz() == want.nnz, what
+        assert (here != there) == (slots and n >= 24_576), what
+
+
+def test_results_past_the_early_room(ctx):
+    # more than two ranges a row: the result is written again once its size is known
+    a = gen.banded(30_000, 3_000, 1.48, 1.0, seed=72)
+    da = ctx.upload(a)
+    assert a.entries.size <= 3 * a.numRows() and a.nnz() <= a.entries.size
+    for _ in range(2):
+        ctx.reset_stats()
+        got = ctx.power(da, 2).download()
+        want = orc.power(omat(a), 2, algo="hbv")
+        assert got.entries.size > 4 * a.numRows()
+        assert np.array_equal(got.rowmap, want.rowmap) and np.array_equal(got.entries, want.entries)
+        assert got.nnz() == want.nnz and ctx.stats()["spgemm_reruns"] == 0
