@@ -50,6 +50,14 @@ constexpr double kChainReach = 1.28;          // branching * steps of a pass's l
 // before its size is known, so that the host waits once.  A second wait and the
 // gap before it are 20 us: from 2^24 rows on, under 3 % of a product.
 constexpr uint32_t kEarlyRows = 1u << 24;
+// Up to so many rows, and for single products as long as their results are written
+// early, the chain's kernels are launched close behind one another: the next one's
+// blocks are placed while the kernel before ends, 2 us a kernel.  Builds of
+// 2e3 nodes 96 -> 82 us, 1e5 158 -> 143, 1.5e6 233 -> 208, 3e6 344 -> 330, but 6e6 511
+// -> 523 and 5e7 2.64 -> 2.94 ms: blocks that wait take places of blocks that work.
+// A^2 at 1.5e6 rows 64 -> 56 us, 6e6 119 -> 114, 1.2e7 193 -> 185.  Kernels of a
+// batch, in a CUDA graph, gained nothing.
+constexpr uint32_t kCloseRows = 1u << 22;
 // A single product goes through slots from so many rows on.  The conversions are
 // launches of their own, 3 to 7 us more than the row kernel's one at 1e4 rows, equal
 // at 2e4; A^2 of a sequence graph's A takes 39 in place of 62 us at 1e5 rows, 54 of
@@ -614,6 +622,15 @@ __device__ __forceinline__ void walk_batch(const ChainArgs& p, WarpSmem& S, uint
   __syncwarp();
 }
 
+// The kernels of a chain follow one another closely: each waits for the kernel before
+// to end, with all that it wrote visible, before it touches memory, and then lets the
+// next one's blocks be placed as soon as all of its own are.  Every block waits, so a
+// kernel's end means the end of all before it.
+__device__ __forceinline__ void follow() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ---- the passes ---------------------------------------------------------------
 // A pass over a large matrix is two kernels.  k_chain_rows streams it: nearly
 // all rows of a sequence graph's powers are a single column, and their part of
@@ -633,6 +650,7 @@ __device__ __forceinline__ void walk_batch(const ChainArgs& p, WarpSmem& S, uint
 // time, held the loads of its other rows back (8.9 and 4.1 ms a build).
 template <bool OUTS, bool OUTC, bool COUNT>
 __global__ void __launch_bounds__(kSThreads, 6) k_chain_rows(const __grid_constant__ ChainArgs p) {
+  follow();
   const uint64_t r0 = (uint64_t(blockIdx.x) * kSWarps + (threadIdx.x >> 5)) * (32 * kSRows);
   if (r0 >= p.n) return;
   const int lane = lane_id();
@@ -663,6 +681,7 @@ __global__ void __launch_bounds__(kSThreads, 6) k_chain_rows(const __grid_consta
 
 template <bool OUTS, bool OUTC, bool COUNT>
 __global__ void __launch_bounds__(kWThreads) k_chain_walk(const __grid_constant__ ChainArgs p) {
+  follow();
   __shared__ WarpSmem smem[kWWarps];
   const int lane = lane_id(), warp = threadIdx.x >> 5;
   WarpSmem& S = smem[warp];
@@ -700,6 +719,7 @@ __global__ void __launch_bounds__(kWThreads) k_chain_walk(const __grid_constant_
 // one kernel, a block kCountRows rows, a warp 32 of them.
 template <bool OUTS, bool OUTC, bool COUNT>
 __global__ void __launch_bounds__(kWThreads) k_chain_small(const __grid_constant__ ChainArgs p) {
+  follow();
   static_assert(kWThreads == kCountRows, "a block's rows are counted together");
   __shared__ WarpSmem smem[kWWarps];
   __shared__ unsigned long long sum[2];
@@ -756,6 +776,7 @@ __device__ __forceinline__ SlotPart my_part(const Parts& q) { return q.table ? q
 // column each, whatever the pass.
 __global__ void __launch_bounds__(kSThreads) k_crs_to_slots(const __grid_constant__ Parts q,
                                                             const __grid_constant__ ChainArgs p) {
+  follow();
   constexpr int kIter = kCrsRows / kSThreads;
   const SlotPart part = my_part(q);
   const int lane = lane_id();
@@ -813,6 +834,7 @@ __global__ void __launch_bounds__(kSThreads) k_crs_to_slots(const __grid_constan
 __global__ void __launch_bounds__(kSThreads) k_slot_sums(const uint32_t* __restrict__ cnt,
                                                          const unsigned long long* __restrict__ nnz, uint64_t groups,
                                                          unsigned long long* __restrict__ sums, DeviceControl* ctl) {
+  follow();
   __shared__ unsigned long long part[2][kSWarps];
   unsigned long long s = 0, z = 0;
   for (uint32_t k = threadIdx.x; k < kSuperGroups; k += kSThreads) {
@@ -845,6 +867,7 @@ __global__ void __launch_bounds__(kSThreads) k_slot_sums(const uint32_t* __restr
 __global__ void __launch_bounds__(kSThreads) k_part_totals(const Parts q, const uint32_t* __restrict__ cnt,
                                                            const unsigned long long* __restrict__ nnz, uint32_t n,
                                                            unsigned long long* __restrict__ totals) {
+  follow();
   __shared__ unsigned long long sum[2][kSWarps];
   const SlotPart part = q.table[blockIdx.x];
   const uint64_t end = min((uint64_t(part.row0) + part.n + kCrsRows - 1) / kCrsRows * kCrsRows, uint64_t(n));
@@ -888,6 +911,7 @@ __global__ void __launch_bounds__(kSThreads, 7) k_slots_to_crs(const __grid_cons
                                                                const unsigned long long* __restrict__ sums,
                                                                const uint32_t* __restrict__ group_cnt,
                                                                DeviceControl* ctl) {
+  follow();
   constexpr int kIter = kCrsRows / kSThreads;
   __shared__ unsigned long long pre[kSWarps];
   __shared__ uint32_t wsum[kSWarps];
@@ -955,24 +979,34 @@ __global__ void __launch_bounds__(kSThreads, 7) k_slots_to_crs(const __grid_cons
   }
 }
 
+// A launch behind another kernel of the chain; `close`: see kCloseRows.
+template <class... P, class... A>
+void launch_next(dvg_context* ctx, bool close, void (*kernel)(P...), uint64_t blocks, int threads, const A&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(blocks));
+  cfg.blockDim = dim3(unsigned(threads));
+  cfg.stream = ctx->stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = close ? 1 : 0;
+  DVG_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+  ctx->stats.kernel_launches++;
+}
+
 template <bool OUTS, bool OUTC, bool COUNT>
-void launch_pass(dvg_context* ctx, const ChainArgs& p) {
+void launch_pass(dvg_context* ctx, bool close, const ChainArgs& p) {
   // one kernel while a warp a 32 rows fits the chip at once; the second
   // kernel's launch costs more than it saves there
   if (p.n <= kSmallRows) {
-    k_chain_small<OUTS, OUTC, COUNT><<<(p.n + kWThreads - 1) / kWThreads, kWThreads, 0, ctx->stream>>>(p);
-    DVG_CUDA(cudaGetLastError());
-    ctx->stats.kernel_launches++;
+    launch_next(ctx, close, k_chain_small<OUTS, OUTC, COUNT>, (uint64_t(p.n) + kWThreads - 1) / kWThreads, kWThreads, p);
     return;
   }
-  k_chain_rows<OUTS, OUTC, COUNT><<<unsigned((uint64_t(p.n) + kSThreads * kSRows - 1) / (kSThreads * kSRows)),
-                                    kSThreads, 0, ctx->stream>>>(p);
-  DVG_CUDA(cudaGetLastError());
+  launch_next(ctx, close, k_chain_rows<OUTS, OUTC, COUNT>,
+              (uint64_t(p.n) + kSThreads * kSRows - 1) / (kSThreads * kSRows), kSThreads, p);
   const uint64_t want = (uint64_t(p.n) + 32 * kWWarps - 1) / (32 * kWWarps);
-  k_chain_walk<OUTS, OUTC, COUNT><<<unsigned(std::min<uint64_t>(want, 7ull * ctx->num_sms)), kWThreads, 0,
-                                    ctx->stream>>>(p);
-  DVG_CUDA(cudaGetLastError());
-  ctx->stats.kernel_launches += 2;
+  launch_next(ctx, close, k_chain_walk<OUTS, OUTC, COUNT>, std::min<uint64_t>(want, 7ull * ctx->num_sms), kWThreads, p);
 }
 
 }  // namespace
@@ -1219,9 +1253,7 @@ void launch_slots(dvg_context* ctx, SlotBuild& sb, const SlotParts& parts, bool 
   ctx->stats.kernel_launches++;
   if (right) {
     p.s = sb.mat[1];
-    k_crs_to_slots<<<conversion_blocks(sb), kSThreads, 0, ctx->stream>>>(Parts{nullptr, nullptr, *right}, p);
-    DVG_CUDA(cudaGetLastError());
-    ctx->stats.kernel_launches++;
+    launch_next(ctx, sb.close, k_crs_to_slots, conversion_blocks(sb), kSThreads, Parts{nullptr, nullptr, *right}, p);
   }
   for (size_t i = 0; i < sb.plan.steps.size(); ++i) {
     const SlotStep& st = sb.plan.steps[i];
@@ -1232,34 +1264,28 @@ void launch_slots(dvg_context* ctx, SlotBuild& sb, const SlotParts& parts, bool 
     p.s = st.s >= 0 ? sb.mat[st.s] : nullptr;
     p.c = st.c >= 0 ? sb.mat[st.c] : nullptr;
     cudaEvent_t ev = timed ? span_begin(ctx) : nullptr;
-    if (i + 1 == sb.plan.steps.size()) launch_pass<false, true, true>(ctx, p);
-    else if (p.s && p.c) launch_pass<true, true, false>(ctx, p);
-    else if (p.s) launch_pass<true, false, false>(ctx, p);
-    else launch_pass<false, true, false>(ctx, p);
+    if (i + 1 == sb.plan.steps.size()) launch_pass<false, true, true>(ctx, sb.close, p);
+    else if (p.s && p.c) launch_pass<true, true, false>(ctx, sb.close, p);
+    else if (p.s) launch_pass<true, false, false>(ctx, sb.close, p);
+    else launch_pass<false, true, false>(ctx, sb.close, p);
     span_end(ctx, ev, kProduct);
   }
   const uint64_t groups = (uint64_t(sb.n) + kCountRows - 1) / kCountRows;
-  k_slot_sums<<<unsigned((groups + kSuperGroups - 1) / kSuperGroups), kSThreads, 0, ctx->stream>>>(
-      sb.group_cnt, sb.group_nnz, groups, sb.sums, sb.ctl);
-  DVG_CUDA(cudaGetLastError());
-  ctx->stats.kernel_launches++;
+  launch_next(ctx, sb.close, k_slot_sums, (groups + kSuperGroups - 1) / kSuperGroups, kSThreads, sb.group_cnt,
+              sb.group_nnz, groups, sb.sums, sb.ctl);
   ctx->stats.host_launch_ns += now_ns() - t0;
 }
 
 void launch_slots_totals(dvg_context* ctx, const SlotBuild& sb, const SlotParts& parts, uint32_t nparts,
                          unsigned long long* totals) {
-  k_part_totals<<<nparts, kSThreads, 0, ctx->stream>>>(Parts{parts.table, parts.part_of, parts.one}, sb.group_cnt,
-                                                       sb.group_nnz, sb.n, totals);
-  DVG_CUDA(cudaGetLastError());
-  ctx->stats.kernel_launches++;
+  launch_next(ctx, sb.close, k_part_totals, nparts, kSThreads, Parts{parts.table, parts.part_of, parts.one},
+              sb.group_cnt, sb.group_nnz, sb.n, totals);
 }
 
 void launch_slots_out(dvg_context* ctx, const SlotBuild& sb, const SlotParts& parts, DeviceControl* ctl) {
-  k_slots_to_crs<<<conversion_blocks(sb), kSThreads, 0, ctx->stream>>>(
-      Parts{parts.table, parts.part_of, parts.one}, sb.mat[sb.plan.out], sb.arena, sb.sums, sb.group_cnt,
-      ctl ? ctl : ctx->d_ctl);
-  DVG_CUDA(cudaGetLastError());
-  ctx->stats.kernel_launches++;
+  launch_next(ctx, sb.close, k_slots_to_crs, conversion_blocks(sb), kSThreads,
+              Parts{parts.table, parts.part_of, parts.one}, sb.mat[sb.plan.out], sb.arena, sb.sums, sb.group_cnt,
+              ctl ? ctl : ctx->d_ctl);
 }
 
 bool check_slots(dvg_context* ctx, const SlotBuild& sb, const SlotCounters& c) {
@@ -1313,6 +1339,7 @@ static dvg_matrix* run_slots(dvg_context* ctx, const SlotPlan& plan, const dvg_m
     return nullptr;
   }
   dvg_matrix* m = nullptr;
+  sb.close = a->nrows <= (plan.steps.size() == 1 ? kEarlyRows : kCloseRows);
   try {
     SlotParts parts{};
     parts.one = whole(a);

@@ -65,6 +65,7 @@ struct SlotBuild {
   std::vector<uint2*> buffers; // theirs
   uint2* arena = nullptr;
   uint64_t arena_cap = 0;      // ranges
+  bool close = false;          // the kernels' blocks are placed while the kernel before ends
   uint64_t early = 0;          // room for the result's ranges before their number is known; 0: none
   void* scratch = nullptr;     // counters | sums of the counts | counts of the result | bitmap
   DeviceControl* ctl = nullptr;
