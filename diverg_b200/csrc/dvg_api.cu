@@ -769,6 +769,7 @@ dvg_status dvg_shutdown(dvg_context* ctx) {
     resolve_spans(ctx);
     for (cudaEvent_t e : ctx->event_pool) cudaEventDestroy(e);
     ctx->event_pool.clear();
+    if (ctx->batch_exec) cudaGraphExecDestroy(ctx->batch_exec);
     for (cudaEvent_t e : ctx->side_events) cudaEventDestroy(e);
     for (cudaStream_t t : ctx->side_streams) cudaStreamDestroy(t);
     DVG_CUDA(cudaFree(ctx->d_ctl));
@@ -853,6 +854,8 @@ dvg_status dvg_trim(dvg_context* ctx) {
     Lock lk(ctx);
     release_cached(ctx);
     DVG_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (ctx->batch_exec) DVG_CUDA(cudaGraphExecDestroy(ctx->batch_exec));
+    ctx->batch_exec = nullptr;
   });
 }
 

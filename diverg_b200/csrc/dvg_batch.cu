@@ -182,6 +182,27 @@ void make_side_streams(dvg_context* ctx, size_t n) {
   }
 }
 
+// Launches the captured graph.  Batches of as many chains with as many passes have
+// the same nodes, so the executable graph of the batch before usually takes over
+// this one's kernels, arguments and grids; where the nodes differ it is instantiated
+// anew.  Instantiating (210 us for the 50 nodes of three windows), the first launch
+// (80 us) and destroying one cost the host more than the chains take: 30 graphs of
+// 1e6 nodes together 995 -> 530 us, 335 of them the GPU's.
+void launch_graph(dvg_context* ctx, cudaGraph_t graph) {
+  cudaGraphExec_t& exec = ctx->batch_exec;
+  if (exec) {
+    cudaGraphExecUpdateResultInfo info;
+    if (cudaGraphExecUpdate(exec, graph, &info) != cudaSuccess) {
+      cudaGetLastError();
+      const cudaGraphExec_t old = exec;
+      exec = nullptr;
+      DVG_CUDA(cudaGraphExecDestroy(old));
+    }
+  }
+  if (!exec) DVG_CUDA(cudaGraphInstantiate(&exec, graph, 0));
+  DVG_CUDA(cudaGraphLaunch(exec, ctx->stream));
+}
+
 // Lays the members' rows side by side, each from a multiple of kSlotPartRows on.
 void lay_out(SlotGroup& g, const dvg_matrix* const* graphs) {
   for (uint32_t k : g.members) {
@@ -336,7 +357,6 @@ void batch_distance_index(dvg_context* ctx, uint32_t ngraphs, const dvg_matrix* 
   void* d_table = nullptr;
   void* d_parts = nullptr;
   cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
   try {
     // ---- the chains' buffers ------------------------------------------------------
     // (before any planned build's: those hand blocks back that their own later
@@ -465,8 +485,7 @@ void batch_distance_index(dvg_context* ctx, uint32_t ngraphs, const dvg_matrix* 
       throw;
     }
     DVG_CUDA(cudaStreamEndCapture(ctx->stream, &graph));
-    DVG_CUDA(cudaGraphInstantiate(&exec, graph, 0));
-    DVG_CUDA(cudaGraphLaunch(exec, ctx->stream));
+    launch_graph(ctx, graph);
     ctx->stats.graph_launches++;
     // ---- results ----------------------------------------------------------------
     for (auto& g : groups) {
@@ -533,8 +552,6 @@ void batch_distance_index(dvg_context* ctx, uint32_t ngraphs, const dvg_matrix* 
       dfree(ctx, d_parts);
       d_parts = nullptr;
     }
-    DVG_CUDA(cudaGraphExecDestroy(exec));
-    exec = nullptr;
     DVG_CUDA(cudaGraphDestroy(graph));
     graph = nullptr;
     // where every graph's index starts in its group's, and its nnz: one
@@ -600,7 +617,6 @@ void batch_distance_index(dvg_context* ctx, uint32_t ngraphs, const dvg_matrix* 
     // graphs that could not join a group
     for (uint32_t k : alone) out[k] = create_distance_index(ctx, graphs[k], dmin[k], dmax[k]);
   } catch (...) {
-    if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
     cleanup();
     if (d_table) dfree(ctx, d_table);

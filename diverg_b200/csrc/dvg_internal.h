@@ -106,6 +106,9 @@ struct dvg_context {
   // use, given back at shutdown
   std::vector<cudaStream_t> side_streams;
   std::vector<cudaEvent_t> side_events;
+  // the last batch's CUDA graph as instantiated (with the pointers of that call, which
+  // every launch replaces); given back by a trim and at shutdown
+  cudaGraphExec_t batch_exec = nullptr;
   // the last cudaMemGetInfo answer, when it was taken, and owned_bytes then
   size_t mi_free = 0, mi_owned = 0;
   uint64_t mi_ns = 0;

@@ -103,3 +103,24 @@ def test_batch_rejects_bad_windows_and_leaves_nothing(ctx):
         ctx.batch_distance_index(dg, [(1, 5), (6, 5)])
     assert e.value.status == N.INVALID_ARG
     assert ctx.batch_distance_index([], []) == []
+
+
+def test_batches_in_turn(ctx):
+    # a batch's CUDA graph takes the place of the one before: the same passes over
+    # other graphs and windows, other numbers of them, dense graphs beside them, and
+    # after a trim
+    rng = np.random.default_rng(71)
+    shapes = [(12, [(100, 300), (0, 50)]), (12, [(90, 290), (0, 45)]), (7, [(100, 300)]), (30, [(100, 300), (0, 50)]),
+              (3, [(100, 300), (0, 50), (3, 3)]), (12, [(100, 300), (0, 50)]), (200, [(100, 300), (0, 50)])]
+    for i, (count, windows) in enumerate(shapes):
+        graphs = [gen.graph_adjacency(gen.small_graph_spec(int(rng.integers(600, 3_000)), seed=710 + 50 * i + k))[0]
+                  for k in range(count)]
+        if i == 4:
+            graphs[1] = gen.random_matrix(500, 2_500, seed=72)
+        ws = [(1, 2) if i == 4 and k == 1 else windows[k % len(windows)] for k in range(count)]
+        dg = [ctx.upload(g) for g in graphs]
+        got = ctx.batch_distance_index(dg, ws)
+        for k in range(count):
+            assert same(got[k].download(), ctx.distance_index(dg[k], *ws[k]).download()), (i, k)
+        if i == 2:
+            ctx.trim()
