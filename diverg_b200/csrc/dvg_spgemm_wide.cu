@@ -16,7 +16,8 @@
 // HBitVector sets runs).  The runs come out of the window with the map01 /
 // map10 boundary masks of hbitvector.hpp:576-597 (gather_chunk); a row wider
 // than the window takes further windows.  The cost is per B range named, not
-// per column.
+// per column.  Where B's rows are named often enough, the product reads bitmaps
+// of unions of B rows instead (BandTables, band_rows): two steps an A range.
 //
 // Chunks of kWRows rows are taken from a ticket by persistent CTAs; the warps
 // of a CTA walk its rows (runs kept in a per-warp buffer), a chunk-local
