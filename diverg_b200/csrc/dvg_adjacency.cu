@@ -24,8 +24,9 @@
 // first.
 //
 // Bound: the matrix's writes, 16 bytes a locus; below ~1e6 loci the launches and
-// the one wait.  1e7 loci of 3.4e4 nodes and 4.6e4 edges: 449 -> 187 us a call, of which
-// k_adj_rows 128 -> 45 us (a binary search over all nodes for every locus before).
+// the one wait.  1e7 loci of 3.4e4 nodes and 4.6e4 edges: 449 -> 163 us a call, of which
+// k_adj_rows 128 -> 45 us (a binary search over all nodes for every locus before)
+// and the two scans 51 -> 11.
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -56,17 +57,20 @@ struct AdjArgs {
   uint64_t* cursor;           // [nnodes]: scatter cursors
   uint32_t* cols;             // [edges of the range]: successor loci
   uint64_t* base;             // [nnodes + 1]: first entry of each node's rows
+  uint64_t* start_n;          // their counts, from [1] on: the same arrays where they
+  uint64_t* eoff_n;           // are scanned in place
+  uint64_t* base_n;
   uint64_t* c_rowmap;
   uint32_t* c_entries;
   DeviceControl* ctl;
 };
 
-// start[v + 1] = node_len[v], eoff[v + 1] = out-degree of node v within the range
-// (scanned afterwards).  Bit 2 of invalid: an endpoint that is no node; bit 1: a
+// start_n[v + 1] = node_len[v], eoff_n[v + 1] = out-degree of node v within the
+// range (scanned afterwards).  Bit 2 of invalid: an endpoint that is no node; bit 1: a
 // successor outside the range of a node inside it (its column would not exist).
 __global__ void k_adj_counts(AdjArgs p, uint32_t all_nodes) {
   const uint64_t t0 = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x, stride = uint64_t(gridDim.x) * blockDim.x;
-  for (uint64_t v = t0; v < p.nnodes; v += stride) p.start[v + 1] = p.node_len[v];
+  for (uint64_t v = t0; v < p.nnodes; v += stride) p.start_n[v + 1] = p.node_len[v];
   for (uint64_t e = t0; e < p.nedges; e += stride) {
     const uint32_t from = p.edges[2 * e], to = p.edges[2 * e + 1];
     if (from < 1 || from > all_nodes || to < 1 || to > all_nodes) {
@@ -78,55 +82,55 @@ __global__ void k_adj_counts(AdjArgs p, uint32_t all_nodes) {
       atomicOr(&p.ctl->invalid, 1ull);
       continue;
     }
-    atomicAdd(reinterpret_cast<unsigned long long*>(p.eoff + (from - p.lower) + 1), 1ull);
+    atomicAdd(reinterpret_cast<unsigned long long*>(p.eoff_n + (from - p.lower) + 1), 1ull);
   }
 }
 
-// In-place inclusive scans of a[1 .. n] and b[1 .. n] (b null: a alone), a block
-// each: for the node counts of most graphs one launch beats the three that a
-// scan over the whole chip takes (two scans of 3.4e4 nodes: 33 -> 18 us).
+// Inclusive scans of a[1 .. n] to to_a and b[1 .. n] to to_b, an element a thread.
+// A block adds up the elements before its own by itself, from L2, so that no block
+// waits for another: for the node counts of most graphs one such launch beats the
+// three that a scan over the whole chip takes (two scans of 3.4e4 nodes:
+// 33 us, 18 by one block each, 5 so).
 constexpr uint32_t kAdjScanThreads = 1024, kAdjScanMax = 1u << 17;
-__global__ void __launch_bounds__(kAdjScanThreads) k_adj_scan(uint64_t* a, uint64_t* b, uint32_t n) {
-  constexpr int kAhead = 8;
-  __shared__ uint64_t warps[kAdjScanThreads / 32];
-  uint64_t* const x = (blockIdx.x ? b : a) + 1;
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // a warp's consecutive elements, 32 at a time
-  const uint32_t per = ((n + kAdjScanThreads - 1) / kAdjScanThreads) * 32, i0 = min(warp * per, n), i1 = min(i0 + per, n);
+__global__ void __launch_bounds__(kAdjScanThreads) k_adj_scan(const uint64_t* __restrict__ a, uint64_t* to_a,
+                                                              const uint64_t* __restrict__ b, uint64_t* to_b,
+                                                              uint32_t n) {
+  constexpr uint32_t kAhead = 8;
+  static_assert(kAdjScanThreads == 32 * 32, "a lane a warp's sums");
+  __shared__ uint64_t sums[32], before[32];
+  const uint64_t* const x = (blockIdx.y ? b : a) + 1;
+  uint64_t* const y = (blockIdx.y ? to_b : to_a) + 1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t i0 = blockIdx.x * kAdjScanThreads, i = i0 + threadIdx.x;
+  const uint64_t mine = i < n ? x[i] : 0;
   uint64_t sum = 0;
-  for (uint32_t i = i0 + lane; i < i1; i += 32 * kAhead) {
+  for (uint32_t j = threadIdx.x; j < i0; j += kAhead * kAdjScanThreads) {
     uint64_t v[kAhead];
 #pragma unroll
-    for (int k = 0; k < kAhead; ++k) v[k] = i + 32 * k < i1 ? x[i + 32 * k] : 0;
+    for (uint32_t k = 0; k < kAhead; ++k) v[k] = j + k * kAdjScanThreads < i0 ? x[j + k * kAdjScanThreads] : 0;
 #pragma unroll
-    for (int k = 0; k < kAhead; ++k) sum += v[k];
+    for (uint32_t k = 0; k < kAhead; ++k) sum += v[k];
   }
   sum = group_sum<32>(kFullMask, sum);
-  if (lane == 0) warps[warp] = sum;
+  const uint64_t incl = group_incl_sum<32>(kFullMask, mine, lane);
+  if (lane == 0) before[warp] = sum;
+  if (lane == 31) sums[warp] = incl;
   __syncthreads();
-  uint64_t run = group_sum<32>(kFullMask, lane < warp ? warps[lane] : uint64_t(0));
-  for (uint32_t i = i0; i < i1; i += 32 * kAhead) {
-    uint64_t v[kAhead];
-#pragma unroll
-    for (int k = 0; k < kAhead; ++k) v[k] = i + 32 * k + lane < i1 ? x[i + 32 * k + lane] : 0;
-#pragma unroll
-    for (int k = 0; k < kAhead; ++k) {
-      v[k] = run + group_incl_sum<32>(kFullMask, v[k], int(lane));
-      run = __shfl_sync(kFullMask, v[k], 31);
-      if (i + 32 * k + lane < i1) x[i + 32 * k + lane] = v[k];
-    }
-  }
+  const uint64_t run = group_sum<32>(kFullMask, before[lane] + (lane < warp ? sums[lane] : uint64_t(0)));
+  if (i < n) y[i] = run + incl;
 }
 
-void scan_nodes(dvg_context* ctx, uint64_t* a, uint64_t* b, uint32_t n) {
+// (counts of more than kAdjScanMax nodes lie in the scanned arrays)
+void scan_nodes(dvg_context* ctx, const uint64_t* a, uint64_t* to_a, const uint64_t* b, uint64_t* to_b, uint32_t n) {
   if (n <= kAdjScanMax) {
-    k_adj_scan<<<b ? 2 : 1, kAdjScanThreads, 0, ctx->stream>>>(a, b, n);
+    k_adj_scan<<<dim3((n + kAdjScanThreads - 1) / kAdjScanThreads, b ? 2 : 1), kAdjScanThreads, 0, ctx->stream>>>(
+        a, to_a, b, to_b, n);
     DVG_CUDA(cudaGetLastError());
     ctx->stats.kernel_launches++;
     return;
   }
-  launch_rowmap_scan(ctx, a, n);
-  if (b) launch_rowmap_scan(ctx, b, n);
+  launch_rowmap_scan(ctx, to_a, n);
+  if (b) launch_rowmap_scan(ctx, to_b, n);
 }
 
 // each edge's successor locus into its source node's segment
@@ -202,7 +206,7 @@ __global__ void k_adj_nodes(AdjArgs p) {
     bool repeated = false;
     const uint64_t r = row_ranges(a, n, repeated);
     if (repeated) atomicOr(&p.ctl->invalid, 16ull);
-    p.base[v + 1] = 2 * (uint64_t(p.node_len[v]) - 1) + 2 * r;
+    p.base_n[v + 1] = 2 * (uint64_t(p.node_len[v]) - 1) + 2 * r;
   }
 }
 
@@ -321,12 +325,16 @@ dvg_matrix* adjacency_from_graph(dvg_context* ctx, uint32_t nnodes, const uint32
     ctx->stats.h2d_bytes += edge_bytes + len_bytes;
     p.edges = reinterpret_cast<const uint32_t*>(d_in);
     p.node_len = reinterpret_cast<const uint32_t*>(d_in + edge_bytes);
-    // start | eoff | cursor | base, all zero at first
-    const size_t words = size_t(m) + 1;
-    p.start = static_cast<uint64_t*>(grab(4 * words * 8));
+    // start | eoff | cursor | base, and the counts that the first, second and last
+    // are scanned from, all zero at first
+    const size_t words = size_t(m) + 1, arrays = m <= kAdjScanMax ? 7 : 4;
+    p.start = static_cast<uint64_t*>(grab(arrays * words * 8));
     p.eoff = p.start + words;
     p.cursor = p.eoff + words;
     p.base = p.cursor + words;
+    p.start_n = arrays > 4 ? p.base + words : p.start;
+    p.eoff_n = arrays > 4 ? p.start_n + words : p.eoff;
+    p.base_n = arrays > 4 ? p.eoff_n + words : p.base;
     uint64_t* h_sizes = reinterpret_cast<uint64_t*>(ctx->h_ctl + 1);
     uint64_t most_edges = nedges;  // of the range
     auto allocate = [&]() {
@@ -339,10 +347,10 @@ dvg_matrix* adjacency_from_graph(dvg_context* ctx, uint32_t nnodes, const uint32
     const bool whole = m == nnodes;
     if (whole) allocate();
     reset_control(ctx);
-    DVG_CUDA(cudaMemsetAsync(p.start, 0, 4 * words * 8, ctx->stream));
+    DVG_CUDA(cudaMemsetAsync(p.start, 0, arrays * words * 8, ctx->stream));
     k_adj_counts<<<adj_grid(ctx, std::max<uint64_t>(m, nedges)), kAdjThreads, 0, ctx->stream>>>(p, nnodes);
     DVG_CUDA(cudaGetLastError());
-    scan_nodes(ctx, p.start, p.eoff, m);
+    scan_nodes(ctx, p.start_n, p.start, p.eoff_n, p.eoff, m);
     if (!whole) {  // a component may hold few of the graph's edges: its own number sizes the result
       DVG_CUDA(cudaMemcpyAsync(h_sizes, p.eoff + m, 8, cudaMemcpyDeviceToHost, ctx->stream));
       read_control(ctx);
@@ -355,7 +363,7 @@ dvg_matrix* adjacency_from_graph(dvg_context* ctx, uint32_t nnodes, const uint32
     }
     k_adj_nodes<<<adj_grid(ctx, m), kAdjThreads, 0, ctx->stream>>>(p);
     DVG_CUDA(cudaGetLastError());
-    scan_nodes(ctx, p.base, nullptr, m);
+    scan_nodes(ctx, p.base_n, p.base, nullptr, nullptr, m);
     k_adj_rows<<<unsigned((nloci + kAdjTile - 1) / kAdjTile), kAdjThreads, 0, ctx->stream>>>(p, nloci);
     DVG_CUDA(cudaGetLastError());
     ctx->stats.kernel_launches += 4 + (nedges ? 1 : 0);
