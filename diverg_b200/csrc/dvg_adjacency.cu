@@ -26,7 +26,7 @@
 // Bound: the matrix's writes, 16 bytes a locus; below ~1e6 loci the launches and
 // the one wait.  1e7 loci of 3.4e4 nodes and 4.6e4 edges: 449 -> 163 us a call, of which
 // k_adj_rows 128 -> 45 us (a binary search over all nodes for every locus before)
-// and the two scans 51 -> 11.
+// and the scans 18 -> 5 each (one block a scan before).
 #include <algorithm>
 #include <cstring>
 #include <vector>
