@@ -69,14 +69,20 @@ constexpr uint32_t kSuperGroups = 512;        // counts that k_slot_sums adds up
 
 __device__ __forceinline__ uint2 empty_slot() { return make_uint2(1u, 0u); }
 __device__ __forceinline__ bool is_multi(uint2 s) { return s.x >= kMulti; }
-__device__ __forceinline__ uint2 ld_slot(const uint2* __restrict__ p, size_t i) { return __ldg(p + i); }
+// Every load of what a kernel of the same chain wrote is an ordinary one: a close
+// chain's kernels (kCloseRows) start while the one before still writes, and the
+// read-only path is for memory that nothing writes from a kernel's start on.  After
+// follow() an ordinary load sees all that the kernels before wrote.  (Read-only loads
+// in a chain that is not close: 170 against 153 us for a build of 1e5 bases, 231
+// against 217 for A^100 of 1e6; ordinary loads by __ldca: 186 and 276.)
+__device__ __forceinline__ uint2 ld_slot(const uint2* p, size_t i) { return p[i]; }
 __device__ __forceinline__ bool is_run(uint2 s) { return s.x <= s.y; }
 __device__ __forceinline__ uint32_t slot_count(uint2 s) {
   return is_run(s) ? 1u : is_multi(s) ? s.x - kMulti : s.x == s.y + 1 ? 0u : 2u;
 }
 // Range t of a slot that has it.
-__device__ __forceinline__ uint2 slot_range(const uint2* __restrict__ arena, uint2 s, uint32_t t) {
-  if (is_multi(s)) return __ldg(arena + s.y + t);
+__device__ __forceinline__ uint2 slot_range(const uint2* arena, uint2 s, uint32_t t) {
+  if (is_multi(s)) return arena[s.y + t];
   if (is_run(s)) return s;
   return t ? make_uint2(s.x, s.x) : make_uint2(s.y, s.y);
 }
@@ -141,7 +147,7 @@ __device__ __forceinline__ uint32_t chain_rows(const ChainArgs& p, uint32_t r0, 
   }
 #pragma unroll 1
   for (uint32_t j = 0; j < p.k; ++j) {
-    const uint2* __restrict__ mat = p.m[j];
+    const uint2* mat = p.m[j];
     const bool last = j + 1 == p.k, gather = OUTC && ((p.bits >> (j + 1)) & 1u);
     uint2 s[U];
 #pragma unroll
@@ -275,8 +281,8 @@ __device__ __noinline__ uint32_t list_merge(uint2* L, uint32_t nr, uint2 v) {
 
 // The nd runs at D |= the rows of `mat` that the ns runs at L name (mat null:
 // the runs themselves).  Returns their new number, or kFull.
-__device__ __noinline__ uint32_t list_product(const uint2* __restrict__ arena, const uint2* L, uint32_t ns,
-                                              const uint2* __restrict__ mat, uint2* D, uint32_t nd) {
+__device__ __noinline__ uint32_t list_product(const uint2* arena, const uint2* L, uint32_t ns, const uint2* mat,
+                                              uint2* D, uint32_t nd) {
   uint2 run = empty_slot();
   for (uint32_t k = 0; k < ns; ++k) {
     const uint2 a = L[k * 32];
@@ -340,7 +346,7 @@ __device__ __forceinline__ bool quick_row(const ChainArgs& p, uint32_t row, uint
   for (uint32_t j = 0;; ++j) {
     const bool gather = OUTC && ((p.bits >> j) & 1u), go = j < p.k;
     if (!gather && !go) break;
-    const uint2* __restrict__ mat = go ? p.m[j] : nullptr;
+    const uint2* mat = go ? p.m[j] : nullptr;
     unsigned long long to = 0;
     uint32_t from = 0;
     auto add_s = [&](uint2 v) {
@@ -422,7 +428,7 @@ __device__ __forceinline__ bool quick_row(const ChainArgs& p, uint32_t row, uint
 // the columns that its ranges cover, the next window starting at the first
 // column past the last one.  Returns the row's slot (uniform).  The arena is
 // read past L1: a slot may be one that this warp has just written.
-__device__ uint2 warp_union(const ChainArgs& p, uint2 left, const uint2* __restrict__ mat, uint2 d, uint2 e,
+__device__ uint2 warp_union(const ChainArgs& p, uint2 left, const uint2* mat, uint2 d, uint2 e,
                             uint32_t* bits, uint32_t* reach) {
   const int lane = lane_id();
   // every range of the union, spread over the lanes
@@ -765,8 +771,8 @@ __global__ void __launch_bounds__(kWThreads) k_chain_small(const __grid_constant
 // works on one of them: block b's is number part_of[b] (a null table: all
 // blocks are `one`'s, the only one).
 struct Parts {
-  const SlotPart* __restrict__ table;
-  const uint32_t* __restrict__ part_of;
+  const SlotPart* table;
+  const uint32_t* part_of;
   SlotPart one;
 };
 __device__ __forceinline__ SlotPart my_part(const Parts& q) { return q.table ? q.table[q.part_of[blockIdx.x]] : q.one; }
@@ -787,8 +793,8 @@ __global__ void __launch_bounds__(kSThreads) k_crs_to_slots(const __grid_constan
     const uint64_t i = b0 + u * kSThreads - part.row0;
     a0[u] = cnt[u] = 0;
     if (i < part.n) {
-      a0[u] = __ldg(part.rowmap + i) >> 1;
-      cnt[u] = (__ldg(part.rowmap + i + 1) >> 1) - a0[u];
+      a0[u] = part.rowmap[i] >> 1;
+      cnt[u] = (part.rowmap[i + 1] >> 1) - a0[u];
     }
   }
   auto range = [&](uint64_t k) {
@@ -831,9 +837,9 @@ __global__ void __launch_bounds__(kSThreads) k_crs_to_slots(const __grid_constan
 }
 
 // Sums of kSuperGroups counts each, a block a sum; the totals of the result.
-__global__ void __launch_bounds__(kSThreads) k_slot_sums(const uint32_t* __restrict__ cnt,
-                                                         const unsigned long long* __restrict__ nnz, uint64_t groups,
-                                                         unsigned long long* __restrict__ sums, DeviceControl* ctl) {
+__global__ void __launch_bounds__(kSThreads) k_slot_sums(const uint32_t* cnt, const unsigned long long* nnz,
+                                                         uint64_t groups, unsigned long long* sums,
+                                                         DeviceControl* ctl) {
   follow();
   __shared__ unsigned long long part[2][kSWarps];
   unsigned long long s = 0, z = 0;
@@ -864,9 +870,9 @@ __global__ void __launch_bounds__(kSThreads) k_slot_sums(const uint32_t* __restr
 
 // Ranges and columns of every part's result, a block a part (its last rows of
 // the identity are no part of it).
-__global__ void __launch_bounds__(kSThreads) k_part_totals(const Parts q, const uint32_t* __restrict__ cnt,
-                                                           const unsigned long long* __restrict__ nnz, uint32_t n,
-                                                           unsigned long long* __restrict__ totals) {
+__global__ void __launch_bounds__(kSThreads) k_part_totals(const Parts q, const uint32_t* cnt,
+                                                           const unsigned long long* nnz, uint32_t n,
+                                                           unsigned long long* totals) {
   follow();
   __shared__ unsigned long long sum[2][kSWarps];
   const SlotPart part = q.table[blockIdx.x];
@@ -906,11 +912,9 @@ __global__ void __launch_bounds__(kSThreads) k_part_totals(const Parts q, const 
 // with the slots requested first and seven blocks an SM (a build of 5e7 rows: 2.78
 // to 2.65 ms).
 __global__ void __launch_bounds__(kSThreads, 7) k_slots_to_crs(const __grid_constant__ Parts q,
-                                                               const uint2* __restrict__ slots,
-                                                               const uint2* __restrict__ arena,
-                                                               const unsigned long long* __restrict__ sums,
-                                                               const uint32_t* __restrict__ group_cnt,
-                                                               DeviceControl* ctl) {
+                                                               const uint2* slots, const uint2* arena,
+                                                               const unsigned long long* sums,
+                                                               const uint32_t* group_cnt, DeviceControl* ctl) {
   follow();
   constexpr int kIter = kCrsRows / kSThreads;
   __shared__ unsigned long long pre[kSWarps];
