@@ -887,11 +887,14 @@ std::string validation_message(unsigned long long bits) {
 
 extern "C" {
 
+// Checks a matrix that came from a caller, and counts its columns: which kernels a
+// product or a build takes goes by that count.
 static void validate_uploaded(dvg_context* ctx, dvg_matrix* m) {
   reset_control(ctx);
   launch_validate(ctx, m->rowmap, m->nrows, m->entries, m->nentries, m->ncols);
   DeviceControl c = read_control(ctx);
   m->canonical = !(c.invalid & 16);
+  m->nnz = c.nnz;
   c.invalid &= ~16ull;
   if (c.invalid) throw Error(DVG_ERR_INVALID_ARG, "malformed range-CRS matrix:" + validation_message(c.invalid));
 }
@@ -917,7 +920,8 @@ dvg_matrix* upload_matrix(dvg_context* ctx, uint32_t nrows, uint32_t ncols, cons
     if (ne) DVG_CUDA(cudaMemcpyAsync(m->entries, entries, ne * 4, cudaMemcpyHostToDevice, ctx->stream));
     ctx->stats.h2d_bytes += (uint64_t(nrows) + 1) * 8 + ne * 4;
     validate_uploaded(ctx, m);
-    m->nnz = nnz ? nnz : count_nnz_host(entries, ne);
+    m->given_nnz = nnz ? nnz : count_nnz_host(entries, ne);
+    m->nnz_given = true;
   } catch (...) {
     free_matrix(ctx, m);
     throw;
@@ -956,7 +960,8 @@ dvg_status dvg_matrix_upload_u32(dvg_context* ctx, uint32_t nrows, uint32_t ncol
       if (ne) DVG_CUDA(cudaMemcpyAsync(m->entries, entries, ne * 4, cudaMemcpyHostToDevice, ctx->stream));
       ctx->stats.h2d_bytes += (uint64_t(nrows) + 1) * 4 + ne * 4;
       validate_uploaded(ctx, m);
-      m->nnz = nnz ? nnz : count_nnz_host(entries, ne);
+      m->given_nnz = nnz ? nnz : count_nnz_host(entries, ne);
+      m->nnz_given = true;
     } catch (...) {
       if (tmp) dfree(ctx, tmp);
       free_matrix(ctx, m);
@@ -987,7 +992,8 @@ dvg_status dvg_matrix_wrap_device(dvg_context* ctx, uint32_t nrows, uint32_t nco
       delete m;
       throw;
     }
-    m->nnz = nnz;
+    m->given_nnz = nnz;
+    m->nnz_given = true;
     *out = m;
   });
 }
@@ -997,7 +1003,7 @@ dvg_status dvg_matrix_info(const dvg_matrix* m, uint32_t* nrows, uint32_t* ncols
   if (nrows) *nrows = m->nrows;
   if (ncols) *ncols = m->ncols;
   if (nentries) *nentries = m->nentries;
-  if (nnz) *nnz = m->nnz;
+  if (nnz) *nnz = m->reported_nnz();
   return DVG_OK;
 }
 

@@ -19,12 +19,16 @@ struct dvg_matrix {
   uint32_t nrows = 0;
   uint32_t ncols = 0;
   uint64_t nentries = 0;
-  uint64_t nnz = 0;
+  uint64_t nnz = 0;         // columns of its ranges, as the device counted them
+  uint64_t given_nnz = 0;   // what the caller said they are, for a matrix that came from one
+  bool nnz_given = false;
   uint64_t* rowmap = nullptr;   // device, nrows + 1
   uint32_t* entries = nullptr;  // device, nentries (allocation padded to 16 B)
   bool owned = true;
   bool canonical = true;  // rows sorted, disjoint and non-adjacent (as SpGEMM emits them)
   int device = 0;
+  // What the caller is told.  Nothing is decided by it: a caller's count may be off.
+  uint64_t reported_nnz() const { return nnz_given ? given_nnz : nnz; }
 };
 
 // Device control block: counters that kernels accumulate into and read back.

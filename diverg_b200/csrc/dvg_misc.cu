@@ -31,9 +31,13 @@ __global__ void k_identity(uint64_t* __restrict__ rowmap, uint32_t* __restrict__
 // bit 4: rowmap[n] != nentries; bit 8: an entry >= ncols.  Not an error:
 // bit 16 marks a matrix whose rows are not canonical (a range with end <
 // start, or a range that does not start past the previous range's end + 1).
+// The columns of its ranges are counted into ctl->nnz.
 __global__ void k_validate(const uint64_t* __restrict__ rowmap, uint32_t nrows, const uint32_t* __restrict__ entries,
                            uint64_t nentries, uint32_t ncols, DeviceControl* ctl) {
-  unsigned long long bad = 0;
+  __shared__ unsigned long long cta_nnz;
+  if (threadIdx.x == 0) cta_nnz = 0;
+  __syncthreads();
+  unsigned long long bad = 0, nnz = 0;
   const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
   const uint64_t tid = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
   for (uint64_t i = tid; i < nrows; i += stride) {
@@ -44,6 +48,7 @@ __global__ void k_validate(const uint64_t* __restrict__ rowmap, uint32_t nrows, 
       for (uint64_t k = a; k < b; k += 2) {
         if (entries[k + 1] < entries[k] || (k > a && uint64_t(entries[k]) <= uint64_t(entries[k - 1]) + 1))
           bad |= 16;
+        if (entries[k + 1] >= entries[k]) nnz += uint64_t(entries[k + 1] - entries[k]) + 1;
       }
     }
   }
@@ -54,6 +59,10 @@ __global__ void k_validate(const uint64_t* __restrict__ rowmap, uint32_t nrows, 
   for (uint64_t i = tid; i < nentries; i += stride)
     if (entries[i] >= ncols) bad |= 8;
   if (bad) atomicOr(&ctl->invalid, bad);
+  nnz = group_sum<32>(kFullMask, nnz);
+  if (lane_id() == 0 && nnz) atomicAdd(&cta_nnz, nnz);
+  __syncthreads();
+  if (threadIdx.x == 0 && cta_nnz) atomicAdd(&ctl->nnz, cta_nnz);
 }
 
 __global__ void k_widen(const uint32_t* __restrict__ src, uint64_t* __restrict__ dst, uint64_t n) {

@@ -680,7 +680,7 @@ dvg_status dvg_server_index_info(dvg_server* s, uint64_t index, uint32_t* nrows,
   }
   if (nrows) *nrows = f->second.m->nrows;
   if (nentries) *nentries = f->second.m->nentries;
-  if (nnz) *nnz = f->second.m->nnz;
+  if (nnz) *nnz = f->second.m->reported_nnz();
   return DVG_OK;
 }
 
