@@ -180,6 +180,26 @@ void free_matrix(dvg_context* ctx, dvg_matrix* m) {
   delete m;
 }
 
+bool give_back(dvg_context* ctx, dvg_matrix* m, uint64_t cap) {
+  if (cap <= m->nentries + m->nentries / 4 + (1u << 18)) return false;
+  uint32_t* exact = nullptr;
+  try {
+    exact = static_cast<uint32_t*>(dalloc(ctx, entries_alloc_bytes(m->nentries)));
+  } catch (const Error& e) {
+    if (e.status != DVG_ERR_OOM) throw;
+    return false;
+  }
+  if (m->nentries) {
+    const cudaError_t e = cudaMemcpyAsync(exact, m->entries, m->nentries * sizeof(uint32_t), cudaMemcpyDeviceToDevice,
+                                          ctx->stream);
+    if (e != cudaSuccess) dfree(ctx, exact);
+    DVG_CUDA(e);
+  }
+  dfree(ctx, m->entries);
+  m->entries = exact;
+  return true;
+}
+
 static cudaEvent_t take_event(dvg_context* ctx) {
   if (!ctx->event_pool.empty()) {
     cudaEvent_t e = ctx->event_pool.back();
@@ -664,7 +684,7 @@ dvg_matrix* create_distance_index(dvg_context* ctx, const dvg_matrix* a, unsigne
   // canonicalise any input
   if (ctx->opt_dindex_schedule == 1 || (dlo == 0 && !a->canonical)) return distance_index_reference(ctx, a, dlo, dup);
   if (ctx->opt_planned && ctx->opt_spgemm_mode == 0 && slots_suit(ctx, a)) {
-    if (dvg_matrix* t = slots_chain(ctx, a, dlo, dup, settled)) return t;
+    if (dvg_matrix* t = slots_chain(ctx, a, dlo, dup, true, settled)) return t;
     ctx->stats.spgemm_reruns++;
   }
   if (ctx->opt_planned && ctx->opt_spgemm_mode != 1 && a->nrows > 0) {
@@ -1105,7 +1125,7 @@ dvg_status dvg_range_power(dvg_context* ctx, const dvg_matrix* a, unsigned k, dv
     dvg_matrix* r = nullptr;
     bool settled = false;
     if (k > 1 && ctx->opt_planned && ctx->opt_spgemm_mode == 0 && slots_suit(ctx, a)) {
-      r = slots_chain(ctx, a, k, k, &settled);
+      r = slots_chain(ctx, a, k, k, false, &settled);
       if (!r) ctx->stats.spgemm_reruns++;
     }
     if (!r) r = range_power(ctx, a, k);

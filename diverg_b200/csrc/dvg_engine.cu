@@ -313,24 +313,15 @@ dvg_matrix* finish_build(dvg_context* ctx, PlannedBuild& pb) {
   m->canonical = true;
   m->device = ctx->device;
   m->rowmap = pb.rowmap[out];
-  // hand the slack of the estimated capacity back: copy into an exact buffer
-  if (pb.cap[out] > m->nentries + m->nentries / 4 + (1u << 18)) {
-    try {
-      m->entries = static_cast<uint32_t*>(dalloc(ctx, entries_alloc_bytes(m->nentries)));
-    } catch (...) {
-      delete m;
-      release_build(ctx, pb);
-      throw;
-    }
-    if (m->nentries)
-      DVG_CUDA(cudaMemcpyAsync(m->entries, pb.entries[out], m->nentries * sizeof(uint32_t),
-                               cudaMemcpyDeviceToDevice, ctx->stream));
-    dfree(ctx, pb.entries[out]);
-  } else {
-    m->entries = pb.entries[out];
-  }
+  m->entries = pb.entries[out];
   pb.live[out] = 0;
   release_build(ctx, pb);
+  try {
+    give_back(ctx, m, pb.cap[out]);  // the slack of the estimated capacity
+  } catch (...) {
+    free_matrix(ctx, m);
+    throw;
+  }
   return m;
 }
 

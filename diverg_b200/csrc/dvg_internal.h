@@ -85,6 +85,7 @@ struct dvg_context {
   double plan_growth = 3.0;           // planned builds: entry capacity per step / input entries
   int64_t opt_slots = 1;              // chains of products over graph-like input run in the row-slot format
   double slot_growth = 4.0;           // row-slot chains: ranges the arena holds / rows
+  double early_growth = 1.125;        // row-slot builds: ranges the result gets room for / rows
   double product_growth = 2.0;        // products with long A ranges: entry capacity / the larger input's entries
   uint64_t max_product_entries = 0;   // largest product output since the last reset (read-back path)
   int64_t opt_autotune = 1;           // batches: tune the row kernel per (window, size class)
@@ -144,6 +145,11 @@ dvg_matrix* adjacency_from_graph(dvg_context* ctx, uint32_t nnodes, const uint32
 // A device matrix owned by the context's allocator.
 dvg_matrix* new_matrix(dvg_context* ctx, uint32_t nrows, uint32_t ncols, uint64_t nentries);
 void free_matrix(dvg_context* ctx, dvg_matrix* m);
+// For a result written to an array of `cap` entries before its size was known: where
+// more than a quarter of them (and 1 MiB) stays empty, its entries move to an array of
+// their size.  Returns whether they do (on the stream: not waited for).  Short of
+// memory, they stay.
+bool give_back(dvg_context* ctx, dvg_matrix* m, uint64_t cap);
 
 // Kernel timing with CUDA events on ctx->stream (active with the "timing"
 // option): span_begin records a start event, span_end its end and the kind.

@@ -48,8 +48,12 @@ constexpr uint32_t kSmallRows = 1u << 17;     // rows up to which a pass is one 
 constexpr double kChainReach = 1.28;          // branching * steps of a pass's left factors
 // A result of up to so many rows gets room for two ranges a row and is written
 // before its size is known, so that the host waits once.  A second wait and the
-// gap before it are 20 us: from 2^24 rows on, under 3 % of a product.
+// gap before it are 20 us: from 2^24 rows on, under 3 % of a product.  An index, which
+// its holder keeps, gets room for an eighth more ranges a row than the context's last
+// one had, and kEarlySpare: rows of windows that a graph's runs fill are one range.
 constexpr uint32_t kEarlyRows = 1u << 24;
+constexpr double kEarlySlack = 1.125;
+constexpr uint64_t kEarlySpare = 1u << 16;
 // Up to so many rows, and for single products as long as their results are written
 // early, the chain's kernels are launched close behind one another: the next one's
 // blocks are placed while the kernel before ends, 2 us a kernel.  Builds of
@@ -1334,7 +1338,7 @@ static SlotPart whole(const dvg_matrix* a) {
 }
 
 static dvg_matrix* run_slots(dvg_context* ctx, const SlotPlan& plan, const dvg_matrix* a, const dvg_matrix* b,
-                             bool* settled) {
+                             bool build, bool* settled) {
   SlotBuild sb;
   try {
     sb = prepare_slots(ctx, plan, a->nrows);
@@ -1343,6 +1347,7 @@ static dvg_matrix* run_slots(dvg_context* ctx, const SlotPlan& plan, const dvg_m
     return nullptr;
   }
   dvg_matrix* m = nullptr;
+  if (build) sb.early = std::min(sb.early, uint64_t(ctx->early_growth * double(a->nrows)) + kEarlySpare);
   sb.close = a->nrows <= (plan.steps.size() == 1 ? kEarlyRows : kCloseRows);
   try {
     SlotParts parts{};
@@ -1375,16 +1380,22 @@ static dvg_matrix* run_slots(dvg_context* ctx, const SlotPlan& plan, const dvg_m
       free_matrix(ctx, m);
       m = nullptr;
     }
+    bool ended = m != nullptr;
     if (m) {
       if (c.ctl.status)
         throw Error(DVG_ERR_DEVICE, "row slots: a result and its counts differ (code " + std::to_string(c.ctl.status) + ")");
-      if (settled) *settled = true;
     } else if (whole_chain) {
       out(c.ctl.total / 2, nullptr);
     }
     if (m) {
+      const uint64_t room = m->nentries;
       m->nentries = c.ctl.total;
       m->nnz = c.ctl.nnz;
+      if (build) {
+        ctx->early_growth = std::clamp(kEarlySlack * double(c.ctl.total / 2) / double(a->nrows), kEarlySlack, 2.0);
+        if (give_back(ctx, m, room)) ended = false;
+      }
+      if (settled) *settled = ended;
     }
   } catch (...) {
     free_matrix(ctx, m);
@@ -1395,8 +1406,8 @@ static dvg_matrix* run_slots(dvg_context* ctx, const SlotPlan& plan, const dvg_m
   return m;
 }
 
-dvg_matrix* slots_chain(dvg_context* ctx, const dvg_matrix* a, unsigned dlo, unsigned dup, bool* settled) {
-  return run_slots(ctx, plan_slots(dlo, dup, branching(a->nnz, a->nrows)), a, nullptr, settled);
+dvg_matrix* slots_chain(dvg_context* ctx, const dvg_matrix* a, unsigned dlo, unsigned dup, bool build, bool* settled) {
+  return run_slots(ctx, plan_slots(dlo, dup, branching(a->nnz, a->nrows)), a, nullptr, build, settled);
 }
 
 bool slots_product_suits(const dvg_context* ctx, const dvg_matrix* a, const dvg_matrix* b) {
@@ -1415,7 +1426,7 @@ dvg_matrix* slots_product(dvg_context* ctx, const dvg_matrix* a, const dvg_matri
   st.bits = 2;
   st.c = pl.out;
   pl.steps.push_back(st);
-  return run_slots(ctx, pl, a, a == b ? nullptr : b, settled);
+  return run_slots(ctx, pl, a, a == b ? nullptr : b, false, settled);
 }
 
 }  // namespace dvg

@@ -96,7 +96,9 @@ void release_slots(dvg_context* ctx, SlotBuild& sb);
 
 // The chain over `a`, waited for once; null when it did not fit its arena.  Sets
 // *settled where that wait has seen all of the result's kernels end, and checked them.
-dvg_matrix* slots_chain(dvg_context* ctx, const dvg_matrix* a, unsigned dlo, unsigned dup, bool* settled);
+// `build`: an index, which holds no more memory than it needs; a power or a product
+// keeps the room that was made for it.
+dvg_matrix* slots_chain(dvg_context* ctx, const dvg_matrix* a, unsigned dlo, unsigned dup, bool build, bool* settled);
 
 // A B alone, where that is faster than the range-CRS row kernel; null and
 // *settled likewise.

@@ -69,3 +69,40 @@ def test_a_wrong_column_count_changes_no_route(form):
             ctx.close()
             del keep
         assert all(route == seen[0][1] for _, route in seen), (what, seen)
+
+
+def used_bytes(ctx):
+    """Device memory in use from CUDA's pool (what contexts allocate from), their caches given back."""
+    from cuda.bindings import runtime as rt
+    ctx.trim()
+    err, pool = rt.cudaDeviceGetDefaultMemPool(0)
+    assert int(err) == 0
+    err, used = rt.cudaMemPoolGetAttribute(pool, rt.cudaMemPoolAttr.cudaMemPoolAttrUsedMemCurrent)
+    assert int(err) == 0
+    return int(used)
+
+
+def block(nbytes):
+    """The size of the block that holds nbytes (the allocator's classes)."""
+    nbytes = (nbytes + 255) // 256 * 256
+    if nbytes <= 1 << 20:
+        return nbytes
+    step = 1 << (nbytes.bit_length() - 3)
+    return (nbytes + step - 1) // step * step
+
+
+@pytest.mark.parametrize("bases,window", [(3_000_000, (400, 600)), (3_000_000, (7, 9)), (40_000, (100, 300))])
+def test_an_index_holds_no_more_than_it_needs(ctx, bases, window):
+    # at most a quarter and 1 MiB more than its entries, whichever route built it
+    a, _ = gen.graph_adjacency(gen.chromosome_graph_spec(bases, seed=84))
+    d = ctx.upload(a)
+    for slots in (1, 0, 1):
+        ctx.set_option("row_slots", slots)
+        ctx.distance_index(d, *window).free()
+        before = used_bytes(ctx)
+        m = ctx.distance_index(d, *window)
+        held = used_bytes(ctx) - before
+        # (a cached block of up to a quarter more may serve the entries)
+        most = block(8 * (m.nrows + 1) + 16) + 5 * block(5 * m.nentries + (1 << 20) + 16) // 4
+        assert held <= most, (slots, held, most)
+        m.free()
