@@ -41,6 +41,9 @@ constexpr int kWWarps = kWThreads / 32;
 constexpr int kSRows = 4;       // rows a lane of k_chain_rows takes
 constexpr int kSRuns = 8;       // runs of a lane's list
 constexpr int kSWin = 256;      // window words of a warp (8,192 columns)
+// A lane's list walk names at most so many columns a factor; the 32 lanes of a warp
+// share the columns of a row of more.
+constexpr uint32_t kLaneColumns = 256;
 constexpr uint32_t kMulti = kSlotMulti;
 constexpr uint32_t kMultiMax = 0xFFFFFFFFu - kMulti - 1;  // ranges of one row
 constexpr uint32_t kCountRows = 32 * kSRows;  // rows whose ranges the last pass counts together
@@ -121,6 +124,9 @@ struct ChainArgs {
   unsigned long long* abort;  // set when the arena is full: the rows that did not fit are left
                               // empty, so that later passes stay in bounds, and the host drops the result
   uint32_t* masks;            // bit r % 32 of word r / 32: k_chain_rows left row r to k_chain_walk
+  uint32_t* queue;            // this pass's rows that a warp walks, + 1 (0: not there yet), and
+  uint32_t* taken;            // how many places were taken (taken[0]) and filled (taken[1])
+  uint32_t queue_cap;
   uint32_t* group_cnt;        // last pass: ranges and columns of c per kCountRows rows
   unsigned long long* group_nnz;
   uint32_t n;
@@ -241,13 +247,20 @@ __device__ __forceinline__ uint32_t chain_rows(const ChainArgs& p, uint32_t r0, 
 
 // A warp's shared memory: the rows it walks next, and the lists of its
 // walks (entry k of lane t at [k * 32 + t]) or, for rows of more runs than
-// those hold, a bitmap window.
+// those hold, a row's bitmaps (bitmap_row) or a bitmap window (warp_union).
+constexpr int kRowWords = 320;  // words of S_j: 10,240 columns
+constexpr int kSumWords = 384;  // and of c: 12,288 columns
+constexpr uint32_t kRowBack = 64 * 32;  // columns that a bitmap has before the first one it gets
 struct WarpSmem {
   union {
     uint2 list[3][kSRuns * 32];
     struct {
       uint32_t bits[kSWin], reach[kSWin];
     } win;
+    struct {
+      uint32_t s[2][kRowWords], c[kSumWords];
+      uint16_t cols[32 * 32];
+    } row;
   };
   uint32_t todo[32];
 };
@@ -284,12 +297,15 @@ __device__ __noinline__ uint32_t list_merge(uint2* L, uint32_t nr, uint2 v) {
 }
 
 // The nd runs at D |= the rows of `mat` that the ns runs at L name (mat null:
-// the runs themselves).  Returns their new number, or kFull.
+// the runs themselves).  Returns their new number, or kFull: too many runs, or too
+// many columns for one lane.
 __device__ __noinline__ uint32_t list_product(const uint2* arena, const uint2* L, uint32_t ns, const uint2* mat,
                                               uint2* D, uint32_t nd) {
   uint2 run = empty_slot();
+  uint32_t named = 0;
   for (uint32_t k = 0; k < ns; ++k) {
     const uint2 a = L[k * 32];
+    if (mat && (named += min(a.y - a.x, kLaneColumns) + 1) > kLaneColumns) return kFull;
     for (uint32_t x = a.x; x <= a.y; ++x) {
       const uint2 s = mat ? ld_slot(mat, x) : a;
       const uint32_t c = slot_count(s);
@@ -450,19 +466,27 @@ __device__ uint2 warp_union(const ChainArgs& p, uint2 left, const uint2* mat, ui
         for (uint32_t t = 0; t < c; ++t) f(range(s, t));
       }
     };
-    if (is_run(left)) {  // one long range: a lane takes single rows
-      rows(uint64_t(left.x) + lane, left.y, 32);
-    } else {  // a lane takes whole ranges of the left row
-      const uint32_t c = slot_count(left);
-      for (uint32_t t = lane; t < c; t += 32) {
-        const uint2 r = range(left, t);
-        rows(r.x, r.y, 1);
+    // a lane takes whole short ranges of the left row; the warp shares the long ones
+    const uint32_t c = slot_count(left);
+    for (uint32_t t0 = 0; t0 < c; t0 += 32) {
+      const uint2 r = t0 + lane < c ? range(left, t0 + lane) : empty_slot();
+      const bool is_long = is_run(r) && r.y - r.x >= 32;
+      if (is_run(r) && !is_long) rows(r.x, r.y, 1);
+      for (unsigned m = __ballot_sync(kFullMask, is_long); m; m &= m - 1) {
+        const int q = __ffs(m) - 1;
+        const uint32_t x = __shfl_sync(kFullMask, r.x, q), y = __shfl_sync(kFullMask, r.y, q);
+        rows(uint64_t(x) + lane, y, 32);
       }
     }
   };
-  uint32_t first = 0xffffffffu;
-  each([&](uint2 v) { first = min(first, v.x); });
-  first = group_min<32>(kFullMask, first);
+  uint32_t first = 0xffffffffu, end = 0;
+  each([&](uint2 v) {
+    first = min(first, v.x);
+    end = max(end, v.y);
+  });
+  __syncwarp();
+  first = __reduce_min_sync(kFullMask, first);
+  end = __reduce_max_sync(kFullMask, end);
   if (first == 0xffffffffu) return empty_slot();
   uint64_t off = 0;
   uint32_t total = 0;
@@ -472,7 +496,9 @@ __device__ uint2 warp_union(const ChainArgs& p, uint2 left, const uint2* mat, ui
     uint32_t next = first;
     while (next != 0xffffffffu) {
       const uint64_t cb = next & ~31u, ce = cb + 32ull * kSWin - 1;
-      for (uint32_t w = lane; w < uint32_t(kSWin); w += 32) bits[w] = reach[w] = 0;
+      // the words that the union can cover, in whole turns of the warp
+      const uint32_t words = min(uint32_t(kSWin), uint32_t((end - cb) / 1024 + 1) * 32);
+      for (uint32_t w = lane; w < words; w += 32) bits[w] = reach[w] = 0;
       __syncwarp();
       uint32_t after = 0xffffffffu;  // the first covered column past the window
       each([&](uint2 v) {
@@ -492,7 +518,7 @@ __device__ uint2 warp_union(const ChainArgs& p, uint2 left, const uint2* mat, ui
       after = group_min<32>(kFullMask, after);
       __syncwarp();
       uint32_t run_reach = 0;
-      for (uint32_t wb = 0; wb < uint32_t(kSWin); wb += 32) {
+      for (uint32_t wb = 0; wb < words; wb += 32) {
         const uint32_t w = wb + lane;
         uint32_t x = bits[w];
         const uint32_t rr = max(group_incl_max<32>(kFullMask, reach[w], lane), run_reach);
@@ -536,11 +562,220 @@ __device__ uint2 warp_union(const ChainArgs& p, uint2 left, const uint2* mat, ui
   return total == 1 ? __ldcg(p.arena + off) : make_uint2(kMulti + total, uint32_t(off));
 }
 
+// The slot of the row whose columns from `base` on the words lo .. hi of W hold, the
+// first and the last of them not empty (lo > hi: no column), by a warp; its ranges and
+// columns to `cnt` and `nnz`.  All uniform but nnz, a lane's share.
+__device__ __forceinline__ uint2 bitmap_slot(const ChainArgs& p, const uint32_t* W, uint32_t base, uint32_t lo,
+                                             uint32_t hi, uint32_t& cnt, unsigned long long& nnz) {
+  const int lane = lane_id();
+  cnt = 0;
+  if (lo > hi) return empty_slot();
+  // a lane's word of 32, and the first and last columns of its runs
+  auto word = [&](uint32_t w, uint32_t& starts, uint32_t& ends) {
+    const uint32_t x = w <= hi ? W[w] : 0u;
+    starts = x & ~(x << 1 | (x && w > lo ? W[w - 1] >> 31 : 0u));
+    ends = x & ~(x >> 1 | (x && w < hi ? W[w + 1] << 31 : 0u));
+    return x;
+  };
+  for (uint32_t g = lo; g <= hi; g += 32) {
+    uint32_t starts, ends;
+    nnz += __popc(word(g + lane, starts, ends));
+    cnt += __popc(starts);
+  }
+  cnt = __reduce_add_sync(kFullMask, cnt);
+  if (cnt == 1) return make_uint2(base + 32 * lo + __ffs(W[lo]) - 1, base + 32 * hi + 31 - __clz(W[hi]));
+  unsigned long long off = 0;
+  if (lane == 0) off = atomicAdd(p.top, (unsigned long long)cnt);
+  off = __shfl_sync(kFullMask, off, 0);
+  if (off + cnt > p.arena_cap) {
+    if (lane == 0) atomicOr(p.abort, 1ull);
+    cnt = 0;
+    return empty_slot();
+  }
+  uint32_t k = 0, q = 0;
+  for (uint32_t g = lo; g <= hi; g += 32) {
+    uint32_t starts, ends;
+    word(g + lane, starts, ends);
+    // (starts and ends up to this lane's word, 16 bits each: a turn has at most 512)
+    const uint32_t mine = __popc(starts) | __popc(ends) << 16;
+    const uint32_t incl = group_incl_sum<32>(kFullMask, mine, lane), all = __shfl_sync(kFullMask, incl, 31);
+    const uint32_t col = base + 32 * (g + lane);
+    uint32_t a = k + ((incl - mine) & 0xffffu), b = q + ((incl - mine) >> 16);
+    for (; starts; starts &= starts - 1) p.arena[off + a++].x = col + uint32_t(__ffs(starts) - 1);
+    for (; ends; ends &= ends - 1) p.arena[off + b++].y = col + uint32_t(__ffs(ends) - 1);
+    k += all & 0xffffu;
+    q += all >> 16;
+  }
+  return make_uint2(kMulti + cnt, uint32_t(off));
+}
+
+// A row by a warp: S_j and c as bitmaps in shared memory, each from a column a little
+// before the first one that it gets.  The columns of S_j are laid out in a list, and a
+// lane takes every 32nd of them: its rows of the factor and of B are requested together,
+// so that a factor is one trip to memory for 32 columns (two, for rows in the arena).
+// False where the columns lie further apart than the bitmaps reach.
+//
+// Bound: those trips, about 1.5 us a factor.  Unions by windows instead (warp_union)
+// read every row three times and scan up to 8,192 columns twice, 8 us each and one for
+// every S_j and sum, all of them kept in the arena.
+template <bool OUTS, bool OUTC>
+__device__ bool bitmap_row(const ChainArgs& p, WarpSmem& M, uint32_t row, uint2& s, uint2& c, uint32_t& nc,
+                           unsigned long long& z) {
+  const int lane = lane_id();
+  uint32_t *S = M.row.s[0], *T = M.row.s[1], *const C = M.row.c;
+  for (uint32_t w = lane; w < uint32_t(kSumWords); w += 32) C[w] = 0;
+  uint32_t sbase = row & ~31u, s_lo = 0, s_hi = 0;  // S's first column; its words that hold any
+  if (lane == 0) S[0] = 1u << (row & 31u);
+  uint32_t cbase = 0, c_lo = 0xffffffffu, c_hi = 0;
+  bool c_any = false;
+  __syncwarp();
+#pragma unroll 1
+  for (uint32_t j = 0;; ++j) {
+    const bool gather = OUTC && ((p.bits >> j) & 1u), go = j < p.k;
+    if (!gather && !go) break;
+    const uint2* mat = go ? p.m[j] : nullptr;
+    for (uint32_t w = lane; go && w < uint32_t(kRowWords); w += 32) T[w] = 0;
+    uint32_t tbase = 0, t_lo = 0xffffffffu, t_hi = 0;
+    bool t_any = false, ok = true;
+    // where a bitmap begins that gets these ranges first
+    auto place = [&](bool has, uint2 v, uint32_t& base, bool& any) {
+      const uint32_t first = __reduce_min_sync(kFullMask, has ? v.x : 0xffffffffu);
+      if (first == 0xffffffffu) return;
+      base = (first & ~31u) > kRowBack ? (first & ~31u) - kRowBack : 0u;
+      any = true;
+    };
+    auto put = [&](uint32_t* W, uint32_t words, uint32_t base, uint2 v, uint32_t& lo, uint32_t& hi) {
+      if (v.x < base || (v.y - base) / 32 >= words) {
+        ok = false;
+        return;
+      }
+      const uint32_t a = v.x - base, b = v.y - base, wa = a / 32, wb = b / 32;
+      for (uint32_t w = wa; w <= wb; ++w)
+        atomicOr(W + w, (w == wa ? ~0u << (a & 31) : ~0u) & (w == wb ? ~0u >> (31 - (b & 31)) : ~0u));
+      lo = min(lo, wa);
+      hi = max(hi, wb);
+    };
+    for (uint32_t g = s_lo; g <= s_hi; g += 32) {
+      uint32_t w = g + lane <= s_hi ? S[g + lane] : 0u;
+      const uint32_t incl = group_incl_sum<32>(kFullMask, uint32_t(__popc(w)), lane);
+      const uint32_t total = __shfl_sync(kFullMask, incl, 31);
+      uint32_t at = incl - __popc(w);
+      for (; w; w &= w - 1) M.row.cols[at++] = uint16_t(32 * (g + lane) + __ffs(w) - 1);
+      __syncwarp();
+      for (uint32_t t0 = 0; t0 < total; t0 += 32) {
+        const bool have = t0 + lane < total;
+        const uint32_t x = have ? sbase + M.row.cols[t0 + lane] : 0u;
+        const uint2 sm = have && go ? ld_slot(mat, x) : empty_slot();
+        const uint2 sb = have && gather ? (p.b ? ld_slot(p.b, x) : make_uint2(x, x)) : empty_slot();
+        const uint32_t nm = slot_count(sm), nb = slot_count(sb);
+        const uint2 m0 = nm ? slot_range(p.arena, sm, 0) : empty_slot();
+        const uint2 b0 = nb ? slot_range(p.arena, sb, 0) : empty_slot();
+        if (go && !t_any) place(nm != 0, m0, tbase, t_any);
+        if (gather && !c_any) place(nb != 0, b0, cbase, c_any);
+        if (nm) put(T, kRowWords, tbase, m0, t_lo, t_hi);
+        for (uint32_t q = 1; q < nm; ++q) put(T, kRowWords, tbase, slot_range(p.arena, sm, q), t_lo, t_hi);
+        if (nb) put(C, kSumWords, cbase, b0, c_lo, c_hi);
+        for (uint32_t q = 1; q < nb; ++q) put(C, kSumWords, cbase, slot_range(p.arena, sb, q), c_lo, c_hi);
+        __syncwarp();
+      }
+      __syncwarp();
+    }
+    if (!__all_sync(kFullMask, ok)) return false;
+    if (!go) break;
+    uint32_t* const last = S;
+    S = T;
+    T = last;
+    sbase = tbase;
+    s_lo = __reduce_min_sync(kFullMask, t_lo);  // (no column: past s_hi, nothing is read)
+    s_hi = __reduce_max_sync(kFullMask, t_hi);
+    __syncwarp();
+  }
+  uint32_t ns = 0;
+  unsigned long long zs = 0;
+  if (OUTS) s = bitmap_slot(p, S, sbase, s_lo, s_hi, ns, zs);
+  if (OUTC) {
+    c_lo = __reduce_min_sync(kFullMask, c_lo);
+    c_hi = __reduce_max_sync(kFullMask, c_hi);
+    c = bitmap_slot(p, C, cbase, c_lo, c_hi, nc, z);
+    z = group_sum<32>(kFullMask, z);
+  }
+  __syncwarp();
+  return true;
+}
+
+// A row by the whole warp, however many runs it has; c's ranges and columns.  (A
+// function of its own, so that its registers are not the lanes' walks'.)
+struct RowCount {
+  uint32_t ranges;
+  unsigned long long columns;
+};
+template <bool OUTS, bool OUTC>
+__device__ __noinline__ RowCount warp_row(const ChainArgs& p, WarpSmem& S, uint32_t r) {
+  const int lane = lane_id();
+  uint2 s = make_uint2(r, r), c = empty_slot();
+  uint32_t k = 0;
+  unsigned long long z = 0;
+  if (!bitmap_row<OUTS, OUTC>(p, S, r, s, c, k, z)) {
+    __syncwarp();
+    s = make_uint2(r, r);
+    c = empty_slot();
+    for (uint32_t j = 0;; ++j) {
+      if (OUTC && ((p.bits >> j) & 1u))
+        c = p.b ? warp_union(p, s, p.b, c, empty_slot(), S.win.bits, S.win.reach)
+                : warp_union(p, s, nullptr, c, s, S.win.bits, S.win.reach);
+      if (j == p.k) break;
+      s = warp_union(p, s, p.m[j], empty_slot(), empty_slot(), S.win.bits, S.win.reach);
+    }
+    k = OUTC ? slot_count(c) : 0;
+    z = 0;
+    for (uint32_t q = lane; q < k; q += 32) {
+      const uint2 v = is_multi(c) ? __ldcg(p.arena + c.y + q) : slot_range(p.arena, c, q);
+      z += v.y - v.x + 1;
+    }
+    z = group_sum<32>(kFullMask, z);
+  }
+  if (OUTS && lane == 0) p.s[r] = s;
+  if (OUTC && lane == 0) p.c[r] = c;
+  __syncwarp();
+  return {k, z};
+}
+
+// Rows that a lane cannot walk are put into the pass's queue, and other warps take rows
+// from it, one at a time, when their own are done: they come in clumps, all 32 of a batch
+// of them, and one after another in their warp would be what the pass lasts.  A^300 of
+// 1e6 bases of a variant-dense graph, 4,172 such rows: 9.9 ms by unions of windows in
+// the row's own warp, 1.2 by bitmaps through the queue; A^100, 52 such rows: 1.72 ms and
+// 0.25; the build for [1000, 1300], 1,910: 4.3 and 0.86.  Where no row needs it, the queue
+// and its clearing cost 3 % of a build of 1e5 bases (152 -> 157 us).  Nobody
+// waits: a place is settled by one exchange each of the warp that puts a row in and of
+// the one that takes it, and where the taker comes first (kGone) the row stays with
+// the warp that had it.  A look into the queue is a trip to memory, at the end of a
+// pass: a warp whose own rows were all quick ones is done before others put rows in,
+// and does not look.
+constexpr uint32_t kGone = 0xffffffffu;
+template <bool OUTS, bool OUTC, class Tally>
+__device__ void take_rows(const ChainArgs& p, WarpSmem& S, Tally&& tally) {
+  for (;;) {
+    const uint2 places = __ldcg(reinterpret_cast<const uint2*>(p.taken));
+    if (__shfl_sync(kFullMask, places.x, 0) >= min(__shfl_sync(kFullMask, places.y, 0), p.queue_cap)) return;
+    uint32_t r = 0;  // row + 1
+    if (lane_id() == 0) {
+      const uint32_t at = atomicAdd(p.taken, 1u);
+      if (at < p.queue_cap) r = atomicExch(p.queue + at, kGone);
+    }
+    r = __shfl_sync(kFullMask, r, 0);
+    if (r == 0) continue;
+    const RowCount n = warp_row<OUTS, OUTC>(p, S, r - 1);
+    if (lane_id() == 0 && n.ranges) tally(r - 1, n.ranges, n.columns);
+  }
+}
+
 // Walks the `batch` rows of the warp's list, a row a lane; rows of more runs
-// than a lane's lists hold go to the whole warp.
+// than a lane's lists hold go to the queue (take_rows), or to the whole warp at once
+// where that is full.  Whether some of them were no quick ones.
 // tally(row, ranges, columns) for each row of c that has any.
 template <bool OUTS, bool OUTC, class Tally>
-__device__ __forceinline__ void walk_batch(const ChainArgs& p, WarpSmem& S, uint32_t batch, Tally&& tally) {
+__device__ __forceinline__ bool walk_batch(const ChainArgs& p, WarpSmem& S, uint32_t batch, Tally&& tally) {
   const int lane = lane_id();
   uint32_t row = 0, ns = 0, nc = 0, cur = 0;
   bool done = false;
@@ -549,7 +784,7 @@ __device__ __forceinline__ void walk_batch(const ChainArgs& p, WarpSmem& S, uint
     row = S.todo[lane];
     done = quick_row<OUTS, OUTC>(p, row, S.list[0] + lane, ns, C, nc);
   }
-  __syncwarp();
+  const bool look = __any_sync(kFullMask, uint32_t(lane) < batch && !done);
   if (uint32_t(lane) < batch && !done) {
     S.list[0][lane] = make_uint2(row, row);
     ns = 1;
@@ -605,31 +840,23 @@ __device__ __forceinline__ void walk_batch(const ChainArgs& p, WarpSmem& S, uint
     }
   }
   __syncwarp();
-  if (left && lane == 0) atomicAdd(&p.ctl->slow_rows, (unsigned long long)__popc(left));
+  if (left) {
+    uint32_t at = 0;
+    if (lane == 0) {
+      atomicAdd(&p.ctl->slow_rows, (unsigned long long)__popc(left));
+      at = atomicAdd(p.taken + 1, uint32_t(__popc(left)));
+    }
+    at = __shfl_sync(kFullMask, at, 0) + __popc(left & ((1u << lane) - 1u));
+    const bool queued = ((left >> lane) & 1u) && at < p.queue_cap && atomicExch(p.queue + at, row + 1) != kGone;
+    left &= ~__ballot_sync(kFullMask, queued);
+  }
   for (; left; left &= left - 1) {
     const uint32_t r = __shfl_sync(kFullMask, row, __ffs(left) - 1);
-    uint2 s = make_uint2(r, r), c = empty_slot();
-    for (uint32_t j = 0;; ++j) {
-      if (OUTC && ((p.bits >> j) & 1u))
-        c = p.b ? warp_union(p, s, p.b, c, empty_slot(), S.win.bits, S.win.reach)
-                : warp_union(p, s, nullptr, c, s, S.win.bits, S.win.reach);
-      if (j == p.k) break;
-      s = warp_union(p, s, p.m[j], empty_slot(), empty_slot(), S.win.bits, S.win.reach);
-    }
-    if (OUTS && lane == 0) p.s[r] = s;
-    if (OUTC) {
-      if (lane == 0) p.c[r] = c;
-      const uint32_t k = slot_count(c);
-      unsigned long long z = 0;
-      for (uint32_t q = lane; q < k; q += 32) {
-        const uint2 v = is_multi(c) ? __ldcg(p.arena + c.y + q) : slot_range(p.arena, c, q);
-        z += v.y - v.x + 1;
-      }
-      z = group_sum<32>(kFullMask, z);
-      if (lane == 0 && k) tally(r, k, z);
-    }
+    const RowCount n = warp_row<OUTS, OUTC>(p, S, r);
+    if (lane == 0 && n.ranges) tally(r, n.ranges, n.columns);
   }
   __syncwarp();
+  return look;
 }
 
 // The kernels of a chain follow one another closely: each waits for the kernel before
@@ -649,7 +876,8 @@ __device__ __forceinline__ void follow() {
 // are in flight to keep HBM busy, and leaves the other rows marked in a
 // bitmap.  k_chain_walk reads the bitmap and walks those, 32 at a time, a row a
 // lane, so that no lane waits for another's longer row and a walk's chain of
-// dependent loads is paid once for 32 rows.
+// dependent loads is paid once for 32 rows; the rows that need a warp go through a
+// queue (take_rows).
 //
 // Bound: HBM, 8 bytes a row for each matrix read and written (all but the first
 // read of a matrix come from L2).  k_chain_rows on 1e7 rows: 51 to 72 us for
@@ -699,6 +927,12 @@ __global__ void __launch_bounds__(kWThreads) k_chain_walk(const __grid_constant_
   // a warp's words lie a grid's width apart, so that each gets its share
   const uint64_t words = (uint64_t(p.n) + 31) / 32, stride = gridDim.x * kWWarps;
   uint64_t next = blockIdx.x * kWWarps + warp;
+  auto tally = [&](uint32_t row, uint32_t cnt, unsigned long long nnz) {
+    if (!COUNT) return;
+    atomicAdd(p.group_cnt + row / kCountRows, cnt);
+    atomicAdd(p.group_nnz + row / kCountRows, nnz);
+  };
+  bool look = false;
   uint32_t x = 0, at = 0;  // a lane's word: its rows still to walk, and the first of its 32
   while (true) {
     const unsigned spent = __ballot_sync(kFullMask, x == 0);
@@ -717,12 +951,9 @@ __global__ void __launch_bounds__(kWThreads) k_chain_walk(const __grid_constant_
     uint32_t k = group_incl_sum<32>(kFullMask, uint32_t(__popc(x)), lane) - __popc(x);
     for (; x && k < 32; x &= x - 1) S.todo[k++] = at + uint32_t(__ffs(x) - 1);
     __syncwarp();
-    walk_batch<OUTS, OUTC>(p, S, min(have, 32u), [&](uint32_t row, uint32_t cnt, unsigned long long nnz) {
-      if (!COUNT) return;
-      atomicAdd(p.group_cnt + row / kCountRows, cnt);
-      atomicAdd(p.group_nnz + row / kCountRows, nnz);
-    });
+    if (walk_batch<OUTS, OUTC>(p, S, min(have, 32u), tally)) look = true;
   }
+  if (look) take_rows<OUTS, OUTC>(p, S, tally);
 }
 
 // A pass over a small matrix, where a launch costs more than the rows: both in
@@ -742,6 +973,7 @@ __global__ void __launch_bounds__(kWThreads) k_chain_small(const __grid_constant
   const uint64_t r0 = uint64_t(blockIdx.x) * kWThreads + warp * 32;
   unsigned long long nnz = 0;
   uint32_t cnt = 0;
+  bool look = false;
   if (r0 < p.n) {
     uint32_t bad;
     if (r0 + 32 <= p.n) bad = chain_rows<OUTS, OUTC, COUNT, 1>(p, uint32_t(r0), cnt, nnz);
@@ -750,11 +982,18 @@ __global__ void __launch_bounds__(kWThreads) k_chain_small(const __grid_constant
     if (bad) S.todo[__popc(who & ((1u << lane) - 1u))] = uint32_t(r0) + lane;
     __syncwarp();
     if (who)
-      walk_batch<OUTS, OUTC>(p, S, __popc(who), [&](uint32_t, uint32_t c, unsigned long long z) {
+      look = walk_batch<OUTS, OUTC>(p, S, __popc(who), [&](uint32_t, uint32_t c, unsigned long long z) {
         cnt += c;
         nnz += z;
       });
   }
+  // (any block's rows: the counts start at zero, and every block adds to them)
+  if (look)
+    take_rows<OUTS, OUTC>(p, S, [&](uint32_t row, uint32_t c, unsigned long long z) {
+      if (!COUNT) return;
+      atomicAdd(p.group_cnt + row / kCountRows, c);
+      atomicAdd(p.group_nnz + row / kCountRows, z);
+    });
   if (COUNT) {
     cnt = __reduce_add_sync(kFullMask, cnt);
     nnz = group_sum<32>(kFullMask, nnz);
@@ -764,8 +1003,8 @@ __global__ void __launch_bounds__(kWThreads) k_chain_small(const __grid_constant
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-      p.group_cnt[blockIdx.x] = uint32_t(sum[0]);
-      p.group_nnz[blockIdx.x] = sum[1];
+      atomicAdd(p.group_cnt + blockIdx.x, uint32_t(sum[0]));
+      atomicAdd(p.group_nnz + blockIdx.x, sum[1]);
     }
   }
 }
@@ -780,6 +1019,13 @@ struct Parts {
   SlotPart one;
 };
 __device__ __forceinline__ SlotPart my_part(const Parts& q) { return q.table ? q.table[q.part_of[blockIdx.x]] : q.one; }
+
+// The chain's first kernel: counters, places, queues and counts of its scratch start at zero.
+__global__ void __launch_bounds__(kSThreads) k_clear(uint4* words, uint32_t n) {
+  follow();
+  for (uint32_t w = blockIdx.x * kSThreads + threadIdx.x; w < n; w += gridDim.x * kSThreads)
+    words[w] = make_uint4(0u, 0u, 0u, 0u);
+}
 
 // Range CRS -> slots.  Canonical input: a row of several ranges is copied to
 // the arena as it is.  Rows past a part's last are rows of the identity: one
@@ -1179,8 +1425,12 @@ SlotBuild prepare_slots(dvg_context* ctx, const SlotPlan& plan, uint32_t n) {
   sb.mat.assign(plan.nmats, nullptr);
   const uint64_t groups = (uint64_t(n) + kCountRows - 1) / kCountRows;
   const uint64_t supers = (groups + kSuperGroups - 1) / kSuperGroups;
-  const size_t sums_off = 512, nnz_off = sums_off + supers * 8, cnt_off = nnz_off + groups * 8;
-  const size_t masks_off = cnt_off + groups * 4;
+  // a pass's rows to be walked by warps: room for its clumps (a row past it is walked at once)
+  sb.queue_cap = uint32_t(std::clamp<uint64_t>(n / 8, 256, 1u << 15));
+  auto round = [](size_t x) { return (x + 15) & ~size_t(15); };
+  const size_t taken_off = 512, queue_off = taken_off + plan.steps.size() * 8;
+  const size_t nnz_off = round(queue_off + plan.steps.size() * sb.queue_cap * 4), cnt_off = nnz_off + groups * 8;
+  const size_t sums_off = round(cnt_off + groups * 4), masks_off = sums_off + supers * 8;
   static_assert(sizeof(SlotCounters) <= 512, "the counters come first");
   std::vector<int> last(plan.nmats, -1);
   auto reads = [&](const SlotStep& s, auto&& f) {
@@ -1207,9 +1457,13 @@ SlotBuild prepare_slots(dvg_context* ctx, const SlotPlan& plan, uint32_t n) {
   try {
     sb.scratch = dalloc(ctx, masks_off + (uint64_t(n) + 31) / 32 * 4);
     char* base = static_cast<char*>(sb.scratch);
+    // (a large pass writes its counts, a small one's blocks add to them)
+    sb.cleared = n <= kSmallRows ? nnz_off + round(groups * 12) : nnz_off;
     sb.ctl = reinterpret_cast<DeviceControl*>(base);
     sb.top = reinterpret_cast<unsigned long long*>(base + 256);
     sb.abort = sb.top + 1;
+    sb.taken = reinterpret_cast<uint32_t*>(base + taken_off);
+    sb.queue = reinterpret_cast<uint32_t*>(base + queue_off);
     sb.sums = reinterpret_cast<unsigned long long*>(base + sums_off);
     sb.group_nnz = reinterpret_cast<unsigned long long*>(base + nnz_off);
     sb.group_cnt = reinterpret_cast<uint32_t*>(base + cnt_off);
@@ -1243,7 +1497,10 @@ void release_slots(dvg_context* ctx, SlotBuild& sb) {
 
 void launch_slots(dvg_context* ctx, SlotBuild& sb, const SlotParts& parts, bool timed, const SlotPart* right) {
   const uint64_t t0 = now_ns();
-  DVG_CUDA(cudaMemsetAsync(sb.scratch, 0, 512, ctx->stream));
+  // (a memset of more than a few KB is 4 us before the next kernel starts)
+  k_clear<<<unsigned(std::min<size_t>(sb.cleared / 4096 + 1, ctx->num_sms)), kSThreads, 0, ctx->stream>>>(
+      static_cast<uint4*>(sb.scratch), uint32_t(sb.cleared / 16));
+  DVG_CUDA(cudaGetLastError());
   ctx->stats.kernel_launches++;
   ChainArgs p{};
   p.arena = sb.arena;
@@ -1252,19 +1509,21 @@ void launch_slots(dvg_context* ctx, SlotBuild& sb, const SlotParts& parts, bool 
   p.ctl = sb.ctl;
   p.abort = sb.abort;
   p.masks = sb.masks;
+  p.queue_cap = sb.queue_cap;
   p.group_cnt = sb.group_cnt;
   p.group_nnz = sb.group_nnz;
   p.n = sb.n;
   p.s = sb.mat[0];
-  k_crs_to_slots<<<conversion_blocks(sb), kSThreads, 0, ctx->stream>>>(Parts{parts.table, parts.part_of, parts.one}, p);
-  DVG_CUDA(cudaGetLastError());
-  ctx->stats.kernel_launches++;
+  launch_next(ctx, sb.close, k_crs_to_slots, conversion_blocks(sb), kSThreads,
+              Parts{parts.table, parts.part_of, parts.one}, p);
   if (right) {
     p.s = sb.mat[1];
     launch_next(ctx, sb.close, k_crs_to_slots, conversion_blocks(sb), kSThreads, Parts{nullptr, nullptr, *right}, p);
   }
   for (size_t i = 0; i < sb.plan.steps.size(); ++i) {
     const SlotStep& st = sb.plan.steps[i];
+    p.taken = sb.taken + 2 * i;
+    p.queue = sb.queue + i * sb.queue_cap;
     p.k = uint32_t(st.k);
     p.bits = st.bits;
     for (int j = 0; j < kChainMax; ++j) p.m[j] = j < st.k ? sb.mat[st.m[j]] : nullptr;

@@ -67,7 +67,12 @@ struct SlotBuild {
   uint64_t arena_cap = 0;      // ranges
   bool close = false;          // the kernels' blocks are placed while the kernel before ends
   uint64_t early = 0;          // room for the result's ranges before their number is known; 0: none
-  void* scratch = nullptr;     // counters | sums of the counts | counts of the result | bitmap
+  // counters | places of each pass | queues | counts of the result | sums of the counts | bitmap
+  void* scratch = nullptr;
+  size_t cleared = 0;          // its first bytes, which the chain's first kernel clears
+  uint32_t queue_cap = 0;
+  uint32_t* taken = nullptr;
+  uint32_t* queue = nullptr;
   DeviceControl* ctl = nullptr;
   unsigned long long* top = nullptr;
   unsigned long long* abort = nullptr;
