@@ -683,7 +683,7 @@ dvg_matrix* create_distance_index(dvg_context* ctx, const dvg_matrix* a, unsigne
   // canonical only for canonical inputs, while the reference's squarings
   // canonicalise any input
   if (ctx->opt_dindex_schedule == 1 || (dlo == 0 && !a->canonical)) return distance_index_reference(ctx, a, dlo, dup);
-  if (ctx->opt_planned && ctx->opt_spgemm_mode == 0 && slots_suit(ctx, a)) {
+  if (ctx->opt_planned && ctx->opt_spgemm_mode == 0 && slots_suit(ctx, a) && slots_due(ctx, slot_key(dlo, dup, a))) {
     if (dvg_matrix* t = slots_chain(ctx, a, dlo, dup, true, settled)) return t;
     ctx->stats.spgemm_reruns++;
   }
@@ -1097,7 +1097,8 @@ dvg_status dvg_range_spgemm(dvg_context* ctx, const dvg_matrix* a, const dvg_mat
     require(a && b && c, "null argument");
     dvg_matrix* r = nullptr;
     bool settled = false;
-    if (ctx->opt_planned && ctx->opt_spgemm_mode == 0 && slots_product_suits(ctx, a, b)) {
+    if (ctx->opt_planned && ctx->opt_spgemm_mode == 0 && slots_product_suits(ctx, a, b) &&
+        slots_due(ctx, product_key(a, b))) {
       r = slots_product(ctx, a, b, &settled);
       if (!r) ctx->stats.spgemm_reruns++;
     }
@@ -1124,7 +1125,8 @@ dvg_status dvg_range_power(dvg_context* ctx, const dvg_matrix* a, unsigned k, dv
     // there is a single product, and with k = 0 none
     dvg_matrix* r = nullptr;
     bool settled = false;
-    if (k > 1 && ctx->opt_planned && ctx->opt_spgemm_mode == 0 && slots_suit(ctx, a)) {
+    if (k > 1 && ctx->opt_planned && ctx->opt_spgemm_mode == 0 && slots_suit(ctx, a) &&
+        slots_due(ctx, slot_key(k, k, a))) {
       r = slots_chain(ctx, a, k, k, false, &settled);
       if (!r) ctx->stats.spgemm_reruns++;
     }

@@ -278,6 +278,12 @@ void batch_distance_index(dvg_context* ctx, uint32_t ngraphs, const dvg_matrix* 
   // ---- validation and grouping -------------------------------------------------
   std::map<std::pair<unsigned, unsigned>, std::vector<uint32_t>> by_window, slots_by_window;
   std::vector<uint32_t> alone;  // built one by one (no rows, or non-canonical input with dmin = 0)
+  std::map<SlotKey, bool> due;  // (a batch counts as one call for all graphs that are alike)
+  auto is_due = [&](const SlotKey& key) {
+    auto it = due.find(key);
+    if (it == due.end()) it = due.emplace(key, slots_due(ctx, key)).first;
+    return it->second;
+  };
   for (uint32_t k = 0; k < ngraphs; ++k) {
     const dvg_matrix* a = graphs[k];
     require(a != nullptr, "batch: null graph");
@@ -288,10 +294,37 @@ void batch_distance_index(dvg_context* ctx, uint32_t ngraphs, const dvg_matrix* 
     if (a->nrows == 0 || (dmin[k] == 0 && !a->canonical) || !ctx->opt_planned || ctx->opt_spgemm_mode == 1 ||
         ctx->opt_dindex_schedule != 0)
       alone.push_back(k);
-    else if (ctx->opt_spgemm_mode == 0 && slots_suit(ctx, a))
+    else if (ctx->opt_spgemm_mode == 0 && slots_suit(ctx, a) && is_due(slot_key(dmin[k], dmax[k], a)))
       slots_by_window[{dmin[k], dmax[k]}].push_back(k);
     else
       by_window[{dmin[k], dmax[k]}].push_back(k);
+  }
+  std::vector<SlotGroup> chains;
+  for (auto& kv : slots_by_window) {
+    // at most as many rows as columns have numbers
+    uint64_t rows = 0;
+    for (uint32_t k : kv.second) {
+      const uint64_t n = (uint64_t(graphs[k]->nrows) + kSlotPartRows - 1) / kSlotPartRows * kSlotPartRows;
+      if (rows == 0 || rows + n >= kSlotMulti) {
+        chains.emplace_back();
+        rows = 0;
+      }
+      chains.back().dlo = kv.first.first;
+      chains.back().dup = kv.first.second;
+      chains.back().members.push_back(k);
+      rows += n;
+    }
+  }
+  for (auto& g : chains) lay_out(g, graphs);
+  for (auto it = chains.begin(); it != chains.end();) {
+    it->sb.key = slot_key(it->dlo, it->dup, it->nnz, it->n);
+    if (is_due(it->sb.key)) {
+      ++it;
+      continue;
+    }
+    auto& others = by_window[{it->dlo, it->dup}];  // together they were given up
+    others.insert(others.end(), it->members.begin(), it->members.end());
+    it = chains.erase(it);
   }
   std::vector<Group> groups;
   for (auto& kv : by_window) {
@@ -312,23 +345,6 @@ void batch_distance_index(dvg_context* ctx, uint32_t ngraphs, const dvg_matrix* 
     }
     if (!cur.members.empty()) groups.push_back(std::move(cur));
   }
-  std::vector<SlotGroup> chains;
-  for (auto& kv : slots_by_window) {
-    // at most as many rows as columns have numbers
-    uint64_t rows = 0;
-    for (uint32_t k : kv.second) {
-      const uint64_t n = (uint64_t(graphs[k]->nrows) + kSlotPartRows - 1) / kSlotPartRows * kSlotPartRows;
-      if (rows == 0 || rows + n >= kSlotMulti) {
-        chains.emplace_back();
-        rows = 0;
-      }
-      chains.back().dlo = kv.first.first;
-      chains.back().dup = kv.first.second;
-      chains.back().members.push_back(k);
-      rows += n;
-    }
-  }
-  for (auto& g : chains) lay_out(g, graphs);
   if (groups.empty() && chains.empty()) {
     try {
       for (uint32_t k : alone) out[k] = create_distance_index(ctx, graphs[k], dmin[k], dmax[k]);
@@ -363,7 +379,9 @@ void batch_distance_index(dvg_context* ctx, uint32_t ngraphs, const dvg_matrix* 
     // steps, on the one stream, still write; a chain beside them must not get one)
     for (auto it = chains.begin(); it != chains.end();) {
       try {
+        const SlotKey key = it->sb.key;
         it->sb = prepare_slots(ctx, plan_slots(it->dlo, it->dup, branching(it->nnz, it->n)), uint32_t(it->n));
+        it->sb.key = key;
         it->ready = true;
         ++it;
       } catch (const Error& e) {

@@ -54,6 +54,13 @@ struct TuneChoice {
   int64_t chunk_rows;  // 0: automatic
 };
 
+// What chains over row slots are alike in (slot_key), and, of one that was given up, how
+// many calls the next ones like it wait, and have still to (slots_missed).
+using SlotKey = std::tuple<unsigned, unsigned, int, int>;
+struct SlotMiss {
+  uint32_t wait = 0, left = 0;
+};
+
 struct dvg_context {
   int device = 0;
   int num_sms = 0;
@@ -85,6 +92,7 @@ struct dvg_context {
   double plan_growth = 3.0;           // planned builds: entry capacity per step / input entries
   int64_t opt_slots = 1;              // chains of products over graph-like input run in the row-slot format
   double slot_growth = 4.0;           // row-slot chains: ranges the arena holds / rows
+  std::map<SlotKey, SlotMiss> slot_misses;
   double early_growth = 1.125;        // row-slot builds: ranges the result gets room for / rows
   double product_growth = 2.0;        // products with long A ranges: entry capacity / the larger input's entries
   uint64_t max_product_entries = 0;   // largest product output since the last reset (read-back path)

@@ -26,6 +26,7 @@
 // 5.0e7 loci, window [400, 600]: 23.05 -> 2.65 ms; 1e6 loci, [0, 250]: 1.26 ->
 // 0.21 ms; 1e5 loci of a variant-dense graph, [100, 300]: 1.01 -> 0.145 ms.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 
 #include "dvg_device.cuh"
@@ -46,6 +47,14 @@ constexpr int kSWin = 256;      // window words of a warp (8,192 columns)
 constexpr uint32_t kLaneColumns = 256;
 constexpr uint32_t kMulti = kSlotMulti;
 constexpr uint32_t kMultiMax = 0xFFFFFFFFu - kMulti - 1;  // ranges of one row
+constexpr unsigned long long kArenaFull = 1, kLongRow = 2, kWideRows = 4;  // why a chain is given up
+// Unions by windows cost a warp about 1 us for every 32 rows that they name and window
+// that they fill, twice.  A chain may spend kWideCost and a sixteenth of its rows on
+// them, and one union name kWideColumns: a few rows that reach far cost little, but with
+// one range of 20,000 columns in 2e5 rows a build for [100, 300] took 364 ms, in range
+// CRS 58.
+constexpr uint64_t kWideCost = 1u << 14;
+constexpr uint32_t kWideColumns = 1u << 12;
 constexpr uint32_t kCountRows = 32 * kSRows;  // rows whose ranges the last pass counts together
 constexpr uint32_t kSmallRows = 1u << 17;     // rows up to which a pass is one kernel
 constexpr double kChainReach = 1.28;          // branching * steps of a pass's left factors
@@ -57,6 +66,7 @@ constexpr double kChainReach = 1.28;          // branching * steps of a pass's l
 constexpr uint32_t kEarlyRows = 1u << 24;
 constexpr double kEarlySlack = 1.125;
 constexpr uint64_t kEarlySpare = 1u << 16;
+constexpr double kSlotGrowthMax = 8.0;  // ranges a row that an arena is made for
 // Up to so many rows, and for single products as long as their results are written
 // early, the chain's kernels are launched close behind one another: the next one's
 // blocks are placed while the kernel before ends, 2 us a kernel.  Builds of
@@ -121,8 +131,12 @@ struct ChainArgs {
   unsigned long long* top;    // ranges taken from the arena
   uint64_t arena_cap;
   DeviceControl* ctl;
-  unsigned long long* abort;  // set when the arena is full: the rows that did not fit are left
-                              // empty, so that later passes stay in bounds, and the host drops the result
+  // Why the chain is given up (kArenaFull, ...), 0: it is not.  The host drops the result;
+  // until then rows that did not fit, and all that are yet to be walked, are left empty, so
+  // that later passes stay in bounds and are over soon.
+  unsigned long long* abort;
+  unsigned long long* wide;   // what unions by windows have cost, and may
+  unsigned long long wide_max;
   uint32_t* masks;            // bit r % 32 of word r / 32: k_chain_rows left row r to k_chain_walk
   uint32_t* queue;            // this pass's rows that a warp walks, + 1 (0: not there yet), and
   uint32_t* taken;            // how many places were taken (taken[0]) and filled (taken[1])
@@ -443,11 +457,14 @@ __device__ __forceinline__ bool quick_row(const ChainArgs& p, uint32_t row, uint
   return true;
 }
 
+__device__ __forceinline__ bool given_up(const ChainArgs& p) { return __ldcg(p.abort) != 0; }
+
 // The union of the rows of `mat` that the slot `left` names (mat null: none)
 // and of the slots d and e, by a warp, any number of runs: bitmap windows over
 // the columns that its ranges cover, the next window starting at the first
-// column past the last one.  Returns the row's slot (uniform).  The arena is
-// read past L1: a slot may be one that this warp has just written.
+// column past the last one.  Returns the row's slot (uniform); of
+// no column where the chain is given up, for the union's own cost or another reason.
+// The arena is read past L1: a slot may be one that this warp has just written.
 __device__ uint2 warp_union(const ChainArgs& p, uint2 left, const uint2* mat, uint2 d, uint2 e,
                             uint32_t* bits, uint32_t* reach) {
   const int lane = lane_id();
@@ -479,6 +496,18 @@ __device__ uint2 warp_union(const ChainArgs& p, uint2 left, const uint2* mat, ui
       }
     }
   };
+  auto give_up = [&](unsigned long long why) {
+    if (lane == 0) atomicOr(p.abort, why);
+    return empty_slot();
+  };
+  if (__shfl_sync(kFullMask, given_up(p), 0)) return empty_slot();
+  uint32_t named = 0;  // rows (at most kWideColumns + 1 counted of a range)
+  for (uint32_t t = lane, c = mat ? slot_count(left) : 0; t < c; t += 32) {
+    const uint2 r = is_multi(left) ? __ldcg(p.arena + left.y + t) : slot_range(p.arena, left, t);
+    named = min(named + min(r.y - r.x, kWideColumns) + 1, kWideColumns + 1);
+  }
+  named = __reduce_add_sync(kFullMask, named);
+  if (named > kWideColumns) return give_up(kWideRows);
   uint32_t first = 0xffffffffu, end = 0;
   each([&](uint2 v) {
     first = min(first, v.x);
@@ -488,6 +517,10 @@ __device__ uint2 warp_union(const ChainArgs& p, uint2 left, const uint2* mat, ui
   first = __reduce_min_sync(kFullMask, first);
   end = __reduce_max_sync(kFullMask, end);
   if (first == 0xffffffffu) return empty_slot();
+  const unsigned long long cost = 2ull * (named / 32 + 1) * ((end - first) / (32 * kSWin) + 1);
+  unsigned long long spent = 0;
+  if (lane == 0) spent = atomicAdd(p.wide, cost);
+  if (__shfl_sync(kFullMask, spent, 0) + cost > p.wide_max) return give_up(kWideRows);
   uint64_t off = 0;
   uint32_t total = 0;
   for (int pass = 0; pass < 2; ++pass) {  // count, then write to the arena
@@ -552,10 +585,8 @@ __device__ uint2 warp_union(const ChainArgs& p, uint2 left, const uint2* mat, ui
       total = count;
       if (lane == 0) off = atomicAdd(p.top, (unsigned long long)total);
       off = __shfl_sync(kFullMask, off, 0);
-      if (total > kMultiMax || off + total > p.arena_cap) {
-        if (lane == 0) atomicOr(p.abort, 1ull);
-        return empty_slot();
-      }
+      if (total > kMultiMax) return give_up(kLongRow);
+      if (off + total > p.arena_cap) return give_up(kArenaFull);
     }
   }
   __syncwarp();
@@ -588,7 +619,7 @@ __device__ __forceinline__ uint2 bitmap_slot(const ChainArgs& p, const uint32_t*
   if (lane == 0) off = atomicAdd(p.top, (unsigned long long)cnt);
   off = __shfl_sync(kFullMask, off, 0);
   if (off + cnt > p.arena_cap) {
-    if (lane == 0) atomicOr(p.abort, 1ull);
+    if (lane == 0) atomicOr(p.abort, kArenaFull);
     cnt = 0;
     return empty_slot();
   }
@@ -757,11 +788,13 @@ template <bool OUTS, bool OUTC, class Tally>
 __device__ void take_rows(const ChainArgs& p, WarpSmem& S, Tally&& tally) {
   for (;;) {
     const uint2 places = __ldcg(reinterpret_cast<const uint2*>(p.taken));
-    if (__shfl_sync(kFullMask, places.x, 0) >= min(__shfl_sync(kFullMask, places.y, 0), p.queue_cap)) return;
+    const bool none = places.x >= min(places.y, p.queue_cap) || given_up(p);
+    if (__shfl_sync(kFullMask, none, 0)) return;
     uint32_t r = 0;  // row + 1
     if (lane_id() == 0) {
       const uint32_t at = atomicAdd(p.taken, 1u);
       if (at < p.queue_cap) r = atomicExch(p.queue + at, kGone);
+      __threadfence();
     }
     r = __shfl_sync(kFullMask, r, 0);
     if (r == 0) continue;
@@ -772,11 +805,21 @@ __device__ void take_rows(const ChainArgs& p, WarpSmem& S, Tally&& tally) {
 
 // Walks the `batch` rows of the warp's list, a row a lane; rows of more runs
 // than a lane's lists hold go to the queue (take_rows), or to the whole warp at once
-// where that is full.  Whether some of them were no quick ones.
+// where that is full.  Whether some of them were no quick ones.  (`dropped`: the chain
+// is given up.)
 // tally(row, ranges, columns) for each row of c that has any.
 template <bool OUTS, bool OUTC, class Tally>
-__device__ __forceinline__ bool walk_batch(const ChainArgs& p, WarpSmem& S, uint32_t batch, Tally&& tally) {
+__device__ __forceinline__ bool walk_batch(const ChainArgs& p, WarpSmem& S, uint32_t batch, bool dropped,
+                                           Tally&& tally) {
   const int lane = lane_id();
+  if (dropped) {
+    if (uint32_t(lane) < batch) {
+      if (OUTS) p.s[S.todo[lane]] = empty_slot();
+      if (OUTC) p.c[S.todo[lane]] = empty_slot();
+    }
+    __syncwarp();
+    return false;
+  }
   uint32_t row = 0, ns = 0, nc = 0, cur = 0;
   bool done = false;
   uint2* const C = S.list[2] + lane;
@@ -817,7 +860,7 @@ __device__ __forceinline__ bool walk_batch(const ChainArgs& p, WarpSmem& S, uint
     if (lane == 31) off = atomicAdd(p.top, (unsigned long long)all);
     off = __shfl_sync(kFullMask, off, 31);
     fits = off + all <= p.arena_cap;
-    if (!fits && lane == 0) atomicOr(p.abort, 1ull);
+    if (!fits && lane == 0) atomicOr(p.abort, kArenaFull);
     off += incl - ws - wc;
   }
   auto put = [&](uint2* to, const uint2* L, uint32_t n, uint32_t want) {
@@ -847,10 +890,16 @@ __device__ __forceinline__ bool walk_batch(const ChainArgs& p, WarpSmem& S, uint
       at = atomicAdd(p.taken + 1, uint32_t(__popc(left)));
     }
     at = __shfl_sync(kFullMask, at, 0) + __popc(left & ((1u << lane) - 1u));
+    if ((left >> lane) & 1u) {  // (rows stay empty that nobody takes: the chain was given up)
+      if (OUTS) p.s[row] = empty_slot();
+      if (OUTC) p.c[row] = empty_slot();
+      __threadfence();
+    }
     const bool queued = ((left >> lane) & 1u) && at < p.queue_cap && atomicExch(p.queue + at, row + 1) != kGone;
     left &= ~__ballot_sync(kFullMask, queued);
   }
   for (; left; left &= left - 1) {
+    if (__shfl_sync(kFullMask, given_up(p), 0)) break;
     const uint32_t r = __shfl_sync(kFullMask, row, __ffs(left) - 1);
     const RowCount n = warp_row<OUTS, OUTC>(p, S, r);
     if (lane == 0 && n.ranges) tally(r, n.ranges, n.columns);
@@ -934,6 +983,7 @@ __global__ void __launch_bounds__(kWThreads) k_chain_walk(const __grid_constant_
   };
   bool look = false;
   uint32_t x = 0, at = 0;  // a lane's word: its rows still to walk, and the first of its 32
+  bool dropped = __shfl_sync(kFullMask, given_up(p), 0);
   while (true) {
     const unsigned spent = __ballot_sync(kFullMask, x == 0);
     uint32_t have = __reduce_add_sync(kFullMask, uint32_t(__popc(x)));
@@ -951,7 +1001,9 @@ __global__ void __launch_bounds__(kWThreads) k_chain_walk(const __grid_constant_
     uint32_t k = group_incl_sum<32>(kFullMask, uint32_t(__popc(x)), lane) - __popc(x);
     for (; x && k < 32; x &= x - 1) S.todo[k++] = at + uint32_t(__ffs(x) - 1);
     __syncwarp();
-    if (walk_batch<OUTS, OUTC>(p, S, min(have, 32u), tally)) look = true;
+    const bool later = given_up(p);  // (for the next batch: it comes while this one is walked)
+    if (walk_batch<OUTS, OUTC>(p, S, min(have, 32u), dropped, tally)) look = true;
+    dropped = __shfl_sync(kFullMask, later, 0);
   }
   if (look) take_rows<OUTS, OUTC>(p, S, tally);
 }
@@ -974,6 +1026,7 @@ __global__ void __launch_bounds__(kWThreads) k_chain_small(const __grid_constant
   unsigned long long nnz = 0;
   uint32_t cnt = 0;
   bool look = false;
+  const bool dropped = given_up(p);
   if (r0 < p.n) {
     uint32_t bad;
     if (r0 + 32 <= p.n) bad = chain_rows<OUTS, OUTC, COUNT, 1>(p, uint32_t(r0), cnt, nnz);
@@ -982,7 +1035,7 @@ __global__ void __launch_bounds__(kWThreads) k_chain_small(const __grid_constant
     if (bad) S.todo[__popc(who & ((1u << lane) - 1u))] = uint32_t(r0) + lane;
     __syncwarp();
     if (who)
-      look = walk_batch<OUTS, OUTC>(p, S, __popc(who), [&](uint32_t, uint32_t c, unsigned long long z) {
+      look = walk_batch<OUTS, OUTC>(p, S, __popc(who), __shfl_sync(kFullMask, dropped, 0), [&](uint32_t, uint32_t c, unsigned long long z) {
         cnt += c;
         nnz += z;
       });
@@ -1074,7 +1127,7 @@ __global__ void __launch_bounds__(kSThreads) k_crs_to_slots(const __grid_constan
       off = __shfl_sync(kFullMask, off, 31) + incl - want;
       if (want) {
         if (want > kMultiMax || off + want > p.arena_cap) {
-          atomicOr(p.abort, 1ull);
+          atomicOr(p.abort, want > kMultiMax ? kLongRow : kArenaFull);
           v[u] = empty_slot();
         } else {
           for (uint64_t k = 0; k < want; ++k) p.arena[off + k] = range(a0[u] + k);
@@ -1416,6 +1469,32 @@ bool slots_suit(const dvg_context* ctx, const dvg_matrix* a) {
          2 * ranges <= 3ull * a->nrows && a->nnz <= 2 * ranges && ctx->opt_slots != 0;
 }
 
+// Chains over such matrices for such a window, as far as whether they fit goes: sizes
+// within a factor of two, densities within a fifth.  (Products: dlo 1, dup 0.)
+SlotKey slot_key(unsigned dlo, unsigned dup, uint64_t nnz, uint64_t nrows) {
+  const double b = branching(nnz, nrows);
+  return {dlo, dup, int(64 - __builtin_clzll(nrows | 1)), b > 0 ? int(std::floor(4 * std::log2(b))) : -1000};
+}
+
+bool slots_due(dvg_context* ctx, const SlotKey& key) {
+  const auto it = ctx->slot_misses.find(key);
+  if (it == ctx->slot_misses.end() || it->second.left == 0) return true;
+  --it->second.left;
+  return false;
+}
+
+// A chain that is given up costs what its passes did until then, so the next ones like
+// it go the range-CRS way at once: 1 call, then 3, 7 and so on up to 63 between two
+// attempts.
+static void slots_missed(dvg_context* ctx, const SlotKey& key) {
+  constexpr size_t kMost = 256;
+  constexpr uint32_t kLongest = 63;
+  if (ctx->slot_misses.size() >= kMost && !ctx->slot_misses.count(key)) ctx->slot_misses.clear();
+  SlotMiss& m = ctx->slot_misses[key];
+  m.wait = std::min(2 * m.wait + 1, kLongest);
+  m.left = m.wait;
+}
+
 static unsigned conversion_blocks(const SlotBuild& sb) { return unsigned((uint64_t(sb.n) + kCrsRows - 1) / kCrsRows); }
 
 SlotBuild prepare_slots(dvg_context* ctx, const SlotPlan& plan, uint32_t n) {
@@ -1462,6 +1541,7 @@ SlotBuild prepare_slots(dvg_context* ctx, const SlotPlan& plan, uint32_t n) {
     sb.ctl = reinterpret_cast<DeviceControl*>(base);
     sb.top = reinterpret_cast<unsigned long long*>(base + 256);
     sb.abort = sb.top + 1;
+    sb.wide = sb.top + 2;
     sb.taken = reinterpret_cast<uint32_t*>(base + taken_off);
     sb.queue = reinterpret_cast<uint32_t*>(base + queue_off);
     sb.sums = reinterpret_cast<unsigned long long*>(base + sums_off);
@@ -1508,6 +1588,8 @@ void launch_slots(dvg_context* ctx, SlotBuild& sb, const SlotParts& parts, bool 
   p.arena_cap = sb.arena_cap;
   p.ctl = sb.ctl;
   p.abort = sb.abort;
+  p.wide = sb.wide;
+  p.wide_max = kWideCost + sb.n / 16;
   p.masks = sb.masks;
   p.queue_cap = sb.queue_cap;
   p.group_cnt = sb.group_cnt;
@@ -1557,11 +1639,15 @@ void launch_slots_out(dvg_context* ctx, const SlotBuild& sb, const SlotParts& pa
 
 bool check_slots(dvg_context* ctx, const SlotBuild& sb, const SlotCounters& c) {
   if (c.abort) {
-    // more rows of several runs than the arena was sized for: the caller takes
-    // the range-CRS path, later chains a larger arena
-    ctx->slot_growth = std::min(2.0 * ctx->slot_growth, 8.0);
+    // the caller takes the range-CRS path; where only the arena was too small, later
+    // chains get a larger one, and otherwise chains like this wait
+    const bool bigger = c.abort == kArenaFull && ctx->slot_growth < kSlotGrowthMax &&
+                        double(sb.arena_cap) >= std::min(ctx->slot_growth * double(sb.n), double(kMulti));
+    if (bigger) ctx->slot_growth = std::min(2.0 * ctx->slot_growth, kSlotGrowthMax);
+    else slots_missed(ctx, sb.key);
     return false;
   }
+  ctx->slot_misses.erase(sb.key);
   // statistics: what every pass had to move, 8 bytes a row for each matrix it
   // reads or writes, and the products that it stands for
   uint64_t bytes = 0, products = 0, adds = 0;
@@ -1597,10 +1683,11 @@ static SlotPart whole(const dvg_matrix* a) {
 }
 
 static dvg_matrix* run_slots(dvg_context* ctx, const SlotPlan& plan, const dvg_matrix* a, const dvg_matrix* b,
-                             bool build, bool* settled) {
+                             const SlotKey& key, bool build, bool* settled) {
   SlotBuild sb;
   try {
     sb = prepare_slots(ctx, plan, a->nrows);
+    sb.key = key;
   } catch (const Error& e) {
     if (e.status != DVG_ERR_OOM) throw;
     return nullptr;
@@ -1666,7 +1753,8 @@ static dvg_matrix* run_slots(dvg_context* ctx, const SlotPlan& plan, const dvg_m
 }
 
 dvg_matrix* slots_chain(dvg_context* ctx, const dvg_matrix* a, unsigned dlo, unsigned dup, bool build, bool* settled) {
-  return run_slots(ctx, plan_slots(dlo, dup, branching(a->nnz, a->nrows)), a, nullptr, build, settled);
+  return run_slots(ctx, plan_slots(dlo, dup, branching(a->nnz, a->nrows)), a, nullptr, slot_key(dlo, dup, a), build,
+                   settled);
 }
 
 bool slots_product_suits(const dvg_context* ctx, const dvg_matrix* a, const dvg_matrix* b) {
@@ -1685,7 +1773,7 @@ dvg_matrix* slots_product(dvg_context* ctx, const dvg_matrix* a, const dvg_matri
   st.bits = 2;
   st.c = pl.out;
   pl.steps.push_back(st);
-  return run_slots(ctx, pl, a, a == b ? nullptr : b, false, settled);
+  return run_slots(ctx, pl, a, a == b ? nullptr : b, product_key(a, b), false, settled);
 }
 
 }  // namespace dvg

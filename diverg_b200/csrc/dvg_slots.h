@@ -1,6 +1,8 @@
 // dvg_slots.h -- chains of products in the row-slot format (dvg_slots.cu).
 #pragma once
 
+#include <algorithm>
+
 #include "dvg_internal.h"
 
 namespace dvg {
@@ -56,10 +58,11 @@ struct SlotParts {
 struct SlotCounters {          // the head of a chain's scratch
   DeviceControl ctl;
   char pad[256 - sizeof(DeviceControl)];
-  unsigned long long top, abort;
+  unsigned long long top, abort, wide;
 };
 struct SlotBuild {
   SlotPlan plan;
+  SlotKey key{};
   uint32_t n = 0;
   std::vector<uint2*> mat;     // per matrix, as the launches use them
   std::vector<uint2*> buffers; // theirs
@@ -76,6 +79,7 @@ struct SlotBuild {
   DeviceControl* ctl = nullptr;
   unsigned long long* top = nullptr;
   unsigned long long* abort = nullptr;
+  unsigned long long* wide = nullptr;
   unsigned long long* sums = nullptr;
   unsigned long long* group_nnz = nullptr;
   uint32_t* group_cnt = nullptr;
@@ -94,8 +98,7 @@ void launch_slots_totals(dvg_context* ctx, const SlotBuild& sb, const SlotParts&
 // The parts' results, into the arrays that the table now names; `ctl` (null: the
 // context's) takes a status where an array is too small.
 void launch_slots_out(dvg_context* ctx, const SlotBuild& sb, const SlotParts& parts, DeviceControl* ctl = nullptr);
-// Books a finished chain's counters; false when its arena ran full and there is
-// no result.
+// Books a finished chain's counters; false when it was given up and there is no result.
 bool check_slots(dvg_context* ctx, const SlotBuild& sb, const SlotCounters& c);
 void release_slots(dvg_context* ctx, SlotBuild& sb);
 
@@ -114,5 +117,13 @@ dvg_matrix* slots_product(dvg_context* ctx, const dvg_matrix* a, const dvg_matri
 inline double branching(uint64_t nnz, uint64_t nrows) {
   return nnz > nrows ? double(nnz - nrows) / double(nrows) : 0.0;
 }
+
+SlotKey slot_key(unsigned dlo, unsigned dup, uint64_t nnz, uint64_t nrows);
+inline SlotKey slot_key(unsigned dlo, unsigned dup, const dvg_matrix* a) { return slot_key(dlo, dup, a->nnz, a->nrows); }
+inline SlotKey product_key(const dvg_matrix* a, const dvg_matrix* b) {
+  return slot_key(1, 0, std::max(a->nnz, b->nnz), a->nrows);
+}
+// Whether a chain is to be tried: chains like it were not just given up.  Counts the call.
+bool slots_due(dvg_context* ctx, const SlotKey& key);
 
 }  // namespace dvg

@@ -106,3 +106,87 @@ def test_an_index_holds_no_more_than_it_needs(ctx, bases, window):
         most = block(8 * (m.nrows + 1) + 16) + 5 * block(5 * m.nentries + (1 << 20) + 16) // 4
         assert held <= most, (slots, held, most)
         m.free()
+
+
+def path_and(n, extra):
+    """The path i -> i + 1, with the ranges `extra` in place of the rows that it names."""
+    i = np.arange(n - 1, dtype=np.uint32)
+    rows = np.split(np.stack([i + 1, i + 1], 1), range(1, n - 1)) + [np.zeros((0, 2), np.uint32)]
+    for r, e in extra.items():
+        rows[r] = np.asarray(e, np.uint32).reshape(-1, 2)
+    rm = np.concatenate(([0], np.cumsum([2 * len(r) for r in rows]))).astype(np.uint64)
+    return CRSMatrix(n, np.concatenate(rows).reshape(-1), rm)
+
+
+def index(ctx, d, m, window):
+    """The index, held against the oracle, and how often its products ran again."""
+    ctx.reset_stats()
+    r = ctx.distance_index(d, *window)
+    again = ctx.stats()["spgemm_reruns"]
+    same(r.download(), orc.dindex(omat(m), *window, algo="hbv"), window)
+    r.free()
+    return again
+
+
+def test_chains_that_do_not_fit_are_not_tried_on_every_call(ctx):
+    # rows of random columns double with every factor, past any arena
+    m = gen.banded(30_000, 30_000, 1.0, 1.0, seed=85)
+    d = ctx.upload(m)
+    ctx.set_option("row_slots", 0)
+    crs = min(index(ctx, d, m, (8, 9)) for _ in range(3))
+    ctx.set_option("row_slots", 1)
+    again = [index(ctx, d, m, (8, 9)) - crs for _ in range(16)]
+    # a larger arena, then 1, 3, 7 calls between two attempts
+    assert 1 <= sum(a > 0 for a in again) <= 5, again
+    # a matrix of another kind is tried
+    g, _ = gen.graph_adjacency(gen.small_graph_spec(30_000, seed=86))
+    assert index(ctx, ctx.upload(g), g, (8, 9)) == 0
+
+
+def test_batches_with_a_graph_that_does_not_fit(ctx):
+    m = gen.banded(30_000, 30_000, 1.0, 1.0, seed=85)
+    g, _ = gen.graph_adjacency(gen.small_graph_spec(20_000, seed=87))
+    graphs = [m, g, g, m]
+    wants = [orc.dindex(omat(x), 8, 9, algo="hbv") for x in graphs]
+    up = [ctx.upload(x) for x in graphs]
+    for _ in range(6):
+        for got, want in zip(ctx.batch_distance_index(up, [(8, 9)] * 4), wants):
+            same(got.download(), want, "batch")
+            got.free()
+
+
+def test_rows_that_reach_far_are_left_to_range_crs(ctx):
+    n = 200_000
+    m = path_and(n, {777: [[778, 20_777]]})
+    d = ctx.upload(m)
+    assert index(ctx, d, m, (40, 60)) >= 1
+    assert index(ctx, d, m, (40, 60)) == 0  # (and not tried at once again)
+    # a few that reach past the bitmaps, and name few columns, stay
+    m = path_and(n, {r: [[r + 1 + 1900 * k, r + 1 + 1900 * k] for k in range(12)] for r in (500, 600, 90_000)})
+    assert index(ctx, ctx.upload(m), m, (3, 5)) == 0
+
+
+def peak_bytes(ctx, call):
+    """The most device memory in use from CUDA's pool during a call."""
+    from cuda.bindings import driver, runtime as rt
+    before = used_bytes(ctx)
+    _, pool = rt.cudaDeviceGetDefaultMemPool(0)
+    high = rt.cudaMemPoolAttr.cudaMemPoolAttrUsedMemHigh
+    err, = rt.cudaMemPoolSetAttribute(pool, high, driver.cuuint64_t(0))
+    assert int(err) == 0
+    call()
+    err, most = rt.cudaMemPoolGetAttribute(pool, high)
+    assert int(err) == 0
+    return int(most) - before
+
+
+def test_a_row_of_too_many_ranges_makes_no_arena_larger(ctx):
+    n = 200_000
+    g = path_and(n, {5: [[6, 6], [9, 9]]})
+    d = ctx.upload(g)
+    build = lambda: ctx.distance_index(d, 20, 30).free()
+    build()
+    usual = peak_bytes(ctx, build)
+    many = path_and(n, {100: [[101 + 2 * k, 101 + 2 * k] for k in range(70_000)]})  # past 65,534
+    assert index(ctx, ctx.upload(many), many, (1, 1)) >= 1
+    assert peak_bytes(ctx, build) <= usual * 1.02
