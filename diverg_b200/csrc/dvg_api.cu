@@ -915,6 +915,7 @@ static void validate_uploaded(dvg_context* ctx, dvg_matrix* m) {
   DeviceControl c = read_control(ctx);
   m->canonical = !(c.invalid & 16);
   m->nnz = c.nnz;
+  m->empty_rows = uint32_t(c.empty_rows);
   c.invalid &= ~16ull;
   if (c.invalid) throw Error(DVG_ERR_INVALID_ARG, "malformed range-CRS matrix:" + validation_message(c.invalid));
 }

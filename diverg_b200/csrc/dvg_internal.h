@@ -22,6 +22,7 @@ struct dvg_matrix {
   uint64_t nnz = 0;         // columns of its ranges, as the device counted them
   uint64_t given_nnz = 0;   // what the caller said they are, for a matrix that came from one
   bool nnz_given = false;
+  uint32_t empty_rows = 0;  // rows without a range, where they were counted (with nnz, of a caller's matrix)
   uint64_t* rowmap = nullptr;   // device, nrows + 1
   uint32_t* entries = nullptr;  // device, nentries (allocation padded to 16 B)
   bool owned = true;
@@ -42,6 +43,7 @@ struct DeviceControl {
   unsigned long long timeout;    // nonzero: a bounded device wait gave up
   unsigned long long tiles_direct;  // tiles that took the direct (unstaged) path
   unsigned long long slow_rows;     // row-mode rows that missed the shared window
+  unsigned long long empty_rows;    // validation: rows without a range
 };
 
 // DeviceControl::status bit of a query that met row pointers outside its

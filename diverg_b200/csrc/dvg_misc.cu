@@ -31,17 +31,21 @@ __global__ void k_identity(uint64_t* __restrict__ rowmap, uint32_t* __restrict__
 // bit 4: rowmap[n] != nentries; bit 8: an entry >= ncols.  Not an error:
 // bit 16 marks a matrix whose rows are not canonical (a range with end <
 // start, or a range that does not start past the previous range's end + 1).
-// The columns of its ranges are counted into ctl->nnz.
+// The columns of its ranges are counted into ctl->nnz, its rows without any into
+// ctl->empty_rows.
 __global__ void k_validate(const uint64_t* __restrict__ rowmap, uint32_t nrows, const uint32_t* __restrict__ entries,
                            uint64_t nentries, uint32_t ncols, DeviceControl* ctl) {
   __shared__ unsigned long long cta_nnz;
-  if (threadIdx.x == 0) cta_nnz = 0;
+  __shared__ uint32_t cta_empty;
+  if (threadIdx.x == 0) cta_nnz = cta_empty = 0;
   __syncthreads();
   unsigned long long bad = 0, nnz = 0;
+  uint32_t empty = 0;
   const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
   const uint64_t tid = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
   for (uint64_t i = tid; i < nrows; i += stride) {
     uint64_t a = rowmap[i], b = rowmap[i + 1];
+    empty += a == b;
     if (b < a || ((b - a) & 1)) {
       bad |= 2;
     } else if (b <= nentries) {
@@ -60,9 +64,12 @@ __global__ void k_validate(const uint64_t* __restrict__ rowmap, uint32_t nrows, 
     if (entries[i] >= ncols) bad |= 8;
   if (bad) atomicOr(&ctl->invalid, bad);
   nnz = group_sum<32>(kFullMask, nnz);
+  empty = __reduce_add_sync(kFullMask, empty);
   if (lane_id() == 0 && nnz) atomicAdd(&cta_nnz, nnz);
+  if (lane_id() == 0 && empty) atomicAdd(&cta_empty, empty);
   __syncthreads();
   if (threadIdx.x == 0 && cta_nnz) atomicAdd(&ctl->nnz, cta_nnz);
+  if (threadIdx.x == 0 && cta_empty) atomicAdd(&ctl->empty_rows, (unsigned long long)cta_empty);
 }
 
 __global__ void k_widen(const uint32_t* __restrict__ src, uint64_t* __restrict__ dst, uint64_t n) {

@@ -1462,17 +1462,26 @@ SlotPlan plan_slots(unsigned dlo, unsigned dup, double branching) {
 // columns on average, the powers' rows soon leave the slots for the arena, or
 // name so many rows that a thread walks them for long: such input, input whose
 // rows are not canonical, and matrices whose columns reach the marker of a
-// several-run row stay with the range-CRS row kernel.
+// several-run row stay with the range-CRS row kernel.  So does large input of more
+// than a quarter of a column a row beyond its first, which no sequence graph has.  At 1e6
+// rows A^2 of a path with skips took 88 us against 110 in range CRS at 0.2 columns, 104
+// against 109 at 0.29 and 160 against 116 at 0.48, of random bands 195 against 146 at 0.3
+// and 364 against 213 at 0.7; A^4 250 against 365, 380 against 410, and of the bands
+// 696 against 581 and 1,856 against 1,074.  Up to 2^18 rows the row kernel's fixed costs
+// are more than that: at 1e5 rows all of these take 0.5 to 0.95 of its time.
+constexpr double kDenseBranching = 0.25;
+constexpr uint32_t kDenseRows = 1u << 18;
 bool slots_suit(const dvg_context* ctx, const dvg_matrix* a) {
   const uint64_t ranges = a->nentries / 2;
   return a->canonical && a->nrows == a->ncols && a->nrows > 0 && a->ncols < kSlotMulti &&
-         2 * ranges <= 3ull * a->nrows && a->nnz <= 2 * ranges && ctx->opt_slots != 0;
+         2 * ranges <= 3ull * a->nrows && a->nnz <= 2 * ranges &&
+         (a->nrows <= kDenseRows || branching(padded_columns(a), a->nrows) <= kDenseBranching) && ctx->opt_slots != 0;
 }
 
 // Chains over such matrices for such a window, as far as whether they fit goes: sizes
 // within a factor of two, densities within a fifth.  (Products: dlo 1, dup 0.)
-SlotKey slot_key(unsigned dlo, unsigned dup, uint64_t nnz, uint64_t nrows) {
-  const double b = branching(nnz, nrows);
+SlotKey slot_key(unsigned dlo, unsigned dup, uint64_t columns, uint64_t nrows) {
+  const double b = branching(columns, nrows);
   return {dlo, dup, int(64 - __builtin_clzll(nrows | 1)), b > 0 ? int(std::floor(4 * std::log2(b))) : -1000};
 }
 
@@ -1753,7 +1762,7 @@ static dvg_matrix* run_slots(dvg_context* ctx, const SlotPlan& plan, const dvg_m
 }
 
 dvg_matrix* slots_chain(dvg_context* ctx, const dvg_matrix* a, unsigned dlo, unsigned dup, bool build, bool* settled) {
-  return run_slots(ctx, plan_slots(dlo, dup, branching(a->nnz, a->nrows)), a, nullptr, slot_key(dlo, dup, a), build,
+  return run_slots(ctx, plan_slots(dlo, dup, branching(padded_columns(a), a->nrows)), a, nullptr, slot_key(dlo, dup, a), build,
                    settled);
 }
 

@@ -190,3 +190,29 @@ def test_a_row_of_too_many_ranges_makes_no_arena_larger(ctx):
     many = path_and(n, {100: [[101 + 2 * k, 101 + 2 * k] for k in range(70_000)]})  # past 65,534
     assert index(ctx, ctx.upload(many), many, (1, 1)) >= 1
     assert peak_bytes(ctx, build) <= usual * 1.02
+
+
+@pytest.mark.parametrize("n,dense_slots", [(1 << 18, True), ((1 << 18) + 1, False), (400_000, False)])
+def test_large_dense_input_stays_in_range_crs(ctx, n, dense_slots):
+    # more than a quarter of a column a row beyond its first, of the rows that have any
+    g, _ = gen.graph_adjacency(gen.small_graph_spec(n - 8_000, seed=88))
+    for what, m, slots in (("graph", g, True), ("1.4 a row", gen.banded(n, 40, 1.2, 1.2, seed=89), dense_slots),
+                           ("0.9 a row", gen.banded(n, 40, 0.9, 1.0, seed=90), dense_slots)):
+        assert m.entries.size <= 3 * m.numRows() and m.nnz() <= m.entries.size, what
+        d = ctx.upload(m)
+        for call in (lambda: ctx.spgemm(d, d), lambda: ctx.power(d, 2), lambda: ctx.distance_index(d, 1, 2)):
+            ctx.set_option("row_slots", 0)
+            call().free()  # (builds in range CRS size themselves by the one before)
+            moved, forms = [], []
+            for on in (1, 0):
+                ctx.set_option("row_slots", on)
+                ctx.reset_stats()
+                r = call()
+                moved.append(ctx.stats()["spgemm_alg_bytes"])
+                forms.append(r.download())
+                r.free()
+            ctx.set_option("row_slots", 1)
+            assert np.array_equal(forms[0].rowmap, forms[1].rowmap), what
+            assert np.array_equal(forms[0].entries, forms[1].entries), what
+            assert (moved[0] != moved[1]) == slots, (what, moved)
+        d.free()
