@@ -1740,7 +1740,11 @@ static dvg_matrix* run_slots(dvg_context* ctx, const SlotPlan& plan, const dvg_m
       if (c.ctl.status)
         throw Error(DVG_ERR_DEVICE, "row slots: a result and its counts differ (code " + std::to_string(c.ctl.status) + ")");
     } else if (whole_chain) {
-      out(c.ctl.total / 2, nullptr);
+      try {
+        out(c.ctl.total / 2, nullptr);
+      } catch (const Error& e) {  // beside the chain's buffers; in range CRS it may fit
+        if (e.status != DVG_ERR_OOM) throw;
+      }
     }
     if (m) {
       const uint64_t room = m->nentries;

@@ -102,7 +102,7 @@ void launch_slots_out(dvg_context* ctx, const SlotBuild& sb, const SlotParts& pa
 bool check_slots(dvg_context* ctx, const SlotBuild& sb, const SlotCounters& c);
 void release_slots(dvg_context* ctx, SlotBuild& sb);
 
-// The chain over `a`, waited for once; null when it did not fit its arena.  Sets
+// The chain over `a`, waited for once; null when it or its result did not fit.  Sets
 // *settled where that wait has seen all of the result's kernels end, and checked them.
 // `build`: an index, which holds no more memory than it needs; a power or a product
 // keeps the room that was made for it.
