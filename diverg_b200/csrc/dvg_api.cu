@@ -347,12 +347,31 @@ static dvg_matrix* range_spgemm_fused(dvg_context* ctx, const dvg_matrix* a, boo
   // product run twice costs more than room for what the last one took
   const bool grows = !a_identity && has_long_ranges(a);
   const uint64_t larger = std::max<uint64_t>({a_ent, b->nentries, 1});
-  const uint64_t usual = cap;
+  uint64_t usual = cap;
   if (grows) {
     const uint64_t want = uint64_t(ctx->product_growth * double(larger));
     if (want > cap && want < (device_free_bytes(ctx) + ctx->cached_bytes) / 16) cap = want;
   }
-  dvg_matrix* c = new_matrix(ctx, n, b->ncols, cap);
+  // the result comes first: short of memory, the guess and then the tables are given up
+  auto make_room = [&](const Error& e) {
+    if (e.status != DVG_ERR_OOM) return false;
+    if (cap > usual) {
+      cap = usual;
+      return true;
+    }
+    if (!band.t.mem) return false;
+    dfree(ctx, band.t.mem);
+    band.t = {};
+    return true;
+  };
+  dvg_matrix* c = nullptr;
+  while (!c) {
+    try {
+      c = new_matrix(ctx, n, b->ncols, cap);
+    } catch (const Error& e) {
+      if (!make_room(e)) throw;
+    }
+  }
   try {
     DVG_CUDA(cudaMemsetAsync(c->rowmap, 0, sizeof(uint64_t), ctx->stream));
     DeviceControl ctl{};
@@ -367,25 +386,21 @@ static dvg_matrix* range_spgemm_fused(dvg_context* ctx, const dvg_matrix* a, boo
       if (!ctl.overflow) break;
       if (attempt == 1) throw Error(DVG_ERR_DEVICE, "range_spgemm: output capacity overflow after resize");
       ctx->stats.spgemm_reruns++;
-      cap = ctl.total;
+      cap = usual = ctl.total;
       dfree(ctx, c->entries);
       c->entries = nullptr;
-      c->entries = static_cast<uint32_t*>(dalloc(ctx, entries_alloc_bytes(cap)));
+      while (!c->entries) {
+        try {
+          c->entries = static_cast<uint32_t*>(dalloc(ctx, entries_alloc_bytes(cap)));
+        } catch (const Error& e) {
+          if (!make_room(e)) throw;
+        }
+      }
     }
     if (grows) ctx->product_growth = std::min(std::max(2.0, 1.25 * double(ctl.total) / double(larger)), 16.0);
-    if (cap > usual && cap / 2 > ctl.total) {  // (the room was for another product's result)
-      auto* exact = static_cast<uint32_t*>(dalloc(ctx, entries_alloc_bytes(ctl.total)));
-      if (ctl.total) {
-        const cudaError_t e = cudaMemcpyAsync(exact, c->entries, ctl.total * sizeof(uint32_t), cudaMemcpyDeviceToDevice,
-                                              ctx->stream);
-        if (e != cudaSuccess) dfree(ctx, exact);
-        DVG_CUDA(e);
-      }
-      DVG_CUDA(cudaStreamSynchronize(ctx->stream));  // the caller waits no more
-      dfree(ctx, c->entries);
-      c->entries = exact;
-    }
     c->nentries = ctl.total;
+    // (room that was guessed from another product's result)
+    if (cap > usual && give_back(ctx, c, cap)) DVG_CUDA(cudaStreamSynchronize(ctx->stream));  // the caller waits no more
     c->nnz = ctl.nnz;
     c->canonical = true;
     ctx->max_product_entries = std::max(ctx->max_product_entries, c->nentries);

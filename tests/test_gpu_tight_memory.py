@@ -53,3 +53,36 @@ m = c.download()
 assert np.array_equal(m.rowmap, 2 * np.minimum(np.arange(n + 1, dtype=np.uint64), n - 2))
 assert np.array_equal(m.entries, np.stack([i[1:], i[1:]], 1).reshape(-1)) and m.nnz() == n - 2
 """)
+
+
+def test_a_long_range_product_without_its_tables():
+    # 2^19 rows of one range of 400 columns: the result is 1.57 GB, the tables of unions
+    # of B's rows 0.25, which no longer fit beside it
+    child("""
+n = 1 << 19
+i = np.arange(n, dtype=np.int64)
+a = CRSMatrix(n, np.stack([i, np.minimum(i + 399, n - 1)], 1).astype(np.uint32).reshape(-1),
+              2 * np.arange(n + 1, dtype=np.uint64))
+# row j: the columns c of [j, j + 350] with c = 2 (j mod 20) modulo 40; never neighbours
+first = i + (2 * (i % 20) - i) % 40
+cols = first[:, None] + 40 * np.arange(9)
+ok = (cols <= i[:, None] + 350) & (cols < n)
+rm = np.concatenate(([0], np.cumsum(2 * ok.sum(1)))).astype(np.uint64)
+b = CRSMatrix(n, np.repeat(cols[ok], 2).astype(np.uint32), rm)
+da, db = ctx.upload(a), ctx.upload(b)
+w = gen.banded(1 << 15, 512, 4.0, 80.0, seed=92)
+dw = ctx.upload(w)
+ctx.spgemm(dw, dw).free()  # (kernels are loaded: these name enough rows for tables)
+dw.free()
+ctx.trim()
+hog = leave(1_740_000_000)
+c = ctx.spgemm(da, db)
+del hog
+ctx.trim()
+m = c.download()
+for j in [0, 1, 63, 64, n // 2 + 5, n - 400, n - 1] + list(range(100_000, 100_040)):
+    want = np.unique(cols[j:j + 400][ok[j:j + 400]])
+    e = m.entries[int(m.rowmap[j]):int(m.rowmap[j + 1])].reshape(-1, 2)
+    assert np.array_equal(e[:, 0], want) and np.array_equal(e[:, 1], want), j
+assert m.entries.size > 700 * n and m.nnz() == m.entries.size // 2
+""")
