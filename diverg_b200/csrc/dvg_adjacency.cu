@@ -20,8 +20,9 @@
 // and counts its ranges, a scan gives every node's first entry, then a thread
 // per locus writes the row map and its row.  The output is allocated for the
 // most entries that so many bases and edges can have (a few more than there
-// are), so nothing is waited for until the end; a node range's edges are counted
-// first.
+// are, in most graphs), so nothing is waited for until the end; a node range's
+// edges are counted first.  Where so much does not fit, the entries are counted
+// before the output is allocated, and where much of it stays empty, it is given back.
 //
 // Bound: the matrix's writes, 16 bytes a locus; below ~1e6 loci the launches and
 // the one wait.  1e7 loci of 3.4e4 nodes and 4.6e4 edges: 449 -> 163 us a call, of which
@@ -337,12 +338,21 @@ dvg_matrix* adjacency_from_graph(dvg_context* ctx, uint32_t nnodes, const uint32
     p.base_n = arrays > 4 ? p.eoff_n + words : p.base;
     uint64_t* h_sizes = reinterpret_cast<uint64_t*>(ctx->h_ctl + 1);
     uint64_t most_edges = nedges;  // of the range
-    auto allocate = [&]() {
-      p.cols = static_cast<uint32_t*>(grab(std::max<uint64_t>(most_edges, 1) * 4));
-      // at most a range a base but the last of a node, and one an edge
-      out = new_matrix(ctx, uint32_t(nloci), uint32_t(nloci), 2 * (nloci - m) + 2 * most_edges);
+    uint64_t cap = 0;              // entries that the result has room for
+    auto make_result = [&](uint64_t entries) {
+      out = new_matrix(ctx, uint32_t(nloci), uint32_t(nloci), entries);
+      cap = entries;
       p.c_rowmap = out->rowmap;
       p.c_entries = out->entries;
+    };
+    auto allocate = [&]() {
+      p.cols = static_cast<uint32_t*>(grab(std::max<uint64_t>(most_edges, 1) * 4));
+      try {
+        // at most a range a base but the last of a node, and one an edge
+        make_result(2 * (nloci - m) + 2 * most_edges);
+      } catch (const Error& e) {
+        if (e.status != DVG_ERR_OOM) throw;  // (counted first, below)
+      }
     };
     const bool whole = m == nnodes;
     if (whole) allocate();
@@ -364,6 +374,11 @@ dvg_matrix* adjacency_from_graph(dvg_context* ctx, uint32_t nnodes, const uint32
     k_adj_nodes<<<adj_grid(ctx, m), kAdjThreads, 0, ctx->stream>>>(p);
     DVG_CUDA(cudaGetLastError());
     scan_nodes(ctx, p.base_n, p.base, nullptr, nullptr, m);
+    if (!out) {
+      DVG_CUDA(cudaMemcpyAsync(h_sizes, p.base + m, 8, cudaMemcpyDeviceToHost, ctx->stream));
+      read_control(ctx);
+      make_result(h_sizes[0]);
+    }
     k_adj_rows<<<unsigned((nloci + kAdjTile - 1) / kAdjTile), kAdjThreads, 0, ctx->stream>>>(p, nloci);
     DVG_CUDA(cudaGetLastError());
     ctx->stats.kernel_launches += 4 + (nedges ? 1 : 0);
@@ -382,6 +397,7 @@ dvg_matrix* adjacency_from_graph(dvg_context* ctx, uint32_t nnodes, const uint32
     out->nentries = h_sizes[0];
     out->canonical = !(c.invalid & 16);
     out->nnz = (nloci - m) + h_sizes[1];
+    if (give_back(ctx, out, cap)) DVG_CUDA(cudaStreamSynchronize(ctx->stream));  // the caller waits no more
   } catch (...) {
     for (void* q : scratch) dfree(ctx, q);
     if (out) free_matrix(ctx, out);

@@ -216,3 +216,21 @@ def test_large_dense_input_stays_in_range_crs(ctx, n, dense_slots):
             assert np.array_equal(forms[0].entries, forms[1].entries), what
             assert (moved[0] != moved[1]) == slots, (what, moved)
         d.free()
+
+
+def test_an_adjacency_matrix_holds_no_more_than_it_needs(ctx):
+    # one range a row, however many edges in a row make it
+    n = 2_000
+    u = np.repeat(np.arange(1, n, dtype=np.uint32), np.arange(n - 1, 0, -1))
+    v = np.concatenate([np.arange(k + 1, n + 1, dtype=np.uint32) for k in range(1, n)])
+    for lower, upper in ((1, 0), (1, n), (5, n + 1)):
+        before = used_bytes(ctx)
+        edges = np.stack([u, v], 1)
+        if upper == n:
+            edges = edges[v < n]  # (none leaves the node range)
+        m = ctx.adjacency_from_graph(np.ones(n, np.uint32), edges, lower, upper)
+        held = used_bytes(ctx) - before
+        assert held <= block(8 * (m.nrows + 1) + 16) + 5 * block(5 * m.nentries + (1 << 20) + 16) // 4, held
+        rows = (upper or n + 1) - lower
+        assert m.nentries == 2 * (rows - 1) and m.nnz == rows * (rows - 1) // 2
+        m.free()

@@ -86,3 +86,26 @@ for j in [0, 1, 63, 64, n // 2 + 5, n - 400, n - 1] + list(range(100_000, 100_04
     assert np.array_equal(e[:, 0], want) and np.array_equal(e[:, 1], want), j
 assert m.entries.size > 700 * n and m.nnz() == m.entries.size // 2
 """)
+
+
+def test_an_adjacency_matrix_of_many_edges_in_a_row():
+    # 1e4 nodes of one base with an edge to every later one: 5e7 edges, 0.60 GB, and one
+    # range a row.  A range an edge would be 0.40 GB more
+    child("""
+n = 10_000
+def edges(n):
+    u = np.repeat(np.arange(1, n, dtype=np.uint32), np.arange(n - 1, 0, -1))
+    at = np.concatenate(([0], np.cumsum(np.arange(n - 1, 0, -1)))).astype(np.int64)
+    v = (np.arange(u.size) - at[u - 1]).astype(np.uint32) + u + 1
+    return np.stack([u, v], 1)
+ctx.adjacency_from_graph(np.ones(100, np.uint32), edges(100)).free()  # (kernels are loaded)
+e = edges(n)
+hog = leave(800_000_000)
+a = ctx.adjacency_from_graph(np.ones(n, np.uint32), e)
+del hog
+m = a.download()
+i = np.arange(n - 1, dtype=np.uint32)
+assert np.array_equal(m.rowmap, 2 * np.minimum(np.arange(n + 1, dtype=np.uint64), n - 1))
+assert np.array_equal(m.entries.reshape(-1, 2), np.stack([i + 1, np.full(n - 1, n - 1, np.uint32)], 1))
+assert m.nnz() == len(e)
+""")
