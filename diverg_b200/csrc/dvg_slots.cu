@@ -1363,28 +1363,33 @@ SlotPlan plan_slots(unsigned dlo, unsigned dup, double branching) {
     return v;
   };
   // passes that multiply by A^v, its factors the largest powers that fit
+  // (counted, not listed: A^v has up to v / have[0] of them)
   auto passes = [&](unsigned v, const std::vector<unsigned>& have) {
-    unsigned n = 0, k = 0;
-    unsigned long long sum = 0;
-    for (size_t j = have.size(); j-- > 0;)
-      for (; v >= have[j]; v -= have[j]) {
-        if (n == 0 || k == kChainMax || sum + have[j] > reach) {
-          ++n;
-          k = 0;
-          sum = 0;
-        }
-        ++k;
-        sum += have[j];
+    uint64_t n = 0, k = 0, sum = 0;  // passes, and the last one's factors and their exponents
+    for (size_t j = have.size(); j-- > 0; v %= have[j]) {
+      const uint64_t e = have[j], fit = std::clamp<uint64_t>(reach / e, 1, kChainMax);
+      uint64_t q = v / e;
+      if (n && q) {
+        const uint64_t more = sum >= reach ? 0 : std::min<uint64_t>({q, kChainMax - k, (reach - sum) / e});
+        q -= more;
+        k += more;
+        sum += more * e;
       }
+      if (q) {
+        n += (q + fit - 1) / fit;
+        k = (q - 1) % fit + 1;
+        sum = k * e;
+      }
+    }
     return n;
   };
   // powers up to half of Q's, and further where that saves passes over A^dlo
   unsigned p_top = q_top > 1 ? q_top / 2 : 1;
   if (rest) p_top = std::max(p_top, 1u << top_bit(rest));
-  unsigned best = ~0u;
+  uint64_t best = ~uint64_t(0);
   for (unsigned long long top = p_top; top <= std::max<unsigned long long>(p_top, dlo); top *= 2) {
     const std::vector<unsigned> have = levels(unsigned(top));
-    unsigned cost = passes(rest, have) + passes(dlo, have);
+    uint64_t cost = passes(rest, have) + passes(dlo, have);
     for (unsigned e = 1; e < std::max(unsigned(top), q_top); ++cost) e *= factor(e, unsigned(top));
     if (cost < best) {
       best = cost;

@@ -1,5 +1,7 @@
 """GPU: which way a call takes, and what it holds on to: matrices whose caller gave
 another column count than the true one, results' memory, chains that do not fit."""
+import time
+
 import numpy as np
 import pytest
 
@@ -234,3 +236,47 @@ def test_an_adjacency_matrix_holds_no_more_than_it_needs(ctx):
         rows = (upper or n + 1) - lower
         assert m.nentries == 2 * (rows - 1) and m.nnz == rows * (rows - 1) // 2
         m.free()
+
+
+def cycle(n, steps):
+    """Row i holds the columns i + s modulo n for the steps s."""
+    cols = np.sort((np.arange(n)[:, None] + np.array(steps)) % n, axis=1)
+    rows = [[(c[0], c[0])] for c in cols] if len(steps) == 1 else None
+    if rows is None:
+        rows = []
+        for c in cols:
+            r = []
+            for x in c:
+                if r and r[-1][1] + 1 == x:
+                    r[-1] = (r[-1][0], x)
+                else:
+                    r.append((x, x))
+            rows.append(r)
+    rm = np.concatenate(([0], np.cumsum([2 * len(r) for r in rows]))).astype(np.uint64)
+    return CRSMatrix(n, np.array([x for r in rows for v in r for x in v], np.uint32), rm)
+
+
+@pytest.mark.parametrize("window", [(2 ** 31 + 5, 2 ** 31 + 5), (3_000_000_000, 3_000_000_002), (2 ** 32 - 1, 2 ** 32 - 1)])
+def test_large_exponents_are_planned_at_once(ctx, window):
+    # a chain over a cycle takes some 40 passes, whatever the exponent
+    m = cycle(1_000, (1,))
+    d = ctx.upload(m)
+    want = orc.dindex(omat(m), *window, algo="hbv")
+    ctx.distance_index(d, 5, 9).free()
+    t = time.perf_counter()
+    r = ctx.distance_index(d, *window)
+    took = time.perf_counter() - t
+    same(r.download(), want, window)
+    assert took < 0.3, took
+
+
+@pytest.mark.parametrize("window", [(0, 2 ** 32 - 1), (2 ** 32 - 1, 2 ** 32 - 1), (2 ** 31 + 1, 2 ** 32 - 1), (7, 2 ** 31)])
+def test_large_exponents_where_a_pass_takes_one_factor(ctx, window):
+    # two columns a row: A^dmin by factors of A alone would take up to 2^32 - 1 passes
+    m = cycle(300, (1, 2))
+    d = ctx.upload(m)
+    t = time.perf_counter()
+    r = ctx.distance_index(d, *window)
+    took = time.perf_counter() - t
+    same(r.download(), orc.dindex(omat(m), *window, algo="hbv"), window)
+    assert took < 1.0, took
