@@ -25,6 +25,7 @@
 #include <cstring>
 
 #include "dvg_internal.h"
+#include "dvg_slots.h"
 
 namespace dvg {
 
@@ -188,8 +189,9 @@ uint64_t predict_build_bytes(double growth, uint32_t n, uint64_t nentries, unsig
   // 2 x 17 x 4 bytes x 2048 rows for each of the 2 CTAs of an SM's 148
   const uint64_t stage = std::min<uint64_t>(136ull * n, 2ull * 148 * 2 * 17 * 4 * 2048);
   const uint64_t scratch = plan.steps.size() * ((uint64_t(n) / 64 + 1) * 32 + 512) + stage;
-  // the input is held twice while a batch lays it out block-diagonally
-  return 2 * input + uint64_t(max_live) * slot + scratch;
+  // the input is held twice while a batch lays it out block-diagonally; a build that
+  // runs as a chain over row slots falls back to the planned one, its buffers given back
+  return std::max(2 * input + uint64_t(max_live) * slot + scratch, predict_slots_bytes(n, nentries, dlo, dup));
 }
 
 void release_build(dvg_context* ctx, PlannedBuild& pb) {

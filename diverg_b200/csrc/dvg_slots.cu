@@ -66,6 +66,7 @@ constexpr double kChainReach = 1.28;          // branching * steps of a pass's l
 constexpr uint32_t kEarlyRows = 1u << 24;
 constexpr double kEarlySlack = 1.125;
 constexpr uint64_t kEarlySpare = 1u << 16;
+constexpr uint32_t kQueueMax = 1u << 15;  // rows that a pass's queue has places for, at most
 constexpr double kSlotGrowthMax = 8.0;  // ranges a row that an arena is made for
 // Up to so many rows, and for single products as long as their results are written
 // early, the chain's kernels are launched close behind one another: the next one's
@@ -1511,6 +1512,52 @@ static void slots_missed(dvg_context* ctx, const SlotKey& key) {
 
 static unsigned conversion_blocks(const SlotBuild& sb) { return unsigned((uint64_t(sb.n) + kCrsRows - 1) / kCrsRows); }
 
+// The buffer of each of a plan's matrices, `count` of them together: a matrix takes that
+// of one whose last reader is an earlier pass (the chain's own buffers only: chains that
+// run side by side share none).
+static std::vector<int> assign_buffers(const SlotPlan& plan, int& count) {
+  std::vector<int> last(plan.nmats, -1), buffer(plan.nmats, 0), spare;
+  auto reads = [&](const SlotStep& s, auto&& f) {
+    for (int j = 0; j < s.k; ++j) f(s.m[j]);
+    if (s.b >= 0) f(s.b);
+  };
+  for (size_t i = 0; i < plan.steps.size(); ++i) reads(plan.steps[i], [&](int k) { last[k] = int(i); });
+  auto take = [&](int k) {
+    if (spare.empty()) spare.push_back(count++);
+    buffer[k] = spare.back();
+    spare.pop_back();
+  };
+  for (int k = 0; k < plan.inputs; ++k) take(k);
+  for (size_t i = 0; i < plan.steps.size(); ++i) {
+    if (plan.steps[i].s >= 0) take(plan.steps[i].s);
+    if (plan.steps[i].c >= 0) take(plan.steps[i].c);
+    std::vector<int> done;
+    reads(plan.steps[i], [&](int k) {
+      if (last[k] == int(i) && k != plan.out && std::find(done.begin(), done.end(), k) == done.end()) done.push_back(k);
+    });
+    for (int k : done) spare.push_back(buffer[k]);
+  }
+  return buffer;
+}
+
+uint64_t predict_slots_bytes(uint32_t nrows, uint64_t nentries, unsigned dlo, unsigned dup) {
+  // (the density decides the passes; the buffers of a few stand for all)
+  int buffers = 0;
+  size_t steps = 0;
+  for (double density : {0.0, 0.001, 0.01, 0.1, 1.0}) {
+    int count = 0;
+    const SlotPlan plan = plan_slots(dlo, dup, density);
+    assign_buffers(plan, count);
+    buffers = std::max(buffers, count);
+    steps = std::max(steps, plan.steps.size());
+  }
+  const uint64_t n = (uint64_t(nrows) + kSlotPartRows - 1) / kSlotPartRows * kSlotPartRows;
+  const uint64_t ranges = std::min<uint64_t>(uint64_t(kSlotGrowthMax * double(n)) + 4096, kMulti);
+  const uint64_t input = 8 * n + 4 * nentries, result = 8 * n + 16 * n, scratch = n + steps * (kQueueMax * 4 + 8);
+  // (blocks are up to a quarter larger than what they hold)
+  return (input + 8 * n * buffers + 8 * ranges + result + scratch) / 4 * 5;
+}
+
 SlotBuild prepare_slots(dvg_context* ctx, const SlotPlan& plan, uint32_t n) {
   SlotBuild sb;
   sb.plan = plan;
@@ -1519,34 +1566,19 @@ SlotBuild prepare_slots(dvg_context* ctx, const SlotPlan& plan, uint32_t n) {
   const uint64_t groups = (uint64_t(n) + kCountRows - 1) / kCountRows;
   const uint64_t supers = (groups + kSuperGroups - 1) / kSuperGroups;
   // a pass's rows to be walked by warps: room for its clumps (a row past it is walked at once)
-  sb.queue_cap = uint32_t(std::clamp<uint64_t>(n / 8, 256, 1u << 15));
+  sb.queue_cap = uint32_t(std::clamp<uint64_t>(n / 8, 256, kQueueMax));
   auto round = [](size_t x) { return (x + 15) & ~size_t(15); };
   const size_t taken_off = 512, queue_off = taken_off + plan.steps.size() * 8;
   const size_t nnz_off = round(queue_off + plan.steps.size() * sb.queue_cap * 4), cnt_off = nnz_off + groups * 8;
   const size_t sums_off = round(cnt_off + groups * 4), masks_off = sums_off + supers * 8;
   static_assert(sizeof(SlotCounters) <= 512, "the counters come first");
-  std::vector<int> last(plan.nmats, -1);
-  auto reads = [&](const SlotStep& s, auto&& f) {
-    for (int j = 0; j < s.k; ++j) f(s.m[j]);
-    if (s.b >= 0) f(s.b);
-  };
-  for (size_t i = 0; i < plan.steps.size(); ++i) reads(plan.steps[i], [&](int k) { last[k] = int(i); });
   // (below kMulti, so that the slot of a row of several runs has y < x)
   sb.arena_cap = std::min<uint64_t>(uint64_t(ctx->slot_growth * double(n)) + 4096, kMulti);
   const double room = 0.5 * double(device_free_bytes(ctx) + ctx->cached_bytes);
   if (double(sb.arena_cap) * 8.0 > room) sb.arena_cap = uint64_t(room / 8.0) + 4096;
   if (n <= kEarlyRows && 16.0 * double(n) < room / 8.0) sb.early = 2ull * n;
-  // a matrix takes the buffer of one whose last reader is an earlier pass (the
-  // chain's own buffers only: chains that run side by side share none)
-  std::vector<uint2*> spare;
-  auto take = [&](int k) {
-    if (spare.empty()) {
-      sb.buffers.push_back(static_cast<uint2*>(dalloc(ctx, size_t(n) * sizeof(uint2))));
-      spare.push_back(sb.buffers.back());
-    }
-    sb.mat[k] = spare.back();
-    spare.pop_back();
-  };
+  int nbuffers = 0;
+  const std::vector<int> buffer = assign_buffers(plan, nbuffers);
   try {
     sb.scratch = dalloc(ctx, masks_off + (uint64_t(n) + 31) / 32 * 4);
     char* base = static_cast<char*>(sb.scratch);
@@ -1563,16 +1595,9 @@ SlotBuild prepare_slots(dvg_context* ctx, const SlotPlan& plan, uint32_t n) {
     sb.group_cnt = reinterpret_cast<uint32_t*>(base + cnt_off);
     sb.masks = reinterpret_cast<uint32_t*>(base + masks_off);
     sb.arena = static_cast<uint2*>(dalloc(ctx, sb.arena_cap * sizeof(uint2)));
-    for (int k = 0; k < plan.inputs; ++k) take(k);
-    for (size_t i = 0; i < plan.steps.size(); ++i) {
-      if (plan.steps[i].s >= 0) take(plan.steps[i].s);
-      if (plan.steps[i].c >= 0) take(plan.steps[i].c);
-      std::vector<int> done;
-      reads(plan.steps[i], [&](int k) {
-        if (last[k] == int(i) && k != plan.out && std::find(done.begin(), done.end(), k) == done.end()) done.push_back(k);
-      });
-      for (int k : done) spare.push_back(sb.mat[k]);
-    }
+    for (int k = 0; k < nbuffers; ++k)
+      sb.buffers.push_back(static_cast<uint2*>(dalloc(ctx, size_t(n) * sizeof(uint2))));
+    for (int k = 0; k < plan.nmats; ++k) sb.mat[k] = sb.buffers[buffer[k]];
   } catch (...) {
     release_slots(ctx, sb);
     throw;

@@ -90,6 +90,8 @@ struct SlotBuild {
 // allocation); issues it (no host round trip: it may be captured).
 // A plan of two inputs takes `right` as its second.
 SlotBuild prepare_slots(dvg_context* ctx, const SlotPlan& plan, uint32_t n);
+// Device memory that an index build as a chain may take, its input and result included.
+uint64_t predict_slots_bytes(uint32_t nrows, uint64_t nentries, unsigned dlo, unsigned dup);
 void launch_slots(dvg_context* ctx, SlotBuild& sb, const SlotParts& parts, bool timed, const SlotPart* right = nullptr);
 // Ranges and columns of each part's result (device, two words a part), once
 // the chain has run.

@@ -280,3 +280,22 @@ def test_large_exponents_where_a_pass_takes_one_factor(ctx, window):
     took = time.perf_counter() - t
     same(r.download(), orc.dindex(omat(m), *window, algo="hbv"), window)
     assert took < 1.0, took
+
+
+@pytest.mark.parametrize("window", [(0, 1), (1, 1), (0, 2), (3, 5), (0, 250), (400, 600)])
+def test_the_server_reserves_what_a_build_takes(window):
+    # a budget below what a build of 4e6 bases takes admits none, even with the largest arena
+    from diverg_b200.serving import Server
+    a, _ = gen.graph_adjacency(gen.chromosome_graph_spec(4_000_000, seed=93))
+    held = 8 * (a.numRows() + 1) + 4 * a.entries.size
+    ctx = Context(0)
+    dense = gen.banded(3_000, 3_000, 1.4, 1.0, seed=64)  # (fills its arena: the next one is larger)
+    dd = ctx.upload(dense)
+    ctx.distance_index(dd, 12, 12).free()
+    d = ctx.upload(a)
+    took = held + peak_bytes(ctx, lambda: ctx.batch_distance_index([d], [window])[0].free())
+    d.free()
+    ctx.close()
+    with Server(hbm_budget_bytes=took - 1) as s:
+        req = s.submit_build(a, *window)
+        assert s.wait([req])[0]["status"] != 0
