@@ -452,7 +452,7 @@ dvg_matrix* range_spadd(dvg_context* ctx, const dvg_matrix* a, const dvg_matrix*
   // the one-pass kernel stages ranges with 8-byte asynchronous copies
   const bool aligned = ((reinterpret_cast<uintptr_t>(a->entries) |
                          reinterpret_cast<uintptr_t>(b_identity ? nullptr : b->entries)) & 7u) == 0;
-  if (ctx->opt_spadd_single && n > 0 && aligned) {
+  if (ctx->opt_spadd_single && n > 0 && aligned && spadd_single_pass_suits(a, b, b_identity)) {
     // one pass: the output never holds more entries than both inputs
     const uint64_t cap = a->nentries + (b_identity ? 2ull * n : b->nentries);
     dvg_matrix* c = new_matrix(ctx, n, a->ncols, cap);

@@ -190,6 +190,8 @@ void launch_spadd(dvg_context* ctx, const dvg_matrix* a, const dvg_matrix* b, bo
 // fully, c_entries up to `cap` entries (a.nentries + b's entries always
 // suffice); the control block receives the total entries, the nnz and a
 // timeout flag.  `scratch`: spadd_single_pass_scratch(a, b, b_identity) bytes.
+// For sums whose rows are not so dense that two passes (launch_spadd) are faster.
+bool spadd_single_pass_suits(const dvg_matrix* a, const dvg_matrix* b, bool b_identity);
 uint64_t spadd_single_pass_scratch(const dvg_matrix* a, const dvg_matrix* b, bool b_identity);
 void launch_spadd_single_pass(dvg_context* ctx, const dvg_matrix* a, const dvg_matrix* b, bool b_identity,
                               uint64_t* c_rowmap, uint32_t* c_entries, uint64_t cap, void* scratch);

@@ -850,11 +850,19 @@ void launch_spadd(dvg_context* ctx, const dvg_matrix* a, const dvg_matrix* b, bo
 // have more ranges than its image on average -- its rows are then merged in place
 // and wait for their offset.  2^20 rows of 8.8, 17.7 and 53 ranges of each operand
 // (64, 16 and 8 rows a chunk): 488 -> 272, 1456 -> 579 and, for 2^19, 3976 -> 979 us.
+// 0: a row alone is more than an image, and every chunk would merge twice.  The sum in
+// two passes (k_spadd) is faster there: 1.4e4 us against 3.4e3 with 2^17 rows of 461
+// ranges of each operand, 8.3e3 against 2.3e3 with 2^16 of 656, 1.8e3 against 1.4e3 with
+// 2^13 of 565.
 static uint32_t add_chunk_rows(const dvg_matrix* a, const dvg_matrix* b, bool b_identity) {
   const uint64_t n = a->nrows, ranges = (a->nentries + (b_identity ? 2 * n : b->nentries)) / 2;
   uint32_t rows = kAddThreads;
-  while (rows > 1 && ranges * rows > n * (8ull * kAddImage / 9)) rows /= 2;
-  return ranges * rows > n * (8ull * kAddImage / 9) ? uint32_t(kAddThreads) : rows;
+  while (rows && ranges * rows > n * (8ull * kAddImage / 9)) rows /= 2;
+  return rows;
+}
+
+bool spadd_single_pass_suits(const dvg_matrix* a, const dvg_matrix* b, bool b_identity) {
+  return add_chunk_rows(a, b, b_identity) > 0;
 }
 
 uint64_t spadd_single_pass_scratch(const dvg_matrix* a, const dvg_matrix* b, bool b_identity) {

@@ -299,3 +299,24 @@ def test_the_server_reserves_what_a_build_takes(window):
     with Server(hbm_budget_bytes=took - 1) as s:
         req = s.submit_build(a, *window)
         assert s.wait([req])[0]["status"] != 0
+
+
+@pytest.mark.parametrize("n", [1, 300, 5_000])
+@pytest.mark.parametrize("ranges,single", [(400, True), (455, True), (456, False), (600, False)])
+def test_sums_of_dense_rows(ctx, n, ranges, single):
+    # up to 910 ranges a row of both operands together in one pass (one launch), denser
+    # rows in two
+    ncols = 4 * ranges + 8
+    rng = np.random.default_rng(94)
+
+    def dense(shift):
+        first = 4 * np.arange(ranges) + shift + rng.integers(0, 2, (n, ranges))
+        e = np.stack([first, first + rng.integers(0, 2, (n, ranges))], 2).astype(np.uint32).reshape(-1)
+        return CRSMatrix(ncols, e, 2 * ranges * np.arange(n + 1, dtype=np.uint64))
+    a, b = dense(0), dense(2)
+    da, db = ctx.upload(a), ctx.upload(b)
+    ctx.reset_stats()
+    c = ctx.spadd(da, db)
+    launches = ctx.stats()["kernel_launches"]
+    same(c.download(), orc.spadd(omat(a), omat(b)), (n, ranges))
+    assert (launches == 1) == single, launches
