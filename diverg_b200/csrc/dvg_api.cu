@@ -799,6 +799,7 @@ dvg_status dvg_shutdown(dvg_context* ctx) {
     if (ctx->d_tile_desc) dfree(ctx, ctx->d_tile_desc);
     if (ctx->d_row_stage) dfree(ctx, ctx->d_row_stage);
     if (ctx->d_ticket) dfree(ctx, ctx->d_ticket);
+    if (ctx->d_slot_queue) dfree(ctx, ctx->d_slot_queue);
     release_cached(ctx);
     DVG_CUDA(cudaStreamSynchronize(ctx->stream));
     resolve_spans(ctx);

@@ -380,7 +380,7 @@ void batch_distance_index(dvg_context* ctx, uint32_t ngraphs, const dvg_matrix* 
     for (auto it = chains.begin(); it != chains.end();) {
       try {
         const SlotKey key = it->sb.key;
-        it->sb = prepare_slots(ctx, plan_slots(it->dlo, it->dup, branching(it->columns, it->n)), uint32_t(it->n));
+        it->sb = prepare_slots(ctx, plan_slots(it->dlo, it->dup, branching(it->columns, it->n)), uint32_t(it->n), true);
         it->sb.key = key;
         it->ready = true;
         ++it;

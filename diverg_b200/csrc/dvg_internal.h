@@ -95,6 +95,8 @@ struct dvg_context {
   int64_t opt_slots = 1;              // chains of products over graph-like input run in the row-slot format
   double slot_growth = 4.0;           // row-slot chains: ranges the arena holds / rows
   std::map<SlotKey, SlotMiss> slot_misses;
+  unsigned long long* d_slot_queue = nullptr;  // rows of chains that warps walk, made on first use
+  uint32_t slot_epoch = 0;                     // the last pass that used it
   double early_growth = 1.125;        // row-slot builds: ranges the result gets room for / rows
   double product_growth = 2.0;        // products with long A ranges: entry capacity / the larger input's entries
   uint64_t max_product_entries = 0;   // largest product output since the last reset (read-back path)

@@ -39,6 +39,7 @@ constexpr int kSThreads = 256;  // streaming kernels
 constexpr int kSWarps = kSThreads / 32;
 constexpr int kWThreads = 128;  // kernels that walk rows
 constexpr int kWWarps = kWThreads / 32;
+constexpr int kWBlocks = 7;     // of them an SM holds at once (72 registers a thread)
 constexpr int kSRows = 4;       // rows a lane of k_chain_rows takes
 constexpr int kSRuns = 8;       // runs of a lane's list
 constexpr int kSWin = 256;      // window words of a warp (8,192 columns)
@@ -66,7 +67,8 @@ constexpr double kChainReach = 1.28;          // branching * steps of a pass's l
 constexpr uint32_t kEarlyRows = 1u << 24;
 constexpr double kEarlySlack = 1.125;
 constexpr uint64_t kEarlySpare = 1u << 16;
-constexpr uint32_t kQueueMax = 1u << 15;  // rows that a pass's queue has places for, at most
+constexpr uint32_t kQueueRows = 1u << 15;  // places of a queue (rows past them are walked at once)
+constexpr size_t kQueueBytes = kQueueRows * sizeof(unsigned long long);
 constexpr double kSlotGrowthMax = 8.0;  // ranges a row that an arena is made for
 // Up to so many rows, and for single products as long as their results are written
 // early, the chain's kernels are launched close behind one another: the next one's
@@ -139,8 +141,9 @@ struct ChainArgs {
   unsigned long long* wide;   // what unions by windows have cost, and may
   unsigned long long wide_max;
   uint32_t* masks;            // bit r % 32 of word r / 32: k_chain_rows left row r to k_chain_walk
-  uint32_t* queue;            // this pass's rows that a warp walks, + 1 (0: not there yet), and
-  uint32_t* taken;            // how many places were taken (taken[0]) and filled (taken[1])
+  unsigned long long* queue;  // rows that a warp walks, and of this pass how many places
+  uint32_t* taken;            // were taken (taken[0]) and filled (taken[1])
+  uint32_t epoch;             // the pass's: what it puts into the queue has it in the upper half
   uint32_t queue_cap;
   uint32_t* group_cnt;        // last pass: ranges and columns of c per kCountRows rows
   unsigned long long* group_nnz;
@@ -501,7 +504,7 @@ __device__ uint2 warp_union(const ChainArgs& p, uint2 left, const uint2* mat, ui
     if (lane == 0) atomicOr(p.abort, why);
     return empty_slot();
   };
-  if (__shfl_sync(kFullMask, given_up(p), 0)) return empty_slot();
+  if (__any_sync(kFullMask, given_up(p))) return empty_slot();
   uint32_t named = 0;  // rows (at most kWideColumns + 1 counted of a range)
   for (uint32_t t = lane, c = mat ? slot_count(left) : 0; t < c; t += 32) {
     const uint2 r = is_multi(left) ? __ldcg(p.arena + left.y + t) : slot_range(p.arena, left, t);
@@ -735,8 +738,15 @@ __device__ bool bitmap_row(const ChainArgs& p, WarpSmem& M, uint32_t row, uint2&
   return true;
 }
 
-// A row by the whole warp, however many runs it has; c's ranges and columns.  (A
-// function of its own, so that its registers are not the lanes' walks'.)
+template <bool OUTS, bool OUTC>
+__device__ __forceinline__ void leave_empty(const ChainArgs& p, uint32_t r) {
+  if (OUTS) p.s[r] = empty_slot();
+  if (OUTC) p.c[r] = empty_slot();
+}
+
+// A row by the whole warp, however many runs it has (none, where the chain is given up);
+// c's ranges and columns.  (A function of its own, so that its registers are not the
+// lanes' walks'.)
 struct RowCount {
   uint32_t ranges;
   unsigned long long columns;
@@ -747,6 +757,11 @@ __device__ __noinline__ RowCount warp_row(const ChainArgs& p, WarpSmem& S, uint3
   uint2 s = make_uint2(r, r), c = empty_slot();
   uint32_t k = 0;
   unsigned long long z = 0;
+  if (__any_sync(kFullMask, given_up(p))) {
+    if (lane == 0) leave_empty<OUTS, OUTC>(p, r);
+    __syncwarp();
+    return {0, 0};
+  }
   if (!bitmap_row<OUTS, OUTC>(p, S, r, s, c, k, z)) {
     __syncwarp();
     s = make_uint2(r, r);
@@ -777,25 +792,30 @@ __device__ __noinline__ RowCount warp_row(const ChainArgs& p, WarpSmem& S, uint3
 // of them, and one after another in their warp would be what the pass lasts.  A^300 of
 // 1e6 bases of a variant-dense graph, 4,172 such rows: 9.9 ms by unions of windows in
 // the row's own warp, 1.2 by bitmaps through the queue; A^100, 52 such rows: 1.72 ms and
-// 0.25; the build for [1000, 1300], 1,910: 4.3 and 0.86.  Where no row needs it, the queue
-// and its clearing cost 3 % of a build of 1e5 bases (152 -> 157 us).  Nobody
-// waits: a place is settled by one exchange each of the warp that puts a row in and of
-// the one that takes it, and where the taker comes first (kGone) the row stays with
-// the warp that had it.  A look into the queue is a trip to memory, at the end of a
-// pass: a warp whose own rows were all quick ones is done before others put rows in,
-// and does not look.
+// 0.24; the build for [1000, 1300], 1,910: 4.3 and 0.86.  Where no row needs it, the queue
+// and the longer code cost 2 to 3 % of a small build (1e5 bases 150 -> 155 us).  Nobody
+// waits: a place is settled by one atomic each of the warp that puts a row in and of the
+// one that takes it, and where the taker comes first (kGone) the row stays with the warp
+// that had it.  What earlier passes left there has another epoch and counts as empty, so
+// the queue is cleared when it is made and never again.  A warp looks into the
+// queue when it has walked rows: one whose rows were all quick ones is done before others
+// put theirs in, and does not.
 constexpr uint32_t kGone = 0xffffffffu;
+__device__ __forceinline__ unsigned long long in_queue(const ChainArgs& p, uint32_t v) {
+  return (unsigned long long)p.epoch << 32 | v;
+}
 template <bool OUTS, bool OUTC, class Tally>
 __device__ void take_rows(const ChainArgs& p, WarpSmem& S, Tally&& tally) {
   for (;;) {
     const uint2 places = __ldcg(reinterpret_cast<const uint2*>(p.taken));
-    const bool none = places.x >= min(places.y, p.queue_cap) || given_up(p);
-    if (__shfl_sync(kFullMask, none, 0)) return;
+    if (__shfl_sync(kFullMask, places.x >= min(places.y, p.queue_cap), 0)) return;
     uint32_t r = 0;  // row + 1
     if (lane_id() == 0) {
       const uint32_t at = atomicAdd(p.taken, 1u);
-      if (at < p.queue_cap) r = atomicExch(p.queue + at, kGone);
-      __threadfence();
+      if (at < p.queue_cap) {
+        const unsigned long long was = atomicExch(p.queue + at, in_queue(p, kGone));
+        if (was >> 32 == p.epoch) r = uint32_t(was);
+      }
     }
     r = __shfl_sync(kFullMask, r, 0);
     if (r == 0) continue;
@@ -806,18 +826,14 @@ __device__ void take_rows(const ChainArgs& p, WarpSmem& S, Tally&& tally) {
 
 // Walks the `batch` rows of the warp's list, a row a lane; rows of more runs
 // than a lane's lists hold go to the queue (take_rows), or to the whole warp at once
-// where that is full.  Whether some of them were no quick ones.  (`dropped`: the chain
-// is given up.)
+// where that is full.  Returns whether rows wait there.  (`dropped`: the chain is given up.)
 // tally(row, ranges, columns) for each row of c that has any.
 template <bool OUTS, bool OUTC, class Tally>
 __device__ __forceinline__ bool walk_batch(const ChainArgs& p, WarpSmem& S, uint32_t batch, bool dropped,
                                            Tally&& tally) {
   const int lane = lane_id();
-  if (dropped) {
-    if (uint32_t(lane) < batch) {
-      if (OUTS) p.s[S.todo[lane]] = empty_slot();
-      if (OUTC) p.c[S.todo[lane]] = empty_slot();
-    }
+  if (__any_sync(kFullMask, dropped)) {
+    if (uint32_t(lane) < batch) leave_empty<OUTS, OUTC>(p, S.todo[lane]);
     __syncwarp();
     return false;
   }
@@ -828,7 +844,7 @@ __device__ __forceinline__ bool walk_batch(const ChainArgs& p, WarpSmem& S, uint
     row = S.todo[lane];
     done = quick_row<OUTS, OUTC>(p, row, S.list[0] + lane, ns, C, nc);
   }
-  const bool look = __any_sync(kFullMask, uint32_t(lane) < batch && !done);
+  const bool slow = __any_sync(kFullMask, uint32_t(lane) < batch && !done);
   if (uint32_t(lane) < batch && !done) {
     S.list[0][lane] = make_uint2(row, row);
     ns = 1;
@@ -846,6 +862,9 @@ __device__ __forceinline__ bool walk_batch(const ChainArgs& p, WarpSmem& S, uint
   }
   __syncwarp();
   unsigned left = __ballot_sync(kFullMask, uint32_t(lane) < batch && !done);
+  // (the look comes while the rows are written)
+  const uint2 places = slow ? __ldcg(reinterpret_cast<const uint2*>(p.taken)) : make_uint2(0u, 0u);
+  const bool put_in = left != 0;
   // places in the arena for the rows of several runs, one request a warp
   // (a row of two columns needs none)
   const uint2* const T = S.list[cur] + lane;
@@ -891,22 +910,17 @@ __device__ __forceinline__ bool walk_batch(const ChainArgs& p, WarpSmem& S, uint
       at = atomicAdd(p.taken + 1, uint32_t(__popc(left)));
     }
     at = __shfl_sync(kFullMask, at, 0) + __popc(left & ((1u << lane) - 1u));
-    if ((left >> lane) & 1u) {  // (rows stay empty that nobody takes: the chain was given up)
-      if (OUTS) p.s[row] = empty_slot();
-      if (OUTC) p.c[row] = empty_slot();
-      __threadfence();
-    }
-    const bool queued = ((left >> lane) & 1u) && at < p.queue_cap && atomicExch(p.queue + at, row + 1) != kGone;
+    const bool queued = ((left >> lane) & 1u) && at < p.queue_cap &&
+                        atomicExch(p.queue + at, in_queue(p, row + 1)) != in_queue(p, kGone);
     left &= ~__ballot_sync(kFullMask, queued);
   }
   for (; left; left &= left - 1) {
-    if (__shfl_sync(kFullMask, given_up(p), 0)) break;
     const uint32_t r = __shfl_sync(kFullMask, row, __ffs(left) - 1);
     const RowCount n = warp_row<OUTS, OUTC>(p, S, r);
     if (lane == 0 && n.ranges) tally(r, n.ranges, n.columns);
   }
   __syncwarp();
-  return look;
+  return put_in || places.x < min(places.y, p.queue_cap);
 }
 
 // The kernels of a chain follow one another closely: each waits for the kernel before
@@ -968,7 +982,7 @@ __global__ void __launch_bounds__(kSThreads, 6) k_chain_rows(const __grid_consta
 }
 
 template <bool OUTS, bool OUTC, bool COUNT>
-__global__ void __launch_bounds__(kWThreads) k_chain_walk(const __grid_constant__ ChainArgs p) {
+__global__ void __launch_bounds__(kWThreads, kWBlocks) k_chain_walk(const __grid_constant__ ChainArgs p) {
   follow();
   __shared__ WarpSmem smem[kWWarps];
   const int lane = lane_id(), warp = threadIdx.x >> 5;
@@ -984,7 +998,7 @@ __global__ void __launch_bounds__(kWThreads) k_chain_walk(const __grid_constant_
   };
   bool look = false;
   uint32_t x = 0, at = 0;  // a lane's word: its rows still to walk, and the first of its 32
-  bool dropped = __shfl_sync(kFullMask, given_up(p), 0);
+  bool dropped = given_up(p);
   while (true) {
     const unsigned spent = __ballot_sync(kFullMask, x == 0);
     uint32_t have = __reduce_add_sync(kFullMask, uint32_t(__popc(x)));
@@ -1004,7 +1018,7 @@ __global__ void __launch_bounds__(kWThreads) k_chain_walk(const __grid_constant_
     __syncwarp();
     const bool later = given_up(p);  // (for the next batch: it comes while this one is walked)
     if (walk_batch<OUTS, OUTC>(p, S, min(have, 32u), dropped, tally)) look = true;
-    dropped = __shfl_sync(kFullMask, later, 0);
+    dropped = later;
   }
   if (look) take_rows<OUTS, OUTC>(p, S, tally);
 }
@@ -1012,7 +1026,7 @@ __global__ void __launch_bounds__(kWThreads) k_chain_walk(const __grid_constant_
 // A pass over a small matrix, where a launch costs more than the rows: both in
 // one kernel, a block kCountRows rows, a warp 32 of them.
 template <bool OUTS, bool OUTC, bool COUNT>
-__global__ void __launch_bounds__(kWThreads) k_chain_small(const __grid_constant__ ChainArgs p) {
+__global__ void __launch_bounds__(kWThreads, kWBlocks) k_chain_small(const __grid_constant__ ChainArgs p) {
   follow();
   static_assert(kWThreads == kCountRows, "a block's rows are counted together");
   __shared__ WarpSmem smem[kWWarps];
@@ -1036,7 +1050,7 @@ __global__ void __launch_bounds__(kWThreads) k_chain_small(const __grid_constant
     if (bad) S.todo[__popc(who & ((1u << lane) - 1u))] = uint32_t(r0) + lane;
     __syncwarp();
     if (who)
-      look = walk_batch<OUTS, OUTC>(p, S, __popc(who), __shfl_sync(kFullMask, dropped, 0), [&](uint32_t, uint32_t c, unsigned long long z) {
+      look = walk_batch<OUTS, OUTC>(p, S, __popc(who), dropped, [&](uint32_t, uint32_t c, unsigned long long z) {
         cnt += c;
         nnz += z;
       });
@@ -1074,13 +1088,6 @@ struct Parts {
 };
 __device__ __forceinline__ SlotPart my_part(const Parts& q) { return q.table ? q.table[q.part_of[blockIdx.x]] : q.one; }
 
-// The chain's first kernel: counters, places, queues and counts of its scratch start at zero.
-__global__ void __launch_bounds__(kSThreads) k_clear(uint4* words, uint32_t n) {
-  follow();
-  for (uint32_t w = blockIdx.x * kSThreads + threadIdx.x; w < n; w += gridDim.x * kSThreads)
-    words[w] = make_uint4(0u, 0u, 0u, 0u);
-}
-
 // Range CRS -> slots.  Canonical input: a row of several ranges is copied to
 // the arena as it is.  Rows past a part's last are rows of the identity: one
 // column each, whatever the pass.
@@ -1091,6 +1098,12 @@ __global__ void __launch_bounds__(kSThreads) k_crs_to_slots(const __grid_constan
   const SlotPart part = my_part(q);
   const int lane = lane_id();
   const uint64_t b0 = uint64_t(blockIdx.x) * kCrsRows + threadIdx.x;
+  // (blocks of a small last pass add to the counts)
+  const uint64_t g = uint64_t(blockIdx.x) * (kCrsRows / kCountRows) + threadIdx.x;
+  if (threadIdx.x < kCrsRows / kCountRows && g * kCountRows < p.n) {
+    p.group_cnt[g] = 0;
+    p.group_nnz[g] = 0;
+  }
   uint64_t a0[kIter], cnt[kIter];
 #pragma unroll
   for (int u = 0; u < kIter; ++u) {
@@ -1314,7 +1327,7 @@ void launch_pass(dvg_context* ctx, bool close, const ChainArgs& p) {
   launch_next(ctx, close, k_chain_rows<OUTS, OUTC, COUNT>,
               (uint64_t(p.n) + kSThreads * kSRows - 1) / (kSThreads * kSRows), kSThreads, p);
   const uint64_t want = (uint64_t(p.n) + 32 * kWWarps - 1) / (32 * kWWarps);
-  launch_next(ctx, close, k_chain_walk<OUTS, OUTC, COUNT>, std::min<uint64_t>(want, 7ull * ctx->num_sms), kWThreads, p);
+  launch_next(ctx, close, k_chain_walk<OUTS, OUTC, COUNT>, std::min<uint64_t>(want, uint64_t(kWBlocks) * ctx->num_sms), kWThreads, p);
 }
 
 }  // namespace
@@ -1553,24 +1566,36 @@ uint64_t predict_slots_bytes(uint32_t nrows, uint64_t nentries, unsigned dlo, un
   }
   const uint64_t n = (uint64_t(nrows) + kSlotPartRows - 1) / kSlotPartRows * kSlotPartRows;
   const uint64_t ranges = std::min<uint64_t>(uint64_t(kSlotGrowthMax * double(n)) + 4096, kMulti);
-  const uint64_t input = 8 * n + 4 * nentries, result = 8 * n + 16 * n, scratch = n + steps * (kQueueMax * 4 + 8);
+  const uint64_t input = 8 * n + 4 * nentries, result = 8 * n + 16 * n, scratch = n + steps * 8 + kQueueBytes;
   // (blocks are up to a quarter larger than what they hold)
   return (input + 8 * n * buffers + 8 * ranges + result + scratch) / 4 * 5;
 }
 
-SlotBuild prepare_slots(dvg_context* ctx, const SlotPlan& plan, uint32_t n) {
+// The context's queue, for chains that run one after another.
+static unsigned long long* slot_queue(dvg_context* ctx, uint32_t passes, uint32_t& epoch) {
+  if (ctx->slot_epoch > 0xffffffffu - passes) ctx->slot_epoch = 0;  // (and cleared once more)
+  if (!ctx->d_slot_queue) ctx->d_slot_queue = static_cast<unsigned long long*>(dalloc(ctx, kQueueBytes));
+  if (ctx->slot_epoch == 0) DVG_CUDA(cudaMemsetAsync(ctx->d_slot_queue, 0, kQueueBytes, ctx->stream));
+  epoch = ctx->slot_epoch + 1;
+  ctx->slot_epoch += passes;
+  return ctx->d_slot_queue;
+}
+
+SlotBuild prepare_slots(dvg_context* ctx, const SlotPlan& plan, uint32_t n, bool own_queue) {
   SlotBuild sb;
   sb.plan = plan;
   sb.n = n;
   sb.mat.assign(plan.nmats, nullptr);
   const uint64_t groups = (uint64_t(n) + kCountRows - 1) / kCountRows;
   const uint64_t supers = (groups + kSuperGroups - 1) / kSuperGroups;
-  // a pass's rows to be walked by warps: room for its clumps (a row past it is walked at once)
-  sb.queue_cap = uint32_t(std::clamp<uint64_t>(n / 8, 256, kQueueMax));
   auto round = [](size_t x) { return (x + 15) & ~size_t(15); };
-  const size_t taken_off = 512, queue_off = taken_off + plan.steps.size() * 8;
-  const size_t nnz_off = round(queue_off + plan.steps.size() * sb.queue_cap * 4), cnt_off = nnz_off + groups * 8;
-  const size_t sums_off = round(cnt_off + groups * 4), masks_off = sums_off + supers * 8;
+  // counters and the passes' places, cleared together
+  const size_t taken_off = sizeof(SlotCounters);
+  sb.cleared = std::max<size_t>(512, round(taken_off + plan.steps.size() * 8));
+  const size_t nnz_off = sb.cleared, cnt_off = nnz_off + groups * 8, sums_off = round(cnt_off + groups * 4);
+  const size_t queue_off = sums_off + supers * 8, masks_off = queue_off + (own_queue ? kQueueBytes : 0);
+  sb.own_queue = own_queue;
+  sb.queue_cap = kQueueRows;
   static_assert(sizeof(SlotCounters) <= 512, "the counters come first");
   // (below kMulti, so that the slot of a row of several runs has y < x)
   sb.arena_cap = std::min<uint64_t>(uint64_t(ctx->slot_growth * double(n)) + 4096, kMulti);
@@ -1582,14 +1607,14 @@ SlotBuild prepare_slots(dvg_context* ctx, const SlotPlan& plan, uint32_t n) {
   try {
     sb.scratch = dalloc(ctx, masks_off + (uint64_t(n) + 31) / 32 * 4);
     char* base = static_cast<char*>(sb.scratch);
-    // (a large pass writes its counts, a small one's blocks add to them)
-    sb.cleared = n <= kSmallRows ? nnz_off + round(groups * 12) : nnz_off;
     sb.ctl = reinterpret_cast<DeviceControl*>(base);
     sb.top = reinterpret_cast<unsigned long long*>(base + 256);
     sb.abort = sb.top + 1;
     sb.wide = sb.top + 2;
     sb.taken = reinterpret_cast<uint32_t*>(base + taken_off);
-    sb.queue = reinterpret_cast<uint32_t*>(base + queue_off);
+    sb.epoch = 1;
+    sb.queue = own_queue ? reinterpret_cast<unsigned long long*>(base + queue_off)
+                         : slot_queue(ctx, uint32_t(plan.steps.size()), sb.epoch);
     sb.sums = reinterpret_cast<unsigned long long*>(base + sums_off);
     sb.group_nnz = reinterpret_cast<unsigned long long*>(base + nnz_off);
     sb.group_cnt = reinterpret_cast<uint32_t*>(base + cnt_off);
@@ -1616,11 +1641,10 @@ void release_slots(dvg_context* ctx, SlotBuild& sb) {
 
 void launch_slots(dvg_context* ctx, SlotBuild& sb, const SlotParts& parts, bool timed, const SlotPart* right) {
   const uint64_t t0 = now_ns();
-  // (a memset of more than a few KB is 4 us before the next kernel starts)
-  k_clear<<<unsigned(std::min<size_t>(sb.cleared / 4096 + 1, ctx->num_sms)), kSThreads, 0, ctx->stream>>>(
-      static_cast<uint4*>(sb.scratch), uint32_t(sb.cleared / 16));
-  DVG_CUDA(cudaGetLastError());
+  // (512 bytes with up to 28 passes; one of more than a few KB takes 4 us longer)
+  DVG_CUDA(cudaMemsetAsync(sb.scratch, 0, sb.cleared, ctx->stream));
   ctx->stats.kernel_launches++;
+  if (sb.own_queue) DVG_CUDA(cudaMemsetAsync(sb.queue, 0, kQueueBytes, ctx->stream));
   ChainArgs p{};
   p.arena = sb.arena;
   p.top = sb.top;
@@ -1630,13 +1654,15 @@ void launch_slots(dvg_context* ctx, SlotBuild& sb, const SlotParts& parts, bool 
   p.wide = sb.wide;
   p.wide_max = kWideCost + sb.n / 16;
   p.masks = sb.masks;
+  p.queue = sb.queue;
   p.queue_cap = sb.queue_cap;
   p.group_cnt = sb.group_cnt;
   p.group_nnz = sb.group_nnz;
   p.n = sb.n;
   p.s = sb.mat[0];
-  launch_next(ctx, sb.close, k_crs_to_slots, conversion_blocks(sb), kSThreads,
-              Parts{parts.table, parts.part_of, parts.one}, p);
+  k_crs_to_slots<<<conversion_blocks(sb), kSThreads, 0, ctx->stream>>>(Parts{parts.table, parts.part_of, parts.one}, p);
+  DVG_CUDA(cudaGetLastError());
+  ctx->stats.kernel_launches++;
   if (right) {
     p.s = sb.mat[1];
     launch_next(ctx, sb.close, k_crs_to_slots, conversion_blocks(sb), kSThreads, Parts{nullptr, nullptr, *right}, p);
@@ -1644,7 +1670,7 @@ void launch_slots(dvg_context* ctx, SlotBuild& sb, const SlotParts& parts, bool 
   for (size_t i = 0; i < sb.plan.steps.size(); ++i) {
     const SlotStep& st = sb.plan.steps[i];
     p.taken = sb.taken + 2 * i;
-    p.queue = sb.queue + i * sb.queue_cap;
+    p.epoch = sb.epoch + uint32_t(i);
     p.k = uint32_t(st.k);
     p.bits = st.bits;
     for (int j = 0; j < kChainMax; ++j) p.m[j] = j < st.k ? sb.mat[st.m[j]] : nullptr;
@@ -1725,7 +1751,7 @@ static dvg_matrix* run_slots(dvg_context* ctx, const SlotPlan& plan, const dvg_m
                              const SlotKey& key, bool build, bool* settled) {
   SlotBuild sb;
   try {
-    sb = prepare_slots(ctx, plan, a->nrows);
+    sb = prepare_slots(ctx, plan, a->nrows, false);
     sb.key = key;
   } catch (const Error& e) {
     if (e.status != DVG_ERR_OOM) throw;

@@ -70,12 +70,14 @@ struct SlotBuild {
   uint64_t arena_cap = 0;      // ranges
   bool close = false;          // the kernels' blocks are placed while the kernel before ends
   uint64_t early = 0;          // room for the result's ranges before their number is known; 0: none
-  // counters | places of each pass | queues | counts of the result | sums of the counts | bitmap
+  // counters | places of each pass | counts of the result | sums of the counts | queue | bitmap
   void* scratch = nullptr;
-  size_t cleared = 0;          // its first bytes, which the chain's first kernel clears
+  size_t cleared = 0;          // its first bytes, which a chain starts by clearing
+  bool own_queue = false;      // the queue is there, cleared for every chain, and not the context's
   uint32_t queue_cap = 0;
   uint32_t* taken = nullptr;
-  uint32_t* queue = nullptr;
+  unsigned long long* queue = nullptr;
+  uint32_t epoch = 0;          // its first pass's
   DeviceControl* ctl = nullptr;
   unsigned long long* top = nullptr;
   unsigned long long* abort = nullptr;
@@ -89,7 +91,8 @@ struct SlotBuild {
 // Allocates what the chain needs (no device work beyond stream-ordered
 // allocation); issues it (no host round trip: it may be captured).
 // A plan of two inputs takes `right` as its second.
-SlotBuild prepare_slots(dvg_context* ctx, const SlotPlan& plan, uint32_t n);
+// Chains that run side by side have queues of their own.
+SlotBuild prepare_slots(dvg_context* ctx, const SlotPlan& plan, uint32_t n, bool own_queue);
 // Device memory that an index build as a chain may take, its input and result included.
 uint64_t predict_slots_bytes(uint32_t nrows, uint64_t nentries, unsigned dlo, unsigned dup);
 void launch_slots(dvg_context* ctx, SlotBuild& sb, const SlotParts& parts, bool timed, const SlotPart* right = nullptr);
