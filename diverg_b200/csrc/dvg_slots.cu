@@ -23,7 +23,7 @@
 // matrix that the reference's sequence of range_spgemm / range_spadd gives.
 //
 // Measured on a B200 against the same builds product by product in range CRS:
-// 5.0e7 loci, window [400, 600]: 23.05 -> 2.65 ms; 1e6 loci, [0, 250]: 1.26 ->
+// 5.0e7 loci, window [400, 600]: 23.05 -> 2.62 ms; 1e6 loci, [0, 250]: 1.26 ->
 // 0.21 ms; 1e5 loci of a variant-dense graph, [100, 300]: 1.01 -> 0.145 ms.
 #include <algorithm>
 #include <cmath>
@@ -69,7 +69,10 @@ constexpr double kEarlySlack = 1.125;
 constexpr uint64_t kEarlySpare = 1u << 16;
 constexpr uint32_t kQueueRows = 1u << 15;  // places of a queue (rows past them are walked at once)
 constexpr size_t kQueueBytes = kQueueRows * sizeof(unsigned long long);
-constexpr double kSlotGrowthMax = 8.0;  // ranges a row that an arena is made for
+// Ranges a row that an arena is made for at most (4 at first: the builds of 1e6 bases of a
+// variant-dense graph take up to 0.3, up to [1000, 1300] 1.1, A^300 1.1 and A^1000 4.3;
+// those of a chromosome 0.05).
+constexpr double kSlotGrowthMax = 8.0;
 // Up to so many rows, and for single products as long as their results are written
 // early, the chain's kernels are launched close behind one another: the next one's
 // blocks are placed while the kernel before ends, 2 us a kernel.  Builds of
@@ -944,11 +947,13 @@ __device__ __forceinline__ void follow() {
 // queue (take_rows).
 //
 // Bound: HBM, 8 bytes a row for each matrix read and written (all but the first
-// read of a matrix come from L2).  k_chain_rows on 1e7 rows: 51 to 72 us for
-// 190 to 300 MB, 3.8 to 5.2 TB/s, issue slots 45 to 60 % busy; six blocks an SM
-// (42 registers) against four: 2.75 and 2.90 ms a 5e7-locus build.  k_chain_walk: 27
-// to 56 us, the latency of a walk, whatever few rows there are.  Walking the
-// rows in the streaming kernel instead, behind a block's barrier or a warp at a
+// read of a matrix come from L2), and instructions.  k_chain_rows on 1e7 rows: 53 to 66
+// us for 180 to 300 MB, 2.8 to 5.5 TB/s with issue slots 43 to 75 % busy -- the first
+// pass, whose sum is of the identity's rows, and the counting one are the busy ones;
+// six blocks an SM (40 registers) against four: 2.75 and 2.90 ms a 5e7-locus build.
+// k_chain_walk: 25 to 45 us, the latency of a walk, whatever few rows there are; 24 to
+// 33 % of an SM's warps are active where 44 % fit, so most have ended by then.  Walking
+// the rows in the streaming kernel instead, behind a block's barrier or a warp at a
 // time, held the loads of its other rows back (8.9 and 4.1 ms a build).
 template <bool OUTS, bool OUTC, bool COUNT>
 __global__ void __launch_bounds__(kSThreads, 6) k_chain_rows(const __grid_constant__ ChainArgs p) {
@@ -1222,8 +1227,9 @@ __global__ void __launch_bounds__(kSThreads) k_part_totals(const Parts q, const 
 // before it in that one, less those before its part, so no block waits for
 // another.  A warp takes 32 consecutive rows at a time.
 //
-// Bound: HBM, 8 bytes a row read and 8 a row and 8 a range written.  Issue slots
-// were 71 % busy at 1e7 rows, 78 us: rows nearly all have at most two ranges, so
+// Bound: HBM, 8 bytes a row read and 8 a row and 8 a range written, and instructions
+// (78 % of the issue slots).  They were 71 % busy at 1e7 rows, 78 us: rows nearly all
+// have at most two ranges, so
 // two ballots give their places in place of a scan, and runs and pairs are written
 // without a loop: 53 us, and 186 in place of 189 us for a product of 1e7 rows
 // with the slots requested first and seven blocks an SM (a build of 5e7 rows: 2.78
@@ -1481,7 +1487,10 @@ SlotPlan plan_slots(unsigned dlo, unsigned dup, double branching) {
 // columns on average, the powers' rows soon leave the slots for the arena, or
 // name so many rows that a thread walks them for long: such input, input whose
 // rows are not canonical, and matrices whose columns reach the marker of a
-// several-run row stay with the range-CRS row kernel.  So does large input of more
+// several-run row stay with the range-CRS row kernel.  (No sharp line: products and
+// powers of 1e5 rows take 0.25 to 0.95 of its time at 1.48 ranges a row; at 1.6 to 2 0.25
+// to 1.05 where the arena holds, and longer chains run full; at 3, and with three
+// columns a range, most of them do.)  So does large input of more
 // than a quarter of a column a row beyond its first, which no sequence graph has.  At 1e6
 // rows A^2 of a path with skips took 88 us against 110 in range CRS at 0.2 columns, 104
 // against 109 at 0.29 and 160 against 116 at 0.48, of random bands 195 against 146 at 0.3

@@ -138,8 +138,11 @@ __device__ void wide_lookback(unsigned long long* out, const FusedArgs& p, uint3
 // ranges than kBandRanges or is wider than the window and has to be walked range
 // by range.
 //
-// Bound: instructions, about 460 a row where an A range takes two steps instead
-// of the 1,300 of ORing each of its ~100 B ranges with two shared atomics.  On the
+// Bound: latency, and instructions: a row's chain of dependent steps (row pointers,
+// ranges, block boxes, table rows, the ORs), with 32 warps an SM to hide it (64 registers
+// a thread) and issue slots 56 % busy.  An A range takes two steps, a row about 460
+// instructions instead of the 1,300 of ORing each of its ~100 B ranges with two shared
+// atomics.  On the
 // banded product of 4.2e6 rows (half-width 512, four ranges of ~32 columns a row)
 // 6.54 -> 4.00 ms, 1.0 of it the tables; 3.2e6 rows whose products hold 16 entries
 // a row, 37.1 -> 3.7 ms.  A warp a row, its window in registers,

@@ -101,9 +101,10 @@ dvg_status dvg_synchronize(dvg_context* ctx);
  * pre-allocated buffers and no host round trip between them, the default; 0 =
  * one read-back per product), "row_slots" (1 = planned builds, powers, and
  * products of 24,576 rows or more, of graph-like input -- canonical rows, at most
- * 1.5 ranges a row and two columns a range on average -- run as passes over
- * matrices of one 8-byte slot a row, the default;
- * 0 = every product in range CRS), "plan_growth" (planned builds: the entry
+ * 1.5 ranges a row and two columns a range on average, and past 2^18 rows at
+ * most 1.25 columns a row that has any -- run as passes over matrices of one
+ * 8-byte slot a row, the default; chains that did not fit are not tried again
+ * at once; 0 = every product in range CRS), "plan_growth" (planned builds: the entry
  * capacity of every step as a percentage of the input's entries, 300 by
  * default and adapted after each build; a step that outgrows it makes the
  * build re-run on the read-back path), "row_slot" (thread-per-row kernel: run-list
@@ -142,7 +143,8 @@ dvg_status dvg_matrix_upload(dvg_context* ctx, uint32_t nrows, uint32_t ncols, c
 dvg_status dvg_matrix_upload_u32(dvg_context* ctx, uint32_t nrows, uint32_t ncols, const uint32_t* rowmap,
                                  const uint32_t* entries, uint64_t nnz, dvg_matrix** out);
 /* Wraps caller-owned device arrays without copying; the arrays must outlive
- * the handle and are not freed by dvg_matrix_free. */
+ * the handle and are not freed by dvg_matrix_free.  nnz, here and above, is what
+ * dvg_matrix_info reports; which kernels run goes by columns counted on the device. */
 dvg_status dvg_matrix_wrap_device(dvg_context* ctx, uint32_t nrows, uint32_t ncols, const uint64_t* d_rowmap,
                                   const uint32_t* d_entries, uint64_t nentries, uint64_t nnz, dvg_matrix** out);
 /* numRows / numCols / rowMap(numRows) / nnz (crs_matrix.hpp:1274-1369, 1980). */
