@@ -150,6 +150,7 @@ struct ChainArgs {
   uint32_t queue_cap;
   uint32_t* group_cnt;        // last pass: ranges and columns of c per kCountRows rows
   unsigned long long* group_nnz;
+  bool add_counts;            // the last pass's blocks add to them (from zero)
   uint32_t n;
 };
 
@@ -796,7 +797,7 @@ __device__ __noinline__ RowCount warp_row(const ChainArgs& p, WarpSmem& S, uint3
 // 1e6 bases of a variant-dense graph, 4,172 such rows: 9.9 ms by unions of windows in
 // the row's own warp, 1.2 by bitmaps through the queue; A^100, 52 such rows: 1.72 ms and
 // 0.24; the build for [1000, 1300], 1,910: 4.3 and 0.86.  Where no row needs it, the queue
-// and the longer code cost 2 to 3 % of a small build (1e5 bases 150 -> 155 us).  Nobody
+// and the longer code cost 2 to 3 % of a small build (1e5 bases 146 -> 148.5 us).  Nobody
 // waits: a place is settled by one atomic each of the warp that puts a row in and of the
 // one that takes it, and where the taker comes first (kGone) the row stays with the warp
 // that had it.  What earlier passes left there has another epoch and counts as empty, so
@@ -831,11 +832,11 @@ __device__ void take_rows(const ChainArgs& p, WarpSmem& S, Tally&& tally) {
 // than a lane's lists hold go to the queue (take_rows), or to the whole warp at once
 // where that is full.  Returns whether rows wait there.  (`dropped`: the chain is given up.)
 // tally(row, ranges, columns) for each row of c that has any.
-template <bool OUTS, bool OUTC, class Tally>
+template <bool OUTS, bool OUTC, bool QUEUE, class Tally>
 __device__ __forceinline__ bool walk_batch(const ChainArgs& p, WarpSmem& S, uint32_t batch, bool dropped,
                                            Tally&& tally) {
   const int lane = lane_id();
-  if (__any_sync(kFullMask, dropped)) {
+  if (QUEUE && __any_sync(kFullMask, dropped)) {
     if (uint32_t(lane) < batch) leave_empty<OUTS, OUTC>(p, S.todo[lane]);
     __syncwarp();
     return false;
@@ -866,7 +867,7 @@ __device__ __forceinline__ bool walk_batch(const ChainArgs& p, WarpSmem& S, uint
   __syncwarp();
   unsigned left = __ballot_sync(kFullMask, uint32_t(lane) < batch && !done);
   // (the look comes while the rows are written)
-  const uint2 places = slow ? __ldcg(reinterpret_cast<const uint2*>(p.taken)) : make_uint2(0u, 0u);
+  const uint2 places = QUEUE && slow ? __ldcg(reinterpret_cast<const uint2*>(p.taken)) : make_uint2(0u, 0u);
   const bool put_in = left != 0;
   // places in the arena for the rows of several runs, one request a warp
   // (a row of two columns needs none)
@@ -906,12 +907,10 @@ __device__ __forceinline__ bool walk_batch(const ChainArgs& p, WarpSmem& S, uint
     }
   }
   __syncwarp();
-  if (left) {
+  if (left && lane == 0) atomicAdd(&p.ctl->slow_rows, (unsigned long long)__popc(left));
+  if (QUEUE && left) {
     uint32_t at = 0;
-    if (lane == 0) {
-      atomicAdd(&p.ctl->slow_rows, (unsigned long long)__popc(left));
-      at = atomicAdd(p.taken + 1, uint32_t(__popc(left)));
-    }
+    if (lane == 0) at = atomicAdd(p.taken + 1, uint32_t(__popc(left)));
     at = __shfl_sync(kFullMask, at, 0) + __popc(left & ((1u << lane) - 1u));
     const bool queued = ((left >> lane) & 1u) && at < p.queue_cap &&
                         atomicExch(p.queue + at, in_queue(p, row + 1)) != in_queue(p, kGone);
@@ -1022,15 +1021,17 @@ __global__ void __launch_bounds__(kWThreads, kWBlocks) k_chain_walk(const __grid
     for (; x && k < 32; x &= x - 1) S.todo[k++] = at + uint32_t(__ffs(x) - 1);
     __syncwarp();
     const bool later = given_up(p);  // (for the next batch: it comes while this one is walked)
-    if (walk_batch<OUTS, OUTC>(p, S, min(have, 32u), dropped, tally)) look = true;
+    if (walk_batch<OUTS, OUTC, true>(p, S, min(have, 32u), dropped, tally)) look = true;
     dropped = later;
   }
   if (look) take_rows<OUTS, OUTC>(p, S, tally);
 }
 
 // A pass over a small matrix, where a launch costs more than the rows: both in
-// one kernel, a block kCountRows rows, a warp 32 of them.
-template <bool OUTS, bool OUTC, bool COUNT>
+// one kernel, a block kCountRows rows, a warp 32 of them.  A product alone does
+// without the queue: a row of it is one factor, and looking and being looked at cost
+// 3 of its 43 us at 1e5 rows.
+template <bool OUTS, bool OUTC, bool COUNT, bool QUEUE>
 __global__ void __launch_bounds__(kWThreads, kWBlocks) k_chain_small(const __grid_constant__ ChainArgs p) {
   follow();
   static_assert(kWThreads == kCountRows, "a block's rows are counted together");
@@ -1046,7 +1047,7 @@ __global__ void __launch_bounds__(kWThreads, kWBlocks) k_chain_small(const __gri
   unsigned long long nnz = 0;
   uint32_t cnt = 0;
   bool look = false;
-  const bool dropped = given_up(p);
+  const bool dropped = QUEUE && given_up(p);
   if (r0 < p.n) {
     uint32_t bad;
     if (r0 + 32 <= p.n) bad = chain_rows<OUTS, OUTC, COUNT, 1>(p, uint32_t(r0), cnt, nnz);
@@ -1055,13 +1056,13 @@ __global__ void __launch_bounds__(kWThreads, kWBlocks) k_chain_small(const __gri
     if (bad) S.todo[__popc(who & ((1u << lane) - 1u))] = uint32_t(r0) + lane;
     __syncwarp();
     if (who)
-      look = walk_batch<OUTS, OUTC>(p, S, __popc(who), dropped, [&](uint32_t, uint32_t c, unsigned long long z) {
+      look = walk_batch<OUTS, OUTC, QUEUE>(p, S, __popc(who), dropped, [&](uint32_t, uint32_t c, unsigned long long z) {
         cnt += c;
         nnz += z;
       });
   }
   // (any block's rows: the counts start at zero, and every block adds to them)
-  if (look)
+  if (QUEUE && look)
     take_rows<OUTS, OUTC>(p, S, [&](uint32_t row, uint32_t c, unsigned long long z) {
       if (!COUNT) return;
       atomicAdd(p.group_cnt + row / kCountRows, c);
@@ -1075,9 +1076,12 @@ __global__ void __launch_bounds__(kWThreads, kWBlocks) k_chain_small(const __gri
       atomicAdd(&sum[1], nnz);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && QUEUE) {
       atomicAdd(p.group_cnt + blockIdx.x, uint32_t(sum[0]));
       atomicAdd(p.group_nnz + blockIdx.x, sum[1]);
+    } else if (threadIdx.x == 0) {
+      p.group_cnt[blockIdx.x] = uint32_t(sum[0]);
+      p.group_nnz[blockIdx.x] = sum[1];
     }
   }
 }
@@ -1103,11 +1107,12 @@ __global__ void __launch_bounds__(kSThreads) k_crs_to_slots(const __grid_constan
   const SlotPart part = my_part(q);
   const int lane = lane_id();
   const uint64_t b0 = uint64_t(blockIdx.x) * kCrsRows + threadIdx.x;
-  // (blocks of a small last pass add to the counts)
-  const uint64_t g = uint64_t(blockIdx.x) * (kCrsRows / kCountRows) + threadIdx.x;
-  if (threadIdx.x < kCrsRows / kCountRows && g * kCountRows < p.n) {
-    p.group_cnt[g] = 0;
-    p.group_nnz[g] = 0;
+  if (p.add_counts && threadIdx.x < kCrsRows / kCountRows) {
+    const uint64_t g = uint64_t(blockIdx.x) * (kCrsRows / kCountRows) + threadIdx.x;
+    if (g * kCountRows < p.n) {
+      p.group_cnt[g] = 0;
+      p.group_nnz[g] = 0;
+    }
   }
   uint64_t a0[kIter], cnt[kIter];
 #pragma unroll
@@ -1323,11 +1328,13 @@ void launch_next(dvg_context* ctx, bool close, void (*kernel)(P...), uint64_t bl
 }
 
 template <bool OUTS, bool OUTC, bool COUNT>
-void launch_pass(dvg_context* ctx, bool close, const ChainArgs& p) {
+void launch_pass(dvg_context* ctx, bool close, const ChainArgs& p, bool alone) {
   // one kernel while a warp a 32 rows fits the chip at once; the second
   // kernel's launch costs more than it saves there
   if (p.n <= kSmallRows) {
-    launch_next(ctx, close, k_chain_small<OUTS, OUTC, COUNT>, (uint64_t(p.n) + kWThreads - 1) / kWThreads, kWThreads, p);
+    const uint64_t blocks = (uint64_t(p.n) + kWThreads - 1) / kWThreads;
+    if (!OUTS && COUNT && alone) launch_next(ctx, close, k_chain_small<false, true, true, false>, blocks, kWThreads, p);
+    else launch_next(ctx, close, k_chain_small<OUTS, OUTC, COUNT, true>, blocks, kWThreads, p);
     return;
   }
   launch_next(ctx, close, k_chain_rows<OUTS, OUTC, COUNT>,
@@ -1663,6 +1670,8 @@ void launch_slots(dvg_context* ctx, SlotBuild& sb, const SlotParts& parts, bool 
   p.wide = sb.wide;
   p.wide_max = kWideCost + sb.n / 16;
   p.masks = sb.masks;
+  const bool alone = sb.plan.steps.size() == 1 && sb.plan.steps[0].k <= 1;  // a product
+  p.add_counts = sb.n <= kSmallRows && !alone;
   p.queue = sb.queue;
   p.queue_cap = sb.queue_cap;
   p.group_cnt = sb.group_cnt;
@@ -1687,10 +1696,10 @@ void launch_slots(dvg_context* ctx, SlotBuild& sb, const SlotParts& parts, bool 
     p.s = st.s >= 0 ? sb.mat[st.s] : nullptr;
     p.c = st.c >= 0 ? sb.mat[st.c] : nullptr;
     cudaEvent_t ev = timed ? span_begin(ctx) : nullptr;
-    if (i + 1 == sb.plan.steps.size()) launch_pass<false, true, true>(ctx, sb.close, p);
-    else if (p.s && p.c) launch_pass<true, true, false>(ctx, sb.close, p);
-    else if (p.s) launch_pass<true, false, false>(ctx, sb.close, p);
-    else launch_pass<false, true, false>(ctx, sb.close, p);
+    if (i + 1 == sb.plan.steps.size()) launch_pass<false, true, true>(ctx, sb.close, p, alone);
+    else if (p.s && p.c) launch_pass<true, true, false>(ctx, sb.close, p, false);
+    else if (p.s) launch_pass<true, false, false>(ctx, sb.close, p, false);
+    else launch_pass<false, true, false>(ctx, sb.close, p, false);
     span_end(ctx, ev, kProduct);
   }
   const uint64_t groups = (uint64_t(sb.n) + kCountRows - 1) / kCountRows;
