@@ -150,7 +150,7 @@ struct SlotGroup {
   std::vector<uint32_t> members;
   std::vector<SlotPart> parts;     // one a member
   std::vector<uint32_t> part_of;   // one a kSlotPartRows rows
-  uint64_t n = 0, columns = 0;
+  uint64_t n = 0, nnz = 0;
   SlotBuild sb;
   SlotParts table{};               // on the device
   unsigned long long* totals = nullptr;
@@ -215,7 +215,7 @@ void lay_out(SlotGroup& g, const dvg_matrix* const* graphs) {
     g.part_of.insert(g.part_of.end(), blocks, uint32_t(g.parts.size()));
     g.parts.push_back(part);
     g.n += uint64_t(blocks) * kSlotPartRows;
-    g.columns += padded_columns(graphs[k]) + (uint64_t(blocks) * kSlotPartRows - part.n);
+    g.nnz += graphs[k]->nnz + (uint64_t(blocks) * kSlotPartRows - part.n);
   }
 }
 
@@ -317,7 +317,7 @@ void batch_distance_index(dvg_context* ctx, uint32_t ngraphs, const dvg_matrix* 
   }
   for (auto& g : chains) lay_out(g, graphs);
   for (auto it = chains.begin(); it != chains.end();) {
-    it->sb.key = slot_key(it->dlo, it->dup, it->columns, it->n);
+    it->sb.key = slot_key(it->dlo, it->dup, it->nnz, it->n);
     if (is_due(it->sb.key)) {
       ++it;
       continue;
@@ -380,7 +380,7 @@ void batch_distance_index(dvg_context* ctx, uint32_t ngraphs, const dvg_matrix* 
     for (auto it = chains.begin(); it != chains.end();) {
       try {
         const SlotKey key = it->sb.key;
-        it->sb = prepare_slots(ctx, plan_slots(it->dlo, it->dup, branching(it->columns, it->n)), uint32_t(it->n), true);
+        it->sb = prepare_slots(ctx, plan_slots(it->dlo, it->dup, branching(it->nnz, it->n)), uint32_t(it->n), true);
         it->sb.key = key;
         it->ready = true;
         ++it;

@@ -43,8 +43,8 @@ constexpr int kWBlocks = 7;     // of them an SM holds at once (72 registers a t
 constexpr int kSRows = 4;       // rows a lane of k_chain_rows takes
 constexpr int kSRuns = 8;       // runs of a lane's list
 constexpr int kSWin = 256;      // window words of a warp (8,192 columns)
-// A lane's list walk names at most so many columns a factor; the 32 lanes of a warp
-// share the columns of a row of more.
+// A run of a lane's list has at most so many columns; the 32 lanes of a warp share the
+// columns of a row with a longer one.
 constexpr uint32_t kLaneColumns = 256;
 constexpr uint32_t kMulti = kSlotMulti;
 constexpr uint32_t kMultiMax = 0xFFFFFFFFu - kMulti - 1;  // ranges of one row
@@ -319,15 +319,14 @@ __device__ __noinline__ uint32_t list_merge(uint2* L, uint32_t nr, uint2 v) {
 }
 
 // The nd runs at D |= the rows of `mat` that the ns runs at L name (mat null:
-// the runs themselves).  Returns their new number, or kFull: too many runs, or too
-// many columns for one lane.
+// the runs themselves).  Returns their new number, or kFull: too many runs, or one
+// too long for a lane.
 __device__ __noinline__ uint32_t list_product(const uint2* arena, const uint2* L, uint32_t ns, const uint2* mat,
                                               uint2* D, uint32_t nd) {
   uint2 run = empty_slot();
-  uint32_t named = 0;
   for (uint32_t k = 0; k < ns; ++k) {
     const uint2 a = L[k * 32];
-    if (mat && (named += min(a.y - a.x, kLaneColumns) + 1) > kLaneColumns) return kFull;
+    if (a.y - a.x >= kLaneColumns && mat) return kFull;
     for (uint32_t x = a.x; x <= a.y; ++x) {
       const uint2 s = mat ? ld_slot(mat, x) : a;
       const uint32_t c = slot_count(s);
@@ -1510,13 +1509,14 @@ bool slots_suit(const dvg_context* ctx, const dvg_matrix* a) {
   const uint64_t ranges = a->nentries / 2;
   return a->canonical && a->nrows == a->ncols && a->nrows > 0 && a->ncols < kSlotMulti &&
          2 * ranges <= 3ull * a->nrows && a->nnz <= 2 * ranges &&
-         (a->nrows <= kDenseRows || branching(padded_columns(a), a->nrows) <= kDenseBranching) && ctx->opt_slots != 0;
+         (a->nrows <= kDenseRows || branching(a->nnz + a->empty_rows, a->nrows) <= kDenseBranching) &&
+         ctx->opt_slots != 0;
 }
 
 // Chains over such matrices for such a window, as far as whether they fit goes: sizes
 // within a factor of two, densities within a fifth.  (Products: dlo 1, dup 0.)
-SlotKey slot_key(unsigned dlo, unsigned dup, uint64_t columns, uint64_t nrows) {
-  const double b = branching(columns, nrows);
+SlotKey slot_key(unsigned dlo, unsigned dup, uint64_t nnz, uint64_t nrows) {
+  const double b = branching(nnz, nrows);
   return {dlo, dup, int(64 - __builtin_clzll(nrows | 1)), b > 0 ? int(std::floor(4 * std::log2(b))) : -1000};
 }
 
@@ -1840,7 +1840,7 @@ static dvg_matrix* run_slots(dvg_context* ctx, const SlotPlan& plan, const dvg_m
 }
 
 dvg_matrix* slots_chain(dvg_context* ctx, const dvg_matrix* a, unsigned dlo, unsigned dup, bool build, bool* settled) {
-  return run_slots(ctx, plan_slots(dlo, dup, branching(padded_columns(a), a->nrows)), a, nullptr, slot_key(dlo, dup, a), build,
+  return run_slots(ctx, plan_slots(dlo, dup, branching(a->nnz, a->nrows)), a, nullptr, slot_key(dlo, dup, a), build,
                    settled);
 }
 

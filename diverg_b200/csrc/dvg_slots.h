@@ -119,18 +119,14 @@ bool slots_product_suits(const dvg_context* ctx, const dvg_matrix* a, const dvg_
 dvg_matrix* slots_product(dvg_context* ctx, const dvg_matrix* a, const dvg_matrix* b, bool* settled);
 
 // Columns of a row beyond its first, on average: how fast rows leave the single column.
-// (`columns`: those of all rows, and one more for each that has none.)
-inline double branching(uint64_t columns, uint64_t nrows) {
-  return columns > nrows ? double(columns - nrows) / double(nrows) : 0.0;
+inline double branching(uint64_t nnz, uint64_t nrows) {
+  return nnz > nrows ? double(nnz - nrows) / double(nrows) : 0.0;
 }
-inline uint64_t padded_columns(const dvg_matrix* a) { return a->nnz + a->empty_rows; }
 
-SlotKey slot_key(unsigned dlo, unsigned dup, uint64_t columns, uint64_t nrows);
-inline SlotKey slot_key(unsigned dlo, unsigned dup, const dvg_matrix* a) {
-  return slot_key(dlo, dup, padded_columns(a), a->nrows);
-}
+SlotKey slot_key(unsigned dlo, unsigned dup, uint64_t nnz, uint64_t nrows);
+inline SlotKey slot_key(unsigned dlo, unsigned dup, const dvg_matrix* a) { return slot_key(dlo, dup, a->nnz, a->nrows); }
 inline SlotKey product_key(const dvg_matrix* a, const dvg_matrix* b) {
-  return slot_key(1, 0, std::max(padded_columns(a), padded_columns(b)), a->nrows);
+  return slot_key(1, 0, std::max(a->nnz, b->nnz), a->nrows);
 }
 // Whether a chain is to be tried: chains like it were not just given up.  Counts the call.
 bool slots_due(dvg_context* ctx, const SlotKey& key);
