@@ -138,8 +138,9 @@ struct ChainArgs {
   uint64_t arena_cap;
   DeviceControl* ctl;
   // Why the chain is given up (kArenaFull, ...), 0: it is not.  The host drops the result;
-  // until then rows that did not fit, and all that are yet to be walked, are left empty, so
-  // that later passes stay in bounds and are over soon.
+  // until then rows that did not fit, and those that a warp would have to walk, are left
+  // empty, so that later passes stay in bounds and are over soon.  (Lanes' walks do not
+  // look: that took up to 4 % of a small chain, A^129 of 2.7e5 bases 163 -> 169 us.)
   unsigned long long* abort;
   unsigned long long* wide;   // what unions by windows have cost, and may
   unsigned long long wide_max;
@@ -796,7 +797,7 @@ __device__ __noinline__ RowCount warp_row(const ChainArgs& p, WarpSmem& S, uint3
 // 1e6 bases of a variant-dense graph, 4,172 such rows: 9.9 ms by unions of windows in
 // the row's own warp, 1.2 by bitmaps through the queue; A^100, 52 such rows: 1.72 ms and
 // 0.24; the build for [1000, 1300], 1,910: 4.3 and 0.86.  Where no row needs it, the queue
-// and the longer code cost 2 to 3 % of a small build (1e5 bases 146 -> 148.5 us).  Nobody
+// and the longer code cost up to 3 % of a small build (2e3 bases 84.0 -> 86.3 us).  Nobody
 // waits: a place is settled by one atomic each of the warp that puts a row in and of the
 // one that takes it, and where the taker comes first (kGone) the row stays with the warp
 // that had it.  What earlier passes left there has another epoch and counts as empty, so
@@ -829,17 +830,11 @@ __device__ void take_rows(const ChainArgs& p, WarpSmem& S, Tally&& tally) {
 
 // Walks the `batch` rows of the warp's list, a row a lane; rows of more runs
 // than a lane's lists hold go to the queue (take_rows), or to the whole warp at once
-// where that is full.  Returns whether rows wait there.  (`dropped`: the chain is given up.)
+// where that is full.  Returns whether rows wait there.
 // tally(row, ranges, columns) for each row of c that has any.
 template <bool OUTS, bool OUTC, bool QUEUE, class Tally>
-__device__ __forceinline__ bool walk_batch(const ChainArgs& p, WarpSmem& S, uint32_t batch, bool dropped,
-                                           Tally&& tally) {
+__device__ __forceinline__ bool walk_batch(const ChainArgs& p, WarpSmem& S, uint32_t batch, Tally&& tally) {
   const int lane = lane_id();
-  if (QUEUE && __any_sync(kFullMask, dropped)) {
-    if (uint32_t(lane) < batch) leave_empty<OUTS, OUTC>(p, S.todo[lane]);
-    __syncwarp();
-    return false;
-  }
   uint32_t row = 0, ns = 0, nc = 0, cur = 0;
   bool done = false;
   uint2* const C = S.list[2] + lane;
@@ -1001,7 +996,6 @@ __global__ void __launch_bounds__(kWThreads, kWBlocks) k_chain_walk(const __grid
   };
   bool look = false;
   uint32_t x = 0, at = 0;  // a lane's word: its rows still to walk, and the first of its 32
-  bool dropped = given_up(p);
   while (true) {
     const unsigned spent = __ballot_sync(kFullMask, x == 0);
     uint32_t have = __reduce_add_sync(kFullMask, uint32_t(__popc(x)));
@@ -1019,9 +1013,7 @@ __global__ void __launch_bounds__(kWThreads, kWBlocks) k_chain_walk(const __grid
     uint32_t k = group_incl_sum<32>(kFullMask, uint32_t(__popc(x)), lane) - __popc(x);
     for (; x && k < 32; x &= x - 1) S.todo[k++] = at + uint32_t(__ffs(x) - 1);
     __syncwarp();
-    const bool later = given_up(p);  // (for the next batch: it comes while this one is walked)
-    if (walk_batch<OUTS, OUTC, true>(p, S, min(have, 32u), dropped, tally)) look = true;
-    dropped = later;
+    if (walk_batch<OUTS, OUTC, true>(p, S, min(have, 32u), tally)) look = true;
   }
   if (look) take_rows<OUTS, OUTC>(p, S, tally);
 }
@@ -1046,7 +1038,6 @@ __global__ void __launch_bounds__(kWThreads, kWBlocks) k_chain_small(const __gri
   unsigned long long nnz = 0;
   uint32_t cnt = 0;
   bool look = false;
-  const bool dropped = QUEUE && given_up(p);
   if (r0 < p.n) {
     uint32_t bad;
     if (r0 + 32 <= p.n) bad = chain_rows<OUTS, OUTC, COUNT, 1>(p, uint32_t(r0), cnt, nnz);
@@ -1055,7 +1046,7 @@ __global__ void __launch_bounds__(kWThreads, kWBlocks) k_chain_small(const __gri
     if (bad) S.todo[__popc(who & ((1u << lane) - 1u))] = uint32_t(r0) + lane;
     __syncwarp();
     if (who)
-      look = walk_batch<OUTS, OUTC, QUEUE>(p, S, __popc(who), dropped, [&](uint32_t, uint32_t c, unsigned long long z) {
+      look = walk_batch<OUTS, OUTC, QUEUE>(p, S, __popc(who), [&](uint32_t, uint32_t c, unsigned long long z) {
         cnt += c;
         nnz += z;
       });
