@@ -280,6 +280,7 @@ void batch_distance_index(dvg_context* ctx, uint32_t ngraphs, const dvg_matrix* 
   std::vector<uint32_t> alone;  // built one by one (no rows, or non-canonical input with dmin = 0)
   std::map<SlotKey, bool> due;  // (a batch counts as one call for all graphs that are alike)
   auto is_due = [&](const SlotKey& key) {
+    if (ctx->slot_misses.empty()) return true;
     auto it = due.find(key);
     if (it == due.end()) it = due.emplace(key, slots_due(ctx, key)).first;
     return it->second;

@@ -1596,13 +1596,13 @@ SlotBuild prepare_slots(dvg_context* ctx, const SlotPlan& plan, uint32_t n, bool
   const uint64_t groups = (uint64_t(n) + kCountRows - 1) / kCountRows;
   const uint64_t supers = (groups + kSuperGroups - 1) / kSuperGroups;
   auto round = [](size_t x) { return (x + 15) & ~size_t(15); };
-  // counters and the passes' places, cleared together
+  // counters, the passes' places and the chain's own queue, cleared together
   const size_t taken_off = sizeof(SlotCounters);
-  sb.cleared = std::max<size_t>(512, round(taken_off + plan.steps.size() * 8));
-  const size_t nnz_off = sb.cleared, cnt_off = nnz_off + groups * 8, sums_off = round(cnt_off + groups * 4);
-  const size_t queue_off = sums_off + supers * 8, masks_off = queue_off + (own_queue ? kQueueBytes : 0);
-  sb.own_queue = own_queue;
-  sb.queue_cap = kQueueRows;
+  const size_t queue_off = std::max<size_t>(512, round(taken_off + plan.steps.size() * 8));
+  sb.queue_cap = own_queue ? uint32_t(std::clamp<uint64_t>(n / 8, 256, kQueueRows)) : kQueueRows;
+  sb.cleared = queue_off + (own_queue ? sb.queue_cap * sizeof(unsigned long long) : 0);
+  const size_t nnz_off = round(sb.cleared), cnt_off = nnz_off + groups * 8, sums_off = round(cnt_off + groups * 4);
+  const size_t masks_off = sums_off + supers * 8;
   static_assert(sizeof(SlotCounters) <= 512, "the counters come first");
   // (below kMulti, so that the slot of a row of several runs has y < x)
   sb.arena_cap = std::min<uint64_t>(uint64_t(ctx->slot_growth * double(n)) + 4096, kMulti);
@@ -1648,10 +1648,9 @@ void release_slots(dvg_context* ctx, SlotBuild& sb) {
 
 void launch_slots(dvg_context* ctx, SlotBuild& sb, const SlotParts& parts, bool timed, const SlotPart* right) {
   const uint64_t t0 = now_ns();
-  // (512 bytes with up to 28 passes; one of more than a few KB takes 4 us longer)
+  // (512 bytes with up to 28 passes and the context's queue; more than a few KB take 4 us longer)
   DVG_CUDA(cudaMemsetAsync(sb.scratch, 0, sb.cleared, ctx->stream));
   ctx->stats.kernel_launches++;
-  if (sb.own_queue) DVG_CUDA(cudaMemsetAsync(sb.queue, 0, kQueueBytes, ctx->stream));
   ChainArgs p{};
   p.arena = sb.arena;
   p.top = sb.top;

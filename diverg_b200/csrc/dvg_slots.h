@@ -70,10 +70,10 @@ struct SlotBuild {
   uint64_t arena_cap = 0;      // ranges
   bool close = false;          // the kernels' blocks are placed while the kernel before ends
   uint64_t early = 0;          // room for the result's ranges before their number is known; 0: none
-  // counters | places of each pass | counts of the result | sums of the counts | queue | bitmap
+  // counters | places of each pass | the queue, where it is the chain's own | counts of the
+  // result | sums of the counts | bitmap
   void* scratch = nullptr;
-  size_t cleared = 0;          // its first bytes, which a chain starts by clearing
-  bool own_queue = false;      // the queue is there, cleared for every chain, and not the context's
+  size_t cleared = 0;          // its first bytes, up to the counts, which a chain starts by clearing
   uint32_t queue_cap = 0;
   uint32_t* taken = nullptr;
   unsigned long long* queue = nullptr;
